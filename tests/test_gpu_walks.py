@@ -1,5 +1,6 @@
-"""GPU: the pairs of a world that is wide on one axis only against all pairs
-of its fat AABBs."""
+"""GPU: the ordered walks of the single-hit queries against the every-hit
+queries (whose walks and casts they do not share), and the pairs of a world
+that is wide on one axis only against all pairs of its fat AABBs."""
 import numpy as np
 import pytest
 
@@ -8,6 +9,8 @@ from bounce_b200 import scene as S
 from bounce_b200.pipeline import CollisionPipeline
 
 pytestmark = pytest.mark.gpu
+
+NONE = 0xFFFFFFFF
 
 
 def stepped(scene, passes=3, **kw):
@@ -18,6 +21,57 @@ def stepped(scene, passes=3, **kw):
             drv.advance()
         pipe.collide(drv.state17())
     return pipe
+
+
+def first_of(index, value, n):
+    """Per query the row of its smallest value, the smaller fixture on a tie (-1: none)."""
+    out = np.full(n, -1, np.int64)
+    order = np.lexsort((index[:, 1], value, index[:, 0]))
+    q, first = np.unique(index[order, 0], return_index=True)
+    out[q] = order[first]
+    return out
+
+
+def world(kind, n):
+    rng = np.random.default_rng(n)
+    if kind == "mixed":
+        return S.mixed_scene(seed=n, n=n, side=max(3.0, 49.0 * (n / 65536.0) ** (1 / 3))).finalize()
+    if kind == "mesh":
+        return S.mesh_terrain_scene(seed=n, n=n).finalize()
+    if kind == "triangles":
+        return S.terrain_scene(seed=n, n=n).finalize()
+    s, _ = S.batched_scene(seed=int(rng.integers(100)), n_worlds=n, lo=4, hi=200)
+    return s.finalize()
+
+
+# One fixture, two, a few; the ends of a warp, of the warp-per-ray range and of
+# a block's share of rays.
+@pytest.mark.parametrize("kind,n,rays", [
+    ("mixed", 1, 40), ("mixed", 2, 33), ("mixed", 3, 1), ("mixed", 700, 31), ("mixed", 3000, 23681),
+    ("mixed", 3000, 23680), ("mixed", 5000, 70001), ("mesh", 600, 500), ("mesh", 600, 30011), ("triangles", 400, 700),
+    ("triangles", 400, 24001), ("worlds", 9, 900), ("worlds", 9, 24500)])
+def test_first_hit(kind, n, rays):
+    sc = world(kind, n)
+    pipe = stepped(sc, max_contacts=max(32 * sc.n_fixtures, 80000))
+    rng = np.random.default_rng(rays)
+    span = np.abs(sc.body_pos).max(axis=0) + 1
+    p1 = rng.uniform(-span, span, (rays, 3))
+    d = rng.normal(size=(rays, 3)) * rng.uniform(0, 8, (rays, 1))
+    d[::17] = np.eye(3)[rng.integers(0, 3, len(d[::17]))] * 6.0  # along one axis
+    d[5::101] = 0.0
+    r = np.concatenate([p1, p1 + d], axis=1).astype(np.float32)
+    worlds = rng.integers(0, sc.n_worlds, rays).astype(np.uint32)
+    fix, hit = pipe.ray_cast_single(r, worlds)
+    idx, hits = pipe.ray_cast(r, worlds)
+    want = first_of(idx.astype(np.int64), hits[:, 6], rays)
+    got = want >= 0
+    assert np.array_equal(fix != NONE, got)
+    if rays > 400:
+        assert got.any()
+    assert np.array_equal(fix[got], idx[want[got], 1])
+    assert np.array_equal(hit[got], hits[want[got]])
+    assert not hit[~got].any()
+    pipe.close()
 
 
 def overlapping(pipe, sc):
