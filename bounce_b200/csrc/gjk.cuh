@@ -116,6 +116,158 @@ __device__ __forceinline__ void bary4(float out[5], V3 A, V3 B, V3 C, V3 D, V3 Q
 	out[4] = sign * divisor;
 }
 
+// What a region test of Solve2 / Solve3 / Solve4 ends with: the vertices
+// that stay (n of them, in the order slots c0, c1, c2) and their
+// barycentric coordinates w / div. The tests only choose; the vertices
+// move once, by selects, after them: the lanes of a warp end in different
+// regions, and a copy of the vertices at each region's own exit ran for
+// one or two lanes at a time and filled the instruction cache.
+struct SimplexRegion
+{
+	uint32_t n; // 0: the simplex stays as it is
+	uint32_t c0, c1, c2;
+	float w0, w1, w2, div;
+
+	__device__ __forceinline__ void keep()
+	{
+		n = 0;
+		c0 = 0, c1 = 1, c2 = 2;
+		w0 = w1 = w2 = 0.0f;
+		div = 1.0f;
+	}
+
+	__device__ __forceinline__ void one(uint32_t a)
+	{
+		n = 1;
+		c0 = a;
+	}
+	__device__ __forceinline__ void two(uint32_t a, uint32_t b, const float w[3])
+	{
+		n = 2;
+		c0 = a, c1 = b;
+		w0 = w[0], w1 = w[1], div = w[2];
+	}
+	__device__ __forceinline__ void three(uint32_t a, uint32_t b, uint32_t c, const float* w, float d)
+	{
+		n = 3;
+		c0 = a, c1 = b, c2 = c;
+		w0 = w[0], w1 = w[1], w2 = w[2], div = d;
+	}
+};
+
+// (gjk.cpp:276-308)
+__device__ __forceinline__ SimplexRegion solve2(V3 A, V3 B)
+{
+	const V3 Q = V3{0.0f, 0.0f, 0.0f};
+	SimplexRegion r;
+	r.keep();
+	float wAB[3];
+	bary2(wAB, A, B, Q);
+	if (wAB[1] <= 0.0f)
+		r.one(0);
+	else if (wAB[0] <= 0.0f)
+		r.one(1);
+	else
+		r.two(0, 1, wAB);
+	return r;
+}
+
+// (gjk.cpp:312-412)
+__device__ __forceinline__ SimplexRegion solve3(V3 A, V3 B, V3 C)
+{
+	const V3 Q = V3{0.0f, 0.0f, 0.0f};
+	SimplexRegion r;
+	r.keep();
+	float wAB[3], wBC[3], wCA[3], wABC[4];
+	bary2(wAB, A, B, Q);
+	bary2(wBC, B, C, Q);
+	bary2(wCA, C, A, Q);
+	bary3(wABC, A, B, C, Q);
+	const float area = wABC[3];
+	if (wAB[1] <= 0.0f && wCA[0] <= 0.0f)
+		r.one(0);
+	else if (wAB[0] <= 0.0f && wBC[1] <= 0.0f)
+		r.one(1);
+	else if (wBC[0] <= 0.0f && wCA[1] <= 0.0f)
+		r.one(2);
+	else if (wAB[0] > 0.0f && wAB[1] > 0.0f && area * wABC[2] <= 0.0f)
+		r.two(0, 1, wAB);
+	else if (wBC[0] > 0.0f && wBC[1] > 0.0f && area * wABC[0] <= 0.0f)
+		r.two(1, 2, wBC);
+	else if (wCA[0] > 0.0f && wCA[1] > 0.0f && area * wABC[1] <= 0.0f)
+		r.two(2, 0, wCA);
+	else if (!(area <= 0.0f))
+		r.three(0, 1, 2, wABC, area);
+	return r;
+}
+
+// (gjk.cpp:416-650). With the origin inside the tetrahedron n is 0 and the
+// four weights go to weight[].
+__device__ __forceinline__ SimplexRegion solve4(V3 A, V3 B, V3 C, V3 D, float weight[4])
+{
+	const V3 Q = V3{0.0f, 0.0f, 0.0f};
+	SimplexRegion r;
+	r.keep();
+	float wAB[3], wAC[3], wAD[3], wBC[3], wCD[3], wDB[3];
+	bary2(wAB, A, B, Q);
+	bary2(wBC, B, C, Q);
+	bary2(wAC, A, C, Q);
+	bary2(wAD, A, D, Q);
+	bary2(wCD, C, D, Q);
+	bary2(wDB, D, B, Q);
+	float wACB[4], wABD[4], wADC[4], wBCD[4];
+	bary3(wACB, A, C, B, Q);
+	bary3(wABD, A, B, D, Q);
+	bary3(wADC, A, D, C, Q);
+	bary3(wBCD, B, C, D, Q);
+	if (wAB[1] <= 0.0f && wAC[1] <= 0.0f && wAD[1] <= 0.0f)
+		r.one(0);
+	else if (wAB[0] <= 0.0f && wDB[0] <= 0.0f && wBC[1] <= 0.0f)
+		r.one(1);
+	else if (wAC[0] <= 0.0f && wBC[0] <= 0.0f && wCD[1] <= 0.0f)
+		r.one(2);
+	else if (wAD[0] <= 0.0f && wCD[0] <= 0.0f && wDB[1] <= 0.0f)
+		r.one(3);
+	else if (wABD[2] <= 0.0f && wACB[1] <= 0.0f && wAB[0] > 0.0f && wAB[1] > 0.0f)
+		r.two(0, 1, wAB);
+	else if (wACB[2] <= 0.0f && wADC[1] <= 0.0f && wAC[0] > 0.0f && wAC[1] > 0.0f)
+		r.two(0, 2, wAC);
+	else if (wADC[2] <= 0.0f && wABD[1] <= 0.0f && wAD[0] > 0.0f && wAD[1] > 0.0f)
+		r.two(0, 3, wAD);
+	else if (wACB[0] <= 0.0f && wBCD[2] <= 0.0f && wBC[0] > 0.0f && wBC[1] > 0.0f)
+		r.two(1, 2, wBC);
+	else if (wADC[0] <= 0.0f && wBCD[0] <= 0.0f && wCD[0] > 0.0f && wCD[1] > 0.0f)
+		r.two(2, 3, wCD);
+	else if (wABD[0] <= 0.0f && wBCD[1] <= 0.0f && wDB[0] > 0.0f && wDB[1] > 0.0f)
+		r.two(3, 1, wDB);
+	else
+	{
+		float wABCD[5];
+		bary4(wABCD, A, B, C, D, Q);
+		if (wABCD[3] <= 0.0f && wACB[0] > 0.0f && wACB[1] > 0.0f && wACB[2] > 0.0f)
+			r.three(0, 2, 1, wACB, (wACB[0] + wACB[1]) + wACB[2]);
+		else if (wABCD[2] <= 0.0f && wABD[0] > 0.0f && wABD[1] > 0.0f && wABD[2] > 0.0f)
+			r.three(0, 1, 3, wABD, (wABD[0] + wABD[1]) + wABD[2]);
+		else if (wABCD[1] <= 0.0f && wADC[0] > 0.0f && wADC[1] > 0.0f && wADC[2] > 0.0f)
+			r.three(0, 3, 2, wADC, (wADC[0] + wADC[1]) + wADC[2]);
+		else if (wABCD[0] <= 0.0f && wBCD[0] > 0.0f && wBCD[1] > 0.0f && wBCD[2] > 0.0f)
+			r.three(1, 2, 3, wBCD, (wBCD[0] + wBCD[1]) + wBCD[2]);
+		else
+		{
+			const float divisor = ((wABCD[0] + wABCD[1]) + wABCD[2]) + wABCD[3];
+			if (!(divisor <= 0.0f))
+			{
+				const float s = 1.0f / divisor;
+				weight[0] = s * wABCD[0];
+				weight[1] = s * wABCD[1];
+				weight[2] = s * wABCD[2];
+				weight[3] = s * wABCD[3];
+			}
+		}
+	}
+	return r;
+}
+
 struct Simplex
 {
 	SVert v[4];
@@ -194,212 +346,54 @@ struct Simplex
 	__device__ void closest_points_from(const XF& xf1, const GProxy& p1, const XF& xf2, const GProxy& p2, V3& P1,
 		V3& P2) const;
 
-	__device__ void set1(const SVert& a)
+	__device__ __forceinline__ SVert picked(uint32_t c, const SVert& a, const SVert& b, const SVert& d, const SVert& e) const
 	{
-		count = 1;
-		v[0] = a;
-		v[0].weight = 1.0f;
-	}
-	__device__ void set2(const SVert& a, float wa, const SVert& b, float wb)
-	{
-		count = 2;
-		v[0] = a;
-		v[0].weight = wa;
-		v[1] = b;
-		v[1].weight = wb;
-	}
-	__device__ void set3(const SVert& a, float wa, const SVert& b, float wb, const SVert& c, float wc)
-	{
-		count = 3;
-		v[0] = a;
-		v[0].weight = wa;
-		v[1] = b;
-		v[1].weight = wb;
-		v[2] = c;
-		v[2].weight = wc;
+		auto f = [&](float x, float y, float z, float w) { return c == 0 ? x : (c == 1 ? y : (c == 2 ? z : w)); };
+		auto u = [&](uint32_t x, uint32_t y, uint32_t z, uint32_t w) { return c == 0 ? x : (c == 1 ? y : (c == 2 ? z : w)); };
+		auto v3_ = [&](V3 x, V3 y, V3 z, V3 w) { return V3{f(x.x, y.x, z.x, w.x), f(x.y, y.y, z.y, w.y), f(x.z, y.z, z.z, w.z)}; };
+		SVert o;
+		o.point1 = v3_(a.point1, b.point1, d.point1, e.point1);
+		o.point2 = v3_(a.point2, b.point2, d.point2, e.point2);
+		o.point = v3_(a.point, b.point, d.point, e.point);
+		o.weight = 0.0f;
+		o.index1 = u(a.index1, b.index1, d.index1, e.index1);
+		o.index2 = u(a.index2, b.index2, d.index2, e.index2);
+		return o;
 	}
 
-	// (gjk.cpp:276-308)
-	__device__ void solve2()
+	__device__ __forceinline__ void take(const SimplexRegion& r)
 	{
-		const V3 Q = V3{0.0f, 0.0f, 0.0f};
-		SVert A = v[0], B = v[1];
-		float wAB[3];
-		bary2(wAB, A.point, B.point, Q);
-		if (wAB[1] <= 0.0f)
-		{
-			set1(A);
+		if (r.n == 0)
 			return;
-		}
-		if (wAB[0] <= 0.0f)
-		{
-			set1(B);
-			return;
-		}
-		float s = 1.0f / wAB[2];
-		set2(A, s * wAB[0], B, s * wAB[1]);
+		const float s = 1.0f / r.div;
+		const SVert A = v[0], B = v[1], C = v[2], D = v[3];
+		v[0] = picked(r.c0, A, B, C, D);
+		v[1] = picked(r.c1, A, B, C, D);
+		v[2] = picked(r.c2, A, B, C, D);
+		v[0].weight = r.n == 1 ? 1.0f : s * r.w0;
+		v[1].weight = s * r.w1;
+		v[2].weight = s * r.w2;
+		count = r.n;
 	}
 
-	// (gjk.cpp:312-412)
-	__device__ void solve3()
+	// Solve2 / Solve3 / Solve4 by the vertex count.
+	__device__ __forceinline__ void solve()
 	{
-		const V3 Q = V3{0.0f, 0.0f, 0.0f};
-		SVert A = v[0], B = v[1], C = v[2];
-		float wAB[3], wBC[3], wCA[3];
-		bary2(wAB, A.point, B.point, Q);
-		bary2(wBC, B.point, C.point, Q);
-		bary2(wCA, C.point, A.point, Q);
-		if (wAB[1] <= 0.0f && wCA[0] <= 0.0f)
+		SimplexRegion r;
+		r.keep();
+		if (count == 2)
+			r = solve2(v[0].point, v[1].point);
+		else if (count == 3)
+			r = solve3(v[0].point, v[1].point, v[2].point);
+		else if (count == 4)
 		{
-			set1(A);
-			return;
+			float w[4] = {v[0].weight, v[1].weight, v[2].weight, v[3].weight};
+			r = solve4(v[0].point, v[1].point, v[2].point, v[3].point, w);
+#pragma unroll
+			for (int i = 0; i < 4; ++i)
+				v[i].weight = w[i];
 		}
-		if (wAB[0] <= 0.0f && wBC[1] <= 0.0f)
-		{
-			set1(B);
-			return;
-		}
-		if (wBC[0] <= 0.0f && wCA[1] <= 0.0f)
-		{
-			set1(C);
-			return;
-		}
-		float wABC[4];
-		bary3(wABC, A.point, B.point, C.point, Q);
-		float area = wABC[3];
-		if (wAB[0] > 0.0f && wAB[1] > 0.0f && area * wABC[2] <= 0.0f)
-		{
-			float s = 1.0f / wAB[2];
-			set2(A, s * wAB[0], B, s * wAB[1]);
-			return;
-		}
-		if (wBC[0] > 0.0f && wBC[1] > 0.0f && area * wABC[0] <= 0.0f)
-		{
-			float s = 1.0f / wBC[2];
-			set2(B, s * wBC[0], C, s * wBC[1]);
-			return;
-		}
-		if (wCA[0] > 0.0f && wCA[1] > 0.0f && area * wABC[1] <= 0.0f)
-		{
-			float s = 1.0f / wCA[2];
-			set2(C, s * wCA[0], A, s * wCA[1]);
-			return;
-		}
-		float divisor = wABC[3];
-		if (divisor <= 0.0f)
-			return;
-		float s = 1.0f / divisor;
-		set3(A, s * wABC[0], B, s * wABC[1], C, s * wABC[2]);
-	}
-
-	// (gjk.cpp:416-650)
-	__device__ void solve4()
-	{
-		const V3 Q = V3{0.0f, 0.0f, 0.0f};
-		SVert A = v[0], B = v[1], C = v[2], D = v[3];
-		float wAB[3], wAC[3], wAD[3], wBC[3], wCD[3], wDB[3];
-		bary2(wAB, A.point, B.point, Q);
-		bary2(wBC, B.point, C.point, Q);
-		bary2(wAC, A.point, C.point, Q);
-		bary2(wAD, A.point, D.point, Q);
-		bary2(wCD, C.point, D.point, Q);
-		bary2(wDB, D.point, B.point, Q);
-		if (wAB[1] <= 0.0f && wAC[1] <= 0.0f && wAD[1] <= 0.0f)
-		{
-			set1(A);
-			return;
-		}
-		if (wAB[0] <= 0.0f && wDB[0] <= 0.0f && wBC[1] <= 0.0f)
-		{
-			set1(B);
-			return;
-		}
-		if (wAC[0] <= 0.0f && wBC[0] <= 0.0f && wCD[1] <= 0.0f)
-		{
-			set1(C);
-			return;
-		}
-		if (wAD[0] <= 0.0f && wCD[0] <= 0.0f && wDB[1] <= 0.0f)
-		{
-			set1(D);
-			return;
-		}
-		float wACB[4], wABD[4], wADC[4], wBCD[4];
-		bary3(wACB, A.point, C.point, B.point, Q);
-		bary3(wABD, A.point, B.point, D.point, Q);
-		bary3(wADC, A.point, D.point, C.point, Q);
-		bary3(wBCD, B.point, C.point, D.point, Q);
-		if (wABD[2] <= 0.0f && wACB[1] <= 0.0f && wAB[0] > 0.0f && wAB[1] > 0.0f)
-		{
-			float s = 1.0f / wAB[2];
-			set2(A, s * wAB[0], B, s * wAB[1]);
-			return;
-		}
-		if (wACB[2] <= 0.0f && wADC[1] <= 0.0f && wAC[0] > 0.0f && wAC[1] > 0.0f)
-		{
-			float s = 1.0f / wAC[2];
-			set2(A, s * wAC[0], C, s * wAC[1]);
-			return;
-		}
-		if (wADC[2] <= 0.0f && wABD[1] <= 0.0f && wAD[0] > 0.0f && wAD[1] > 0.0f)
-		{
-			float s = 1.0f / wAD[2];
-			set2(A, s * wAD[0], D, s * wAD[1]);
-			return;
-		}
-		if (wACB[0] <= 0.0f && wBCD[2] <= 0.0f && wBC[0] > 0.0f && wBC[1] > 0.0f)
-		{
-			float s = 1.0f / wBC[2];
-			set2(B, s * wBC[0], C, s * wBC[1]);
-			return;
-		}
-		if (wADC[0] <= 0.0f && wBCD[0] <= 0.0f && wCD[0] > 0.0f && wCD[1] > 0.0f)
-		{
-			float s = 1.0f / wCD[2];
-			set2(C, s * wCD[0], D, s * wCD[1]);
-			return;
-		}
-		if (wABD[0] <= 0.0f && wBCD[1] <= 0.0f && wDB[0] > 0.0f && wDB[1] > 0.0f)
-		{
-			float s = 1.0f / wDB[2];
-			set2(D, s * wDB[0], B, s * wDB[1]);
-			return;
-		}
-		float wABCD[5];
-		bary4(wABCD, A.point, B.point, C.point, D.point, Q);
-		if (wABCD[3] <= 0.0f && wACB[0] > 0.0f && wACB[1] > 0.0f && wACB[2] > 0.0f)
-		{
-			float s = 1.0f / ((wACB[0] + wACB[1]) + wACB[2]);
-			set3(A, s * wACB[0], C, s * wACB[1], B, s * wACB[2]);
-			return;
-		}
-		if (wABCD[2] <= 0.0f && wABD[0] > 0.0f && wABD[1] > 0.0f && wABD[2] > 0.0f)
-		{
-			float s = 1.0f / ((wABD[0] + wABD[1]) + wABD[2]);
-			set3(A, s * wABD[0], B, s * wABD[1], D, s * wABD[2]);
-			return;
-		}
-		if (wABCD[1] <= 0.0f && wADC[0] > 0.0f && wADC[1] > 0.0f && wADC[2] > 0.0f)
-		{
-			float s = 1.0f / ((wADC[0] + wADC[1]) + wADC[2]);
-			set3(A, s * wADC[0], D, s * wADC[1], C, s * wADC[2]);
-			return;
-		}
-		if (wABCD[0] <= 0.0f && wBCD[0] > 0.0f && wBCD[1] > 0.0f && wBCD[2] > 0.0f)
-		{
-			float s = 1.0f / ((wBCD[0] + wBCD[1]) + wBCD[2]);
-			set3(B, s * wBCD[0], C, s * wBCD[1], D, s * wBCD[2]);
-			return;
-		}
-		float divisor = ((wABCD[0] + wABCD[1]) + wABCD[2]) + wABCD[3];
-		if (divisor <= 0.0f)
-			return;
-		float s = 1.0f / divisor;
-		count = 4;
-		v[0].weight = s * wABCD[0];
-		v[1].weight = s * wABCD[1];
-		v[2].weight = s * wABCD[2];
-		v[3].weight = s * wABCD[3];
+		take(r);
 	}
 };
 
@@ -461,12 +455,7 @@ __device__ __forceinline__ uint32_t gjk_loop(Simplex& sx, const XF& xf1, const G
 			save1[i] = sx.v[i].index1;
 			save2[i] = sx.v[i].index2;
 		}
-		if (sx.count == 2)
-			sx.solve2();
-		else if (sx.count == 3)
-			sx.solve3();
-		else if (sx.count == 4)
-			sx.solve4();
+		sx.solve();
 		if (sx.count == 4)
 			break;
 		V3 d = sx.search_dir();

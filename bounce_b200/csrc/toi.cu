@@ -706,12 +706,7 @@ __device__ bool gjk_ray_cast(const XF& xf1, const GProxy& p1, const XF& xf2, con
 			save1[i] = sx.v[i].index1;
 			save2[i] = sx.v[i].index2;
 		}
-		if (sx.count == 2)
-			sx.solve2();
-		else if (sx.count == 3)
-			sx.solve3();
-		else if (sx.count == 4)
-			sx.solve4();
+		sx.solve();
 		if (sx.count == 4)
 			break;
 		v = sx.closest();
