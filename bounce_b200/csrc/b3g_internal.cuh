@@ -170,6 +170,7 @@ struct Buffers
 	uint32_t* leafOf;     // per proxy: its sorted leaf (set when the LBVH is built)
 	float4* walkNodes;    // the tree as the world queries walk it: 4 float4 per inner node (queries.cu)
 	float4* walkLeaves;   // and 4 float4 per sorted leaf
+	uint32_t* walkTurned; // a triangle fixture lies outside its box (queries.cu)
 	uint32_t* leafCount;  // pair count per sorted leaf (then exclusive offsets)
 	uint32_t* pairScratch; // first contact records (A, B) found per leaf, slot-major (B3G_TRAV_SLOTS x n uint2)
 	uint32_t* scanAux;

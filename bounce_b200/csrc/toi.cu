@@ -9,7 +9,7 @@
 // b3Sweep::GetTransform (sweep.h:43-63).
 #include <algorithm>
 
-#include "collide_common.cuh"
+#include "lane_gjk.cuh"
 
 static_assert(sizeof(b3g_toi_input) == 272, "b3g_toi_input: 68 words");
 static_assert(sizeof(b3g_gjk_cast_input) == 192, "b3g_gjk_cast_input: 48 words");
@@ -179,69 +179,11 @@ enum : uint32_t
 	ST_SEPARATED
 };
 
-// One query on a lane. Its record stays in shared memory (one column of its
-// warp's array: word w of lane l at w * TOI_ROW + l).
+// One query on a lane: its record stays in the lane's column of its warp's
+// shared memory (lane_gjk.cuh).
 constexpr uint32_t TOI_WORDS = sizeof(b3g_toi_input) / 4;
-constexpr uint32_t TOI_ROW = 33; // so that a row and a column are both free of bank conflicts
-
-// A proxy of the query: a hull's vertices, or the shape's own, which are the
-// first words of its params (sphere, capsule and triangle alike).
-struct ToiProxy
-{
-	const float4* gv; // hull vertices or nullptr
-	const float* lv;  // the lane's column at the shape's params
-	uint32_t count;
-
-	__device__ __forceinline__ V3 vertex(uint32_t i) const
-	{
-		if (gv)
-		{
-			const float4 w = __ldg(gv + i);
-			return V3{w.x, w.y, w.z};
-		}
-		return V3{lv[3 * i * TOI_ROW], lv[(3 * i + 1) * TOI_ROW], lv[(3 * i + 2) * TOI_ROW]};
-	}
-
-	// b3GJKProxy::GetSupportIndex (gjk_proxy.h:72-86): first maximum. A
-	// hull's vertices load four at a time. Out of line: one copy for both
-	// proxies.
-	__device__ __noinline__ uint32_t support(V3 d) const
-	{
-		uint32_t index = 0;
-		if (gv)
-		{
-			float best = 0.0f;
-			for (uint32_t i0 = 0; i0 < count; i0 += 4)
-			{
-				float4 w[4];
-#pragma unroll
-				for (uint32_t k = 0; k < 4; ++k)
-					w[k] = __ldg(gv + min(i0 + k, count - 1u));
-#pragma unroll
-				for (uint32_t k = 0; k < 4; ++k)
-				{
-					const float proj = dot(d, V3{w[k].x, w[k].y, w[k].z});
-					// The last vertex repeats past the end: never above itself.
-					const bool take = i0 + k == 0u || proj > best;
-					best = take ? proj : best;
-					index = take ? i0 + k : index;
-				}
-			}
-			return index;
-		}
-		float best = dot(d, vertex(0));
-		for (uint32_t i = 1; i < count; ++i)
-		{
-			const float proj = dot(d, vertex(i));
-			if (proj > best)
-			{
-				best = proj;
-				index = i;
-			}
-		}
-		return index;
-	}
-};
+constexpr uint32_t TOI_ROW = LANE_ROW;
+using ToiProxy = LaneProxy<TOI_ROW>;
 
 // b3SeparationFunction (time_of_impact.cpp:26-461) for the feature pair the
 // GJK ended with.
@@ -602,15 +544,10 @@ constexpr uint32_t TOI_WARPS = 2;
 constexpr uint32_t TOI_BLOCKS = 6; // per SM: 4 took 2.92 ms, 8 (128 registers, spills) 2.94 ms
 constexpr uint32_t TOI_REFILL = 4; // lanes without a query before the warp brings new ones: 8 took 3.00 ms
 
-// The simplex in the rows after the query: per vertex the point (3), the
-// weight and the two support indices.
-constexpr uint32_t TOI_SX = TOI_WORDS;
-constexpr uint32_t TOI_SX_VERT = 6;
-
 __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevScene S, const float* in, uint32_t n,
 	uint32_t share, uint32_t* out)
 {
-	__shared__ float record[TOI_WARPS][(TOI_WORDS + 4 * TOI_SX_VERT) * TOI_ROW];
+	__shared__ float record[TOI_WARPS][(TOI_WORDS + LANE_SIMPLEX_WORDS) * TOI_ROW];
 	const uint32_t lane = threadIdx.x & 31u;
 	float* const W = record[threadIdx.x >> 5];
 	float* const mine = W + lane;
@@ -619,23 +556,17 @@ __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevSc
 	const uint32_t end = min(next + share, n);
 	const float tolerance = 0.25f * B3G_LINEAR_SLOP;
 
-	auto word = [&](uint32_t v, uint32_t k) -> float& { return mine[(TOI_SX + TOI_SX_VERT * v + k) * TOI_ROW]; };
-	auto point = [&](uint32_t v) { return V3{word(v, 0), word(v, 1), word(v, 2)}; };
-	auto set_sx = [&](uint32_t v, V3 p, float w, uint32_t i1, uint32_t i2) {
-		word(v, 0) = p.x, word(v, 1) = p.y, word(v, 2) = p.z;
-		word(v, 3) = w;
-		word(v, 4) = __uint_as_float(i1), word(v, 5) = __uint_as_float(i2);
-	};
-	auto sx_index1 = [&](uint32_t v) { return __float_as_uint(word(v, 4)); };
-	auto sx_index2 = [&](uint32_t v) { return __float_as_uint(word(v, 5)); };
-
-	uint32_t state = TOI_IDLE, query = 0, count = 0;
+	uint32_t state = TOI_IDLE, query = 0;
+	LaneSimplex sx;
+	sx.mine = mine + TOI_WORDS * TOI_ROW;
+	sx.count = sx.steps = sx.saveCount = 0;
+	sx.metric = 0.0f;
 	ToiProxy pA, pB;
 	pA.gv = pB.gv = nullptr;
 	pA.lv = mine + 4 * TOI_ROW;
 	pB.lv = mine + 16 * TOI_ROW;
 	pA.count = pB.count = 0;
-	float target = 0.0f, tMax = 0.0f, t1 = 0.0f, t2 = 0.0f, a1 = 0.0f, a2 = 0.0f, s1 = 0.0f, s2 = 0.0f, metric = 0.0f;
+	float target = 0.0f, tMax = 0.0f, t1 = 0.0f, t2 = 0.0f, a1 = 0.0f, a2 = 0.0f, s1 = 0.0f, s2 = 0.0f;
 	float tRoot = 0.0f;
 	uint32_t kind = VALUE_MIN;
 	uint32_t iteration = 0, pushBack = 0, steps = 0, indexA = 0, indexB = 0; // steps: of the GJK or the root finder
@@ -646,20 +577,6 @@ __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevSc
 	XF xfA, xfB;
 	xfA.p = xfB.p = V3{0.0f, 0.0f, 0.0f};
 	xfA.q = xfB.q = Q4{V3{0.0f, 0.0f, 0.0f}, 1.0f};
-
-	auto simplex_size = [&]() -> float {
-		// b3Simplex::GetMetric (gjk.cpp:881-912).
-		if (count < 2u)
-			return 0.0f;
-		const V3 A = point(0), E1 = point(1) - A;
-		if (count == 2u)
-			return len(A - point(1));
-		const V3 E2 = point(2) - A;
-		if (count == 3u)
-			return len(cross(E1, E2));
-		const float det = det3(E1, E2, point(3) - A);
-		return signf_(det) * det;
-	};
 
 	for (;;)
 	{
@@ -686,28 +603,15 @@ __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevSc
 			if (state == TOI_IDLE && first + rank < next)
 			{
 				query = first + rank;
-				// b3GJKProxy::Set (gjk.cpp:37-95); the radius follows the vertices.
-				auto set = [&](ToiProxy& p, uint32_t type, uint32_t hull) -> float {
-					p.gv = nullptr;
-					if (type <= B3G_SHAPE_TRIANGLE)
-					{
-						p.count = type + 1u; // sphere 1, capsule 2, triangle 3
-						return p.lv[3 * p.count * TOI_ROW];
-					}
-					const HullDesc h = S.hulls[hull];
-					p.gv = S.hverts + h.vOff;
-					p.count = h.vCnt;
-					return p.lv[0];
-				};
-				static_assert(B3G_SHAPE_SPHERE == 0 && B3G_SHAPE_CAPSULE == 1 && B3G_SHAPE_TRIANGLE == 2, "vertex counts");
-				const float rA = set(pA, __float_as_uint(mine[0]), __float_as_uint(mine[TOI_ROW]));
-				const float rB = set(pB, __float_as_uint(mine[2 * TOI_ROW]), __float_as_uint(mine[3 * TOI_ROW]));
+				const float rA = pA.set(S, __float_as_uint(mine[0]), __float_as_uint(mine[TOI_ROW]), mine + 4 * TOI_ROW);
+				const float rB =
+					pB.set(S, __float_as_uint(mine[2 * TOI_ROW]), __float_as_uint(mine[3 * TOI_ROW]), mine + 16 * TOI_ROW);
 				target = fmaxr(B3G_LINEAR_SLOP, (rA + rB) - 3.0f * B3G_LINEAR_SLOP);
 				tMax = mine[64 * TOI_ROW];
 				t1 = 0.0f;
 				iteration = 0;
-				count = 0;
-				metric = 0.0f;
+				sx.count = 0;
+				sx.metric = 0.0f;
 				state = TOI_START;
 			}
 			__syncwarp();
@@ -754,27 +658,7 @@ __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevSc
 		{
 			if (active)
 			{
-				// b3Simplex::ReadCache (gjk.cpp:820-868): the last simplex's
-				// support points at these transforms, dropped when their metric
-				// changed by more than a factor of two or vanished.
-#pragma unroll 1
-				for (uint32_t i = 0; i < count; ++i)
-				{
-					const uint32_t i1 = sx_index1(i), i2 = sx_index2(i);
-					set_sx(i, xmul(xfB, pB.vertex(i2)) - xmul(xfA, pA.vertex(i1)), 0.0f, i1, i2);
-				}
-				if (count > 1u)
-				{
-					const float now = simplex_size();
-					if (now < 0.5f * metric || 2.0f * metric < now || now < B3G_EPSILON)
-						count = 0;
-				}
-				if (count == 0u)
-				{
-					set_sx(0, xmul(xfB, pB.vertex(0)) - xmul(xfA, pA.vertex(0)), 1.0f, 0u, 0u);
-					count = 1;
-				}
-				steps = 0;
+				sx.start(pA, pB, xfA, xfB);
 				state = TOI_GJK;
 			}
 		}
@@ -783,61 +667,12 @@ __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevSc
 			// One GJK iteration (gjk.cpp:683-768), or the points of minimum
 			// separation: both end in support scans.
 			V3 dA = V3{0.0f, 0.0f, 0.0f}, dB = dA;
-			uint32_t save1[4], save2[4];
-			const uint32_t saveCount = count;
 			bool scanA = false, scanB = false;
 			if (active && step == TOI_GJK)
 			{
-				SimplexRegion r;
-				r.keep();
-				const V3 A = point(0), B = point(1), C = point(2);
-#pragma unroll
-				for (uint32_t i = 0; i < 4; ++i)
-				{
-					save1[i] = sx_index1(i);
-					save2[i] = sx_index2(i);
-				}
-				if (count == 2u)
-					r = solve2(A, B);
-				else if (count == 3u)
-					r = solve3(A, B, C);
-				else if (count == 4u)
-				{
-					float w[4] = {word(0, 3), word(1, 3), word(2, 3), word(3, 3)};
-					r = solve4(A, B, C, point(3), w);
-					word(0, 3) = w[0], word(1, 3) = w[1], word(2, 3) = w[2], word(3, 3) = w[3];
-				}
-				if (r.n != 0u)
-				{
-					const V3 P0 = point(r.c0), P1 = point(r.c1), P2 = point(r.c2);
-					const uint32_t i0 = sx_index1(r.c0), i1 = sx_index1(r.c1), i2 = sx_index1(r.c2);
-					const uint32_t j0 = sx_index2(r.c0), j1 = sx_index2(r.c1), j2 = sx_index2(r.c2);
-					const float s = 1.0f / r.div;
-					set_sx(0, P0, r.n == 1u ? 1.0f : s * r.w0, i0, j0);
-					set_sx(1, P1, s * r.w1, i1, j1);
-					set_sx(2, P2, s * r.w2, i2, j2);
-					count = r.n;
-				}
-				// b3Simplex::GetSearchDirection
-				V3 d = V3{0.0f, 0.0f, 0.0f};
-				if (count < 4u)
-				{
-					const V3 X = point(0), E = point(1) - X, O = V3{0.0f, 0.0f, 0.0f} - X;
-					d = O;
-					if (count == 2u)
-						d = cross(cross(E, O), E);
-					else if (count == 3u)
-					{
-						d = cross(E, point(2) - X);
-						if (!(dot(d, O) > 0.0f))
-							d = -d;
-					}
-				}
-				scanA = scanB = !(count == 4u || dot(d, d) < B3G_EPSILON * B3G_EPSILON);
+				scanA = scanB = sx.directions(xfA, xfB, dA, dB);
 				if (!scanA)
 					state = TOI_END;
-				dA = rotc(xfA.q, -d);
-				dB = rotc(xfB.q, d);
 			}
 			else if (active)
 			{
@@ -860,22 +695,8 @@ __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevSc
 				kind = VALUE_MIN;
 				state = TOI_VALUE;
 			}
-			else if (active && scanA)
-			{
-				++steps;
-				bool duplicate = false;
-#pragma unroll
-				for (uint32_t i = 0; i < 4; ++i)
-					if (i < saveCount && ia == save1[i] && ib == save2[i])
-						duplicate = true;
-				if (duplicate || steps == 20u)
-					state = TOI_END;
-				if (!duplicate)
-				{
-					set_sx(count, xmul(xfB, pB.vertex(ib)) - xmul(xfA, pA.vertex(ia)), 0.0f, ia, ib);
-					++count;
-				}
-			}
+			else if (active && scanA && !sx.add(pA, pB, xfA, xfB, ia, ib))
+				state = TOI_END;
 		}
 		else if (step == TOI_VALUE)
 		{
@@ -950,21 +771,9 @@ __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevSc
 		}
 		else if (active)
 		{
-			// The witness points and the distance (gjk.cpp:770-812).
-			V3 P1 = V3{0.0f, 0.0f, 0.0f}, P2 = P1;
-#pragma unroll 1
-			for (uint32_t i = 0; i < count; ++i)
-			{
-				const float w = word(i, 3);
-				const V3 x1 = xmul(xfA, pA.vertex(sx_index1(i))), x2 = xmul(xfB, pB.vertex(sx_index2(i)));
-				const V3 q1 = count == 1u ? x1 : w * x1, q2 = count == 1u ? x2 : w * x2;
-				P1 = i == 0u ? q1 : P1 + q1;
-				P2 = i == 0u ? q2 : P2 + q2;
-			}
-			if (count == 4u)
-				P2 = P1;
+			V3 P1, P2;
+			sx.end(pA, pB, xfA, xfB, P1, P2);
 			const float distance = len(P1 - P2);
-			metric = simplex_size();
 			if (distance == 0.0f)
 			{
 				how = ST_OVERLAPPED;
@@ -975,12 +784,12 @@ __global__ void __launch_bounds__(TOI_WARPS * 32, TOI_BLOCKS) k_toi_sweeps(DevSc
 			else
 			{
 				GJKCache cache;
-				cache.count = count;
+				cache.count = sx.count;
 #pragma unroll
 				for (uint32_t i = 0; i < 4; ++i)
 				{
-					cache.index1[i] = sx_index1(i);
-					cache.index2[i] = sx_index2(i);
+					cache.index1[i] = sx.index1(i);
+					cache.index2[i] = sx.index2(i);
 				}
 				sep.init(cache, pA, pB, xfA, xfB);
 				if (sep.type == SEP_NONE)

@@ -596,8 +596,7 @@ int b3g_shape_cast_single(b3g_ctx* ctx, uint32_t n, const b3g_shape_cast_input* 
 /* b3g_shape_cast_single on device buffers (casts, fixture, hit as above, all
  * device memory), asynchronous on stream (NULL: the context's stream), for
  * callers that keep their casts on the GPU. The casts are not checked: every
- * hull index must be below the hull count. Nothing is copied; the scratch of
- * the cast ordering is the context's query scratch (grown on first use). */
+ * hull index must be below the hull count. Nothing is copied or allocated. */
 int b3g_shape_cast_single_device(b3g_ctx* ctx, uint32_t n, const b3g_shape_cast_input* casts, uint32_t* fixture,
 	float* hit, void* stream);
 

@@ -74,6 +74,52 @@ def test_first_hit(kind, n, rays):
     pipe.close()
 
 
+def casts_of(sc, n, seed):
+    rng = np.random.default_rng(seed)
+    pick = rng.integers(0, sc.n_fixtures, n)
+    pick = pick[sc.fix_type[pick] != N.SHAPE_MESH]
+    pick = rng.choice(pick, n)
+    c = np.zeros(n, N.SHAPE_CAST_DTYPE)
+    c["type"], c["hull"], c["params"] = sc.fix_type[pick], sc.fix_hull[pick], sc.fix_params.reshape(-1, 12)[pick]
+    span = np.abs(sc.body_pos).max(axis=0) + 0.5
+    c["position"] = rng.uniform(-span, span, (n, 3))
+    c["rotation"] = S.random_quats(rng, n)
+    c["displacement"] = rng.normal(size=(n, 3)) * rng.uniform(0, 2.5, (n, 1))
+    c["displacement"][::29] = 0.0
+    c["world"] = rng.integers(0, sc.n_worlds, n)
+    return c
+
+
+# Lanes per cast go from 32 to 1 over these counts; triangle fixtures on bodies
+# away from the identity lie outside their boxes (the reference's quirk).
+@pytest.mark.parametrize("kind,n,casts", [
+    ("mixed", 1, 3), ("mixed", 2, 33), ("mixed", 700, 1), ("mixed", 2000, 2368), ("mixed", 2000, 2369),
+    ("mixed", 2000, 9500), ("mixed", 2000, 40001), ("mixed", 500, 80001), ("mesh", 500, 300), ("mesh", 500, 20000),
+    ("triangles", 300, 500), ("turned", 300, 500), ("turned", 300, 9000), ("worlds", 7, 6000)])
+def test_first_cast(kind, n, casts):
+    sc = world("triangles" if kind == "turned" else kind, n)
+    if kind == "turned":
+        sc.body_pos[0] = (0.4, 0.3, -0.2)
+    pipe = stepped(sc, max_contacts=max(32 * sc.n_fixtures, 90000))
+    c = casts_of(sc, casts, n + casts)
+    fix, hit = pipe.shape_cast_single(c)
+    idx, hits = pipe.shape_cast(c)
+    key = idx.astype(np.int64)
+    # Of equal fractions the smaller fixture, then triangle.
+    order = np.lexsort((key[:, 2], key[:, 1], hits[:, 6], key[:, 0]))
+    q, first = np.unique(key[order, 0], return_index=True)
+    want = np.full(casts, -1, np.int64)
+    want[q] = order[first]
+    got = want >= 0
+    assert np.array_equal(fix[:, 0] != NONE, got)
+    if casts > 400:
+        assert got.any()
+    assert np.array_equal(fix[got], idx[want[got], 1:])
+    assert np.array_equal(hit[got], hits[want[got]])
+    assert not hit[~got].any()
+    pipe.close()
+
+
 def overlapping(pipe, sc):
     """Contacts every pass must hold: overlapping fat AABBs of two bodies, one of them dynamic."""
     box = pipe.fat_aabbs()
