@@ -215,7 +215,8 @@ struct Buffers
 	// mesh contacts (allocated when the scene has meshes)
 	float4* meshAABB[2];      // per contact: the other shape's fat AABB in mesh space (2 float4)
 	DevManifold* extraMan[2]; // per contact: manifolds 1 and 2 of a mesh contact
-	uint32_t* meshCount;      // per contact: overlapping triangles, then exclusive offsets
+	uint32_t* meshList;       // the pass's mesh contacts, skipped ones included
+	uint2* meshItems;         // per mesh contact: its first work item and their number
 	uint32_t* meshPairC;      // per (contact, triangle) work item: contact
 	uint32_t* meshPairT;      // ... triangle
 	DevManifold* meshPairMan; // ... its b3Manifold (triangleKey set)
@@ -309,7 +310,8 @@ enum
 	CTR_HC_POST = 34,       // hull-capsule contacts past their GJK (k_hull_capsule_post): at a distance
 	CTR_HC_DEEP = 35,       // ... and overlapping
 	CTR_HS_POST = 36,       // hull-sphere contacts past their face scan (k_hull_sphere_gjk)
-	CTR_COUNT = 37
+	CTR_MESH_ALL = 37,      // mesh contacts of the pass, skipped ones included
+	CTR_COUNT = 38
 };
 static_assert(CTR_BUCKET0 + BK_COUNT <= CTR_ASLEEP, "bucket counters overlap");
 

@@ -149,9 +149,22 @@ __global__ void __launch_bounds__(BUCKET_THREADS) k_bucket(DevScene S, Buffers B
 			uint32_t ba = S.fixBody[fa], bb = S.fixBody[fb];
 			bool activeA = S.bodyAwake[ba] && S.bodyType[ba] != B3G_BODY_STATIC;
 			bool activeB = S.bodyAwake[bb] && S.bodyType[bb] != B3G_BODY_STATIC;
+			const bool mesh = S.fixType[fa] == B3G_SHAPE_MESH || S.fixType[fb] == B3G_SHAPE_MESH;
+			if (mesh)
+			{
+				// Every mesh contact keeps its box in mesh space up to date
+				// (k_mesh_sync), skipped or not.
+				const uint32_t peers = __activemask();
+				const uint32_t leader = __ffs(peers) - 1;
+				uint32_t at = 0;
+				if (lane == leader)
+					at = atomicAdd(&B.counters[CTR_MESH_ALL], (uint32_t)__popc(peers));
+				at = __shfl_sync(peers, at, leader) + __popc(peers & ((1u << lane) - 1u));
+				B.meshList[at] = c;
+			}
 			if (!activeA && !activeB)
 				bk = BK_INACTIVE;
-			else if (S.fixType[fa] == B3G_SHAPE_MESH || S.fixType[fb] == B3G_SHAPE_MESH)
+			else if (mesh)
 				bk = BK_MESH; // b3MeshContact, sensors included (its TestOverlap runs per triangle)
 			else if ((S.fixFlags[fa] | S.fixFlags[fb]) & B3G_FIXTURE_SENSOR)
 				bk = BK_SENSOR;
@@ -418,20 +431,21 @@ void launch_narrowphase(b3g_ctx* c, cudaStream_t s)
 {
 	Buffers& B = c->buf;
 	uint32_t cap = c->cfg.max_contacts;
-	// Mesh midphase on its own stream beside the bucketing and the convex
-	// and hull kernels (joined before the mesh work items).
+	k_bucket<<<persistent_blocks(8), BUCKET_THREADS, 0, s>>>(c->scene, B, c->cur, cap);
+	prof_mark(c, PM_BUCKETED, s);
+	// The mesh contacts (midphase, work items, clustering) on a stream of their
+	// own beside the convex and hull kernels.
 	const bool meshSide = !c->profiling && c->nMeshFix;
-	cudaStream_t ms = meshSide ? c->meshStream : s;
+	const uint32_t* meshList = B.bucketList + (size_t)BK_MESH * cap;
+	const uint32_t* meshCount = B.counters + CTR_BUCKET0 + BK_MESH;
 	if (meshSide)
 	{
 		cudaEventRecord(c->meshFork, s);
-		cudaStreamWaitEvent(ms, c->meshFork, 0);
+		cudaStreamWaitEvent(c->meshStream, c->meshFork, 0);
+		launch_mesh_prepare(c, c->meshStream);
+		launch_mesh_collide(c, meshList, meshCount, c->meshStream);
+		cudaEventRecord(c->meshJoin, c->meshStream);
 	}
-	launch_mesh_prepare(c, ms);
-	if (meshSide)
-		cudaEventRecord(c->meshJoin, ms);
-	k_bucket<<<persistent_blocks(8), BUCKET_THREADS, 0, s>>>(c->scene, B, c->cur, cap);
-	prof_mark(c, PM_BUCKETED, s);
 	NPArgs a = make_np_args(c);
 	// The buckets are disjoint sets of contacts: the hull-hull and
 	// hull-triangle kernels run on a second stream beside the convex ones
@@ -464,7 +478,11 @@ void launch_narrowphase(b3g_ctx* c, cudaStream_t s)
 	}
 	if (meshSide)
 		cudaStreamWaitEvent(s, c->meshJoin, 0);
-	launch_mesh_collide(c, B.bucketList + (size_t)BK_MESH * cap, B.counters + CTR_BUCKET0 + BK_MESH, s);
+	else
+	{
+		launch_mesh_prepare(c, s);
+		launch_mesh_collide(c, meshList, meshCount, s);
+	}
 	prof_mark(c, PM_MESH, s);
 }
 

@@ -120,6 +120,35 @@ def test_first_cast(kind, n, casts):
     pipe.close()
 
 
+# Spheres whose box covers none, some, more than a warp's row (128) and all of
+# a fine mesh's triangles: a work item per triangle whose box the sphere's fat
+# box in mesh space overlaps, and no other.
+@pytest.mark.parametrize("radius", [0.05, 0.6, 1.2, 2.5, 9.0])
+def test_mesh_items(radius):
+    V, T = S.grid_mesh(41, 41, 0.25, 3)
+    sc = S.Scene()
+    sc.mesh_arrays = dict(desc=np.array([0, len(V), 0, len(T)], np.uint32), verts=np.ascontiguousarray(V.reshape(-1)),
+                          tris=np.ascontiguousarray(T.reshape(-1), np.uint32), max_pairs=200000)
+    g = sc.add_body(0, N.BODY_STATIC, (0, 0, 0), (0, 0, 0, 1))
+    sc.add_fixture(g, N.SHAPE_MESH, [1.0, 1.0, 1.0, 0.0])
+    rng = np.random.default_rng(7)
+    p = np.concatenate([rng.uniform(-5, 5, (30, 1)), rng.uniform(-1, 1, (30, 1)), rng.uniform(-5, 5, (30, 1))], 1)
+    for x in p:
+        b = sc.add_body(0, N.BODY_DYNAMIC, x, (0, 0, 0, 1))
+        sc.add_fixture(b, N.SHAPE_SPHERE, [0, 0, 0, radius])
+    sc.finalize()
+    pipe = CollisionPipeline(sc)
+    pipe.collide(S.KinematicDriver(sc).state17())
+    F = np.float32
+    lo, hi = V[T].min(axis=1) - F(0.005), V[T].max(axis=1) + F(0.005)
+    want = 0
+    for x in sc.body_pos[1:]:
+        l, h = (x - F(radius)) - F(0.2), (x + F(radius)) + F(0.2)
+        want += int(np.all((lo <= h) & (hi >= l), axis=1).sum())
+    assert pipe.pass_stats()["mesh_items"] == want
+    pipe.close()
+
+
 def overlapping(pipe, sc):
     """Contacts every pass must hold: overlapping fat AABBs of two bodies, one of them dynamic."""
     box = pipe.fat_aabbs()
