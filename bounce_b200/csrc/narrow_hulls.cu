@@ -50,6 +50,41 @@ __device__ void warp_query_faces(const XF& xf1, const HullRef& h1, const XF& xf2
 	XF xf = xmult(xf2, xf1);
 	float best = -B3G_MAX_SCALAR;
 	uint32_t bi = 0xFFFFFFFFu;
+	// Few faces against many vertices (a triangle's two against a hull): the
+	// vertices go on the lanes instead, one face after the other. A face costs
+	// about 25 instructions of reduction then, and 12 per 32 vertices, where
+	// a lane per face costs 12 per vertex: it pays from 3 faces and 12
+	// vertices down and up. Measured on 13,870 items of 64-vertex hulls
+	// against triangles, with the launch shape below: 140 -> 130 us.
+	if (h1.fCnt <= 3 && h2.vCnt >= 12)
+	{
+		for (uint32_t i = 0; i < h1.fCnt; ++i)
+		{
+			PL plane = pmul(xf, hp(h1, i));
+			V3 d = -plane.n;
+			float sp = -INFINITY;
+			uint32_t si = 0xFFFFFFFFu;
+			for (uint32_t k = lane; k < h2.vCnt; k += 32)
+			{
+				float proj = dot(d, hv(h2, k));
+				if (si == 0xFFFFFFFFu || proj > sp)
+				{
+					si = k;
+					sp = proj;
+				}
+			}
+			warp_argmax(sp, si);
+			float s = pdist(hv(h2, si), plane);
+			if (s > best)
+			{
+				best = s;
+				bi = i;
+			}
+		}
+		index = bi == 0xFFFFFFFFu ? 0u : bi;
+		sep = best;
+		return;
+	}
 	for (uint32_t i = lane; i < h1.fCnt; i += 32)
 	{
 		PL plane = pmul(xf, hp(h1, i));
@@ -158,10 +193,19 @@ __host__ __device__ __forceinline__ uint32_t sat_warp_recs(uint32_t maxUE)
 	return maxUE > 2 * (SAT_FLAT_EDGES - 1) ? maxUE : 2 * (SAT_FLAT_EDGES - 1);
 }
 
+// The warps that share one hull pair's edge query: this one is `part` of
+// `parts`, they meet at barrier `bar` of their block, and slot[] holds one
+// (separation, pair) per part in shared memory.
+struct EdgeParts
+{
+	uint32_t part, parts, bar;
+	float2* slot;
+};
+
 // b3QueryEdgeSeparation(hull, hull) (sat.cpp:111-174). recs holds
 // sat_warp_recs(maxUE) records.
 __device__ void warp_query_edges(const XF& xf1, const HullRef& h1, const XF& xf2, const HullRef& h2,
-	uint32_t lane, EdgeRec* recs, uint32_t maxUE, uint32_t& index1, uint32_t& index2, float& sep)
+	uint32_t lane, EdgeRec* recs, uint32_t maxUE, const EdgeParts& P, uint32_t& index1, uint32_t& index2, float& sep)
 {
 	XF xf = xmult(xf2, xf1);
 	V3 C1 = xmul(xf, h1.centroid);
@@ -201,7 +245,8 @@ __device__ void warp_query_edges(const XF& xf1, const HullRef& h1, const XF& xf2
 		const bool rows1 = n1 >= n2;
 		const uint32_t nl = rows1 ? n1 : n2, nb = rows1 ? n2 : n1;
 		EdgeRec* rb = recs;
-		for (uint32_t b = lane; b < nb; b += 32)
+		const uint32_t b0 = nb * P.part / P.parts, b1 = nb * (P.part + 1) / P.parts;
+		for (uint32_t b = b0 + lane; b < b1; b += 32)
 		{
 			if (rows1)
 				edge_rec_2(rb[b], h2, 2 * b);
@@ -219,7 +264,7 @@ __device__ void warp_query_edges(const XF& xf1, const HullRef& h1, const XF& xf2
 				edge_rec_1(mine, xf, h1, le);
 			else
 				edge_rec_2(mine, h2, le);
-			for (uint32_t b = 0; b < nb; ++b)
+			for (uint32_t b = b0; b < b1; ++b)
 			{
 				const EdgeRec other = rb[b];
 				if (!valid)
@@ -232,8 +277,9 @@ __device__ void warp_query_edges(const XF& xf1, const HullRef& h1, const XF& xf2
 	else
 	{
 		// (i, j) of k = i n2 + j, stepped without a division per pair.
-		uint32_t i = n2 ? lane / n2 : 0u, j = lane - i * n2;
-		for (uint32_t k = lane; k < total; k += 32, j += 32)
+		const uint32_t k0 = lane + 32 * P.part, step = 32 * P.parts;
+		uint32_t i = n2 ? k0 / n2 : 0u, j = k0 - i * n2;
+		for (uint32_t k = k0; k < total; k += step, j += step)
 		{
 			while (j >= n2)
 			{
@@ -256,6 +302,23 @@ __device__ void warp_query_edges(const XF& xf1, const HullRef& h1, const XF& xf2
 		}
 	}
 	warp_argmax(best, bk);
+	if (P.parts > 1)
+	{
+		// First maximum over the parts: as over the lanes.
+		if (lane == 0)
+			P.slot[P.part] = make_float2(best, __uint_as_float(bk));
+		asm volatile("bar.sync %0, %1;" ::"r"(P.bar), "r"(32u * P.parts) : "memory");
+		for (uint32_t q = 0; q < P.parts; ++q)
+		{
+			const float2 o = P.slot[q];
+			const uint32_t ok = __float_as_uint(o.y);
+			if (o.x > best || (o.x == best && ok < bk))
+			{
+				best = o.x;
+				bk = ok;
+			}
+		}
+	}
 	if (bk == 0xFFFFFFFFu)
 	{
 		index1 = 0;
@@ -379,6 +442,15 @@ struct WarpClip
 __host__ __device__ __forceinline__ size_t sat_warp_bytes(uint32_t maxUE)
 {
 	size_t recs = (size_t)sat_warp_recs(maxUE) * sizeof(EdgeRec);
+	return recs > sizeof(WarpClip) ? recs : sizeof(WarpClip);
+}
+
+// The same where the second hull is a triangle: it has 3 edges, so a flat edge
+// query holds at most SAT_FLAT_EDGES - 1 + 3 records and a broadcast one 3,
+// however large the hulls are.
+__host__ __device__ __forceinline__ size_t sat_triangle_warp_bytes()
+{
+	size_t recs = (SAT_FLAT_EDGES + 2) * sizeof(EdgeRec);
 	return recs > sizeof(WarpClip) ? recs : sizeof(WarpClip);
 }
 
@@ -693,6 +765,7 @@ struct HullCtx
 	uint32_t maxUE;
 	uint32_t* status;
 	WarpClip* clip; // the warp's shared clip buffers
+	EdgeParts parts;
 };
 
 // Lane 0 builds, the warp learns the point count.
@@ -717,7 +790,7 @@ __device__ void collide_hulls_nocache(DevManifold& m, const HullCtx& H, uint32_t
 	warp_query_faces(H.xf2, H.h2, H.xf1, H.h1, lane, fi2, fs2);
 	if (fs2 > totalRadius)
 		return;
-	warp_query_edges(H.xf1, H.h1, H.xf2, H.h2, lane, H.recs, H.maxUE, ei1, ei2, es);
+	warp_query_edges(H.xf1, H.h1, H.xf2, H.h2, lane, H.recs, H.maxUE, H.parts, ei1, ei2, es);
 	if (es > totalRadius)
 		return;
 	const float kRelEdgeTol = 0.90f;
@@ -839,12 +912,14 @@ __device__ void sat_after_miss(DevManifold& m, const HullCtx& H, uint4& cache, u
 		cache = make_uint4(CT_SEPARATION, FT_FACE2, fi2, fi2);
 		return;
 	}
-	warp_query_edges(H.xf1, H.h1, H.xf2, H.h2, lane, H.recs, H.maxUE, ei1, ei2, es);
+	warp_query_edges(H.xf1, H.h1, H.xf2, H.h2, lane, H.recs, H.maxUE, H.parts, ei1, ei2, es);
 	if (es > totalRadius)
 	{
 		cache = make_uint4(CT_SEPARATION, FT_EDGES, ei1, ei2);
 		return;
 	}
+	if (H.parts.part != 0)
+		return; // the contact is the first part's
 	const float kRelEdgeTol = 0.90f;
 	const float kRelFaceTol = 0.98f;
 	const float kAbsTol = 0.5f * B3G_LINEAR_SLOP;
@@ -907,6 +982,7 @@ __device__ __forceinline__ void load_hull_ctx(const NPArgs& a, uint32_t c, HullC
 	H.recs = nullptr;
 	H.maxUE = 0;
 	H.clip = nullptr;
+	H.parts = EdgeParts{0, 1, 0, nullptr};
 }
 
 // Pass 1: one thread per hull-hull contact reads its feature cache.
@@ -996,6 +1072,12 @@ __device__ __forceinline__ bool stage_wait(unsigned long long* bar, uint32_t pha
 // over the other hull's vertices waited on each load. Shared memory per block:
 // W barriers (16-byte rounded), then per warp its query / clip area
 // (sat_warp_bytes), then per warp its staging area (sat_stage_bytes).
+//
+// With fewer pairs than half (a quarter) of the warps, 2 (4) warps of a block
+// share a pair: each runs the face queries and its part of the edge pairs (93
+// x 93 of them between two 64-vertex hulls, most of the time), and the first
+// goes on with the contact. Measured on 77 pairs of 12-64-vertex hulls: 158 us
+// with a warp each, 62 us with 4.
 template <int W, bool STAGE>
 __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 {
@@ -1018,14 +1100,18 @@ __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 		}
 		__syncwarp();
 	}
+	__shared__ float2 partBest[2][W];
 	uint32_t n = *a.missCount;
-	uint32_t gw = blockIdx.x * W + warp;
 	uint32_t nw = gridDim.x * W;
-	for (uint32_t t = gw; t < n; t += nw)
+	const uint32_t parts = !a.convexCache ? 1u : (W >= 4 && 4u * n <= nw ? 4u : (2u * n <= nw ? 2u : 1u));
+	uint32_t turn = 0;
+	for (uint32_t t = (blockIdx.x * W + warp) / parts; t < n; t += nw / parts, turn ^= 1u)
 	{
 		uint32_t c = a.missList[t];
 		HullCtx H;
 		load_hull_ctx(a, c, H);
+		// The slots alternate: a warp may be a pair ahead of one still reading.
+		H.parts = EdgeParts{warp % parts, parts, 1u + warp / parts, &partBest[turn][warp / parts * parts]};
 		H.recs = recs;
 		H.clip = reinterpret_cast<WarpClip*>(wsm);
 		H.maxUE = maxUE;
@@ -1076,7 +1162,7 @@ __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 		else
 			collide_hulls_nocache(m, H, lane);
 		__syncwarp();
-		if (lane == 0)
+		if (lane == 0 && H.parts.part == 0)
 		{
 			finish_convex(a, c, m);
 			a.cache[c] = cache;
@@ -1166,6 +1252,7 @@ __global__ void __launch_bounds__(W * 32) k_hull_triangle(NPArgs a, uint32_t max
 		H.recs = recs;
 		H.clip = reinterpret_cast<WarpClip*>(wsm);
 		H.maxUE = maxUE;
+		H.parts = EdgeParts{0, 1, 0, nullptr};
 		DevManifold& m = a.man[c];
 		if (lane == 0)
 			man_clear(m);
@@ -1190,11 +1277,11 @@ __global__ void __launch_bounds__(W * 32) k_hull_triangle(NPArgs a, uint32_t max
 // (hull_mesh_contact.cpp:42-50), points tagged with the triangle. Sensor
 // contacts record the triangle's overlap in pointCount.
 template <int W>
-__global__ void __launch_bounds__(W * 32) k_mesh_items_hull(NPArgs a, Buffers B, uint32_t maxUE)
+__global__ void __launch_bounds__(W * 32, 4) k_mesh_items_hull(NPArgs a, Buffers B, uint32_t maxUE)
 {
 	extern __shared__ float4 smem[];
 	const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	char* wsm = reinterpret_cast<char*>(smem) + (size_t)warp * sat_warp_bytes(maxUE);
+	char* wsm = reinterpret_cast<char*>(smem) + (size_t)warp * sat_triangle_warp_bytes();
 	EdgeRec* recs = reinterpret_cast<EdgeRec*>(wsm);
 	uint32_t n = min(B.counters[CTR_MESH_PAIRS], B.meshPairCap);
 	for (uint32_t i = blockIdx.x * W + warp; i < n; i += gridDim.x * W)
@@ -1216,6 +1303,7 @@ __global__ void __launch_bounds__(W * 32) k_mesh_items_hull(NPArgs a, Buffers B,
 		H.recs = recs;
 		H.clip = reinterpret_cast<WarpClip*>(wsm);
 		H.maxUE = maxUE;
+		H.parts = EdgeParts{0, 1, 0, nullptr};
 		DevManifold& m = B.meshPairMan[i];
 		if (lane == 0)
 			man_clear(m);
@@ -1371,8 +1459,6 @@ size_t hull_sat_smem(int warps, uint32_t maxUE)
 void launch_mesh_items_hull(const NPArgs& a, const Buffers& B, uint32_t maxUE, const Tune& tune, cudaStream_t s)
 {
 	uint32_t ue = maxUE > 3 ? maxUE : 3;
-	size_t smem = hull_sat_smem(4, ue);
-	if (smem > 48 * 1024)
-		cudaFuncSetAttribute(k_mesh_items_hull<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-	k_mesh_items_hull<4><<<persistent_blocks((int)tune.v[B3G_TUNE_SAT_BLOCKS]), 128, smem, s>>>(a, B, ue);
+	// As many blocks as 128 registers allow (with 80 or 255 it takes longer).
+	k_mesh_items_hull<4><<<persistent_blocks(4), 128, 4 * sat_triangle_warp_bytes(), s>>>(a, B, ue);
 }
