@@ -480,9 +480,6 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 	step(dalloc(&B.nodeFirst, 2 * P), "alloc");
 	step(dalloc(&B.leafData, P), "alloc");
 	step(dalloc(&B.leafOf, P), "alloc");
-	step(dalloc(&B.walkNodes, 4 * (size_t)P), "alloc");
-	step(dalloc(&B.walkLeaves, 4 * (size_t)P), "alloc");
-	step(dalloc(&B.walkTurned, 1), "alloc");
 	step(dalloc(&B.nodeParent, 2 * P), "alloc");
 	step(dalloc(&B.nodeEnd, P), "alloc");
 	step(dalloc(&B.splitRight, P), "alloc");
@@ -591,9 +588,6 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 	dfree(B.nodeFirst);
 	dfree(B.leafData);
 	dfree(B.leafOf);
-	dfree(B.walkNodes);
-	dfree(B.walkLeaves);
-	dfree(B.walkTurned);
 	dfree(B.nodeParent);
 	dfree(B.nodeEnd);
 	dfree(B.splitRight);

@@ -168,11 +168,9 @@ struct Buffers
 	uint32_t* proxyInfo;  // per proxy: body (bits 0-27), dynamic body (bit 28), shape type (bits 29-31)
 	uint2* leafData;      // per sorted leaf: its proxy's proxyInfo word and fixture key
 	uint32_t* leafOf;     // per proxy: its sorted leaf (set when the LBVH is built)
-	float4* walkNodes;    // the tree as the world queries walk it: 4 float4 per inner node (queries.cu)
-	float4* walkLeaves;   // and 4 float4 per sorted leaf
-	uint32_t* walkTurned; // a triangle fixture lies outside its box (queries.cu)
 	uint32_t* leafCount;  // pair count per sorted leaf (then exclusive offsets)
-	uint32_t* pairScratch; // first contact records (A, B) found per leaf, slot-major (B3G_TRAV_SLOTS x n uint2)
+	uint32_t* pairScratch; // first contact records (A, B) found per leaf, slot-major (B3G_TRAV_SLOTS x n uint2);
+	                       // between passes the tree as the world queries walk it (queries.cu)
 	uint32_t* scanAux;
 	uint32_t* rawA;       // overlapping pairs in traversal order (this pass)
 	uint32_t* rawB;
@@ -311,7 +309,8 @@ enum
 	CTR_HC_DEEP = 35,       // ... and overlapping
 	CTR_HS_POST = 36,       // hull-sphere contacts past their face scan (k_hull_sphere_gjk)
 	CTR_MESH_ALL = 37,      // mesh contacts of the pass, skipped ones included
-	CTR_COUNT = 38
+	CTR_WALK_TURNED = 38,   // a triangle fixture lies outside its box (queries.cu)
+	CTR_COUNT = 39
 };
 static_assert(CTR_BUCKET0 + BK_COUNT <= CTR_ASLEEP, "bucket counters overlap");
 

@@ -1046,16 +1046,18 @@ __global__ void __launch_bounds__(32) k_ray_first_warp(QueryCtx q, WalkTree tree
 // 124 and 286 us; at 40,000: 459 and 317 us.
 constexpr uint32_t RAY_WARP_MAX = 148u * 160u;
 
-// The tree laid out for the ordered walks, in the context's own records.
+// The tree laid out for the ordered walks, in the scratch of the pair search,
+// which holds nothing between passes.
 WalkTree launch_walk_tree(b3g_ctx* c, const QueryCtx& q, uint32_t* turned, cudaStream_t s)
 {
 	WalkTree t;
-	t.nodes = c->buf.walkNodes;
-	t.leaves = c->buf.walkLeaves;
+	static_assert(sizeof(uint2) * B3G_TRAV_SLOTS >= 8 * sizeof(float4), "two records per proxy");
+	float4* nodes = reinterpret_cast<float4*>(c->buf.pairScratch);
+	float4* leaves = nodes + 4 * (size_t)c->cfg.max_proxies;
+	t.nodes = nodes;
+	t.leaves = leaves;
 	t.count = q.leaves;
-	if (turned)
-		cudaMemsetAsync(turned, 0, sizeof(uint32_t), s);
-	k_walk_tree<<<(q.leaves + 127) / 128, 128, 0, s>>>(q, c->buf.walkNodes, c->buf.walkLeaves, turned);
+	k_walk_tree<<<(q.leaves + 127) / 128, 128, 0, s>>>(q, nodes, leaves, turned);
 	return t;
 }
 
@@ -1719,7 +1721,9 @@ __global__ void __launch_bounds__(CAST_WARPS * 32, CAST_BLOCKS) k_shape_cast_fir
 void launch_shape_cast_first(b3g_ctx* c, const QueryCtx& q, const float* casts, uint32_t n, uint32_t* fix, float* hit,
 	cudaStream_t s)
 {
-	uint32_t* turned = c->anyTriangle ? c->buf.walkTurned : nullptr;
+	// Cleared by each pass and only set here, so that calls on several streams,
+	// which write the same records, never see it go back to 0.
+	uint32_t* turned = c->anyTriangle ? c->buf.counters + CTR_WALK_TURNED : nullptr;
 	const WalkTree t = launch_walk_tree(c, q, turned, s);
 	// As many lanes to a cast as leave the GPU about 16 warps per SM: 16,384
 	// casts took 1.17 ms with 4 lanes each, 1.23 ms with 16.
