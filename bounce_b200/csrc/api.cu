@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "collide_common.cuh"
+#include "scan.cuh"
 
 namespace {
 
@@ -99,17 +100,24 @@ uint32_t pow2_at_least(uint32_t v)
 	return p;
 }
 
-__global__ void k_pass_begin(uint32_t* counters, int havePass, uint32_t cap)
+// What a pass counts in or scans over starts at 0: the counters (the previous
+// pass's contact count moves to CTR_PREV_PAIRS; CTR_PAIRS itself stays until
+// the contact list is laid out), the new contacts' groups, the scans' states
+// and the previous contacts' found flags. One kernel for what were seven
+// memsets between the pass's kernels, about 2.5 us each on the stream.
+__global__ void k_pass_begin(Buffers B, int havePass, uint32_t cap, uint32_t nf)
 {
-	uint32_t i = threadIdx.x;
-	if (i >= CTR_COUNT)
-		return;
-	uint32_t pairs = counters[CTR_PAIRS];
-	__syncthreads();
-	if (i == CTR_PREV_PAIRS)
-		counters[i] = havePass ? min(pairs, cap) : 0u;
-	else
-		counters[i] = 0;
+	const uint32_t prev = havePass ? min(B.counters[CTR_PAIRS], cap) : 0u;
+	const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+	if (first < CTR_COUNT && first != CTR_PAIRS)
+		B.counters[first] = first == CTR_PREV_PAIRS ? prev : 0u;
+	for (uint32_t i = first; i <= nf; i += stride)
+		B.newOff[i] = B.newFill[i] = 0;
+	const uint32_t words = (nf + 1 + SC_TILE - 1) / SC_TILE + (prev + SC_TILE - 1) / SC_TILE + 2;
+	for (uint32_t i = first; i < words; i += stride)
+		B.passScan[i] = 0;
+	for (uint32_t i = first; i < prev; i += stride)
+		B.prevFound[i] = 0;
 }
 
 // b3TriangleHull::Set (triangle_hull.h:36-69) for every triangle fixture:
@@ -486,9 +494,11 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 	step(dalloc(&B.refitFlag, P), "alloc");
 	step(dalloc(&B.worldEnd, P), "alloc");
 	step(dalloc(&B.proxyInfo, P), "alloc");
-	step(dalloc(&B.leafCount, std::max(P, C)), "alloc");
+	step(dalloc(&B.outOff, C), "alloc");
 	step(dalloc(&B.pairScratch, 2 * B3G_TRAV_SLOTS * (size_t)P), "alloc"); // uint2 records per leaf
-	step(dalloc(&B.scanAux, scan_aux_words(std::max(P, C) + 1)), "alloc");
+	const size_t scanWords = scan_aux_words(std::max(P, C) + 1);
+	step(dalloc(&B.scanAux, scanWords + scan_aux_words(P + 1) + scan_aux_words(C)), "alloc");
+	B.passScan = reinterpret_cast<unsigned long long*>(B.scanAux + scanWords);
 	for (int k = 0; k < 2; ++k)
 	{
 		step(dalloc(&B.pairA[k], C), "alloc");
@@ -508,7 +518,6 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 	step(dalloc(&B.prevFound, C), "alloc");
 	step(dalloc(&B.rawA, C), "alloc");
 	step(dalloc(&B.rawB, C), "alloc");
-	step(dalloc(&B.travOverflow, C), "alloc");
 	step(dalloc(&B.newList, C), "alloc");
 	step(dalloc(&B.newOff, (size_t)P + 1), "alloc");
 	step(dalloc(&B.newFill, (size_t)P + 1), "alloc");
@@ -594,7 +603,7 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 	dfree(B.refitFlag);
 	dfree(B.worldEnd);
 	dfree(B.proxyInfo);
-	dfree(B.leafCount);
+	dfree(B.outOff);
 	dfree(B.pairScratch);
 	dfree(B.scanAux);
 	for (int k = 0; k < 2; ++k)
@@ -613,7 +622,6 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 	dfree(B.prevFound);
 	dfree(B.rawA);
 	dfree(B.rawB);
-	dfree(B.travOverflow);
 	dfree(B.newList);
 	dfree(B.newOff);
 	dfree(B.newFill);
@@ -1528,7 +1536,8 @@ static void issue_pass(b3g_ctx* c, cudaStream_t s, const float* state, size_t by
 		if (cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &deps, &nd) == cudaSuccess && nd == 1)
 			*copyNode = deps[0];
 	}
-	k_pass_begin<<<1, CTR_COUNT, 0, s>>>(c->buf.counters, c->havePass ? 1 : 0, c->cfg.max_contacts);
+	k_pass_begin<<<work_blocks(std::max<uint64_t>(c->nFixtures + 1, c->cfg.max_contacts), 256, 4), 256, 0, s>>>(c->buf,
+		c->havePass ? 1 : 0, c->cfg.max_contacts, c->nFixtures);
 	prof_mark(c, PM_UPLOADED, s);
 	launch_sync(c, s);
 	prof_mark(c, PM_SYNCED, s);
@@ -1693,7 +1702,7 @@ extern "C" int b3g_collide(b3g_ctx* c, const float* state, int onDevice, void* s
 			c->candFetched = false;
 			c->passStream = s;
 			// pass begin, sync, broadphase, candidates; the rest in b3g_finish_pass
-			c->launches += 1 + 1 + (c->creationPass && c->nMeshFix ? 1 : 0) + broadphase_launches(c) + 2;
+			c->launches += 1 + 1 + (c->creationPass && c->nMeshFix ? 1 : 0) + broadphase_launches(c) + 1;
 			CK(cudaGetLastError());
 			tree_pass_issued(c);
 			return B3G_OK;
@@ -2010,7 +2019,7 @@ extern "C" int b3g_fetch_touching(b3g_ctx* c, uint32_t* index, void* manifolds, 
 	Buffers& B = c->buf;
 	if (n == 0)
 		return 0;
-	uint32_t* offsets = B.leafCount; // sized max(P, C)
+	uint32_t* offsets = B.outOff;
 	const DevManifold* extra = B.extraMan[c->cur] ? B.extraMan[c->cur] : B.man[c->cur];
 	wait_copies(c, c->stream);
 	k_touch_flags<<<(n + 255) / 256, 256, 0, c->stream>>>(B.man[c->cur], extra, B.cstate[c->cur], n, offsets);
@@ -2065,7 +2074,7 @@ extern "C" int b3g_fetch_results_async(b3g_ctx* c, uint32_t* contacts, uint32_t 
 	wait_copies(c, c->stream);
 	if (n && touchCapacity)
 	{
-		uint32_t* offsets = B.leafCount;
+		uint32_t* offsets = B.outOff;
 		const DevManifold* extra = B.extraMan[c->cur] ? B.extraMan[c->cur] : B.man[c->cur];
 		k_touch_flags<<<(n + 255) / 256, 256, 0, c->stream>>>(B.man[c->cur], extra, B.cstate[c->cur], n, offsets);
 		scan_exclusive(offsets, n, B.scanAux, B.counters + CTR_TOUCH_OUT, B.counters + CTR_STATUS, c->stream);
@@ -2126,11 +2135,11 @@ extern "C" int b3g_fetch_results_packed_async(b3g_ctx* c, uint32_t* contacts, ui
 	if (n && touchCapacity)
 	{
 		const DevManifold* extra = B.extraMan[c->cur] ? B.extraMan[c->cur] : B.man[c->cur];
-		k_pack_sizes<<<(n + 255) / 256, 256, 0, c->stream>>>(B.man[c->cur], extra, B.cstate[c->cur], n, B.leafCount,
+		k_pack_sizes<<<(n + 255) / 256, 256, 0, c->stream>>>(B.man[c->cur], extra, B.cstate[c->cur], n, B.outOff,
 			c->touchBytes);
-		scan_exclusive(B.leafCount, n, B.scanAux, B.counters + CTR_TOUCH_OUT, B.counters + CTR_STATUS, c->stream);
+		scan_exclusive(B.outOff, n, B.scanAux, B.counters + CTR_TOUCH_OUT, B.counters + CTR_STATUS, c->stream);
 		scan_exclusive(c->touchBytes, n, B.scanAux, B.counters + CTR_SCRATCH, B.counters + CTR_STATUS, c->stream);
-		k_pack_scatter<<<(n + 255) / 256, 256, 0, c->stream>>>(B.man[c->cur], extra, B.cstate[c->cur], n, B.leafCount,
+		k_pack_scatter<<<(n + 255) / 256, 256, 0, c->stream>>>(B.man[c->cur], extra, B.cstate[c->cur], n, B.outOff,
 			c->touchBytes, B.touchIndex, reinterpret_cast<unsigned long long*>(B.touchMan));
 	}
 	CK(cudaEventRecord(c->copyReady, c->stream));
@@ -2836,7 +2845,10 @@ extern "C" int b3g_autotune(b3g_ctx* c, uint32_t reps, void* stream, uint32_t* o
 		if (h[CTR_BUCKET0 + convexBucket[k]] == 0)
 			continue;
 		pick(c->tune.v[B3G_TUNE_CONVEX + k], kBlocksPerSM, 5,
-			[&] { launch_convex_one(k, a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s); });
+			[&] {
+				reset_post_counts(B, s);
+				launch_convex_one(k, a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
+			});
 	}
 	const uint32_t* hullList = B.bucketList + (size_t)BK_HULLS * cap;
 	const uint32_t* hullCount = B.counters + CTR_BUCKET0 + BK_HULLS;
@@ -2863,7 +2875,11 @@ extern "C" int b3g_autotune(b3g_ctx* c, uint32_t reps, void* stream, uint32_t* o
 		probeSat();
 	}
 	if (rc == B3G_OK)
-		pick(c->tune.v[B3G_TUNE_TRAVERSE], kTraverse, 3, [&] { launch_traverse(c, s); });
+		pick(c->tune.v[B3G_TUNE_TRAVERSE], kTraverse, 3, [&] {
+			cudaMemsetAsync(B.counters + CTR_RAW, 0, sizeof(uint32_t), s);
+			cudaMemsetAsync(B.counters + CTR_TRAV_OVERFLOW, 0, sizeof(uint32_t), s);
+			launch_traverse(c, s);
+		});
 	cudaEventDestroy(e0);
 	cudaEventDestroy(e1);
 	CK(cudaStreamSynchronize(s));

@@ -168,13 +168,13 @@ struct Buffers
 	uint32_t* proxyInfo;  // per proxy: body (bits 0-27), dynamic body (bit 28), shape type (bits 29-31)
 	uint2* leafData;      // per sorted leaf: its proxy's proxyInfo word and fixture key
 	uint32_t* leafOf;     // per proxy: its sorted leaf (set when the LBVH is built)
-	uint32_t* leafCount;  // pair count per sorted leaf (then exclusive offsets)
+	uint32_t* outOff;     // per contact: offsets of the touching output
 	uint32_t* pairScratch; // first contact records (A, B) found per leaf, slot-major (B3G_TRAV_SLOTS x n uint2);
 	                       // between passes the tree as the world queries walk it (queries.cu)
-	uint32_t* scanAux;
+	uint32_t* scanAux;    // scan state
+	unsigned long long* passScan; // scan states of the contact list (order.cu), cleared when the pass begins
 	uint32_t* rawA;       // overlapping pairs in traversal order (this pass)
 	uint32_t* rawB;
-	uint4* travOverflow;  // records past a leaf's scratch slots: A, B, leaf, index in the leaf
 
 	// contact-list order: new contacts, then the kept previous ones
 	uint32_t* newList;    // raw indices of pairs without a previous contact
@@ -546,3 +546,10 @@ void launch_contact_constraints(b3g_ctx* c, const ConstraintCall& q, cudaStream_
 
 // Grid size for grid-stride loops over device-side counts.
 inline int persistent_blocks(int perSM = 8) { return 148 * perSM; }
+// The same, but no more than `items` at most give work to: a grid of 1,184
+// blocks for the few contacts of a small scene takes 1 us longer to come and go.
+inline int work_blocks(uint64_t items, uint32_t perBlock, int perSM)
+{
+	const uint64_t b = (items + perBlock - 1) / perBlock;
+	return (int)(b < 1 ? 1 : (b < 148ull * perSM ? b : 148ull * perSM));
+}

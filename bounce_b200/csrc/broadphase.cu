@@ -24,6 +24,7 @@
 #include <cuda/atomic>
 
 #include "collide_common.cuh"
+#include "scan.cuh"
 
 namespace {
 
@@ -769,8 +770,7 @@ __device__ __forceinline__ uint2 canon_pair_keys(uint32_t pa, uint32_t keyA, uin
 // (leafData) load beside it, so a found pair costs no further dependent
 // load. The walk counts the filtered
 // overlaps, keeps the first TRAV_SLOTS contact records in the leaf's scratch
-// slots (slot-major) and appends the others, with their leaf and index, to
-// the overflow list. MW: several worlds share the tree, so the walk stops at
+// slots (slot-major) and appends the others to the pair list one by one. MW: several worlds share the tree, so the walk stops at
 // the first node past the query's world (worlds are contiguous in
 // depth-first order).
 constexpr uint32_t TRAV_SLOTS = B3G_TRAV_SLOTS;
@@ -820,9 +820,13 @@ __device__ __forceinline__ uint32_t walk(const DevScene& S, Buffers& B, int n, i
 					scratch[(size_t)count * n + j] = p;
 				else
 				{
-					uint32_t o = atomicAdd(&B.counters[CTR_TRAV_OVERFLOW], 1u);
+					atomicAdd(&B.counters[CTR_TRAV_OVERFLOW], 1u);
+					const uint32_t o = atomicAdd(&B.counters[CTR_RAW], 1u);
 					if (o < cap)
-						B.travOverflow[o] = make_uint4(p.x, p.y, (uint32_t)j, count);
+					{
+						B.rawA[o] = p.x;
+						B.rawB[o] = p.y;
+					}
 				}
 				++count;
 			}
@@ -850,7 +854,8 @@ __global__ void k_traverse_count(DevScene S, Buffers B, int n, uint32_t cur, uin
 	const uint32_t live = min(32u, (uint32_t)n - ((uint32_t)j - lane));
 	const uint32_t mask = live == 32u ? 0xFFFFFFFFu : (1u << live) - 1u;
 	__syncwarp(mask);
-	uint32_t incl = count;
+	const uint32_t kept = min(count, TRAV_SLOTS);
+	uint32_t incl = kept;
 	for (uint32_t o = 1; o < 32u; o <<= 1)
 	{
 		const uint32_t y = __shfl_up_sync(mask, incl, o);
@@ -860,10 +865,8 @@ __global__ void k_traverse_count(DevScene S, Buffers B, int n, uint32_t cur, uin
 	uint32_t base = 0;
 	if (lane == live - 1u)
 		base = atomicAdd(&B.counters[CTR_RAW], incl);
-	base = __shfl_sync(mask, base, live - 1u) + incl - count;
-	B.leafCount[j] = base;
+	base = __shfl_sync(mask, base, live - 1u) + incl - kept;
 	const uint2* scratch = reinterpret_cast<const uint2*>(B.pairScratch);
-	const uint32_t kept = min(count, TRAV_SLOTS);
 	for (uint32_t k = 0; k < kept; ++k)
 	{
 		const uint32_t slot = base + k;
@@ -876,150 +879,18 @@ __global__ void k_traverse_count(DevScene S, Buffers B, int n, uint32_t cur, uin
 	}
 }
 
-// The overflow records: record k of leaf j goes to leafCount[j] + k. A list
-// longer than the contact capacity means more pairs than contacts fit, which
-// the status already reports.
-__global__ void k_traverse_overflow(Buffers B, uint32_t cap)
-{
-	uint32_t n = min(B.counters[CTR_TRAV_OVERFLOW], cap);
-	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-	{
-		uint4 r = B.travOverflow[t];
-		uint32_t slot = B.leafCount[r.z] + r.w;
-		if (slot < cap)
-		{
-			B.rawA[slot] = r.x;
-			B.rawB[slot] = r.y;
-		}
-	}
-}
-
-// One-pass exclusive scan of u32 in place (decoupled look-back, as the
-// one-sweep sort): a block takes the next tile through a counter, reduces its
-// SC_TILE entries, publishes the tile's sum, adds up the sums of the tiles
-// before it (walking back until a tile that already published its inclusive
-// prefix; bounded wait) and writes its entries' offsets. n: *nPtr (at most
-// cap) when nPtr is set, else nHost. state: the tile counter, then one word
-// per tile (flag in bits 62-63, sum in bits 0-31), zeroed before the launch.
-// The tile holding the last entry writes the total (0 for an empty scan).
-constexpr int SC_THREADS = 256;
-constexpr int SC_ITEMS = 8;
-constexpr uint32_t SC_TILE = SC_THREADS * SC_ITEMS;
-constexpr unsigned long long SC_AGG = 1ull << 62;
-constexpr unsigned long long SC_INC = 2ull << 62;
-constexpr uint32_t SC_SPIN = 1u << 22;
-
+// Scan in place of *nPtr entries (at most cap) when nPtr is set, else nHost.
 __global__ void __launch_bounds__(SC_THREADS) k_scan_tiles(uint32_t* data, const uint32_t* nPtr, uint32_t nHost,
 	uint32_t cap, unsigned long long* state, uint32_t* total, uint32_t* err)
 {
-	__shared__ uint32_t sTile, sPrefix;
-	__shared__ uint32_t warpSums[SC_THREADS / 32];
-	const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
 	const uint32_t n = nPtr ? min(*nPtr, cap) : nHost;
-	if (t == 0)
-		sTile = atomicAdd(reinterpret_cast<unsigned int*>(state), 1u);
-	__syncthreads();
-	const uint32_t tile = sTile;
-	const uint32_t numTiles = (n + SC_TILE - 1) / SC_TILE;
-	if (tile >= numTiles)
-	{
-		if (tile == 0 && t == 0 && total)
-			*total = 0u;
-		return;
-	}
-	// Thread t owns entries [t * SC_ITEMS, t * SC_ITEMS + SC_ITEMS) of the tile.
-	const uint32_t first = tile * SC_TILE + t * SC_ITEMS;
-	uint32_t v[SC_ITEMS];
-	uint32_t sum = 0;
+	scan_tile(
+		[=](uint32_t first, uint32_t* v) {
 #pragma unroll
-	for (int r = 0; r < SC_ITEMS; ++r)
-	{
-		v[r] = first + r < n ? data[first + r] : 0u;
-		sum += v[r];
-	}
-	uint32_t incl = sum;
-#pragma unroll
-	for (int o = 1; o < 32; o <<= 1)
-	{
-		uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-		if (lane >= (uint32_t)o)
-			incl += y;
-	}
-	if (lane == 31)
-		warpSums[warp] = incl;
-	__syncthreads();
-	if (warp == 0)
-	{
-		uint32_t w = lane < SC_THREADS / 32 ? warpSums[lane] : 0u;
-		uint32_t wi = w;
-#pragma unroll
-		for (int o = 1; o < SC_THREADS / 32; o <<= 1)
-		{
-			uint32_t y = __shfl_up_sync(0xFFFFFFFFu, wi, o);
-			if (lane >= (uint32_t)o)
-				wi += y;
-		}
-		const uint32_t agg = __shfl_sync(0xFFFFFFFFu, wi, SC_THREADS / 32 - 1);
-		if (lane < SC_THREADS / 32)
-			warpSums[lane] = wi - w;
-		// Look-back by the whole warp: lane k reads the tile k + 1 places
-		// back, so a round trip covers 32 tiles. A window is taken once every
-		// tile in it has published; the nearest inclusive prefix in it ends
-		// the walk (tiles before the first one count as an inclusive 0).
-		volatile unsigned long long* st = state + 1;
-		if (lane == 0)
-			st[tile] = (tile == 0 ? SC_INC : SC_AGG) | agg;
-		uint32_t prefix = 0;
-		int32_t look = (int32_t)tile - 1;
-		uint32_t spins = 0;
-		while (tile > 0)
-		{
-			const int32_t idx = look - (int32_t)lane;
-			unsigned long long w8 = 2ull << 62; // before tile 0: an inclusive 0
-			if (idx >= 0)
-				w8 = st[idx];
-			if (!__all_sync(0xFFFFFFFFu, (w8 >> 62) != 0ull))
-			{
-				if (++spins > SC_SPIN)
-				{
-					if (lane == 0)
-						atomicOr(err, B3G_ST_WAIT_TIMEOUT);
-					break;
-				}
-				continue;
-			}
-			const uint32_t inc = __ballot_sync(0xFFFFFFFFu, (w8 & SC_INC) != 0ull);
-			const uint32_t last = inc ? (uint32_t)(__ffs(inc) - 1) : 31u;
-			uint32_t v = lane <= last ? (uint32_t)w8 : 0u;
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1)
-				v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-			prefix += v;
-			if (inc)
-				break;
-			look -= 32;
-		}
-		if (lane == 0)
-		{
-			if (tile > 0)
-			{
-				__threadfence();
-				st[tile] = SC_INC | (uint32_t)(prefix + agg);
-			}
-			sPrefix = prefix;
-			if (tile == numTiles - 1 && total)
-				*total = prefix + agg;
-		}
-	}
-	__syncthreads();
-	uint32_t run = sPrefix + warpSums[warp] + incl - sum;
-#pragma unroll
-	for (int r = 0; r < SC_ITEMS; ++r)
-	{
-		if (first + r < n)
-			data[first + r] = run;
-		run += v[r];
-	}
+			for (int r = 0; r < SC_ITEMS; ++r)
+				v[r] = first + r < n ? data[first + r] : 0u;
+		},
+		data, n, state, total, err);
 }
 
 } // namespace
@@ -1027,23 +898,14 @@ __global__ void __launch_bounds__(SC_THREADS) k_scan_tiles(uint32_t* data, const
 // Words of scan state (u32) a scan of up to n entries needs in aux.
 uint32_t scan_aux_words(uint32_t n)
 {
-	return 2u * ((n + SC_TILE - 1) / SC_TILE + 1u);
+	return 2u * (scan_tiles(n) + 1u);
 }
 
 void scan_exclusive(uint32_t* data, uint32_t n, uint32_t* aux, uint32_t* total, uint32_t* err, cudaStream_t s)
 {
-	const uint32_t tiles = (n + SC_TILE - 1) / SC_TILE;
+	const uint32_t tiles = scan_tiles(n);
 	cudaMemsetAsync(aux, 0, sizeof(unsigned long long) * (tiles + 1u), s);
 	k_scan_tiles<<<tiles ? tiles : 1u, SC_THREADS, 0, s>>>(data, nullptr, n, n,
-		reinterpret_cast<unsigned long long*>(aux), total, err);
-}
-
-void scan_exclusive_device(uint32_t* data, const uint32_t* nPtr, uint32_t cap, uint32_t* aux, uint32_t* total,
-	uint32_t* err, cudaStream_t s)
-{
-	const uint32_t tiles = (cap + SC_TILE - 1) / SC_TILE;
-	cudaMemsetAsync(aux, 0, sizeof(unsigned long long) * (tiles + 1u), s);
-	k_scan_tiles<<<tiles ? tiles : 1u, SC_THREADS, 0, s>>>(data, nPtr, 0u, cap,
 		reinterpret_cast<unsigned long long*>(aux), total, err);
 }
 
@@ -1107,12 +969,11 @@ uint32_t broadphase_launches(const b3g_ctx* c)
 	while ((1u << wb) < c->nWorlds)
 		++wb;
 	uint32_t passes = 4 + (wb + 7) / 8;
-	// traversal: walk (with the pair list's ranges), overflow records
 	if (!c->treeRebuild)
-		return 2; // the tree refit by the sync kernel
+		return 1; // the walk; the tree is refit by the sync kernel
 	// bounds init, bounds, Morton; sort: histogram, scan, one kernel per
-	// pass; build; leaves, refit
-	return 3 + (passes + 2) + (n > 1 ? 1 : 0) + 2 + 2;
+	// pass; build; leaves, refit; walk
+	return 3 + (passes + 2) + (n > 1 ? 1 : 0) + 2 + 1;
 }
 
 void launch_broadphase(b3g_ctx* c, cudaStream_t s)
@@ -1121,10 +982,7 @@ void launch_broadphase(b3g_ctx* c, cudaStream_t s)
 	int n = (int)c->nFixtures;
 	c->treeLeaves = (uint32_t)n;
 	if (n == 0)
-	{
-		cudaMemsetAsync(B.counters + CTR_RAW, 0, sizeof(uint32_t), s);
 		return;
-	}
 	if (!c->treeRebuild)
 	{
 		// Same tree as the last pass, refit by k_sync (grow_leaf): walk.
@@ -1183,8 +1041,8 @@ void launch_broadphase(b3g_ctx* c, cudaStream_t s)
 	prof_mark(c, PM_TRAVERSED, s);
 }
 
-// LBVH traversal (count, offsets, emit) of the tree built by this pass; the
-// count kernel runs with the tuned block size. Re-running it on the same tree
+// LBVH traversal of the tree built by this pass, with the tuned block size;
+// CTR_RAW and CTR_TRAV_OVERFLOW start at 0. Re-running it on the same tree
 // writes the same pairs.
 void launch_traverse(b3g_ctx* c, cudaStream_t s)
 {
@@ -1194,13 +1052,10 @@ void launch_traverse(b3g_ctx* c, cudaStream_t s)
 	if (n == 0)
 		return;
 	const int tb = (int)c->tune.v[B3G_TUNE_TRAVERSE];
-	cudaMemsetAsync(B.counters + CTR_TRAV_OVERFLOW, 0, sizeof(uint32_t), s);
-	cudaMemsetAsync(B.counters + CTR_RAW, 0, sizeof(uint32_t), s);
 	if (c->nWorlds > 1)
 		k_traverse_count<true><<<(n + tb - 1) / tb, tb, 0, s>>>(c->scene, B, n, cur, c->cfg.max_contacts,
 			c->walkLimit);
 	else
 		k_traverse_count<false><<<(n + tb - 1) / tb, tb, 0, s>>>(c->scene, B, n, cur, c->cfg.max_contacts,
 			c->walkLimit);
-	k_traverse_overflow<<<persistent_blocks(2), 256, 0, s>>>(B, c->cfg.max_contacts);
 }

@@ -967,8 +967,6 @@ __device__ __forceinline__ HullRef mesh_tri_ref(const MeshTri& t)
 	return r;
 }
 
-void scan_exclusive_device(uint32_t* data, const uint32_t* nPtr, uint32_t cap, uint32_t* aux, uint32_t* total,
-	uint32_t* err, cudaStream_t s);
 void launch_apart(const NPArgs& a, const uint32_t* list, const uint32_t* count, cudaStream_t s);
 void launch_mesh_items_convex(const NPArgs& a, const Buffers& B, cudaStream_t s);
 void launch_mesh_items_hull(const NPArgs& a, const Buffers& B, uint32_t maxUE, const Tune& tune, cudaStream_t s);
@@ -983,6 +981,12 @@ void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const u
 // contacts in this context's pass: the triangle buckets need triangle
 // fixtures, the sensor bucket sensors, the inactive bucket a sleeping body.
 bool convex_bucket_possible(const b3g_ctx* c, int k);
+// Before a bucket kernel runs once more in a pass.
+inline void reset_post_counts(const Buffers& B, cudaStream_t s)
+{
+	static_assert(CTR_HC_DEEP == CTR_HC_POST + 1 && CTR_HS_POST == CTR_HC_POST + 2, "one memset");
+	cudaMemsetAsync(B.counters + CTR_HC_POST, 0, 3 * sizeof(uint32_t), s);
+}
 void launch_hulls(const NPArgs& base, const uint32_t* list, const uint32_t* count, uint32_t maxUE, const Tune& tune,
 	cudaStream_t s);
 void launch_hulls_probe(const NPArgs& base, const uint32_t* list, const uint32_t* count, const Tune& tune,

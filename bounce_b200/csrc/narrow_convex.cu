@@ -1066,7 +1066,8 @@ __global__ void __launch_bounds__(128) k_mesh_items_convex(NPArgs a, Buffers B)
 
 } // namespace
 
-// Bucket kernel k of launch_convex_buckets (the order of B3G_TUNE_CONVEX).
+// Bucket kernel k of launch_convex_buckets (the order of B3G_TUNE_CONVEX). The
+// counts of the contacts handed on (hsPostCount, hcPostCount) start at 0.
 void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap,
 	const Tune& tune, cudaStream_t s)
 {
@@ -1076,7 +1077,7 @@ void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const u
 	NPArgs a = base;
 	a.list = lists + (size_t)bk * cap;
 	a.listCount = counts + bk;
-	const int blocks = persistent_blocks((int)tune.v[B3G_TUNE_CONVEX + k]);
+	const int blocks = work_blocks(cap, 128, (int)tune.v[B3G_TUNE_CONVEX + k]);
 	switch (k)
 	{
 	case 0:
@@ -1095,14 +1096,12 @@ void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const u
 		k_convex<BK_TRIANGLE_CAPSULE><<<blocks, 128, 0, s>>>(a);
 		break;
 	case 5:
-		cudaMemsetAsync(a.hsPostCount, 0, sizeof(uint32_t), s);
 		k_convex<BK_HULL_SPHERE><<<blocks, 128, 0, s>>>(a);
-		k_hull_sphere_gjk<<<persistent_blocks(4), 128, 0, s>>>(a);
+		k_hull_sphere_gjk<<<work_blocks(cap, 128, 4), 128, 0, s>>>(a);
 		break;
 	case 6:
-		cudaMemsetAsync(a.hcPostCount, 0, 2 * sizeof(uint32_t), s);
 		k_convex<BK_HULL_CAPSULE><<<blocks, 128, 0, s>>>(a);
-		k_hull_capsule_post<HC_POST_LANES><<<persistent_blocks(HC_POST_BLOCKS), 128, 0, s>>>(a);
+		k_hull_capsule_post<HC_POST_LANES><<<work_blocks(cap, 128 / HC_POST_LANES, HC_POST_BLOCKS), 128, 0, s>>>(a);
 		break;
 	case 7:
 		k_sensor<<<blocks, 128, 0, s>>>(a);
@@ -1125,7 +1124,7 @@ void launch_apart(const NPArgs& base, const uint32_t* list, const uint32_t* coun
 	NPArgs a = base;
 	a.list = list;
 	a.listCount = count;
-	k_apart<<<persistent_blocks(4), 128, 0, s>>>(a);
+	k_apart<<<work_blocks(a.hcPostCap, 128, 4), 128, 0, s>>>(a);
 }
 
 void launch_mesh_items_convex(const NPArgs& a, const Buffers& B, cudaStream_t s)

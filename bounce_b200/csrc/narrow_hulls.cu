@@ -1389,7 +1389,8 @@ void launch_sat_kernel(const NPArgs& a, uint32_t maxUE, int blocksPerSM, size_t 
 		cudaFuncSetAttribute(k_hulls_sat<W, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 		configured = smem;
 	}
-	k_hulls_sat<W, STAGE><<<persistent_blocks(blocksPerSM), W * 32, smem, s>>>(a, maxUE);
+	// Up to 4 warps share a pair.
+	k_hulls_sat<W, STAGE><<<work_blocks(4ull * a.hcPostCap, W, blocksPerSM), W * 32, smem, s>>>(a, maxUE);
 }
 
 // The staged kernel when its shared memory fits a block, else the kernel
@@ -1447,7 +1448,7 @@ void launch_hulls_probe(const NPArgs& base, const uint32_t* list, const uint32_t
 	NPArgs a = base;
 	a.list = list;
 	a.listCount = count;
-	k_hulls_probe<<<persistent_blocks((int)tune.v[B3G_TUNE_PROBE]), 128, 0, s>>>(a);
+	k_hulls_probe<<<work_blocks(a.hcPostCap, 128, (int)tune.v[B3G_TUNE_PROBE]), 128, 0, s>>>(a);
 }
 
 // Dynamic shared memory of the SAT kernel with `warps` warps per block.

@@ -28,6 +28,7 @@
 // point is the walk's result.
 
 #include "collide_common.cuh"
+#include "scan.cuh"
 
 namespace {
 
@@ -50,11 +51,10 @@ __device__ __forceinline__ uint32_t hash_mask_for(const Buffers& B, uint32_t con
 	return min(slots, B.hashCap) - 1u;
 }
 
-// Clears the slots the table of this pass will use (total contacts, or the
-// pass's new plus kept contacts when total is ~0u) and records its size.
-__global__ void k_hash_clear(Buffers B, uint32_t cur, uint32_t cap, uint32_t total)
+// Clears the slots that the table of this pass will use for n contacts and
+// records its size.
+__device__ __forceinline__ void clear_table(Buffers& B, uint32_t cur, uint32_t n)
 {
-	const uint32_t n = total == ~0u ? min(B.counters[CTR_BEGUN] + B.counters[CTR_KEPT], cap) : total;
 	const uint32_t mask = hash_mask_for(B, n);
 	if (blockIdx.x == 0 && threadIdx.x == 0)
 		B.hashMask[cur] = mask;
@@ -62,9 +62,16 @@ __global__ void k_hash_clear(Buffers B, uint32_t cur, uint32_t cap, uint32_t tot
 		B.hashKeys[cur][i] = B3G_EMPTY_KEY;
 }
 
-// New contacts grouped by the smaller key rank, reversed (descending order).
-__global__ void k_new_scatter(DevScene S, Buffers B, uint32_t nf)
+__global__ void k_hash_clear(Buffers B, uint32_t cur, uint32_t total)
 {
+	clear_table(B, cur, total);
+}
+
+// The pass's table cleared, and the new contacts grouped by the smaller key
+// rank, reversed (descending order).
+__global__ void k_new_scatter(DevScene S, Buffers B, uint32_t cur, uint32_t cap, uint32_t nf)
+{
+	clear_table(B, cur, min(B.counters[CTR_BEGUN] + B.counters[CTR_KEPT], cap));
 	uint32_t n = B.counters[CTR_BEGUN];
 	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
 	{
@@ -79,10 +86,9 @@ __global__ void k_new_scatter(DevScene S, Buffers B, uint32_t nf)
 
 // Final place of each new contact: its group's offset plus the number of
 // group members with a larger key (the ranks in a group are distinct).
-__global__ void k_new_place(DevScene S, Buffers B, uint32_t cur, uint32_t nf, int havePrev)
+__device__ __forceinline__ void place_new(const DevScene& S, Buffers& B, uint32_t cur, uint32_t nf, uint32_t mask)
 {
 	uint32_t n = B.counters[CTR_BEGUN];
-	const uint32_t mask = B.hashMask[cur];
 	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
 	{
 		uint32_t c = B.newTmp[t];
@@ -100,8 +106,6 @@ __global__ void k_new_place(DevScene S, Buffers B, uint32_t cur, uint32_t nf, in
 		B.posKey[pos] = pos;
 		insert_contact(B, cur, mask, a, b, pos);
 	}
-	if (!havePrev && blockIdx.x == 0 && threadIdx.x == 0)
-		B.counters[CTR_PAIRS] = n;
 }
 
 __device__ __forceinline__ bool body_active(const DevScene& S, uint32_t b)
@@ -115,33 +119,90 @@ __device__ __forceinline__ bool body_active(const DevScene& S, uint32_t b)
 // that the caller's filter rejects is destroyed whatever its bodies' state:
 // UpdateContacts tests both before the inactive skip
 // (contact_manager.cpp:176-199).
-__global__ void k_kept(DevScene S, Buffers B, FilterArgs F, uint32_t cur, uint32_t cap)
+//
+// A warp's lanes take neighbouring contacts (their words and flags load in
+// whole lines) and leave 32 flags as one word; thread t then takes its own
+// SC_ITEMS = 8 entries as byte t of the tile's words. With each thread loading
+// its 8 entries itself the scan of 1.2 million contacts took 85 us.
+struct KeptFlags
 {
-	uint32_t prevBuf = cur ^ 1u;
-	uint32_t n = min(B.counters[CTR_PREV_PAIRS], cap);
-	for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
+	// References: a copy of these structures would be indexed in local memory.
+	const DevScene& S;
+	const FilterArgs& F;
+	const uint32_t *pairA, *pairB, *prevFound;
+	uint32_t n;
+	uint32_t* sBits; // SC_TILE / 32 words of shared memory
+
+	__device__ __forceinline__ void operator()(uint32_t first, uint32_t* v) const
 	{
-		uint32_t kept = 1;
-		uint32_t fa = B.pairA[prevBuf][p], fb = B.pairB[prevBuf][p];
-		if (S.fixLife[fa] != FIX_LIVE || S.fixLife[fb] != FIX_LIVE)
-			kept = 0; // a fixture was replaced or removed by a scene update
-		else if (F.mode != 0 && ((F.vetoPrev && p < F.nVeto && F.vetoPrev[p]) ||
-									joint_excluded(F, S.fixBody[fa], S.fixBody[fb])))
-			kept = 0;
-		else if (!B.prevFound[p])
+		static_assert(SC_ITEMS == 8, "a byte per thread");
+		const uint32_t t = threadIdx.x;
+		const uint32_t tile = first - t * SC_ITEMS;
+		uint32_t fa[SC_ITEMS], fb[SC_ITEMS], found[SC_ITEMS], live[SC_ITEMS];
+		// The loads of all entries before any is used.
+#pragma unroll
+		for (int r = 0; r < SC_ITEMS; ++r)
 		{
-			uint32_t ba = S.fixBody[fa], bb = S.fixBody[fb];
-			kept = (body_active(S, ba) || body_active(S, bb)) ? 0u : 1u;
+			const uint32_t p = tile + r * SC_THREADS + t;
+			const bool in = p < n;
+			fa[r] = in ? pairA[p] : 0u;
+			fb[r] = in ? pairB[p] : 0u;
+			found[r] = in ? prevFound[p] : 1u;
 		}
-		B.keptScan[p] = kept;
+#pragma unroll
+		for (int r = 0; r < SC_ITEMS; ++r)
+			live[r] = S.fixLife[fa[r]] == FIX_LIVE && S.fixLife[fb[r]] == FIX_LIVE ? 1u : 0u;
+#pragma unroll
+		for (int r = 0; r < SC_ITEMS; ++r)
+		{
+			const uint32_t p = tile + r * SC_THREADS + t;
+			// A fixture that is not live was replaced or removed by a scene update.
+			bool kept = p < n && live[r];
+			if (kept && F.mode != 0 && ((F.vetoPrev && p < F.nVeto && F.vetoPrev[p]) ||
+										   joint_excluded(F, S.fixBody[fa[r]], S.fixBody[fb[r]])))
+				kept = false;
+			if (kept && !found[r])
+				kept = !body_active(S, S.fixBody[fa[r]]) && !body_active(S, S.fixBody[fb[r]]);
+			const uint32_t bits = __ballot_sync(0xffffffffu, kept);
+			if ((t & 31u) == 0)
+				sBits[(r * SC_THREADS + t) / 32u] = bits;
+		}
+		__syncthreads();
+		const uint32_t byte = sBits[t / 4u] >> (8u * (t & 3u));
+#pragma unroll
+		for (int r = 0; r < SC_ITEMS; ++r)
+			v[r] = byte >> r & 1u;
 	}
+};
+
+// Both offset scans of the contact list: the first newTiles blocks take the
+// new contacts' groups, the others the previous contacts' kept flags.
+__global__ void __launch_bounds__(SC_THREADS) k_order_scan(DevScene S, Buffers B, FilterArgs F, uint32_t cur,
+	uint32_t cap, uint32_t nf, uint32_t newTiles)
+{
+	uint32_t* err = B.counters + CTR_STATUS;
+	if (blockIdx.x < newTiles)
+	{
+		const uint32_t* data = B.newOff;
+		scan_tile(
+			[=](uint32_t first, uint32_t* v) {
+#pragma unroll
+				for (int r = 0; r < SC_ITEMS; ++r)
+					v[r] = first + r <= nf ? data[first + r] : 0u;
+			},
+			B.newOff, nf + 1, B.passScan, nullptr, err);
+		return;
+	}
+	const uint32_t n = min(B.counters[CTR_PREV_PAIRS], cap);
+	__shared__ uint32_t sBits[SC_TILE / 32];
+	const KeptFlags flags{S, F, B.pairA[cur ^ 1u], B.pairB[cur ^ 1u], B.prevFound, n, sBits};
+	scan_tile(flags, B.keptScan, n, B.passScan + newTiles + 1, B.counters + CTR_KEPT, err);
 }
 
 // Kept previous contacts follow the new ones in their previous order; the
 // others are destroyed, listed in list order.
-__global__ void k_layout_prev(Buffers B, uint32_t cur, uint32_t cap)
+__device__ __forceinline__ void place_kept(Buffers& B, uint32_t cur, uint32_t cap, uint32_t mask)
 {
-	const uint32_t mask = B.hashMask[cur];
 	uint32_t prevBuf = cur ^ 1u;
 	uint32_t n = min(B.counters[CTR_PREV_PAIRS], cap);
 	uint32_t numNew = B.counters[CTR_BEGUN];
@@ -179,6 +240,16 @@ __global__ void k_layout_prev(Buffers B, uint32_t cur, uint32_t cap)
 		B.counters[CTR_PAIRS] = min(total, cap);
 		B.counters[CTR_ENDED] = n - keptTotal;
 	}
+}
+
+__global__ void k_place(DevScene S, Buffers B, uint32_t cur, uint32_t cap, uint32_t nf, int havePrev)
+{
+	const uint32_t mask = B.hashMask[cur];
+	place_new(S, B, cur, nf, mask);
+	if (havePrev)
+		place_kept(B, cur, cap, mask);
+	else if (blockIdx.x == 0 && threadIdx.x == 0)
+		B.counters[CTR_PAIRS] = B.counters[CTR_BEGUN];
 }
 
 // ---------------------------------------------------------------------------
@@ -409,27 +480,18 @@ void launch_order(b3g_ctx* c, cudaStream_t s)
 	Buffers& B = c->buf;
 	const uint32_t cap = c->cfg.max_contacts, cur = c->cur, nf = c->nFixtures;
 	const int havePrev = c->havePass ? 1 : 0;
-	scan_exclusive(B.newOff, nf + 1, B.scanAux, B.counters + CTR_SCRATCH, B.counters + CTR_STATUS, s);
-	if (havePrev)
-	{
-		k_kept<<<persistent_blocks(8), 256, 0, s>>>(c->scene, B, make_filter_args(c), cur, cap);
-		scan_exclusive_device(B.keptScan, B.counters + CTR_PREV_PAIRS, cap, B.scanAux, B.counters + CTR_KEPT,
-			B.counters + CTR_STATUS, s);
-	}
+	const uint32_t newTiles = scan_tiles(nf + 1), prevTiles = havePrev ? std::max(scan_tiles(cap), 1u) : 0u;
+	k_order_scan<<<newTiles + prevTiles, SC_THREADS, 0, s>>>(c->scene, B, make_filter_args(c), cur, cap, nf, newTiles);
 	// New and kept counts known: the pass's table, filled as the contacts
 	// take their places.
-	k_hash_clear<<<persistent_blocks(8), 256, 0, s>>>(B, cur, cap, ~0u);
-	k_new_scatter<<<persistent_blocks(4), 256, 0, s>>>(c->scene, B, nf);
-	k_new_place<<<persistent_blocks(4), 256, 0, s>>>(c->scene, B, cur, nf, havePrev);
-	if (havePrev)
-		k_layout_prev<<<persistent_blocks(8), 256, 0, s>>>(B, cur, cap);
+	k_new_scatter<<<work_blocks(2 * (uint64_t)cap, 256, 8), 256, 0, s>>>(c->scene, B, cur, cap, nf);
+	k_place<<<work_blocks(cap, 256, 8), 256, 0, s>>>(c->scene, B, cur, cap, nf, havePrev);
 }
 
-uint32_t order_launches(const b3g_ctx* c)
+uint32_t order_launches(const b3g_ctx*)
 {
-	// scan, scatter, place; kept, scan, layout of the previous contacts;
-	// the table's clear
-	return 3 + (c->havePass ? 3 : 0) + 1;
+	// scans, scatter (with the table's clear), place
+	return 3;
 }
 
 // Host-driven replay of the wake-ups; runs only when some non-static body is
@@ -466,6 +528,7 @@ int resolve_wakeups(b3g_ctx* c, cudaStream_t s)
 			cudaMemsetAsync(B.counters + CTR_BUCKET0, 0, sizeof(uint32_t) * BK_COUNT, s);
 			cudaMemsetAsync(B.counters + CTR_WAKE_ACTIVATED, 0, sizeof(uint32_t), s);
 			cudaMemsetAsync(B.counters + CTR_HULL_MISS, 0, sizeof(uint32_t), s);
+			reset_post_counts(B, s);
 			k_wake_activate<<<persistent_blocks(4), 256, 0, s>>>(c->scene, B, cur, cap, nInactive);
 			++launches;
 			if (!fetch())
@@ -525,7 +588,7 @@ int resolve_wakeups(b3g_ctx* c, cudaStream_t s)
 		}
 		k_compact_move<<<persistent_blocks(4), 256, 0, s>>>(B, cur, cap, np, numNew, copied, kept2, kept2Total);
 		const uint32_t total = std::min(numNew + kept2Total, cap);
-		k_hash_clear<<<persistent_blocks(8), 256, 0, s>>>(B, cur, cap, total);
+		k_hash_clear<<<persistent_blocks(8), 256, 0, s>>>(B, cur, total);
 		k_rehash<<<persistent_blocks(8), 256, 0, s>>>(B, cur, total);
 		k_set_counts<<<1, 1, 0, s>>>(B, total, np - kept2Total);
 		launches += 1 + 3 + 1 + 1 + 1 + 1;

@@ -41,8 +41,24 @@ __device__ __forceinline__ bool filter_drop(const DevScene& S, const Buffers& B,
 	return B.moved[a] == 0 && B.moved[b] == 0;
 }
 
-__global__ void k_diff(DevScene S, Buffers B, FilterArgs F, uint32_t cur, uint32_t cap, uint32_t nf, int havePrev)
+// The pair list is complete (more pairs than contacts fit is an overflow); the
+// pass has no contacts until they are laid out (order.cu).
+__device__ __forceinline__ void begin_contacts(Buffers& B, uint32_t cap)
 {
+	if (blockIdx.x == 0 && threadIdx.x == 0)
+	{
+		if (B.counters[CTR_RAW] > cap)
+			atomicOr(&B.counters[CTR_STATUS], B3G_ST_PAIR_OVERFLOW);
+		B.counters[CTR_PAIRS] = 0;
+	}
+}
+
+constexpr int DIFF_THREADS = 256;
+
+__global__ void __launch_bounds__(DIFF_THREADS) k_diff(DevScene S, Buffers B, FilterArgs F, uint32_t cur, uint32_t cap,
+	uint32_t nf, int havePrev)
+{
+	begin_contacts(B, cap);
 	uint32_t n = min(B.counters[CTR_RAW], cap);
 	uint32_t prevBuf = cur ^ 1u;
 	const uint32_t lane = threadIdx.x & 31;
@@ -61,7 +77,7 @@ __global__ void k_diff(DevScene S, Buffers B, FilterArgs F, uint32_t cur, uint32
 				drop = filter_drop(S, B, F, a, b, prev);
 			if (drop)
 			{
-				// No contact: a previous one is destroyed (k_kept), none is created.
+				// No contact: a previous one is destroyed (k_order_scan), none is created.
 			}
 			else if (prev >= 0)
 				B.prevFound[prev] = 1;
@@ -80,6 +96,24 @@ __global__ void k_diff(DevScene S, Buffers B, FilterArgs F, uint32_t cur, uint32
 		if (isNew)
 			B.newList[slot + __popc(ballot & ((1u << lane) - 1u))] = c;
 	}
+	// The proxies the broadphase re-inserted, one atomic per block.
+	__shared__ uint32_t sMoved[DIFF_THREADS / 32];
+	uint32_t m = 0;
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x)
+		m += B.moved[i];
+	for (int o = 16; o > 0; o >>= 1)
+		m += __shfl_xor_sync(0xffffffffu, m, o);
+	if (lane == 0)
+		sMoved[threadIdx.x >> 5] = m;
+	__syncthreads();
+	if (threadIdx.x == 0)
+	{
+		m = 0;
+		for (uint32_t w = 0; w < DIFF_THREADS / 32; ++w)
+			m += sMoved[w];
+		if (m)
+			atomicAdd(&B.counters[CTR_MOVED], m);
+	}
 }
 
 // Contact filter (mode 2), before the contact list: the drop flag of every
@@ -88,6 +122,7 @@ __global__ void k_diff(DevScene S, Buffers B, FilterArgs F, uint32_t cur, uint32
 __global__ void k_candidates(DevScene S, Buffers B, FilterArgs F, uint32_t* cand, uint32_t cur, uint32_t cap,
 	int havePrev)
 {
+	begin_contacts(B, cap);
 	uint32_t n = min(B.counters[CTR_RAW], cap);
 	uint32_t prevBuf = cur ^ 1u;
 	for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
@@ -303,38 +338,6 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(DevScene S, Buffers B,
 	}
 }
 
-// The pair-overflow status; with clearFound, also clears the previous
-// contacts' found flags (k_diff sets them), only as many as the previous pass
-// had.
-__global__ void k_overflow_check(Buffers B, uint32_t cap, int clearFound, uint32_t nf)
-{
-	if (blockIdx.x == 0 && threadIdx.x == 0 && B.counters[CTR_RAW] > cap)
-		atomicOr(&B.counters[CTR_STATUS], B3G_ST_PAIR_OVERFLOW);
-	if (!clearFound)
-		return;
-	const uint32_t n = min(B.counters[CTR_PREV_PAIRS], cap);
-	for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
-		B.prevFound[p] = 0;
-	// The proxies the broadphase re-inserted, one atomic per block.
-	__shared__ uint32_t sMoved[32];
-	uint32_t m = 0;
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x)
-		m += B.moved[i];
-	for (int o = 16; o > 0; o >>= 1)
-		m += __shfl_xor_sync(0xffffffffu, m, o);
-	if ((threadIdx.x & 31) == 0)
-		sMoved[threadIdx.x >> 5] = m;
-	__syncthreads();
-	if (threadIdx.x == 0)
-	{
-		m = 0;
-		for (uint32_t w = 0; w < blockDim.x / 32; ++w)
-			m += sMoved[w];
-		if (m)
-			atomicAdd(&B.counters[CTR_MOVED], m);
-	}
-}
-
 } // namespace
 
 FilterArgs make_filter_args(const b3g_ctx* c)
@@ -354,8 +357,7 @@ void launch_candidates(b3g_ctx* c, cudaStream_t s)
 {
 	Buffers& B = c->buf;
 	uint32_t cap = c->cfg.max_contacts;
-	k_overflow_check<<<1, 1, 0, s>>>(B, cap, 0, 0);
-	k_candidates<<<persistent_blocks(8), 256, 0, s>>>(c->scene, B, make_filter_args(c), c->dCand, c->cur, cap,
+	k_candidates<<<work_blocks(cap, 256, 8), 256, 0, s>>>(c->scene, B, make_filter_args(c), c->dCand, c->cur, cap,
 		c->havePass ? 1 : 0);
 }
 
@@ -377,18 +379,14 @@ void launch_pairs_diff(b3g_ctx* c, cudaStream_t s)
 	uint32_t cap = c->cfg.max_contacts;
 	uint32_t cur = c->cur;
 	uint32_t nf = c->nFixtures;
-	cudaMemsetAsync(B.newOff, 0, sizeof(uint32_t) * (nf + 1), s);
-	cudaMemsetAsync(B.newFill, 0, sizeof(uint32_t) * (nf + 1), s);
-	k_overflow_check<<<persistent_blocks(2), 256, 0, s>>>(B, cap, 1, nf);
-	k_diff<<<persistent_blocks(8), 256, 0, s>>>(c->scene, B, make_filter_args(c), cur, cap, nf,
+	k_diff<<<work_blocks(std::max(cap, nf), DIFF_THREADS, 8), DIFF_THREADS, 0, s>>>(c->scene, B, make_filter_args(c), cur, cap, nf,
 		c->havePass ? 1 : 0);
 	launch_order(c, s);
 }
 
 uint32_t pairs_diff_launches(const b3g_ctx* c)
 {
-	// overflow check (with the found flags and the moved count), diff, order
-	return 2 + order_launches(c);
+	return 1 + order_launches(c);
 }
 
 NPArgs make_np_args(b3g_ctx* c)
@@ -427,11 +425,13 @@ NPArgs make_np_args(b3g_ctx* c)
 	return a;
 }
 
+constexpr int CONVEX_HULL_CAPSULE = 6; // launch_convex_one
+
 void launch_narrowphase(b3g_ctx* c, cudaStream_t s)
 {
 	Buffers& B = c->buf;
 	uint32_t cap = c->cfg.max_contacts;
-	k_bucket<<<persistent_blocks(8), BUCKET_THREADS, 0, s>>>(c->scene, B, c->cur, cap);
+	k_bucket<<<work_blocks(cap, BUCKET_THREADS, 8), BUCKET_THREADS, 0, s>>>(c->scene, B, c->cur, cap);
 	prof_mark(c, PM_BUCKETED, s);
 	// The mesh contacts (midphase, work items, clustering) on a stream of their
 	// own beside the convex and hull kernels.
@@ -463,22 +463,33 @@ void launch_narrowphase(b3g_ctx* c, cudaStream_t s)
 		launch_hull_triangles(a, B.bucketList + (size_t)BK_HULL_TRIANGLE * cap,
 			B.counters + CTR_BUCKET0 + BK_HULL_TRIANGLE, c->maxUniqueEdges, c->tune, side);
 	prof_mark(c, PM_HULLS, s);
-	launch_apart(a, B.bucketList + (size_t)BK_APART * cap, B.counters + CTR_BUCKET0 + BK_APART, s);
 	// The convex kernels (hull-sphere and hull-capsule each a scan kernel and
 	// a follow-up kernel on the contacts the scan hands on) run beside the
-	// hull-hull probe and SAT: the two branches take about as long.
+	// hull-hull probe and SAT. The hull-capsule pair, the longest of them, gets
+	// the stream that the mesh work leaves free: each kernel ends in a tail
+	// of slow warps that the others fill (a pass of 454, 16,000 and 65,536 mixed
+	// bodies: 212, 338 and 647 us without the third branch, 176, 301 and 626
+	// with it).
+	const bool third = side != s && !meshSide;
+	if (third)
+	{
+		cudaStreamWaitEvent(c->meshStream, c->forkEvent, 0);
+		launch_convex_one(CONVEX_HULL_CAPSULE, a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, c->meshStream);
+		cudaEventRecord(c->meshJoin, c->meshStream);
+	}
 	for (int k = 0; k < B3G_CONVEX_KERNELS; ++k)
-		if (convex_bucket_possible(c, k))
+		if (convex_bucket_possible(c, k) && !(third && k == CONVEX_HULL_CAPSULE))
 			launch_convex_one(k, a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
+	launch_apart(a, B.bucketList + (size_t)BK_APART * cap, B.counters + CTR_BUCKET0 + BK_APART, s);
 	prof_mark(c, PM_CONVEX, s);
 	if (side != s)
 	{
 		cudaEventRecord(c->joinEvent, side);
 		cudaStreamWaitEvent(s, c->joinEvent, 0);
 	}
-	if (meshSide)
+	if (meshSide || third)
 		cudaStreamWaitEvent(s, c->meshJoin, 0);
-	else
+	if (!meshSide)
 	{
 		launch_mesh_prepare(c, s);
 		launch_mesh_collide(c, meshList, meshCount, s);
@@ -504,6 +515,6 @@ bool convex_bucket_possible(const b3g_ctx* c, int k)
 
 void launch_finalize(b3g_ctx* c, cudaStream_t s)
 {
-	k_finalize<<<persistent_blocks(4), FIN_THREADS, 0, s>>>(c->scene, c->buf, c->cur, c->cfg.max_contacts,
+	k_finalize<<<work_blocks(std::max(c->cfg.max_contacts, c->nFixtures), FIN_THREADS, 4), FIN_THREADS, 0, s>>>(c->scene, c->buf, c->cur, c->cfg.max_contacts,
 		c->nFixtures);
 }
