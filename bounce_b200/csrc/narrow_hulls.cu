@@ -358,8 +358,9 @@ __device__ void build_edge_contact(DevManifold& m, const XF& xf1, uint32_t index
 	m.points[0].edgeContact = 1;
 }
 
-// b3BuildFaceContact (collide_hulls.cpp:75-187). Runs on one lane.
-__device__ void build_face_contact(DevManifold& m, const XF& xf1, uint32_t index1, const HullRef& h1, float r1,
+// b3BuildFaceContact (collide_hulls.cpp:75-187) on one thread, for the
+// polygons that do not fit the rings of rebuild_faces.
+__device__ __noinline__ void build_face_contact(DevManifold& m, const XF& xf1, uint32_t index1, const HullRef& h1, float r1,
 	const XF& xf2, const HullRef& h2, float r2, bool flipNormal, uint32_t* status)
 {
 	float totalRadius = r1 + r2;
@@ -709,10 +710,8 @@ __device__ void rebuild_edge_contact(DevManifold& m, const XF& xf1, uint32_t ind
 	}
 }
 
-// b3RebuildFaceContact (collide_hulls.cpp:323-353).
-__device__ void rebuild_face_contact(DevManifold& m, const XF& xf1, uint32_t index1, const HullRef& h1, float r1,
-	const XF& xf2, const HullRef& h2, float r2, bool flipNormal, const XF& xf01, const XF& xf02,
-	uint32_t* status)
+// The orientation test of b3RebuildFaceContact (collide_hulls.cpp:323-353).
+__device__ __forceinline__ bool face_contact_persists(const XF& xf1, const XF& xf2, const XF& xf01, const XF& xf02)
 {
 	Q4 q01 = xf01.q, q1 = xf1.q;
 	Q4 q02 = xf02.q, q2 = xf2.q;
@@ -720,8 +719,7 @@ __device__ void rebuild_face_contact(DevManifold& m, const XF& xf1, uint32_t ind
 	Q4 dq = qmul(conj(q1), q2);
 	Q4 q = qmul(conj(dq0), dq);
 	const float kCosTol = 0.995f;
-	if (fabsr(q.s) > kCosTol)
-		build_face_contact(m, xf1, index1, h1, r1, xf2, h2, r2, flipNormal, status);
+	return fabsr(q.s) > kCosTol;
 }
 
 enum
@@ -831,55 +829,6 @@ __device__ uint32_t read_face_thread(const XF& xf1, const HullRef& h1, const XF&
 	return s > totalRadius ? CT_SEPARATION : CT_OVERLAP;
 }
 
-// The cache half of b3CollideHullsCache (collide_hulls.cpp:367-415), one
-// thread per contact: b3FeatureCache::ReadState (sat.cpp:178-207), then the
-// separation hit, or the overlap hit that rebuilds the cached edge or face
-// contact. Returns true when the contact is finished; otherwise the cache is
-// flushed (cacheType = empty, the feature fields as ReadState left them) and
-// the contact needs the SAT. The face rebuild clips on this thread: the
-// polygons are small (3 or 4 vertices on these hulls), and a warp per rebuild
-// measured slower than the threads that do it here.
-__device__ bool probe_cache(DevManifold& m, const HullCtx& H, uint4& cache)
-{
-	float totalRadius = H.r1 + H.r2;
-	uint32_t state0 = cache.x;
-	if (cache.x == CT_EMPTY)
-	{
-		cache.x = CT_SEPARATION;
-		cache.y = FT_FACE1;
-		cache.z = 0;
-		cache.w = 0;
-	}
-	// A face of either hull is read by one call with the hulls in the face's
-	// order, so the lanes of a warp with face caches of hull 1 and of hull 2
-	// run it together rather than one group after the other.
-	const bool face = cache.y == FT_FACE1 || cache.y == FT_FACE2;
-	const bool f2 = cache.y == FT_FACE2;
-	const XF xa = f2 ? H.xf2 : H.xf1, xb = f2 ? H.xf1 : H.xf2;
-	const HullRef ha = f2 ? H.h2 : H.h1, hb = f2 ? H.h1 : H.h2;
-	uint32_t state1;
-	if (cache.y == FT_EDGES)
-		state1 = read_edges(H.xf1, H.h1, H.xf2, H.h2, cache.z, cache.w, totalRadius);
-	else if (face)
-		state1 = read_face_thread(xa, ha, xb, hb, cache.z, totalRadius);
-	else
-		state1 = CT_EMPTY;
-	if (state0 == CT_SEPARATION && state1 == CT_SEPARATION)
-		return true; // separation cache hit
-	if (state0 == CT_OVERLAP && state1 == CT_OVERLAP)
-	{
-		if (cache.y == FT_EDGES)
-			rebuild_edge_contact(m, H.xf1, cache.z, H.h1, H.xf2, cache.w, H.h2);
-		else if (face)
-			rebuild_face_contact(m, xa, cache.z, ha, f2 ? H.r2 : H.r1, xb, hb, f2 ? H.r1 : H.r2, f2,
-				f2 ? H.xf02 : H.xf01, f2 ? H.xf01 : H.xf02, H.status);
-		if (m.pointCount > 0)
-			return true; // overlap cache hit
-	}
-	cache.x = CT_EMPTY;
-	return false;
-}
-
 // Warp-aggregated append of c to a list (the calling lanes of the warp).
 __device__ __forceinline__ void warp_append(uint32_t* list, uint32_t* count, uint32_t c)
 {
@@ -985,29 +934,446 @@ __device__ __forceinline__ void load_hull_ctx(const NPArgs& a, uint32_t c, HullC
 	H.parts = EdgeParts{0, 1, 0, nullptr};
 }
 
-// Pass 1: one thread per hull-hull contact reads its feature cache.
-__global__ void __launch_bounds__(128) k_hulls_probe(NPArgs a)
+constexpr int PROBE_THREADS = 128;
+constexpr int PROBE_BLOCKS = 4;
+constexpr uint32_t CLIP_SLOTS = 16; // a power of two
+
+// A thread's clip polygon: a ring of vertices in shared memory, one column of
+// words per thread. A vertex's edge pair takes two words of two 16-bit edges
+// (0xFFFF: none).
+struct ClipRings
 {
-	uint32_t n = *a.listCount;
-	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+	float x[CLIP_SLOTS][PROBE_THREADS], y[CLIP_SLOTS][PROBE_THREADS], z[CLIP_SLOTS][PROBE_THREADS];
+	uint32_t pair1[CLIP_SLOTS][PROBE_THREADS], pair2[CLIP_SLOTS][PROBE_THREADS];
+
+	__device__ __forceinline__ V3 pos(uint32_t i) const
 	{
-		uint32_t c = a.list[t];
-		int32_t prev = a.prevIndex[c];
-		uint4 cache = prev >= 0 ? a.prevCache[prev] : make_uint4(CT_EMPTY, FT_FACE1, 0, 0);
-		DevManifold& m = a.man[c];
-		man_clear(m);
-		bool done = false;
-		if (a.convexCache)
+		const uint32_t s = i % CLIP_SLOTS, t = threadIdx.x;
+		return V3{x[s][t], y[s][t], z[s][t]};
+	}
+	__device__ __forceinline__ void put(uint32_t i, V3 p, uint32_t p1, uint32_t p2)
+	{
+		const uint32_t s = i % CLIP_SLOTS, t = threadIdx.x;
+		x[s][t] = p.x;
+		y[s][t] = p.y;
+		z[s][t] = p.z;
+		pair1[s][t] = p1;
+		pair2[s][t] = p2;
+	}
+};
+__device__ __forceinline__ uint32_t ring_edges(uint32_t in, uint32_t out) { return in | out << 16; }
+__device__ __forceinline__ uint32_t ring_edge(uint32_t e) { return e == 0xFFFFu ? B3G_NULL_EDGE : e; }
+
+// Leaves a contact that its cache does not resolve to the SAT kernel.
+__device__ __forceinline__ void probe_miss(const NPArgs& a, uint32_t c, uint4 cache)
+{
+	a.cache[c] = cache;
+	warp_append(a.missList, a.missCount, c);
+}
+// ... flushed: the feature fields stay as ReadState left them.
+__device__ __forceinline__ void probe_flush(const NPArgs& a, uint32_t c, uint4 cache)
+{
+	cache.x = CT_EMPTY;
+	probe_miss(a, c, cache);
+}
+
+// b3BuildFaceContact (collide_hulls.cpp:75-187) of a cached face, a contact
+// per lane; live: the lane's contact is its own (the others repeat one of
+// them and write nothing). The warp takes each side plane and each vertex in
+// step, over the largest polygon of its lanes.
+__device__ void rebuild_faces(const NPArgs& a, uint32_t c, bool live, ClipRings& R)
+{
+	uint4 cache = a.prevCache[a.prevIndex[c]];
+	HullCtx H;
+	load_hull_ctx(a, c, H);
+	const bool flip = cache.y == FT_FACE2;
+	const XF xf1 = flip ? H.xf2 : H.xf1, xf2 = flip ? H.xf1 : H.xf2;
+	const HullRef h1 = flip ? H.h2 : H.h1, h2 = flip ? H.h1 : H.h2;
+	const float totalRadius = (flip ? H.r2 : H.r1) + (flip ? H.r1 : H.r2);
+	const uint32_t index1 = cache.z;
+	const PL plane1 = pmul(xf1, hp(h1, index1));
+	uint32_t head = 0, cnt = 0;
+	// A polygon that outgrows the ring, or edges that do not fit 16 bits: the
+	// thread builds the contact on its own.
+	bool big = h1.eCnt > 0xFFFFu || h2.eCnt > 0xFFFFu;
+	bool failed = false;
+	{
+		// b3BuildPolygon (clip.cpp:33-58).
+		V3 normal1 = rotc(xf2.q, plane1.n);
+		const uint32_t begin = h2.f[hull_support_face(h2, -normal1)];
+		uint32_t edge = begin;
+		do
 		{
-			HullCtx H;
-			load_hull_ctx(a, c, H);
-			done = probe_cache(m, H, cache);
+			if (cnt == CLIP_SLOTS)
+				big = true;
+			if (big)
+				break;
+			const uint4 e = h2.e[edge];
+			R.put(cnt++, xmul(xf2, hv(h2, e.x)), ~0u, ring_edges(e.z, edge));
+			edge = e.w;
+		} while (edge != begin);
+	}
+	__syncwarp();
+	// b3ClipPolygonToFaceSidePlanes (clip.cpp:244-281), b3ClipPolygonToPlane
+	// (clip.cpp:101-150): vertices leave the ring's head and the clipped
+	// polygon grows behind its tail.
+	const uint32_t begin = h1.f[index1];
+	uint32_t edge = begin, guard = 0;
+	bool run = !big;
+	while (__any_sync(0xffffffffu, run))
+	{
+		PL cp = plane1;
+		V3 p1 = plane1.n;
+		float d1 = 0.0f;
+		uint32_t out1 = 0, n = 0, outN = 0;
+		const uint32_t tail = head + cnt;
+		if (run && ++guard > h1.eCnt)
+		{
+			failed = true; // face loops are validated on upload; never loop forever
+			run = false;
 		}
-		a.cache[c] = cache;
-		if (done)
-			finish_convex(a, c, m);
-		else
-			warp_append(a.missList, a.missCount, c);
+		if (run)
+		{
+			PL plane = hull_edge_side_plane(h1, edge);
+			plane.d += totalRadius;
+			cp = pmul(xf1, plane);
+			n = cnt;
+			p1 = R.pos(tail - 1);
+			out1 = R.pair2[(tail - 1) % CLIP_SLOTS][threadIdx.x] >> 16;
+			d1 = pdist(p1, cp);
+		}
+		const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+		for (uint32_t i = 0; i < most; ++i)
+		{
+			if (i < n)
+			{
+				const uint32_t s = (head + i) % CLIP_SLOTS;
+				const V3 p2 = R.pos(s);
+				const uint32_t e1 = R.pair1[s][threadIdx.x], e2 = R.pair2[s][threadIdx.x];
+				const float d2 = pdist(p2, cp);
+				const bool leaves = d1 <= 0.0f && d2 > 0.0f, enters = d1 > 0.0f && d2 <= 0.0f;
+				const bool stays = d1 <= 0.0f && d2 <= 0.0f;
+				const uint32_t adds = (leaves || enters ? 1u : 0u) + (enters || stays ? 1u : 0u);
+				if (outN + adds + (n - i - 1) > CLIP_SLOTS)
+				{
+					big = true;
+					run = false;
+					n = 0;
+				}
+				else
+				{
+					if (leaves || enters)
+					{
+						const float fraction = d1 / (d1 - d2);
+						R.put(tail + outN++, p1 + fraction * (p2 - p1),
+							leaves ? ring_edges(edge, 0xFFFFu) : ring_edges(0xFFFFu, edge),
+							leaves ? ring_edges(out1, 0xFFFFu) : ring_edges(0xFFFFu, e2 & 0xFFFFu));
+					}
+					if (enters || stays)
+						R.put(tail + outN++, p2, e1, e2);
+				}
+				p1 = p2;
+				d1 = d2;
+				out1 = e2 >> 16;
+			}
+			__syncwarp();
+		}
+		if (run)
+		{
+			head = tail;
+			cnt = outN;
+			edge = he_next(h1, edge);
+			run = cnt > 0 && edge != begin;
+		}
+	}
+	if (big || failed)
+		cnt = 0;
+	// The vertices on or behind the reference face, moved up to the head.
+	uint32_t n1 = 0, minIndex = 0;
+	float minSep = B3G_MAX_SCALAR;
+	for (uint32_t i = 0; i < cnt; ++i)
+	{
+		const uint32_t s = (head + i) % CLIP_SLOTS;
+		const V3 p = R.pos(s);
+		const float sep = pdist(p, plane1);
+		if (sep <= totalRadius)
+		{
+			if (sep < minSep)
+			{
+				minIndex = n1;
+				minSep = sep;
+			}
+			R.put(head + n1, p, R.pair1[s][threadIdx.x], R.pair2[s][threadIdx.x]);
+			++n1;
+		}
+	}
+	__syncwarp();
+	// b3ReducePolygon (cluster.cpp:59-200) of their projections on the face:
+	// o[k] is the projection of vertex at[k].
+	auto get = [&](uint32_t k) { return pclosest(R.pos(head + k), plane1); };
+	const V3 oriented = flip ? -plane1.n : plane1.n;
+	V3 o[4];
+	uint32_t at[4];
+	uint32_t pc, sorted;
+	if (n1 <= 4)
+	{
+#pragma unroll
+		for (uint32_t k = 0; k < 4; ++k)
+		{
+			at[k] = k;
+			o[k] = k < n1 ? get(k) : oriented;
+		}
+		pc = sorted = n1;
+	}
+	else
+	{
+		pc = 1;
+		sorted = 0;
+		at[0] = minIndex;
+		at[1] = at[2] = at[3] = 0;
+		o[0] = get(minIndex);
+		o[1] = o[2] = o[3] = o[0];
+		float mx = -B3G_MAX_SCALAR;
+		for (uint32_t i = 0; i < n1; ++i)
+		{
+			if (i == at[0])
+				continue;
+			const V3 v = get(i) - o[0];
+			const float dd = dot(v, v);
+			if (dd > mx)
+			{
+				mx = dd;
+				at[1] = i;
+			}
+		}
+		if (!(mx < B3G_EPSILON * B3G_EPSILON))
+		{
+			pc = 2;
+			o[1] = get(at[1]);
+			mx = -B3G_MAX_SCALAR;
+			for (uint32_t i = 0; i < n1; ++i)
+			{
+				if (i == at[0] || i == at[1])
+					continue;
+				const V3 nn = cross(o[1] - o[0], get(i) - o[0]);
+				const float a2 = fabsr(dot(nn, oriented));
+				if (a2 > mx)
+				{
+					mx = a2;
+					at[2] = i;
+				}
+			}
+			const float kAreaTol = 0.01f;
+			if (!(mx < 2.0f * kAreaTol))
+			{
+				pc = 3;
+				o[2] = get(at[2]);
+				const uint32_t c0 = at[0], c1 = at[1];
+				if (!is_ccw(o[0], o[1], o[2], oriented))
+				{
+					const V3 v = o[0];
+					o[0] = o[1];
+					o[1] = v;
+					at[0] = c1;
+					at[1] = c0;
+				}
+				float mn = B3G_MAX_SCALAR;
+				for (uint32_t i = 0; i < n1; ++i)
+				{
+					if (i == c0 || i == c1 || i == at[2])
+						continue;
+					const V3 nn = cross(o[1] - o[0], get(i) - o[0]);
+					const float sa2 = dot(nn, oriented);
+					if (sa2 < mn)
+					{
+						mn = sa2;
+						at[3] = i;
+					}
+				}
+				if (!(fabsr(mn) < 2.0f * kAreaTol))
+				{
+					pc = sorted = 4;
+					o[3] = get(at[3]);
+				}
+			}
+		}
+	}
+	__syncwarp();
+	// b3SortPolygon (cluster.cpp:34-57).
+#pragma unroll
+	for (uint32_t i = 1; i < 4; ++i)
+	{
+		const V3 B = o[i];
+#pragma unroll
+		for (uint32_t j = i + 1; j < 4; ++j)
+			if (j < sorted && !is_ccw(o[0], B, o[j], oriented))
+			{
+				const V3 v = o[i];
+				o[i] = o[j];
+				o[j] = v;
+				const uint32_t k = at[i];
+				at[i] = at[j];
+				at[j] = k;
+			}
+	}
+	if (!live)
+		return;
+	DevManifold& m = a.man[c];
+	if (big)
+	{
+		build_face_contact(m, xf1, index1, h1, flip ? H.r2 : H.r1, xf2, h2, flip ? H.r1 : H.r2, flip, a.status);
+		pc = m.pointCount;
+	}
+	else
+	{
+		if (failed)
+			atomicOr(a.status, B3G_ST_POLY_OVERFLOW);
+		const XF xm1 = flip ? xf2 : xf1, xm2 = flip ? xf1 : xf2;
+		const V3 normal = rotc(xm1.q, oriented);
+#pragma unroll
+		for (uint32_t i = 0; i < 4; ++i)
+		{
+			if (i >= pc)
+				break;
+			const uint32_t s = (head + at[i]) % CLIP_SLOTS;
+			const V3 v2 = R.pos(s);
+			const uint32_t e1 = R.pair1[s][threadIdx.x], e2 = R.pair2[s][threadIdx.x];
+			const uint32_t q1 = flip ? e2 : e1, q2 = flip ? e1 : e2;
+			set_point(m.points[i], normal, xmult(xm1, flip ? v2 : o[i]), xmult(xm2, flip ? o[i] : v2));
+			set_id(m.points[i], mkpair(ring_edge(q1 & 0xFFFFu), ring_edge(q1 >> 16), ring_edge(q2 & 0xFFFFu),
+				ring_edge(q2 >> 16)));
+		}
+		m.pointCount = pc;
+	}
+	if (pc > 0)
+	{
+		a.cache[c] = cache; // overlap cache hit
+		finish_convex(a, c, m);
+	}
+	else
+		probe_flush(a, c, cache);
+}
+
+// Pass 1, the cache half of b3CollideHullsCache (collide_hulls.cpp:367-415):
+// b3FeatureCache::ReadState (sat.cpp:178-207), then the separation hit, or the
+// overlap hit that rebuilds the cached edge or face contact. What a cache does
+// not resolve goes to the SAT kernel.
+//
+// A block takes a tile of contacts and sorts them by what their caches hold,
+// so that a warp reads faces or edges and not some of each; the face contacts
+// to rebuild queue up until the block is full of them (or the contacts run
+// out) and rebuild on a lane each, in step, their polygons in shared memory.
+// With everything on the contact's own thread, 5.6 lanes of a warp were active
+// and the polygons lived in local memory: a pass of 512 worlds with 572,000 hull
+// pairs took 1,288 us, now 1,113. Blocks of 64 threads, or 5 blocks an SM
+// with 96 registers, take 10 % of that longer.
+__global__ void __launch_bounds__(PROBE_THREADS, PROBE_BLOCKS) k_hulls_probe(NPArgs a)
+{
+	__shared__ ClipRings rings;
+	__shared__ uint32_t sRead[PROBE_THREADS], sFace[2 * PROBE_THREADS];
+	__shared__ uint32_t sFaces, sEdges, sQueue;
+	const uint32_t n = *a.listCount;
+	const uint32_t tid = threadIdx.x, lane = tid & 31u;
+	if (tid == 0)
+		sQueue = 0;
+	for (uint32_t base = blockIdx.x * PROBE_THREADS;; base += gridDim.x * PROBE_THREADS)
+	{
+		const bool more = base < n;
+		if (more)
+		{
+			if (tid == 0)
+				sFaces = sEdges = 0;
+			__syncthreads();
+			uint32_t c = 0;
+			bool face = false, edges = false;
+			if (base + tid < n)
+			{
+				c = a.list[base + tid];
+				const int32_t prev = a.prevIndex[c];
+				const uint4 cache = prev >= 0 ? a.prevCache[prev] : make_uint4(CT_EMPTY, FT_FACE1, 0, 0);
+				man_clear(a.man[c]);
+				const bool hit = a.convexCache && (cache.x == CT_SEPARATION || cache.x == CT_OVERLAP);
+				face = hit && (cache.y == FT_FACE1 || cache.y == FT_FACE2);
+				edges = hit && cache.y == FT_EDGES;
+				if (!a.convexCache)
+					probe_miss(a, c, cache);
+				else if (cache.x == CT_EMPTY)
+					probe_miss(a, c, make_uint4(CT_EMPTY, FT_FACE1, 0, 0));
+				else if (!face && !edges)
+					probe_flush(a, c, cache);
+			}
+			__syncwarp();
+			const uint32_t below = (1u << lane) - 1u;
+			const uint32_t fm = __ballot_sync(0xffffffffu, face), em = __ballot_sync(0xffffffffu, edges);
+			uint32_t f0 = 0, e0 = 0;
+			if (lane == 0)
+			{
+				f0 = fm ? atomicAdd(&sFaces, (uint32_t)__popc(fm)) : 0u;
+				e0 = em ? atomicAdd(&sEdges, (uint32_t)__popc(em)) : 0u;
+			}
+			f0 = __shfl_sync(0xffffffffu, f0, 0);
+			e0 = __shfl_sync(0xffffffffu, e0, 0);
+			// Faces from the front, edges from the back.
+			if (face)
+				sRead[f0 + __popc(fm & below)] = c;
+			if (edges)
+				sRead[PROBE_THREADS - 1 - (e0 + __popc(em & below))] = c;
+			__syncthreads();
+			if (tid < sFaces)
+			{
+				// A face of either hull is read with the hulls in the face's order.
+				c = sRead[tid];
+				const uint4 cache = a.prevCache[a.prevIndex[c]];
+				HullCtx H;
+				load_hull_ctx(a, c, H);
+				const bool f2 = cache.y == FT_FACE2;
+				const uint32_t state = read_face_thread(f2 ? H.xf2 : H.xf1, f2 ? H.h2 : H.h1, f2 ? H.xf1 : H.xf2,
+					f2 ? H.h1 : H.h2, cache.z, H.r1 + H.r2);
+				if (cache.x == CT_SEPARATION && state == CT_SEPARATION)
+				{
+					a.cache[c] = cache; // separation cache hit
+					finish_convex(a, c, a.man[c]);
+				}
+				else if (cache.x == CT_OVERLAP && state == CT_OVERLAP &&
+					face_contact_persists(f2 ? H.xf2 : H.xf1, f2 ? H.xf1 : H.xf2, f2 ? H.xf02 : H.xf01,
+						f2 ? H.xf01 : H.xf02))
+					sFace[atomicAdd(&sQueue, 1u)] = c;
+				else
+					probe_flush(a, c, cache);
+			}
+			else if (tid >= PROBE_THREADS - sEdges)
+			{
+				c = sRead[tid];
+				const uint4 cache = a.prevCache[a.prevIndex[c]];
+				HullCtx H;
+				load_hull_ctx(a, c, H);
+				const uint32_t state = read_edges(H.xf1, H.h1, H.xf2, H.h2, cache.z, cache.w, H.r1 + H.r2);
+				DevManifold& m = a.man[c];
+				bool done = cache.x == CT_SEPARATION && state == CT_SEPARATION;
+				if (cache.x == CT_OVERLAP && state == CT_OVERLAP)
+				{
+					rebuild_edge_contact(m, H.xf1, cache.z, H.h1, H.xf2, cache.w, H.h2);
+					done = m.pointCount > 0;
+				}
+				if (done)
+				{
+					a.cache[c] = cache;
+					finish_convex(a, c, m);
+				}
+				else
+					probe_flush(a, c, cache);
+			}
+		}
+		__syncthreads();
+		const uint32_t queued = sQueue;
+		const uint32_t take = more && queued < PROBE_THREADS ? 0u : min(queued, (uint32_t)PROBE_THREADS);
+		if ((tid & ~31u) < take)
+			rebuild_faces(a, sFace[queued - take + min(tid, take - 1u)], tid < take, rings);
+		__syncthreads();
+		if (tid == 0)
+			sQueue = queued - take;
+		if (!more && queued == take)
+			break;
 	}
 }
 
@@ -1448,7 +1814,7 @@ void launch_hulls_probe(const NPArgs& base, const uint32_t* list, const uint32_t
 	NPArgs a = base;
 	a.list = list;
 	a.listCount = count;
-	k_hulls_probe<<<work_blocks(a.hcPostCap, 128, (int)tune.v[B3G_TUNE_PROBE]), 128, 0, s>>>(a);
+	k_hulls_probe<<<work_blocks(a.hcPostCap, PROBE_THREADS, (int)tune.v[B3G_TUNE_PROBE]), PROBE_THREADS, 0, s>>>(a);
 }
 
 // Dynamic shared memory of the SAT kernel with `warps` warps per block.

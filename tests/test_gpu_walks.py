@@ -170,3 +170,77 @@ def test_pairs_of_flat_and_narrow_worlds(scale):
     got = {(min(a, b), max(a, b)) for a, b, _ in pipe.contacts().tolist()}
     assert got == overlapping(pipe, sc)
     pipe.close()
+
+
+def prism(n, radius, height):
+    """A prism over a regular n-gon as packed hull arrays, its caps one face each."""
+    a = 2 * np.pi * np.arange(n) / n
+    ring = radius * np.stack([np.cos(a), np.zeros(n), np.sin(a)], -1)
+    v = np.concatenate([ring + [0, height, 0], ring - [0, height, 0]]).astype(np.float32)
+    # Outward loops: the top, the bottom, then the sides.
+    loops = [list(range(n))[::-1], [n + i for i in range(n)]]
+    loops += [[i, (i + 1) % n, n + (i + 1) % n, n + i] for i in range(n)]
+    at, edges = {}, []
+    for loop in loops:
+        for k, x in enumerate(loop):
+            y = loop[(k + 1) % len(loop)]
+            if (y, x) in at:
+                at[(x, y)] = at[(y, x)] ^ 1
+            else:
+                at[(x, y)] = len(edges)
+                edges += [None, None]
+    for f, loop in enumerate(loops):
+        ids = [at[(x, loop[(k + 1) % len(loop)])] for k, x in enumerate(loop)]
+        for k, e in enumerate(ids):
+            edges[e] = [loop[k], e ^ 1, f, ids[k - 1], ids[(k + 1) % len(ids)]]
+    faces = [at[(loop[0], loop[1])] for loop in loops]
+    planes = []
+    for loop in loops:
+        p = v[loop].astype(np.float64)
+        nrm = np.cross(p[1] - p[0], p[2] - p[1])
+        nrm /= np.linalg.norm(nrm)
+        planes.append([*nrm, nrm @ p[0]])
+    return dict(desc=np.array([0, 2 * n, 0, len(edges), 0, len(loops)], np.uint32), verts=v.reshape(-1),
+                edges=np.array(edges, np.uint32).reshape(-1), faces=np.array(faces, np.uint32),
+                planes=np.array(planes, np.float32).reshape(-1), centroids=np.zeros(3, np.float32))
+
+
+# A pair at rest: the pass that finds the contact builds it from the separating
+# axes (a warp per contact), the next rebuilds it from the feature cache (a
+# lane per contact, rings of 16 clip vertices), and both give the same points.
+# Faces below, at and beyond what a ring holds; more pairs than a block takes.
+@pytest.mark.parametrize("sides", [(3, 3), (4, 4), (4, 9), (3, 15), (15, 3), (16, 4), (8, 16), (17, 4), (30, 30),
+                                   (4, 40)])
+@pytest.mark.parametrize("pairs", [1, 33, 700])
+def test_rebuilt_face_contacts(sides, pairs):
+    rng = np.random.default_rng(sides[0] * 100 + sides[1])
+    sc = S.Scene()
+    low, top = (sc.hulls.extend(prism(n, r, 0.5)) for n, r in zip(sides, (1.0, 0.9)))
+    for k in range(pairs):
+        x = np.array([5.0 * (k % 30), 0, 5.0 * (k // 30)])
+        b = sc.add_body(0, N.BODY_STATIC, x, (0, 0, 0, 1))
+        sc.add_fixture(b, N.SHAPE_HULL, [0.02], hull=low)
+        turn = rng.uniform(-3, 3) / 2
+        x = x + [rng.uniform(-0.6, 0.6), 0.98 + rng.uniform(0, 0.05), rng.uniform(-0.6, 0.6)]
+        tilt = np.array([rng.uniform(-0.01, 0.01), np.sin(turn), rng.uniform(-0.01, 0.01), np.cos(turn)])
+        b = sc.add_body(0, N.BODY_DYNAMIC, x, tilt / np.linalg.norm(tilt))
+        sc.add_fixture(b, N.SHAPE_HULL, [0.02], hull=top)
+    sc.finalize()
+    pipe = CollisionPipeline(sc, max_contacts=4096)
+    state = S.KinematicDriver(sc).state17()
+    rounds = []
+    for _ in range(2):
+        pipe.collide(state)
+        index, m = pipe.touching()
+        order = np.argsort(index)
+        rounds.append((pipe.contacts()[index][order], m[order]))
+    assert pipe.pass_stats()["hull_miss"] < len(rounds[0][0])
+    (f0, m0), (f1, m1) = rounds
+    assert len(f0) >= 0.9 * pairs
+    assert np.array_equal(f0[:, :2], f1[:, :2])
+    assert np.array_equal(m0["pointCount"], m1["pointCount"])
+    for field in ("n", "p1", "p2", "triangleKey", "key", "edgeContact"):
+        for i in range(4):
+            has = m0["pointCount"] > i
+            assert np.array_equal(m0["points"][field][has, i], m1["points"][field][has, i]), field
+    pipe.close()
