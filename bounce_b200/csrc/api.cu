@@ -710,6 +710,7 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 		cudaFree(c->edgeBuf);
 	dfree(c->dFixMaterial);
 	dfree(c->ciTiles);
+	dfree(c->ciItems);
 	if (c->ciHost)
 		cudaFree(c->ciHost);
 	if (c->toiScratch)
@@ -2264,8 +2265,11 @@ extern "C" int b3g_contact_constraints_device(b3g_ctx* c, uint32_t count, const 
 	if (c->ciTileCap < words)
 	{
 		dfree(c->ciTiles);
+		dfree(c->ciItems);
 		c->ciTileCap = 0;
 		CK(dalloc(&c->ciTiles, words));
+		CK(dalloc(&c->ciItems, c->cfg.max_contacts));
+		CK(cudaMemsetAsync(c->ciTiles, 0, sizeof(unsigned long long) * words, stream ? (cudaStream_t)stream : c->stream));
 		c->ciTileCap = words;
 	}
 	ConstraintCall q;
@@ -2276,6 +2280,7 @@ extern "C" int b3g_contact_constraints_device(b3g_ctx* c, uint32_t count, const 
 	q.dtRatio = dtRatio;
 	q.warm = warm ? 1 : 0;
 	q.tiles = c->ciTiles;
+	q.items = c->ciItems;
 	q.counts = counts;
 	q.constraints = constraints;
 	q.constraintCap = constraints ? cCap : 0;

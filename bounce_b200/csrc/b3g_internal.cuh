@@ -370,6 +370,7 @@ struct b3g_ctx
 	size_t qScratchBytes;
 	float2* dFixMaterial;         // per fixture: friction, restitution (b3g_set_materials)
 	unsigned long long* ciTiles;  // b3g_contact_constraints_device: tile counter and states (allocated on first use)
+	uint4* ciItems;               // ... and the selected contacts
 	uint32_t ciTileCap;
 	void* ciHost;                 // b3g_contact_constraints: device copies of its host buffers
 	size_t ciHostBytes;
@@ -535,6 +536,7 @@ struct ConstraintCall
 	float dtRatio;
 	int warm;
 	unsigned long long* tiles;
+	uint4* items;
 	uint32_t* counts;
 	b3g_contact_constraint* constraints;
 	uint32_t constraintCap;

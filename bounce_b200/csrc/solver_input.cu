@@ -10,15 +10,18 @@
 // b3g_manifold_constraint), the manifolds of consecutive constraints stored
 // consecutively.
 //
-// One kernel of resident blocks. Each block takes tiles of 1,024 items
-// (contacts of the list, or the caller's list entries) in order through a
-// counter until none is left, counts the constraints and manifolds its items
-// produce, and finds the counts of the tiles before it by decoupled look-back (Merrill & Garland: publish the
-// tile's own count, add the published counts of earlier tiles until one that
-// holds its inclusive prefix, 32 tiles per probe; bounded waits). The tile's
-// selected items are compacted in shared memory in constraint order and
-// handed out to quads: the four lanes of a quad build one constraint, lane q
-// taking manifold point q, so consecutive quads write consecutive records.
+// Two kernels. k_constraint_items takes tiles of 1,024 items (contacts of the
+// list, or the caller's list entries) in order through a counter, counts the
+// constraints and manifolds its items produce, finds the counts of the tiles
+// before it by decoupled look-back (Merrill & Garland: publish the tile's own
+// count, add the published counts of earlier tiles until one that holds its
+// inclusive prefix, 32 tiles per probe; bounded waits) and writes the selected
+// items in constraint order. k_contact_constraints hands those out to quads:
+// the four lanes of a quad build one constraint, lane q taking manifold point
+// q, so consecutive quads write consecutive records. In one kernel the scan's
+// barriers and the 125 registers of the second half left the loads of both
+// waiting: 183 us for the 330,000 constraints of 1.2 million contacts, now 25
+// and 126; 97 us for 65,536 mixed bodies, now 13 and 54.
 // Every expression keeps the reference's operand order (the library is built
 // with -fmad=false), so the records are the reference's bit for bit.
 #include "collide_common.cuh"
@@ -52,12 +55,14 @@ struct CIArgs
 	const uint32_t* fixBody;
 	const uint32_t* fixType;
 	const uint32_t* fixFlags;
+	bool sensors;             // some fixture is a sensor
 	const float4* fixParams;
 	const float2* material;   // per fixture: friction, restitution
 	const float4* bodies;     // b3g_solver_body records (7 float4 each)
 	float dtRatio;
 	int warm;
-	unsigned long long* tileState; // [0]: tile counter, [1 + t]: status of tile t (zeroed per call)
+	unsigned long long* tileState; // [0]: tile counter, [1 + t]: status of tile t (0 between calls)
+	uint4* items;             // selected items in constraint order (Selected)
 	uint32_t* counts;         // device: constraints, manifolds (zeroed per call)
 	float4* cOut;             // b3g_contact_constraint records (8 float4 each)
 	uint32_t cCap;
@@ -76,43 +81,46 @@ __device__ __forceinline__ uint32_t item_count(const CIArgs& a)
 // holds; an index past the contact list gets a record without manifolds);
 // by default a contact gets one when it is touching and neither fixture is a
 // sensor (the island filter of b3World::Solve, world.cpp:336-348). A selected
-// contact's fixtures and bodies are looked up here, four items per thread in
-// flight, rather than at the head of its quad's dependent loads.
+// contact's bodies are looked up here, four items per thread in flight, rather
+// than at the head of its quad's dependent loads.
 struct Item
 {
-	uint32_t c, flag, mc, fa, fb, ba, bb;
+	uint32_t c, flag, mc, ba, bb;
 };
 
-__device__ __forceinline__ Item item_counts(const CIArgs& a, uint32_t i, uint32_t n)
+// A selected item: x = contact (0xFFFFFFFF: a record without manifolds),
+// y = first manifold (bits 0-29) and manifold count (bits 30-31; at most 3),
+// z, w = bodies.
+__device__ __forceinline__ uint4 selected(const Item& it, uint32_t firstManifold)
 {
-	Item it{0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u, 0u};
+	return make_uint4(it.c, firstManifold | it.mc << 30, it.ba, it.bb);
+}
+
+// st: the contact's state word where the items are the contacts themselves.
+__device__ __forceinline__ Item item_counts(const CIArgs& a, uint32_t i, uint32_t n, uint32_t st)
+{
+	Item it{0xFFFFFFFFu, 0u, 0u, 0u, 0u};
 	if (i >= n)
 		return it;
-	const uint32_t nc = min(*a.nContacts, a.maxContacts);
-	uint32_t c;
+	uint32_t c = i;
 	if (a.list)
 	{
 		c = a.list[i];
 		it.flag = 1;
-		if (c >= nc)
+		if (c >= min(*a.nContacts, a.maxContacts))
 			return it;
+		st = a.cstate[c];
 	}
-	else
-	{
-		c = i;
-	}
-	const uint32_t st = a.cstate[c];
 	if (!a.list && (st & 1u) == 0)
 		return it;
-	it.fa = a.pairA[c];
-	it.fb = a.pairB[c];
-	if (!a.list && ((a.fixFlags[it.fa] | a.fixFlags[it.fb]) & B3G_FIXTURE_SENSOR) != 0)
+	const uint32_t fa = a.pairA[c], fb = a.pairB[c];
+	if (!a.list && a.sensors && ((a.fixFlags[fa] | a.fixFlags[fb]) & B3G_FIXTURE_SENSOR) != 0)
 		return it;
 	it.c = c;
 	it.flag = 1;
 	it.mc = min((st >> 8) & 0xFFu, 3u);
-	it.ba = a.fixBody[it.fa];
-	it.bb = a.fixBody[it.fb];
+	it.ba = a.fixBody[fa];
+	it.bb = a.fixBody[fb];
 	return it;
 }
 
@@ -212,17 +220,20 @@ __device__ __forceinline__ float u2f(uint32_t u) { return __uint_as_float(u); }
 // One manifold, built by the four lanes of a quad (lane `sub` = point sub):
 // the velocity-constraint manifold of the constructor (contact_solver.cpp:87-147)
 // completed by InitializeVelocityConstraints (:219-302), and the
-// position-constraint points (:127-130). Every lane of the quad calls this.
+// position-constraint points (:127-130). Every lane of the quad calls this;
+// out is the record in shared memory.
 __device__ void quad_manifold(const CIArgs& a, const DevManifold* m, uint32_t k, const float4* BA, const float4* BB,
 	float radiusA, float radiusB, float rest, uint32_t sub, uint32_t mask, float4* out)
 {
 	const uint32_t pc = min(m->pointCount, 4u);
 	const bool has = sub < pc;
-	const DevPoint* p = m->points + sub;
-	const V3 ln = v3(p->n[0], p->n[1], p->n[2]);
-	const V3 lp1 = v3(p->p1[0], p->p1[1], p->p1[2]);
-	const V3 lp2 = v3(p->p2[0], p->p2[1], p->p2[2]);
-	const float lni = p->normalImpulse;
+	// A point is n, p1, p2, normalImpulse: 40 bytes, 8-byte aligned.
+	const float2* p = reinterpret_cast<const float2*>(m->points + sub);
+	const float2 f0 = p[0], f1 = p[1], f2 = p[2], f3 = p[3], f5 = p[4];
+	const V3 ln = v3(f0.x, f0.y, f1.x);
+	const V3 lp1 = v3(f1.y, f2.x, f2.y);
+	const V3 lp2 = v3(f3.x, f3.y, f5.x);
+	const float lni = f5.y;
 	// b3WorldManifoldPoint::Initialize (collision.cpp:63-76) for this lane's point.
 	V3 point = v3(0.0f, 0.0f, 0.0f), nA = v3(0.0f, 0.0f, 0.0f);
 	if (has)
@@ -366,39 +377,26 @@ __device__ void quad_manifold(const CIArgs& a, const DevManifold* m, uint32_t k,
 	out[2 * sub + 1] = w1;
 }
 
-// One constraint, built by a quad (every lane calls this with the same item).
-__device__ void quad_contact(const CIArgs& a, uint32_t c, uint32_t k, uint32_t ms, uint32_t mc, uint32_t fa,
-	uint32_t fb, uint32_t ba, uint32_t bb, uint32_t sub, uint32_t mask)
+// One constraint record, written by a quad. c = 0xFFFFFFFF: one without a
+// contact.
+__device__ __forceinline__ void quad_constraint(const CIArgs& a, uint4 item, uint32_t k, const float4* BA,
+	const float4* BB, float radiusA, float radiusB, float2 matA, float2 matB, float rest, uint32_t sub)
 {
-	if (c == 0xFFFFFFFFu)
+	const uint32_t ms = item.y & 0x3FFFFFFFu, mc = item.y >> 30;
+	float4 w0 = f4(0.0f, 0.0f, 0.0f, 0.0f), w1 = w0;
+	if (item.x == 0xFFFFFFFFu)
 	{
-		if (k < a.cCap)
-		{
-			float4* o = a.cOut + 8 * (size_t)k;
-			float4 w0 = f4(0.0f, 0.0f, 0.0f, 0.0f), w1 = w0;
-			if (sub == 0)
-				w0 = f4(u2f(0xFFFFFFFFu), u2f(0xFFFFFFFFu), u2f(ms), u2f(0u));
-			if (sub == 3)
-				w1 = f4(u2f(c), 0.0f, 0.0f, 0.0f);
-			o[2 * sub] = w0;
-			o[2 * sub + 1] = w1;
-		}
-		return;
+		if (sub == 0)
+			w0 = f4(u2f(0xFFFFFFFFu), u2f(0xFFFFFFFFu), u2f(ms), u2f(0u));
+		if (sub == 3)
+			w1 = f4(u2f(item.x), 0.0f, 0.0f, 0.0f);
 	}
-	const float4* BA = a.bodies + 7 * (size_t)ba;
-	const float4* BB = a.bodies + 7 * (size_t)bb;
-	const float radiusA = shape_radius(a, fa), radiusB = shape_radius(a, fb);
-	const float2 matA = a.material[fa], matB = a.material[fb];
-	// b3MixRestitution (contact.h:40-43).
-	const float rest = fmaxr(matA.y, matB.y);
-	if (k < a.cCap)
-	{
-		float4 w0, w1;
+	else
 		switch (sub)
 		{
 		case 0:
 			// b3MixFriction (contact.h:33-36).
-			w0 = f4(u2f(ba), u2f(bb), u2f(ms), u2f(mc));
+			w0 = f4(u2f(item.z), u2f(item.w), u2f(ms), u2f(mc));
 			w1 = f4(BA[3].y, BB[3].y, sqrtf(matA.x * matB.x), rest);
 			break;
 		case 1:
@@ -411,31 +409,21 @@ __device__ void quad_contact(const CIArgs& a, uint32_t c, uint32_t k, uint32_t m
 			break;
 		default:
 			w0 = f4(BB[6].x, BB[6].y, radiusA, radiusB);
-			w1 = f4(u2f(c), 0.0f, 0.0f, 0.0f);
+			w1 = f4(u2f(item.x), 0.0f, 0.0f, 0.0f);
 			break;
 		}
-		float4* o = a.cOut + 8 * (size_t)k;
-		o[2 * sub] = w0;
-		o[2 * sub + 1] = w1;
-	}
-	for (uint32_t j = 0; j < mc; ++j)
-	{
-		if (ms + j >= a.mCap)
-			break;
-		const DevManifold* m = j == 0 ? a.man + c : a.extra + 2 * (size_t)c + j - 1;
-		quad_manifold(a, m, k, BA, BB, radiusA, radiusB, rest, sub, mask, a.mOut + 29 * (size_t)(ms + j));
-	}
+	float4* o = a.cOut + 8 * (size_t)k;
+	o[2 * sub] = w0;
+	o[2 * sub + 1] = w1;
 }
 
-__global__ void __launch_bounds__(CI_BLOCK) k_contact_constraints(CIArgs a)
+__global__ void __launch_bounds__(CI_BLOCK) k_constraint_items(CIArgs a)
 {
 	__shared__ uint32_t sTile;
 	__shared__ unsigned long long sPrefix;
-	__shared__ uint32_t sItem[7][CI_TILE]; // per selected item: c, ms, mc, fa, fb, ba, bb
 	const uint32_t t = threadIdx.x, lane = t & 31u;
 	const uint32_t n = item_count(a);
 	const uint32_t tiles = max((n + CI_TILE - 1) / CI_TILE, 1u);
-	const uint32_t sub = lane & 3u, mask = 0xFu << (lane & ~3u);
 	for (;;)
 	{
 		if (t == 0)
@@ -445,12 +433,26 @@ __global__ void __launch_bounds__(CI_BLOCK) k_contact_constraints(CIArgs a)
 		if (tile >= tiles)
 			break;
 		// Thread t holds items 4t .. 4t + 3 of the tile.
+		static_assert(CI_ITEMS == 4, "one load of states per thread");
 		Item it[CI_ITEMS];
+		const uint32_t first = tile * CI_TILE + CI_ITEMS * t;
+		uint32_t st[CI_ITEMS] = {0u, 0u, 0u, 0u};
+		if (!a.list && first + CI_ITEMS <= n)
+		{
+			const uint4 w = *reinterpret_cast<const uint4*>(a.cstate + first);
+			st[0] = w.x;
+			st[1] = w.y;
+			st[2] = w.z;
+			st[3] = w.w;
+		}
+		else if (!a.list)
+			for (int r = 0; r < CI_ITEMS; ++r)
+				st[r] = first + r < n ? a.cstate[first + r] : 0u;
 		unsigned long long sum = 0;
 #pragma unroll
 		for (int r = 0; r < CI_ITEMS; ++r)
 		{
-			it[r] = item_counts(a, tile * CI_TILE + CI_ITEMS * t + r, n);
+			it[r] = item_counts(a, first + r, n, st[r]);
 			sum += ((unsigned long long)it[r].flag << 32) | it[r].mc;
 		}
 		unsigned long long total;
@@ -522,30 +524,94 @@ __global__ void __launch_bounds__(CI_BLOCK) k_contact_constraints(CIArgs a)
 				}
 			}
 		}
+		__syncthreads();
 		// The tile's selected items in constraint order.
+		run += sPrefix;
 #pragma unroll
 		for (int r = 0; r < CI_ITEMS; ++r)
 		{
 			if (it[r].flag)
-			{
-				const uint32_t kl = (uint32_t)(run >> 32);
-				sItem[0][kl] = it[r].c;
-				sItem[1][kl] = (uint32_t)(run & 0xFFFFFFFFull);
-				sItem[2][kl] = it[r].mc;
-				sItem[3][kl] = it[r].fa;
-				sItem[4][kl] = it[r].fb;
-				sItem[5][kl] = it[r].ba;
-				sItem[6][kl] = it[r].bb;
-			}
+				a.items[(uint32_t)(run >> 32)] = selected(it[r], (uint32_t)(run & 0xFFFFFFFFull));
 			run += ((unsigned long long)it[r].flag << 32) | it[r].mc;
 		}
 		__syncthreads();
-		const uint32_t k0 = (uint32_t)(sPrefix >> 32), ms0 = (uint32_t)(sPrefix & 0xFFFFFFFFull);
-		const uint32_t count = (uint32_t)(total >> 32);
-		for (uint32_t e = t >> 2; e < count; e += CI_BLOCK / 4)
-			quad_contact(a, sItem[0][e], k0 + e, ms0 + sItem[1][e], sItem[2][e], sItem[3][e], sItem[4][e],
-				sItem[5][e], sItem[6][e], sub, mask);
-		__syncthreads();
+	}
+}
+
+// The records. A warp builds the manifolds of 8 constraints in shared memory
+// and writes them out together: written from the quads, 44 of a manifold's 116
+// words went out one by one, 36 bytes apart. Bound by the loads of the bodies
+// and manifolds, two to four deep, with 20 warps an SM to hide them (4 and 6
+// blocks an SM take 1 % longer).
+constexpr int CC_WARPS = 4;
+constexpr int CC_BLOCKS = 5;
+
+__global__ void __launch_bounds__(CC_WARPS * 32, CC_BLOCKS) k_contact_constraints(CIArgs a, uint32_t tiles)
+{
+	__shared__ float4 sOut[CC_WARPS][8][29];
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	const uint32_t sub = lane & 3u, quad = lane >> 2, mask = 0xFu << (lane & ~3u);
+	// The tile states are zero again for the next call.
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= tiles; i += gridDim.x * blockDim.x)
+		a.tileState[i] = 0ull;
+	const uint32_t n = a.counts[0];
+	if (n == 0xFFFFFFFFu)
+		return; // a wait ran out: no counts to go by
+	// Each warp's next items are on their way while it builds these.
+	const uint32_t step = gridDim.x * CC_WARPS * 8u;
+	const uint4 none = make_uint4(0xFFFFFFFFu, 0u, 0u, 0u);
+	uint32_t k = (blockIdx.x * CC_WARPS + warp) * 8u + quad;
+	uint4 next = k < n ? a.items[k] : none;
+	uint32_t nextA = next.x != 0xFFFFFFFFu ? a.pairA[next.x] : 0u;
+	uint32_t nextB = next.x != 0xFFFFFFFFu ? a.pairB[next.x] : 0u;
+	for (; k - quad < n; k += step)
+	{
+		const bool valid = k < n;
+		const uint4 item = next;
+		next = k + step < n ? a.items[k + step] : none;
+		const uint32_t c = item.x, ms = item.y & 0x3FFFFFFFu, mc = item.y >> 30;
+		const float4* BA = a.bodies + 7 * (size_t)item.z;
+		const float4* BB = a.bodies + 7 * (size_t)item.w;
+		float radiusA = 0.0f, radiusB = 0.0f, rest = 0.0f;
+		float2 matA = make_float2(0.0f, 0.0f), matB = matA;
+		if (c != 0xFFFFFFFFu)
+		{
+			const uint32_t fa = nextA, fb = nextB;
+			radiusA = shape_radius(a, fa);
+			radiusB = shape_radius(a, fb);
+			matA = a.material[fa];
+			matB = a.material[fb];
+			// b3MixRestitution (contact.h:40-43).
+			rest = fmaxr(matA.y, matB.y);
+		}
+		if (valid && k < a.cCap)
+			quad_constraint(a, item, k, BA, BB, radiusA, radiusB, matA, matB, rest, sub);
+		if (next.x != 0xFFFFFFFFu)
+		{
+			nextA = a.pairA[next.x];
+			nextB = a.pairB[next.x];
+		}
+		const uint32_t most = __reduce_max_sync(0xffffffffu, mc);
+		for (uint32_t j = 0; j < most; ++j)
+		{
+			const bool has = j < mc && ms + j < a.mCap;
+			if (has)
+			{
+				const DevManifold* m = j == 0 ? a.man + c : a.extra + 2 * (size_t)c + j - 1;
+				quad_manifold(a, m, k, BA, BB, radiusA, radiusB, rest, sub, mask, sOut[warp][quad]);
+			}
+			__syncwarp();
+			const uint32_t to = has ? ms + j : 0xFFFFFFFFu;
+			for (uint32_t base = 0; base < 8u * 29u; base += 32u)
+			{
+				const uint32_t e = base + lane;
+				const uint32_t row = min(e / 29u, 7u);
+				const uint32_t m = __shfl_sync(0xffffffffu, to, 4u * row);
+				if (e < 8u * 29u && m != 0xFFFFFFFFu)
+					a.mOut[29 * (size_t)m + (e - 29u * row)] = sOut[warp][row][e - 29u * row];
+			}
+			__syncwarp();
+		}
 	}
 }
 
@@ -553,9 +619,8 @@ __global__ void __launch_bounds__(CI_BLOCK) k_contact_constraints(CIArgs a)
 
 uint32_t contact_constraint_tiles(uint32_t items) { return std::max((items + CI_TILE - 1) / CI_TILE, 1u); }
 
-// Zeroes the tile states and the counts, then launches the kernel on s over
-// the tiles of the item capacity (the list length, or max_contacts for the
-// default selection).
+// Zeroes the counts, then launches the kernels on s over the tiles of the item
+// capacity (the list length, or max_contacts for the default selection).
 void launch_contact_constraints(b3g_ctx* c, const ConstraintCall& q, cudaStream_t s)
 {
 	Buffers& B = c->buf;
@@ -572,12 +637,14 @@ void launch_contact_constraints(b3g_ctx* c, const ConstraintCall& q, cudaStream_
 	a.fixBody = c->scene.fixBody;
 	a.fixType = c->scene.fixType;
 	a.fixFlags = c->scene.fixFlags;
+	a.sensors = c->anySensor;
 	a.fixParams = c->scene.fixParams;
 	a.material = q.material;
 	a.bodies = reinterpret_cast<const float4*>(q.bodies);
 	a.dtRatio = q.dtRatio;
 	a.warm = q.warm;
 	a.tileState = q.tiles;
+	a.items = q.items;
 	a.counts = q.counts;
 	a.cOut = reinterpret_cast<float4*>(q.constraints);
 	a.cCap = q.constraints ? q.constraintCap : 0;
@@ -586,15 +653,9 @@ void launch_contact_constraints(b3g_ctx* c, const ConstraintCall& q, cudaStream_
 	const uint32_t tiles = contact_constraint_tiles(q.list ? q.listCount : c->cfg.max_contacts);
 	// Persistent blocks (as many as are resident at once) take the tiles in
 	// order through the counter until they run out.
-	static int perSM = 0;
-	if (perSM == 0 &&
-		(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_contact_constraints, CI_BLOCK, 0) != cudaSuccess ||
-			perSM < 1))
-		perSM = 1;
-	int sms = 148;
-	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-	const uint32_t blocks = std::min<uint32_t>(tiles, (uint32_t)(perSM * sms));
-	cudaMemsetAsync(q.tiles, 0, sizeof(unsigned long long) * ((size_t)tiles + 1), s);
+	const uint32_t blocks = (uint32_t)work_blocks(tiles, 1, 5);
 	cudaMemsetAsync(q.counts, 0, 2 * sizeof(uint32_t), s);
-	k_contact_constraints<<<blocks, CI_BLOCK, 0, s>>>(a);
+	k_constraint_items<<<blocks, CI_BLOCK, 0, s>>>(a);
+	const uint32_t most = q.list ? q.listCount : c->cfg.max_contacts;
+	k_contact_constraints<<<work_blocks(most, 8 * CC_WARPS, CC_BLOCKS), CC_WARPS * 32, 0, s>>>(a, tiles);
 }
