@@ -495,7 +495,7 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 	step(dalloc(&B.worldEnd, P), "alloc");
 	step(dalloc(&B.proxyInfo, P), "alloc");
 	step(dalloc(&B.outOff, C), "alloc");
-	step(dalloc(&B.pairScratch, 2 * B3G_TRAV_SLOTS * (size_t)P), "alloc"); // uint2 records per leaf
+	step(dalloc(&B.walkTree, 8 * (size_t)P), "alloc");
 	const size_t scanWords = scan_aux_words(std::max(P, C) + 1);
 	step(dalloc(&B.scanAux, scanWords + scan_aux_words(P + 1) + scan_aux_words(C)), "alloc");
 	B.passScan = reinterpret_cast<unsigned long long*>(B.scanAux + scanWords);
@@ -604,7 +604,7 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 	dfree(B.worldEnd);
 	dfree(B.proxyInfo);
 	dfree(B.outOff);
-	dfree(B.pairScratch);
+	dfree(B.walkTree);
 	dfree(B.scanAux);
 	for (int k = 0; k < 2; ++k)
 	{

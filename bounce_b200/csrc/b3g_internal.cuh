@@ -169,8 +169,7 @@ struct Buffers
 	uint2* leafData;      // per sorted leaf: its proxy's proxyInfo word and fixture key
 	uint32_t* leafOf;     // per proxy: its sorted leaf (set when the LBVH is built)
 	uint32_t* outOff;     // per contact: offsets of the touching output
-	uint32_t* pairScratch; // first contact records (A, B) found per leaf, slot-major (B3G_TRAV_SLOTS x n uint2);
-	                       // between passes the tree as the world queries walk it (queries.cu)
+	float4* walkTree;     // the tree as the world queries walk it: 8 float4 per proxy (queries.cu)
 	uint32_t* scanAux;    // scan state
 	unsigned long long* passScan; // scan states of the contact list (order.cu), cleared when the pass begins
 	uint32_t* rawA;       // overlapping pairs in traversal order (this pass)
@@ -276,8 +275,7 @@ __device__ __forceinline__ bool joint_excluded(const FilterArgs& F, uint32_t ba,
 	return lo < F.nJoints && F.jointKeys[lo] == k;
 }
 
-// Contact records a leaf's walk keeps in its scratch slots; leaves with more
-// partners walk again for the rest.
+// The pairs of one leaf after which CTR_TRAV_OVERFLOW counts the rest.
 #define B3G_TRAV_SLOTS 32u
 
 // Counter slots in Buffers::counters.
@@ -303,7 +301,7 @@ enum
 	CTR_ASLEEP = 29,    // non-static bodies still asleep after the wake-ups
 	CTR_SCRATCH = 30,
 	CTR_MESH_PAIRS = 31, // (contact, triangle) work items of the pass
-	CTR_TRAV_OVERFLOW = 32, // traversal records past the scratch slots
+	CTR_TRAV_OVERFLOW = 32, // pairs of a leaf past its first B3G_TRAV_SLOTS
 	CTR_CANDIDATES = 33,    // new pairs handed to the caller's contact filter
 	CTR_HC_POST = 34,       // hull-capsule contacts past their GJK (k_hull_capsule_post): at a distance
 	CTR_HC_DEEP = 35,       // ... and overlapping

@@ -1046,13 +1046,11 @@ __global__ void __launch_bounds__(32) k_ray_first_warp(QueryCtx q, WalkTree tree
 // 124 and 286 us; at 40,000: 459 and 317 us.
 constexpr uint32_t RAY_WARP_MAX = 148u * 160u;
 
-// The tree laid out for the ordered walks, in the scratch of the pair search,
-// which holds nothing between passes.
+// The tree laid out for the ordered walks, in the context's own records.
 WalkTree launch_walk_tree(b3g_ctx* c, const QueryCtx& q, uint32_t* turned, cudaStream_t s)
 {
 	WalkTree t;
-	static_assert(sizeof(uint2) * B3G_TRAV_SLOTS >= 8 * sizeof(float4), "two records per proxy");
-	float4* nodes = reinterpret_cast<float4*>(c->buf.pairScratch);
+	float4* nodes = c->buf.walkTree;
 	float4* leaves = nodes + 4 * (size_t)c->cfg.max_proxies;
 	t.nodes = nodes;
 	t.leaves = leaves;

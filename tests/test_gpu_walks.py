@@ -244,3 +244,30 @@ def test_rebuilt_face_contacts(sides, pairs):
             has = m0["pointCount"] > i
             assert np.array_equal(m0["points"][field][has, i], m1["points"][field][has, i]), field
     pipe.close()
+
+
+# More overlapping nodes than a warp's stack holds (every box meets every other,
+# the lanes go on along the ropes), the fewest leaves, and several worlds whose
+# boxes lie on top of one another.
+@pytest.mark.parametrize("n,worlds", [(1, 1), (2, 1), (3, 2), (5, 1), (129, 1), (1500, 1), (1200, 7)])
+def test_pairs_of_heaped_worlds(n, worlds):
+    sc = S.Scene()
+    rng = np.random.default_rng(n)
+    for k in range(n):
+        b = sc.add_body(k % worlds, N.BODY_DYNAMIC, rng.uniform(-0.2, 0.2, 3), (0, 0, 0, 1))
+        sc.add_fixture(b, N.SHAPE_SPHERE, [0, 0, 0, 0.5])
+    sc.finalize()
+    pipe = CollisionPipeline(sc, max_contacts=max(64, n * n))
+    state = S.KinematicDriver(sc).state17()
+    for _ in range(2):
+        pipe.collide(state)
+    got = pipe.contacts()[:, :2].astype(np.int64)
+    world = np.arange(n) % worlds
+    a, b = np.triu_indices(n, 1)
+    same = world[a] == world[b]
+    want = a[same] * n + b[same]
+    assert np.array_equal(np.sort(got.min(axis=1) * n + got.max(axis=1)), np.sort(want))
+    per_leaf = 32
+    over = sum(max(0, c - 1 - i - per_leaf) for w in range(worlds) for c in [np.sum(world == w)] for i in range(c))
+    assert pipe.pass_stats()["trav_overflow"] == over
+    pipe.close()
