@@ -459,6 +459,17 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 			rc = fail(c, B3G_E_CUDA, "%s: %s", what, cudaGetErrorString(e));
 	};
 	step(cudaSetDevice(cfg->device), "cudaSetDevice");
+	if (rc == B3G_OK)
+	{
+		carveout_api();
+		carveout_broadphase();
+		carveout_pairs();
+		carveout_order();
+		carveout_narrow_convex();
+		carveout_narrow_hulls();
+		carveout_mesh();
+		carveout_solver_input();
+	}
 	step(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate");
 	step(cudaStreamCreateWithFlags(&c->copyStream, cudaStreamNonBlocking), "cudaStreamCreate");
 	step(cudaEventCreateWithFlags(&c->copyReady, cudaEventDisableTiming), "cudaEventCreate");
@@ -2896,4 +2907,10 @@ extern "C" int b3g_autotune(b3g_ctx* c, uint32_t reps, void* stream, uint32_t* o
 		for (int k = 0; k < B3G_TUNE_COUNT; ++k)
 			out[k] = c->tune.v[k];
 	return B3G_OK;
+}
+
+void carveout_api()
+{
+	set_carveout({
+		(const void*)k_pass_begin, (const void*)k_pack_sizes, (const void*)k_pack_scatter});
 }

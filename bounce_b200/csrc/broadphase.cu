@@ -784,7 +784,7 @@ __device__ __forceinline__ uint2 canon_pair_keys(uint32_t pa, uint32_t keyA, uin
 // MW: several worlds share the tree. They are contiguous in its order, so a
 // right child past the last leaf of the query's world is not entered; its
 // first leaf is its own index (a left child begins where its parent does).
-constexpr uint32_t WALK_STACK = 256;
+constexpr uint32_t WALK_STACK = 128; // 256: 1 % longer, for the shared memory it takes from the others
 struct WalkWarp
 {
 	uint32_t left[WALK_STACK], right[WALK_STACK]; // children of the nodes to search
@@ -1224,4 +1224,14 @@ void launch_traverse(b3g_ctx* c, cudaStream_t s)
 	auto* walk = c->nWorlds > 1 ? (c->walkLimit ? k_traverse<true, true> : k_traverse<true, false>)
 								: (c->walkLimit ? k_traverse<false, true> : k_traverse<false, false>);
 	walk<<<blocks, tb, smem, s>>>(c->scene, B, (uint32_t)n, leaves, c->cfg.max_contacts, c->walkLimit);
+}
+
+void carveout_broadphase()
+{
+	set_carveout({
+		(const void*)k_sync, (const void*)k_bounds_init, (const void*)k_bounds, (const void*)k_morton,
+		(const void*)k_os_hist, (const void*)k_os_scan, (const void*)k_onesweep, (const void*)k_build,
+		(const void*)k_leaves, (const void*)k_refit, (const void*)k_traverse<false, false>,
+		(const void*)k_traverse<false, true>, (const void*)k_traverse<true, false>,
+		(const void*)k_traverse<true, true>, (const void*)k_scan_tiles});
 }

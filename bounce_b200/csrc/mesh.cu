@@ -1032,3 +1032,9 @@ uint32_t mesh_launches(const b3g_ctx* c)
 	// sync with the work items; two evaluation kernels, cluster
 	return c->nMeshFix ? 1 + 2 + 1 : 0;
 }
+
+void carveout_mesh()
+{
+	set_carveout({
+		(const void*)k_mesh_sync, (const void*)k_mesh_cluster});
+}

@@ -936,7 +936,11 @@ __device__ __forceinline__ void load_hull_ctx(const NPArgs& a, uint32_t c, HullC
 
 constexpr int PROBE_THREADS = 128;
 constexpr int PROBE_BLOCKS = 4;
-constexpr uint32_t CLIP_SLOTS = 16; // a power of two
+// A power of two. Faces have 3 or 4 vertices and gain one per side plane that
+// cuts them; with 16 slots the rings fill the SM's shared memory: three contexts
+// at once took 415 us a pass of 65,536 mixed bodies and 879 of 512 worlds, with
+// 8 they take 392 and 831, though more polygons are left to build_face_contact.
+constexpr uint32_t CLIP_SLOTS = 8;
 
 // A thread's clip polygon: a ring of vertices in shared memory, one column of
 // words per thread. A vertex's edge pair takes two words of two 16-bit edges
@@ -1828,4 +1832,13 @@ void launch_mesh_items_hull(const NPArgs& a, const Buffers& B, uint32_t maxUE, c
 	uint32_t ue = maxUE > 3 ? maxUE : 3;
 	// As many blocks as 128 registers allow (with 80 or 255 it takes longer).
 	k_mesh_items_hull<4><<<persistent_blocks(4), 128, 4 * sat_triangle_warp_bytes(), s>>>(a, B, ue);
+}
+
+void carveout_narrow_hulls()
+{
+	set_carveout({
+		(const void*)k_hulls_probe, (const void*)k_hulls_sat<2, true>, (const void*)k_hulls_sat<4, true>,
+		(const void*)k_hulls_sat<8, true>, (const void*)k_hulls_sat<2, false>, (const void*)k_hulls_sat<4, false>,
+		(const void*)k_hulls_sat<8, false>, (const void*)k_hull_triangle<2>, (const void*)k_hull_triangle<4>,
+		(const void*)k_hull_triangle<8>, (const void*)k_mesh_items_hull<4>});
 }

@@ -610,3 +610,10 @@ int resolve_wakeups(b3g_ctx* c, cudaStream_t s)
 	c->launches += launches;
 	return cudaGetLastError() == cudaSuccess ? B3G_OK : B3G_E_CUDA;
 }
+
+void carveout_order()
+{
+	set_carveout({
+		(const void*)k_order_scan, (const void*)k_new_scatter, (const void*)k_place, (const void*)k_wake_events,
+		(const void*)k_wake_activate, (const void*)k_awake_out});
+}

@@ -521,3 +521,9 @@ void launch_finalize(b3g_ctx* c, cudaStream_t s)
 	k_finalize<<<work_blocks(std::max(c->cfg.max_contacts, c->nFixtures), FIN_THREADS, 4), FIN_THREADS, 0, s>>>(c->scene, c->buf, c->cur, c->cfg.max_contacts,
 		c->nFixtures);
 }
+
+void carveout_pairs()
+{
+	set_carveout({
+		(const void*)k_diff, (const void*)k_bucket, (const void*)k_finalize});
+}

@@ -659,3 +659,9 @@ void launch_contact_constraints(b3g_ctx* c, const ConstraintCall& q, cudaStream_
 	const uint32_t most = q.list ? q.listCount : c->cfg.max_contacts;
 	k_contact_constraints<<<work_blocks(most, 8 * CC_WARPS, CC_BLOCKS), CC_WARPS * 32, 0, s>>>(a, tiles);
 }
+
+void carveout_solver_input()
+{
+	set_carveout({
+		(const void*)k_constraint_items, (const void*)k_contact_constraints});
+}

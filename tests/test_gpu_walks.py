@@ -207,7 +207,7 @@ def prism(n, radius, height):
 
 # A pair at rest: the pass that finds the contact builds it from the separating
 # axes (a warp per contact), the next rebuilds it from the feature cache (a
-# lane per contact, rings of 16 clip vertices), and both give the same points.
+# lane per contact, rings of a few clip vertices), and both give the same points.
 # Faces below, at and beyond what a ring holds; more pairs than a block takes.
 @pytest.mark.parametrize("sides", [(3, 3), (4, 4), (4, 9), (3, 15), (15, 3), (16, 4), (8, 16), (17, 4), (30, 30),
                                    (4, 40)])
