@@ -278,6 +278,8 @@ __device__ __forceinline__ bool joint_excluded(const FilterArgs& F, uint32_t ba,
 
 // The pairs of one leaf after which CTR_TRAV_OVERFLOW counts the rest.
 #define B3G_TRAV_SLOTS 32u
+// Each of the pinned buffers of reserve_stage.
+#define B3G_STAGE_BYTES ((size_t)1 << 18)
 
 // Counter slots in Buffers::counters.
 enum
@@ -292,26 +294,30 @@ enum
 	CTR_MOVED,
 	CTR_STATUS,
 	CTR_TOUCH_OUT,
-	CTR_HULL_MISS,      // hull-hull contacts the feature cache did not resolve
 	CTR_RAW,            // overlapping pairs found by the traversal
 	CTR_KEPT,           // previous contacts kept
 	CTR_WAKE_EVENTS,
-	CTR_WAKE_ACTIVATED,
 	CTR_LATE_DESTROYED,
 	CTR_BUCKET0 = 16,   // BK_COUNT bucket sizes
-	CTR_ASLEEP = 29,    // non-static bodies still asleep after the wake-ups
-	CTR_SCRATCH = 30,
-	CTR_MESH_PAIRS = 31, // (contact, triangle) work items of the pass
-	CTR_TRAV_OVERFLOW = 32, // pairs of a leaf past its first B3G_TRAV_SLOTS
-	CTR_CANDIDATES = 33,    // new pairs handed to the caller's contact filter
-	CTR_HC_POST = 34,       // hull-capsule contacts past their GJK (k_hull_capsule_post): at a distance
-	CTR_HC_DEEP = 35,       // ... and overlapping
-	CTR_HS_POST = 36,       // hull-sphere contacts past their face scan (k_hull_sphere_gjk)
-	CTR_MESH_ALL = 37,      // mesh contacts of the pass, skipped ones included
-	CTR_WALK_TURNED = 38,   // a triangle fixture lies outside its box (queries.cu)
-	CTR_COUNT = 39
+	// The buckets and the counters up to CTR_ASLEEP start at 0 in each wake-up
+	// round (order.cu).
+	CTR_HULL_MISS = CTR_BUCKET0 + BK_COUNT, // hull-hull contacts the feature cache did not resolve
+	CTR_HC_POST,        // hull-capsule contacts past their GJK (k_hull_capsule_post): at a distance
+	CTR_HC_DEEP,        // ... and overlapping
+	CTR_HS_POST,        // hull-sphere contacts past their face scan (k_hull_sphere_gjk)
+	CTR_WAKE_ACTIVATED,
+	CTR_ASLEEP,         // non-static bodies still asleep after the wake-ups
+	CTR_SCRATCH,
+	CTR_MESH_PAIRS,     // (contact, triangle) work items of the pass
+	CTR_TRAV_OVERFLOW,  // pairs of a leaf past its first B3G_TRAV_SLOTS
+	CTR_CANDIDATES,     // new pairs handed to the caller's contact filter
+	CTR_MESH_ALL,       // mesh contacts of the pass, skipped ones included
+	CTR_WALK_TURNED,    // a triangle fixture lies outside its box (queries.cu)
+	CTR_WAKE_INACTIVE,  // contacts the pass skipped as inactive
+	CTR_WAKE_SAVE,      // the counters from CTR_BUCKET0 to CTR_WAKE_ACTIVATED as the pass left them
+	CTR_COUNT = CTR_WAKE_SAVE + (CTR_WAKE_ACTIVATED - CTR_BUCKET0) + 1
 };
-static_assert(CTR_BUCKET0 + BK_COUNT <= CTR_ASLEEP, "bucket counters overlap");
+static_assert(CTR_LATE_DESTROYED < CTR_BUCKET0, "named counters overlap the buckets");
 
 // Launch shapes of the tunable kernels (include/b3g.h, B3G_TUNE_*).
 #define B3G_CONVEX_KERNELS 9
@@ -359,7 +365,12 @@ struct b3g_ctx
 	cudaEvent_t copyReady;    // results of the pass ready to copy
 	cudaEvent_t copyDone;     // those copies finished
 	bool copyPending;
-	uint32_t* touchBytes;     // per contact: packed bytes of its manifolds
+	uint2* packList;          // b3g_fetch_results_packed_async: manifolds with points (k_pack_list)
+	unsigned long long* packStates; // ... its scan's states, 0 between calls
+	cudaEvent_t countsReady;  // the last fetch's counts are on the host
+	bool countsFetched;       // hCounters are those of the last pass, which has ended
+	char *stageOut, *stageImpulses, *stageAwake; // pinned, B3G_STAGE_BYTES each (allocated on first use)
+	cudaEvent_t impulsesStaged, awakeStaged;     // the copies from them
 	void* edgeBuf;            // b3g_fetch_fixture_contacts scratch (allocated on first use)
 	size_t edgeBytes;
 	cudaStream_t sideStream;  // hull-hull / hull-triangle narrowphase, beside the convex buckets
@@ -421,6 +432,7 @@ struct b3g_ctx
 	uint32_t* dUpdateBad;        // a device-side scene update skipped invalid records
 	bool fixTypeStale;           // hFixType lags device-side scene updates
 	std::vector<uint8_t> hAwake; // host copy of the awake flags (sleep count)
+	uint32_t awakeStale;         // its first flags that the last pass may have changed (refresh_awake)
 	float4* dFixParams;
 	float4* dFixBound;
 

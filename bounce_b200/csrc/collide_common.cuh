@@ -977,6 +977,7 @@ void launch_convex_buckets(const NPArgs& base, const uint32_t* lists, const uint
 	const Tune& tune, cudaStream_t s);
 void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap,
 	const Tune& tune, cudaStream_t s);
+constexpr int CONVEX_HULL_CAPSULE = 6, CONVEX_INACTIVE = 8;
 // Whether convex bucket kernel k (the order of B3G_TUNE_CONVEX) can have
 // contacts in this context's pass: the triangle buckets need triangle
 // fixtures, the sensor bucket sensors, the inactive bucket a sleeping body.

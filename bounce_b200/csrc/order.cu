@@ -324,13 +324,38 @@ __device__ __forceinline__ bool woken_before(const DevScene& S, const Buffers& B
 	return S.bodyType[body] != B3G_BODY_STATIC && B.tWake[body] < pos;
 }
 
+// Before the rounds: nobody woken, the skipped contacts set aside (the bucket
+// lists are reused for the contacts each round activates).
+__global__ void k_wake_begin(Buffers B, uint32_t cap, uint32_t nb)
+{
+	const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+	const uint32_t nInactive = B.counters[CTR_BUCKET0 + BK_INACTIVE], n = min(B.counters[CTR_PAIRS], cap);
+	for (uint32_t b = first; b < nb; b += stride)
+		B.tWake[b] = 0xFFFFFFFFu;
+	for (uint32_t t = first; t < nInactive; t += stride)
+	{
+		B.inactiveSave[t] = B.bucketList[(size_t)BK_INACTIVE * cap + t];
+		B.activated[t] = 0;
+	}
+	for (uint32_t c = first; c < n; c += stride)
+		B.lateDestroyed[c] = 0;
+	if (first <= CTR_WAKE_ACTIVATED - CTR_BUCKET0)
+		B.counters[CTR_WAKE_SAVE + first] = B.counters[CTR_BUCKET0 + first];
+	if (first == 0)
+		B.counters[CTR_WAKE_INACTIVE] = nInactive;
+}
+
 // Skipped contacts whose body was woken at an earlier list position become
 // active: a contact whose pair still overlaps runs the narrowphase (appended
 // to the bucket lists and to wakeList), a retained one whose pair does not is
-// destroyed now and wakes its bodies if it had points.
-__global__ void k_wake_activate(DevScene S, Buffers B, uint32_t cur, uint32_t cap, uint32_t nInactive)
+// destroyed now and wakes its bodies if it had points. Also counts the bodies
+// still asleep, which holds once no contact changes any more.
+__global__ void k_wake_activate(DevScene S, Buffers B, uint32_t cur, uint32_t cap, uint32_t nb)
 {
-	uint32_t events = 0;
+	uint32_t events = 0, asleep = 0;
+	const uint32_t nInactive = B.counters[CTR_WAKE_INACTIVE];
+	for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
+		asleep += S.bodyAwake[b] == 0 && B.tWake[b] == 0xFFFFFFFFu && S.bodyType[b] != B3G_BODY_STATIC ? 1u : 0u;
 	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nInactive; t += gridDim.x * blockDim.x)
 	{
 		if (B.activated[t])
@@ -368,27 +393,21 @@ __global__ void k_wake_activate(DevScene S, Buffers B, uint32_t cur, uint32_t ca
 		B.wakeList[w] = c;
 	}
 	for (int o = 16; o > 0; o >>= 1)
+	{
 		events += __shfl_xor_sync(0xffffffffu, events, o);
+		asleep += __shfl_xor_sync(0xffffffffu, asleep, o);
+	}
 	if ((threadIdx.x & 31) == 0 && events)
 		atomicAdd(&B.counters[CTR_WAKE_EVENTS], events);
-}
-
-// Awake flags after the pass (written back for the next pass) and the count
-// of non-static bodies still asleep.
-__global__ void k_awake_out(DevScene S, Buffers B, uint8_t* awake, uint32_t nb)
-{
-	uint32_t asleep = 0;
-	for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
-	{
-		uint8_t on = (S.bodyAwake[b] != 0 || B.tWake[b] != 0xFFFFFFFFu) ? 1 : 0;
-		awake[b] = on;
-		if (!on && S.bodyType[b] != B3G_BODY_STATIC)
-			++asleep;
-	}
-	for (int o = 16; o > 0; o >>= 1)
-		asleep += __shfl_xor_sync(0xffffffffu, asleep, o);
 	if ((threadIdx.x & 31) == 0 && asleep)
 		atomicAdd(&B.counters[CTR_ASLEEP], asleep);
+}
+
+// Awake flags after the pass, written back for the next pass.
+__global__ void k_awake_out(DevScene S, Buffers B, uint8_t* awake, uint32_t nb)
+{
+	for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
+		awake[b] = (S.bodyAwake[b] != 0 || B.tWake[b] != 0xFFFFFFFFu) ? 1 : 0;
 }
 
 // Compaction after late destructions: keep flags without them (into kept2).
@@ -495,65 +514,64 @@ uint32_t order_launches(const b3g_ctx*)
 }
 
 // Host-driven replay of the wake-ups; runs only when some non-static body is
-// asleep at the start of the pass. Reads the counters back once per round.
+// asleep at the start of the pass. The host waits once per round, and the first
+// round is issued with the events that start it: a pass whose events wake
+// nobody else waits once, one with a round of activated contacts twice (three
+// and five times when each step waited for its own count).
 int resolve_wakeups(b3g_ctx* c, cudaStream_t s)
 {
 	Buffers& B = c->buf;
-	const uint32_t cap = c->cfg.max_contacts, cur = c->cur;
+	const uint32_t cap = c->cfg.max_contacts, cur = c->cur, nb = c->nBodies;
 	uint32_t launches = 0;
-	uint32_t h[CTR_COUNT];
+	const uint32_t* h = c->hCounters;
 	auto fetch = [&]() -> bool {
-		return cudaMemcpyAsync(h, B.counters, sizeof(h), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+		return cudaMemcpyAsync(c->hCounters, B.counters, sizeof(uint32_t) * CTR_COUNT, cudaMemcpyDeviceToHost, s) ==
+			cudaSuccess &&
 			cudaStreamSynchronize(s) == cudaSuccess;
 	};
-	cudaMemsetAsync(B.tWake, 0xFF, sizeof(uint32_t) * c->nBodies, s);
-	k_wake_events<<<persistent_blocks(4), 256, 0, s>>>(c->scene, B, cur, cap, nullptr, nullptr,
-		c->havePass ? 1 : 0);
-	++launches;
-	if (!fetch())
-		return B3G_E_CUDA;
-	const uint32_t nInactive = h[CTR_BUCKET0 + BK_INACTIVE];
+	const int most = work_blocks(std::max(cap, nb), 256, 4);
+	k_wake_begin<<<most, 256, 0, s>>>(B, cap, nb);
+	k_wake_events<<<most, 256, 0, s>>>(c->scene, B, cur, cap, nullptr, nullptr, c->havePass ? 1 : 0);
+	launches += 2;
 	uint32_t late = 0;
-	if (h[CTR_WAKE_EVENTS] != 0 && nInactive != 0)
+	NPArgs a = make_np_args(c);
+	// Every round but the last activates at least one skipped contact.
+	for (uint32_t round = 0;; ++round)
 	{
-		// The bucket lists are reused for the contacts each round activates.
-		cudaMemcpyAsync(B.inactiveSave, B.bucketList + (size_t)BK_INACTIVE * cap, sizeof(uint32_t) * nInactive,
-			cudaMemcpyDeviceToDevice, s);
-		cudaMemsetAsync(B.activated, 0, sizeof(uint32_t) * nInactive, s);
-		cudaMemsetAsync(B.lateDestroyed, 0, sizeof(uint32_t) * cap, s);
-		NPArgs a = make_np_args(c);
-		// Every round but the last activates at least one skipped contact.
-		for (uint32_t round = 0; round <= nInactive; ++round)
+		cudaMemsetAsync(B.counters + CTR_BUCKET0, 0, sizeof(uint32_t) * (CTR_ASLEEP - CTR_BUCKET0 + 1), s);
+		k_wake_activate<<<most, 256, 0, s>>>(c->scene, B, cur, cap, nb);
+		++launches;
+		if (!fetch())
+			return B3G_E_CUDA;
+		const uint32_t act = h[CTR_WAKE_ACTIVATED];
+		const bool lateNow = h[CTR_LATE_DESTROYED] != late;
+		late = h[CTR_LATE_DESTROYED];
+		if ((act == 0 && !lateNow) || round > h[CTR_WAKE_INACTIVE])
+			break;
+		if (act)
 		{
-			cudaMemsetAsync(B.counters + CTR_BUCKET0, 0, sizeof(uint32_t) * BK_COUNT, s);
-			cudaMemsetAsync(B.counters + CTR_WAKE_ACTIVATED, 0, sizeof(uint32_t), s);
-			cudaMemsetAsync(B.counters + CTR_HULL_MISS, 0, sizeof(uint32_t), s);
-			reset_post_counts(B, s);
-			k_wake_activate<<<persistent_blocks(4), 256, 0, s>>>(c->scene, B, cur, cap, nInactive);
-			++launches;
-			if (!fetch())
-				return B3G_E_CUDA;
-			const uint32_t act = h[CTR_WAKE_ACTIVATED];
-			const bool lateNow = h[CTR_LATE_DESTROYED] != late;
-			late = h[CTR_LATE_DESTROYED];
-			if (act == 0 && !lateNow)
-				break;
-			if (act)
-			{
-				launch_convex_buckets(a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
-				launch_hulls(a, B.bucketList + (size_t)BK_HULLS * cap, B.counters + CTR_BUCKET0 + BK_HULLS,
-					c->maxUniqueEdges, c->tune, s);
+			for (int k = 0; k < B3G_CONVEX_KERNELS; ++k)
+				if (k != CONVEX_INACTIVE && convex_bucket_possible(c, k))
+				{
+					launch_convex_one(k, a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
+					++launches;
+				}
+			launch_hulls(a, B.bucketList + (size_t)BK_HULLS * cap, B.counters + CTR_BUCKET0 + BK_HULLS,
+				c->maxUniqueEdges, c->tune, s);
+			if (c->anyTriangle)
 				launch_hull_triangles(a, B.bucketList + (size_t)BK_HULL_TRIANGLE * cap,
 					B.counters + CTR_BUCKET0 + BK_HULL_TRIANGLE, c->maxUniqueEdges, c->tune, s);
-				launch_mesh_collide(c, B.bucketList + (size_t)BK_MESH * cap, B.counters + CTR_BUCKET0 + BK_MESH, s);
-				launches += c->nMeshFix ? 3 : 0;
-				k_wake_events<<<persistent_blocks(4), 256, 0, s>>>(c->scene, B, cur, cap, B.wakeList,
-					B.counters + CTR_WAKE_ACTIVATED, 0);
-				launches += B3G_CONVEX_KERNELS + 2 + 1 + 1;
-			}
+			launch_mesh_collide(c, B.bucketList + (size_t)BK_MESH * cap, B.counters + CTR_BUCKET0 + BK_MESH, s);
+			k_wake_events<<<most, 256, 0, s>>>(c->scene, B, cur, cap, B.wakeList, B.counters + CTR_WAKE_ACTIVATED, 0);
+			launches += 2 + (c->anyTriangle ? 1 : 0) + (c->nMeshFix ? 3 : 0) + 1;
 		}
-		cudaMemsetAsync(B.counters + CTR_BUCKET0, 0, sizeof(uint32_t) * BK_COUNT, s);
 	}
+	// The work lists are the pass's own where no skipped contact could wake,
+	// and gone where the rounds went through them.
+	if (h[CTR_WAKE_EVENTS] == 0 || h[CTR_WAKE_INACTIVE] == 0)
+		cudaMemcpyAsync(B.counters + CTR_BUCKET0, B.counters + CTR_WAKE_SAVE,
+			sizeof(uint32_t) * (CTR_WAKE_ACTIVATED - CTR_BUCKET0 + 1), cudaMemcpyDeviceToDevice, s);
+	c->asleep = h[CTR_ASLEEP];
 	if (late)
 	{
 		// Rare: a retained contact whose pair no longer overlaps was destroyed
@@ -593,17 +611,11 @@ int resolve_wakeups(b3g_ctx* c, cudaStream_t s)
 		k_set_counts<<<1, 1, 0, s>>>(B, total, np - kept2Total);
 		launches += 1 + 3 + 1 + 1 + 1 + 1;
 	}
-	cudaMemsetAsync(B.counters + CTR_ASLEEP, 0, sizeof(uint32_t), s);
 	const int nbBlocks = (int)std::min<uint32_t>((c->nBodies + 255) / 256, 148u * 4u);
 	k_awake_out<<<nbBlocks, 256, 0, s>>>(c->scene, B, c->dBodyAwake, c->nBodies);
 	++launches;
-	if (!fetch())
-		return B3G_E_CUDA;
-	c->asleep = h[CTR_ASLEEP];
+	c->awakeStale = std::max(c->awakeStale, c->nBodies);
 	// Bodies past the processed prefix keep their flags.
-	if (c->hAwake.size() >= c->nBodies &&
-		cudaMemcpy(c->hAwake.data(), c->dBodyAwake, c->nBodies, cudaMemcpyDeviceToHost) != cudaSuccess)
-		return B3G_E_CUDA;
 	for (uint32_t b = c->nBodies; b < c->hAwake.size(); ++b)
 		if (c->hAwake[b] == 0 && c->hBodyType[b] != B3G_BODY_STATIC)
 			++c->asleep;

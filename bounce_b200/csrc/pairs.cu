@@ -428,7 +428,6 @@ NPArgs make_np_args(b3g_ctx* c)
 	return a;
 }
 
-constexpr int CONVEX_HULL_CAPSULE = 6; // launch_convex_one
 
 void launch_narrowphase(b3g_ctx* c, cudaStream_t s)
 {

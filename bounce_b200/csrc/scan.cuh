@@ -132,3 +132,91 @@ __device__ __forceinline__ void scan_tile(const Load& load, uint32_t* out, uint3
 		run += v[r];
 	}
 }
+
+// The same over pairs of counts packed in a u64 (the first in bits 32 and up,
+// below 2^30). Tile status words: state in bits 62-63, the pair below.
+constexpr unsigned long long SC_PAIR = SC_AGG - 1ull;
+
+// Block-wide exclusive scan of one u64 per thread; returns the thread's
+// exclusive prefix and leaves the block total in *total.
+__device__ __forceinline__ unsigned long long block_scan(unsigned long long v, unsigned long long* total)
+{
+	__shared__ unsigned long long warpSum[SC_THREADS / 32];
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	unsigned long long x = v;
+	for (int off = 1; off < 32; off <<= 1)
+	{
+		unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+		if (lane >= (uint32_t)off)
+			x += y;
+	}
+	if (lane == 31)
+		warpSum[warp] = x;
+	__syncthreads();
+	if (warp == 0)
+	{
+		unsigned long long w = lane < SC_THREADS / 32 ? warpSum[lane] : 0ull;
+		for (int off = 1; off < 32; off <<= 1)
+		{
+			unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, w, off);
+			if (lane >= (uint32_t)off)
+				w += y;
+		}
+		if (lane < SC_THREADS / 32)
+			warpSum[lane] = w;
+	}
+	__syncthreads();
+	unsigned long long before = warp ? warpSum[warp - 1] : 0ull;
+	*total = warpSum[SC_THREADS / 32 - 1];
+	return before + x - v;
+}
+
+// Called by the first warp of a block: publishes tile's total and returns the
+// sum of the tiles before it; st: the status words, 0 before the launch.
+__device__ __forceinline__ unsigned long long look_back_pairs(volatile unsigned long long* st, uint32_t tile,
+	unsigned long long total, bool& timedOut)
+{
+	const uint32_t lane = threadIdx.x & 31u;
+	unsigned long long prefix = 0;
+	if (tile == 0)
+	{
+		if (lane == 0)
+			st[0] = SC_INC | total;
+		return prefix;
+	}
+	if (lane == 0)
+		st[tile] = SC_AGG | total;
+	int32_t hi = (int32_t)tile - 1;
+	uint32_t spins = 0;
+	while (true)
+	{
+		const int32_t idx = hi - (int32_t)lane;
+		const unsigned long long v = idx >= 0 ? (unsigned long long)st[idx] : (unsigned long long)SC_INC;
+		const uint32_t notReady = __ballot_sync(0xFFFFFFFFu, (v & ~SC_PAIR) == 0ull);
+		const uint32_t inc = __ballot_sync(0xFFFFFFFFu, (v & SC_INC) != 0ull);
+		const uint32_t last = inc ? (uint32_t)__ffs(inc) - 1u : 31u;
+		const uint32_t need = last == 31u ? 0xFFFFFFFFu : (2u << last) - 1u;
+		if (notReady & need)
+		{
+			if (++spins > SC_SPIN)
+			{
+				timedOut = true;
+				break;
+			}
+			continue;
+		}
+		unsigned long long part = lane <= last ? (v & SC_PAIR) : 0ull;
+		for (int off = 16; off > 0; off >>= 1)
+			part += __shfl_xor_sync(0xFFFFFFFFu, part, off);
+		prefix += part;
+		if (inc)
+			break;
+		hi -= 32;
+	}
+	if (lane == 0)
+	{
+		__threadfence();
+		st[tile] = SC_INC | (prefix + total);
+	}
+	return prefix;
+}

@@ -25,6 +25,7 @@
 // Every expression keeps the reference's operand order (the library is built
 // with -fmad=false), so the records are the reference's bit for bit.
 #include "collide_common.cuh"
+#include "scan.cuh"
 
 static_assert(sizeof(b3g_solver_body) == 112, "b3g_solver_body: 7 float4");
 static_assert(sizeof(b3g_contact_constraint) == 128, "b3g_contact_constraint: 8 float4");
@@ -32,15 +33,9 @@ static_assert(sizeof(b3g_manifold_constraint) == 464, "b3g_manifold_constraint: 
 
 namespace {
 
-constexpr int CI_BLOCK = 256;
+constexpr int CI_BLOCK = SC_THREADS;
 constexpr int CI_ITEMS = 4;
 constexpr uint32_t CI_TILE = CI_BLOCK * CI_ITEMS;
-// Tile status words: state in bits 62-63, (constraints << 32 | manifolds) below.
-constexpr unsigned long long CI_AGG = 1ull << 62;
-constexpr unsigned long long CI_INC = 2ull << 62;
-constexpr unsigned long long CI_VAL = CI_AGG - 1ull;
-constexpr uint32_t CI_SPIN = 1u << 22;
-
 struct CIArgs
 {
 	const uint32_t* pairA;
@@ -122,40 +117,6 @@ __device__ __forceinline__ Item item_counts(const CIArgs& a, uint32_t i, uint32_
 	it.ba = a.fixBody[fa];
 	it.bb = a.fixBody[fb];
 	return it;
-}
-
-// Block-wide exclusive scan of one u64 per thread; returns the thread's
-// exclusive prefix and leaves the block total in *total.
-__device__ __forceinline__ unsigned long long block_scan(unsigned long long v, unsigned long long* total)
-{
-	__shared__ unsigned long long warpSum[CI_BLOCK / 32];
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	unsigned long long x = v;
-	for (int off = 1; off < 32; off <<= 1)
-	{
-		unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, off);
-		if (lane >= (uint32_t)off)
-			x += y;
-	}
-	if (lane == 31)
-		warpSum[warp] = x;
-	__syncthreads();
-	if (warp == 0)
-	{
-		unsigned long long w = lane < CI_BLOCK / 32 ? warpSum[lane] : 0ull;
-		for (int off = 1; off < 32; off <<= 1)
-		{
-			unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, w, off);
-			if (lane >= (uint32_t)off)
-				w += y;
-		}
-		if (lane < CI_BLOCK / 32)
-			warpSum[lane] = w;
-	}
-	__syncthreads();
-	unsigned long long before = warp ? warpSum[warp - 1] : 0ull;
-	*total = warpSum[CI_BLOCK / 32 - 1];
-	return before + x - v;
 }
 
 // b3g_solver_body as 7 float4: (x, q0) (q1 q2 q3, v0) (v1 v2, w0 w1)
@@ -459,55 +420,8 @@ __global__ void __launch_bounds__(CI_BLOCK) k_constraint_items(CIArgs a)
 		unsigned long long run = block_scan(sum, &total);
 		if (t < 32)
 		{
-			// Publish the tile's counts, then look back 32 tiles at a time:
-			// the counts of the tiles up to the nearest one holding its
-			// inclusive prefix (tiles before the first count as such a tile
-			// holding 0).
-			volatile unsigned long long* st = a.tileState + 1;
-			unsigned long long prefix = 0;
 			bool timedOut = false;
-			if (tile == 0)
-			{
-				if (lane == 0)
-					st[0] = CI_INC | total;
-			}
-			else
-			{
-				if (lane == 0)
-					st[tile] = CI_AGG | total;
-				int32_t hi = (int32_t)tile - 1;
-				uint32_t spins = 0;
-				while (true)
-				{
-					const int32_t idx = hi - (int32_t)lane;
-					const unsigned long long v = idx >= 0 ? (unsigned long long)st[idx] : (unsigned long long)CI_INC;
-					const uint32_t notReady = __ballot_sync(0xFFFFFFFFu, (v & ~CI_VAL) == 0ull);
-					const uint32_t inc = __ballot_sync(0xFFFFFFFFu, (v & CI_INC) != 0ull);
-					const uint32_t last = inc ? (uint32_t)__ffs(inc) - 1u : 31u;
-					const uint32_t need = last == 31u ? 0xFFFFFFFFu : (2u << last) - 1u;
-					if (notReady & need)
-					{
-						if (++spins > CI_SPIN)
-						{
-							timedOut = true;
-							break;
-						}
-						continue;
-					}
-					unsigned long long part = lane <= last ? (v & CI_VAL) : 0ull;
-					for (int off = 16; off > 0; off >>= 1)
-						part += __shfl_xor_sync(0xFFFFFFFFu, part, off);
-					prefix += part;
-					if (inc)
-						break;
-					hi -= 32;
-				}
-				if (lane == 0)
-				{
-					__threadfence();
-					st[tile] = CI_INC | (prefix + total);
-				}
-			}
+			const unsigned long long prefix = look_back_pairs(a.tileState + 1, tile, total, timedOut);
 			if (lane == 0)
 			{
 				sPrefix = prefix;

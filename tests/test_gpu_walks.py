@@ -271,3 +271,48 @@ def test_pairs_of_heaped_worlds(n, worlds):
     over = sum(max(0, c - 1 - i - per_leaf) for w in range(worlds) for c in [np.sum(world == w)] for i in range(c))
     assert pipe.pass_stats()["trav_overflow"] == over
     pipe.close()
+
+
+# The packed results and the impulses of worlds on both sides of what travels
+# through the small pinned buffers (256 KB), to pageable and to pinned memory;
+# mesh contacts bring contacts of several manifolds.
+@pytest.mark.parametrize("kind,n", [("mixed", 1), ("mixed", 40), ("mixed", 900), ("mixed", 9000), ("mesh", 700)])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_results_through_small_buffers(kind, n, pinned):
+    torch = pytest.importorskip("torch")
+    sc = world(kind, n)
+    pipe = CollisionPipeline(sc, max_contacts=max(40 * sc.n_fixtures, 64))
+    drv = S.KinematicDriver(sc)
+    cap = 4 * sc.n_fixtures + 64
+    make = lambda shape, dt: torch.zeros(shape, dtype=dt, pin_memory=pinned).numpy()
+    contacts = make((40 * sc.n_fixtures + 64, 3), torch.int32).view(np.uint32)
+    index, packed = make((cap,), torch.int32).view(np.uint32), make((cap * 320,), torch.uint8)
+    rng = np.random.default_rng(n)
+    for k in range(3):
+        pipe.collide(drv.state17())
+        c = pipe.fetch_results_packed_async(contacts, index, packed)
+        pipe.wait_results()
+        assert np.array_equal(contacts[: c["contacts"]], pipe.contacts())
+        want_index, want = pipe.touching()
+        assert np.array_equal(index[: c["manifolds"]], want_index)
+        at = 0
+        for m in want:
+            points = int(m["pointCount"])
+            assert packed[at : at + 32].tobytes() == m.tobytes()[288:]
+            assert packed[at + 32 : at + 32 + 72 * points].tobytes() == m["points"][:points].tobytes()
+            at += 32 + 72 * points
+        assert at == 32 * c["manifolds"] + 72 * c["points"]
+        # What the solver hands back reaches the next pass's first manifolds.
+        c0 = pipe.contacts()[:, :2]
+        imp = rng.uniform(0, 1, len(c0)).astype(np.float32)
+        pipe.load_impulses(np.zeros((len(c0), 4), np.float32), np.zeros((len(c0), 2), np.float32), imp)
+        pipe.collide(drv.state17())
+        flags = pipe.contacts()
+        man = pipe.manifolds()
+        old = {tuple(p): float(x) for p, x in zip(c0.tolist(), imp)}
+        both = [(float(m["motorImpulse"]), old[tuple(p[:2])]) for p, m in zip(flags.tolist(), man)
+                if tuple(p[:2]) in old and not p[2] & 2 and m["pointCount"] and sc.fix_type[p[0]] != N.SHAPE_MESH
+                and sc.fix_type[p[1]] != N.SHAPE_MESH]
+        assert all(a == b for a, b in both) and (both or n < 100)
+        drv.advance()
+    pipe.close()
