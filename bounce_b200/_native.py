@@ -194,6 +194,14 @@ assert TOI_INPUT_DTYPE.itemsize == 272 and GJK_CAST_DTYPE.itemsize == 192
 assert SOLVER_BODY_DTYPE.itemsize == 112 and CONTACT_CONSTRAINT_DTYPE.itemsize == 128
 assert MANIFOLD_CONSTRAINT_DTYPE.itemsize == 464
 
+
+class WorldTemplates(ctypes.Structure):
+    """b3g_world_templates (include/b3g.h)."""
+
+    _fields_ = [(k, ctypes.c_void_p) for k in ("body_type", "fixture_body", "shape_type", "hull", "flags", "params",
+                                               "state", "motion")]
+
+
 EXPORTED = [
     "b3g_create",
     "b3g_destroy",
@@ -254,6 +262,7 @@ EXPORTED = [
     "b3g_set_active",
     "b3g_world_counts",
     "b3g_kinematic_step",
+    "b3g_swap_worlds",
     "b3g_set_tuning",
     "b3g_get_tuning",
     "b3g_hull_from_points",
@@ -347,6 +356,8 @@ def load():
                                      ctypes.c_uint32, vp, vp], ctypes.c_int),
         "b3g_set_active": ([ctx, ctypes.c_uint32, ctypes.c_uint32], ctypes.c_int),
         "b3g_world_counts": ([ctx, ctypes.c_uint32, vp, vp], ctypes.c_int),
+        "b3g_swap_worlds": ([ctx, ctypes.c_uint32, vp, ctypes.c_uint32, vp, ctypes.POINTER(WorldTemplates), vp, vp, vp],
+                            ctypes.c_int),
         "b3g_kinematic_step": ([vp, vp, ctypes.c_uint32, ctypes.c_float, vp], ctypes.c_int),
         "b3g_set_tuning": ([ctx, u32p], ctypes.c_int),
         "b3g_get_tuning": ([ctx, u32p], ctypes.c_int),

@@ -1274,68 +1274,144 @@ __global__ void k_retire(DevScene S, UpdateArgs u, UpdateLimits lim)
 	}
 }
 
-__global__ void k_scatter(DevScene S, UpdateArgs u, UpdateLimits lim, uint32_t* world, uint32_t* btype,
-	uint8_t* awake, uint32_t* fbody, uint32_t* ftype, uint32_t* fhull, uint32_t* fflags, float4* fparams,
-	float4* fbound)
+// The scene's arrays an update writes.
+struct UpdateTargets
+{
+	uint32_t *world, *btype;
+	uint8_t* awake;
+	uint32_t *fbody, *ftype, *fhull, *fflags;
+	float4 *fparams, *fbound;
+};
+
+__device__ __forceinline__ void write_body(const UpdateLimits& lim, const UpdateTargets& to, uint32_t b, uint32_t world,
+	uint32_t type, uint8_t awake)
+{
+	if (b >= lim.bodies || world >= lim.worlds || type > B3G_BODY_DYNAMIC)
+	{
+		atomicOr(lim.bad, 1u);
+		return;
+	}
+	to.world[b] = world;
+	to.btype[b] = type;
+	to.awake[b] = awake;
+}
+
+__device__ __forceinline__ void write_fixture(const DevScene& S, const UpdateLimits& lim, const UpdateTargets& to,
+	uint32_t f, uint32_t body, uint32_t type, uint32_t hull, uint32_t flags, const float* p)
+{
+	if (f >= lim.fixtures || body >= lim.bodies ||
+		!(type == B3G_SHAPE_SPHERE || type == B3G_SHAPE_CAPSULE || type == B3G_SHAPE_HULL) ||
+		(type == B3G_SHAPE_HULL && hull >= lim.hulls))
+	{
+		atomicOr(lim.bad, 1u);
+		return;
+	}
+	to.fbody[f] = body;
+	to.ftype[f] = type;
+	to.fhull[f] = hull;
+	to.fflags[f] = flags;
+	for (int k = 0; k < 3; ++k)
+		to.fparams[3 * (size_t)f + k] = make_float4(p[4 * k], p[4 * k + 1], p[4 * k + 2], p[4 * k + 3]);
+	to.fbound[f] = fixture_bound(S, type, hull, p);
+	S.fixLife[f] = FIX_FRESH;
+}
+
+__global__ void k_scatter(DevScene S, UpdateArgs u, UpdateLimits lim, UpdateTargets to)
 {
 	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < u.nb + u.nf; t += gridDim.x * blockDim.x)
 	{
 		if (t < u.nb)
 		{
-			uint32_t b = u.bIdx[t];
-			if (b >= lim.bodies || u.bWorld[t] >= lim.worlds || u.bType[t] > B3G_BODY_DYNAMIC)
-			{
-				atomicOr(lim.bad, 1u);
-				continue;
-			}
-			world[b] = u.bWorld[t];
-			btype[b] = u.bType[t];
-			awake[b] = u.bAwake ? u.bAwake[t] : 1;
+			write_body(lim, to, u.bIdx[t], u.bWorld[t], u.bType[t], u.bAwake ? u.bAwake[t] : 1);
 			continue;
 		}
-		uint32_t j = t - u.nb;
-		uint32_t f = u.fIdx[j];
-		uint32_t ty = u.fType[j];
-		if (f >= lim.fixtures || u.fBody[j] >= lim.bodies ||
-			!(ty == B3G_SHAPE_SPHERE || ty == B3G_SHAPE_CAPSULE || ty == B3G_SHAPE_HULL) ||
-			(ty == B3G_SHAPE_HULL && u.fHull[j] >= lim.hulls))
-		{
-			atomicOr(lim.bad, 1u);
-			continue;
-		}
-		const float* p = u.fParams + 12 * (size_t)j;
-		fbody[f] = u.fBody[j];
-		ftype[f] = u.fType[j];
-		fhull[f] = u.fHull[j];
-		fflags[f] = u.fFlags[j];
-		for (int k = 0; k < 3; ++k)
-			fparams[3 * (size_t)f + k] = make_float4(p[4 * k], p[4 * k + 1], p[4 * k + 2], p[4 * k + 3]);
-		fbound[f] = fixture_bound(S, u.fType[j], u.fHull[j], p);
-		S.fixLife[f] = FIX_FRESH;
+		const uint32_t j = t - u.nb;
+		write_fixture(S, lim, to, u.fIdx[j], u.fBody[j], u.fType[j], u.fHull[j], u.fFlags[j],
+			u.fParams + 12 * (size_t)j);
 	}
 }
 
+// Worlds in and out (b3g_swap_worlds): the ranges travel as kernel arguments,
+// a block takes 256 slots of one range. A serving step of 192 worlds admits
+// and retires 22: as index vectors built and gathered by 45 library kernels
+// the update took 750 us of host time, longer than the pass.
+constexpr uint32_t SWAP_RANGES = 64;
+struct WorldRanges
+{
+	uint32_t start[SWAP_RANGES], count[SWAP_RANGES], offset[SWAP_RANGES], world[SWAP_RANGES];
+};
+
+__global__ void k_retire_ranges(DevScene S, UpdateLimits lim, WorldRanges r)
+{
+	const uint32_t k = blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
+	if (t >= r.count[k])
+		return;
+	const uint32_t f = r.start[k] + t;
+	if (f >= lim.fixtures)
+		atomicOr(lim.bad, 1u);
+	else
+		S.fixLife[f] = FIX_DEAD;
+}
+
+__global__ void k_admit_ranges(DevScene S, UpdateLimits lim, UpdateTargets to, WorldRanges r, b3g_world_templates from,
+	float* state, float* motion)
+{
+	const uint32_t k = blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
+	const uint32_t start = r.start[k], count = r.count[k], offset = r.offset[k];
+	if (t < count)
+	{
+		const uint32_t j = offset + t;
+		write_body(lim, to, start + t, r.world[k], from.body_type[j], 1);
+		write_fixture(S, lim, to, start + t, start + from.fixture_body[j], from.shape_type[j], from.hull[j],
+			from.flags[j], from.params + 12 * (size_t)j);
+	}
+	// The block's rows, 17 floats each, word by word.
+	const uint32_t first = blockIdx.x * blockDim.x;
+	const uint32_t rows = first < count ? min(count - first, blockDim.x) : 0u;
+	const size_t to0 = 17 * (size_t)(start + first), from0 = 17 * (size_t)(offset + first);
+#pragma unroll 4
+	for (uint32_t w = threadIdx.x; w < 17u * rows; w += blockDim.x)
+	{
+		state[to0 + w] = from.state[from0 + w];
+		motion[to0 + w] = from.motion[from0 + w];
+	}
+}
+
+// Per world: contacts touching, manifolds with points, points. The contacts of
+// a world lie together in the list, so a warp's contacts of one world take one
+// atomic per count (a contact each: 26 us for 190,000 contacts, most of it
+// waiting for the atomics, now 6).
 __global__ void k_world_counts(DevScene S, Buffers B, uint32_t cur, uint32_t cap, uint32_t worlds, uint32_t* out)
 {
-	uint32_t n = min(B.counters[CTR_PAIRS], cap);
+	const uint32_t n = min(B.counters[CTR_PAIRS], cap);
 	for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
 	{
-		uint32_t w = S.bodyWorld[S.fixBody[B.pairA[cur][c]]];
-		if (w >= worlds)
+		const uint32_t st = B.cstate[cur][c];
+		if ((st & 1u) == 0)
+			continue; // no points without touching
+		const uint32_t w = S.bodyWorld[S.fixBody[B.pairA[cur][c]]];
+		const uint32_t pc = ((st >> 8) & 0xFFu) ? B.man[cur][c].pointCount : 0u;
+		const uint32_t peers = __match_any_sync(__activemask(), w);
+		const uint32_t manifolds = __popc(__ballot_sync(peers, pc != 0));
+		const uint32_t points = __reduce_add_sync(peers, pc);
+		if (w >= worlds || (threadIdx.x & 31u) != (uint32_t)__ffs(peers) - 1u)
 			continue;
-		uint32_t st = B.cstate[cur][c];
-		uint32_t pc = ((st >> 8) & 0xFFu) ? B.man[cur][c].pointCount : 0u;
-		if (st & 1u)
-			atomicAdd(&out[3 * w + 0], 1u);
-		if (pc)
+		atomicAdd(&out[3 * w + 0], (uint32_t)__popc(peers));
+		if (manifolds)
 		{
-			atomicAdd(&out[3 * w + 1], 1u);
-			atomicAdd(&out[3 * w + 2], pc);
+			atomicAdd(&out[3 * w + 1], manifolds);
+			atomicAdd(&out[3 * w + 2], points);
 		}
 	}
 }
 
 } // namespace
+
+static UpdateTargets update_targets(b3g_ctx* c)
+{
+	return UpdateTargets{c->dBodyWorld, c->dBodyType, c->dBodyAwake, c->dFixBody, c->dFixType, c->dFixHull,
+		c->dFixFlags, c->dFixParams, c->dFixBound};
+}
 
 static void launch_update(b3g_ctx* c, const UpdateArgs& u, cudaStream_t s)
 {
@@ -1344,8 +1420,7 @@ static void launch_update(b3g_ctx* c, const UpdateArgs& u, cudaStream_t s)
 	if (u.nr)
 		k_retire<<<blocks, 256, 0, s>>>(c->scene, u, lim);
 	if (u.nb + u.nf)
-		k_scatter<<<blocks, 256, 0, s>>>(c->scene, u, lim, c->dBodyWorld, c->dBodyType, c->dBodyAwake,
-			c->dFixBody, c->dFixType, c->dFixHull, c->dFixFlags, c->dFixParams, c->dFixBound);
+		k_scatter<<<blocks, 256, 0, s>>>(c->scene, u, lim, update_targets(c));
 }
 
 static bool pageable(const void* p)
@@ -1393,6 +1468,19 @@ static cudaError_t wait_staged(b3g_ctx* c, cudaStream_t s)
 	return e == cudaSuccess ? cudaStreamWaitEvent(s, c->awakeStaged, 0) : e;
 }
 
+// After an update whose records the host has not seen.
+static void device_updated(b3g_ctx* c)
+{
+	c->treeForce = true; // fixtures created, replaced or retired: new leaves
+	// The written fixtures' types and flags stay on the device.
+	c->anyTriangle = c->anySensor = true;
+	// The host copy of fixture types is refreshed when the stand-alone
+	// narrowphase next needs it; written bodies are awake, so the sleep count
+	// can only have dropped (it stays an upper bound until the next wake-up
+	// replay recounts it).
+	c->fixTypeStale = true;
+}
+
 extern "C" int b3g_update_scene_device(b3g_ctx* c, uint32_t nb, const uint32_t* bodyIndex, const uint32_t* world,
 	const uint32_t* type, uint32_t nf, const uint32_t* fixIndex, const uint32_t* body, const uint32_t* shapeType,
 	const uint32_t* hull, const float* params, const uint32_t* flags, uint32_t nr, const uint32_t* retireIndex,
@@ -1430,14 +1518,65 @@ extern "C" int b3g_update_scene_device(b3g_ctx* c, uint32_t nb, const uint32_t* 
 	CK(wait_staged(c, s));
 	launch_update(c, u, s);
 	CK(cudaGetLastError());
-	c->treeForce = true; // fixtures created, replaced or retired: new leaves
-	// The written fixtures' types and flags stay on the device.
-	c->anyTriangle = c->anySensor = true;
-	// The host copy of fixture types is refreshed when the stand-alone
-	// narrowphase next needs it; written bodies are awake, so the sleep count
-	// can only have dropped (it stays an upper bound until the next wake-up
-	// replay recounts it).
-	c->fixTypeStale = true;
+	device_updated(c);
+	return B3G_OK;
+}
+
+extern "C" int b3g_swap_worlds(b3g_ctx* c, uint32_t nRetire, const uint32_t* retire, uint32_t nAdmit,
+	const uint32_t* admit, const b3g_world_templates* from, float* state, float* motion, void* stream)
+{
+	if (!c)
+		return B3G_E_INVALID;
+	if ((nRetire && !retire) || (nAdmit && (!admit || !from || !state || !motion)))
+		return fail(c, B3G_E_INVALID, "b3g_swap_worlds: null argument");
+	if (c->capFixtures == 0 || c->capBodies == 0)
+		return fail(c, B3G_E_STATE, "b3g_swap_worlds: no scene");
+	if (!c->keysAreIndex)
+		return fail(c, B3G_E_STATE, "b3g_swap_worlds: needs proxy keys equal to fixture indices");
+	auto past = [](uint32_t start, uint32_t count, uint32_t cap) { return start > cap || count > cap - start; };
+	for (uint32_t i = 0; i < nRetire; ++i)
+		if (past(retire[2 * i], retire[2 * i + 1], c->capFixtures))
+			return fail(c, B3G_E_INVALID, "b3g_swap_worlds: retired range %u", i);
+	for (uint32_t i = 0; i < nAdmit; ++i)
+		if (past(admit[4 * i], admit[4 * i + 1], std::min(c->capFixtures, c->capBodies)))
+			return fail(c, B3G_E_INVALID, "b3g_swap_worlds: admitted range %u", i);
+	if (nRetire + nAdmit == 0)
+		return B3G_OK;
+	CK(cudaSetDevice(c->device));
+	cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
+	CK(refresh_awake(c));
+	CK(wait_staged(c, s));
+	const UpdateLimits lim{c->capBodies, c->capFixtures, c->nWorlds, c->nHulls, c->dUpdateBad};
+	WorldRanges r;
+	// All that leave before any that enter: a range may be given out again.
+	for (int pass = 0; pass < 2; ++pass)
+	{
+		const uint32_t n = pass == 0 ? nRetire : nAdmit, words = pass == 0 ? 2 : 4;
+		const uint32_t* in = pass == 0 ? retire : admit;
+		for (uint32_t i = 0; i < n; i += SWAP_RANGES)
+		{
+			const uint32_t m = std::min(n - i, SWAP_RANGES);
+			uint32_t most = 0;
+			for (uint32_t k = 0; k < m; ++k)
+			{
+				const uint32_t* w = in + (size_t)words * (i + k);
+				r.start[k] = w[0];
+				r.count[k] = w[1];
+				r.offset[k] = pass == 0 ? 0u : w[2];
+				r.world[k] = pass == 0 ? 0u : w[3];
+				most = std::max(most, w[1]);
+			}
+			if (most == 0)
+				continue;
+			const dim3 grid((most + 255) / 256, m);
+			if (pass == 0)
+				k_retire_ranges<<<grid, 256, 0, s>>>(c->scene, lim, r);
+			else
+				k_admit_ranges<<<grid, 256, 0, s>>>(c->scene, lim, update_targets(c), r, *from, state, motion);
+		}
+	}
+	CK(cudaGetLastError());
+	device_updated(c);
 	return B3G_OK;
 }
 

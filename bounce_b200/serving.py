@@ -162,7 +162,6 @@ class ServingEngine:
         self.counts_dev = torch.zeros((ring, max_worlds, 3), dtype=torch.int32, device=self.dev)
         self.counts_host = torch.zeros((ring, max_worlds, 3), dtype=torch.int32, pin_memory=True)
         self.ring = ring
-        self._keep = None
         self.events = collections.deque()  # (step, ring slot, event, finished requests)
         self.stream = torch.cuda.Stream(device=self.dev)
         self.sptr = self.stream.cuda_stream
@@ -251,59 +250,21 @@ class ServingEngine:
         self.st_motion = cat([mo for _, _, mo in rows], F)
         return templates
 
-    def _expand(self, starts, counts, offsets=None):
-        """Device index vectors of the ranges (start_i, count_i): for each
-        element its destination, its source (offset_i + local) and its range."""
-        torch = self.torch
-        total = int(sum(counts))
-        c = torch.tensor(counts, dtype=torch.int64).to(self.dev, non_blocking=True)
-        st = torch.tensor(starts, dtype=torch.int64).to(self.dev, non_blocking=True)
-        rep = torch.repeat_interleave(torch.arange(len(counts), device=self.dev), c, output_size=total)
-        base = torch.cumsum(c, 0) - c
-        local = torch.arange(total, device=self.dev) - base[rep]
-        dst = st[rep] + local
-        src = None
-        if offsets is not None:
-            src = torch.tensor(offsets, dtype=torch.int64).to(self.dev, non_blocking=True)[rep] + local
-        return dst, src, rep, st
-
     def _flush_updates(self):
-        torch = self.torch
         adm = self.pending_admit
         ret = self.pending_retire
         if not adm and not ret:
             return
-        with torch.cuda.stream(self.stream):
-            keep = []
-            nb = nr = 0
-            z = self.st_btype[:0]
-            bidx = world = btype = fbody = ftype = fhull = fflags = rix = z
-            params = self.st_params[:0]
-            if adm:
-                dst, src, rep, st = self._expand([r.start for r in adm], [r.tmpl.n for r in adm],
-                                                 [r.tmpl.offset for r in adm])
-                wids = torch.tensor([r.world for r in adm], dtype=torch.int32).to(self.dev, non_blocking=True)
-                bidx = dst.to(torch.int32)
-                world = wids[rep]
-                btype = self.st_btype[src]
-                fbody = (st[rep] + self.st_fbody[src]).to(torch.int32)
-                ftype = self.st_ftype[src]
-                fhull = self.st_fhull[src]
-                fflags = self.st_fflags[src]
-                params = self.st_params[src].contiguous()
-                self.state.index_copy_(0, dst, self.st_state[src])
-                self.motion.index_copy_(0, dst, self.st_motion[src])
-                nb = len(bidx)
-            if ret:
-                rdst, _, _, _ = self._expand([a for a, _ in ret], [n for _, n in ret])
-                rix = rdst.to(torch.int32)
-                nr = len(rix)
-            keep = [bidx, world, btype, fbody, ftype, fhull, fflags, params, rix]
-            p = lambda t: ctypes.c_void_p(t.data_ptr()) if t.numel() else None
-            self._check(self.lib.b3g_update_scene_device(
-                self.ctx, nb, p(bidx), p(world), p(btype), nb, p(bidx), p(fbody), p(ftype), p(fhull), p(params),
-                p(fflags), nr, p(rix), ctypes.c_void_p(self.sptr)))
-            self._keep = keep  # alive until the next update (stream order covers their use)
+        rows = np.array([(r.start, r.tmpl.n, r.tmpl.offset, r.world) for r in adm], np.uint32)
+        gone = np.array(ret, np.uint32)
+        from_ = None
+        if adm:
+            from_ = ctypes.byref(N.WorldTemplates(*(t.data_ptr() for t in (
+                self.st_btype, self.st_fbody, self.st_ftype, self.st_fhull, self.st_fflags, self.st_params,
+                self.st_state, self.st_motion))))
+        self._check(self.lib.b3g_swap_worlds(
+            self.ctx, len(ret), gone.ctypes.data, len(adm), rows.ctypes.data, from_, self.state.data_ptr(),
+            self.motion.data_ptr(), ctypes.c_void_p(self.sptr)))
         self.pending_admit = []
         self.pending_retire = []
 

@@ -216,6 +216,30 @@ int b3g_update_scene_device(b3g_ctx* ctx, uint32_t body_count, const uint32_t* b
 	uint32_t fixture_count, const uint32_t* fixture_index, const uint32_t* body,
 	const uint32_t* shape_type, const uint32_t* hull, const float* params, const uint32_t* flags,
 	uint32_t retire_count, const uint32_t* retire_index, void* stream);
+/* Worlds in and out of the scene by ranges, for hosts that keep the worlds they
+ * may admit in device memory (the serving loop). A world is a range of slots,
+ * one body and one fixture each, at the same index. retire: nRetire times
+ * (start, count); admit: nAdmit times (start, count, offset, world): slots
+ * [start, start + count) take templates [offset, offset + count), the fixture's
+ * body index being relative to the range. Retired ranges go first. The admitted
+ * bodies are awake; their rows of the templates' state and motion (17 floats
+ * each, see b3g_kinematic_step) are copied to those of state and motion. The
+ * range lists are host memory, read before the call returns; all else is
+ * device memory, and invalid records are treated as b3g_update_scene_device
+ * treats them. Asynchronous on stream. */
+typedef struct b3g_world_templates
+{
+	const uint32_t* body_type;
+	const uint32_t* fixture_body;
+	const uint32_t* shape_type;
+	const uint32_t* hull;
+	const uint32_t* flags;
+	const float* params; /* 12 per fixture */
+	const float* state;
+	const float* motion;
+} b3g_world_templates;
+int b3g_swap_worlds(b3g_ctx* ctx, uint32_t retire_count, const uint32_t* retire, uint32_t admit_count,
+	const uint32_t* admit, const b3g_world_templates* templates, float* state, float* motion, void* stream);
 int b3g_set_active(b3g_ctx* ctx, uint32_t bodies, uint32_t fixtures);
 int b3g_world_counts(b3g_ctx* ctx, uint32_t worlds, uint32_t* out, void* stream);
 

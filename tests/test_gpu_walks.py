@@ -1,11 +1,14 @@
 """GPU: the ordered walks of the single-hit queries against the every-hit
 queries (whose walks and casts they do not share), and the pairs of a world
 that is wide on one axis only against all pairs of its fat AABBs."""
+import ctypes
+
 import numpy as np
 import pytest
 
 from bounce_b200 import _native as N
 from bounce_b200 import scene as S
+from bounce_b200 import serving as V
 from bounce_b200.pipeline import CollisionPipeline
 
 pytestmark = pytest.mark.gpu
@@ -316,3 +319,55 @@ def test_results_through_small_buffers(kind, n, pinned):
         assert all(a == b for a, b in both) and (both or n < 100)
         drv.advance()
     pipe.close()
+
+
+def flush_by_lists(e, torch):
+    """ServingEngine._flush_updates through b3g_update_scene_device's index lists."""
+    adm, ret = e.pending_admit, e.pending_retire
+    dev = lambda x, dt: torch.from_numpy(np.ascontiguousarray(x, dt)).to(e.dev)
+    cat = lambda xs: np.concatenate(xs) if xs else np.zeros(0)
+    slots = cat([r.start + np.arange(r.tmpl.n) for r in adm])
+    a = [dev(slots, np.int32), dev(cat([np.full(r.tmpl.n, r.world) for r in adm]), np.int32),
+         dev(cat([r.tmpl.body_type for r in adm]), np.int32), dev(cat([r.start + r.tmpl.fix_body for r in adm]), np.int32),
+         dev(cat([r.tmpl.fix_type for r in adm]), np.int32), dev(cat([r.tmpl.fix_hull for r in adm]), np.int32),
+         dev(cat([r.tmpl.fix_params.reshape(-1) for r in adm]), np.float32),
+         dev(cat([r.tmpl.fix_flags for r in adm]), np.int32),
+         dev(cat([np.arange(s, s + n) for s, n in ret]), np.int32)]
+    for r in adm:
+        rows = slice(r.tmpl.offset, r.tmpl.offset + r.tmpl.n)
+        e.state[r.start:r.start + r.tmpl.n] = e.st_state[rows]
+        e.motion[r.start:r.start + r.tmpl.n] = e.st_motion[rows]
+    torch.cuda.synchronize()
+    b, w, bt, fb, ft, fh, fp, ff, rx = [ctypes.c_void_p(x.data_ptr()) for x in a]
+    e._check(e.lib.b3g_update_scene_device(e.ctx, len(a[0]), b, w, bt, len(a[0]), b, fb, ft, fh, fp, ff, len(a[8]), rx,
+                                           ctypes.c_void_p(e.sptr)))
+    torch.cuda.synchronize()
+    e.pending_admit, e.pending_retire = [], []
+
+
+# More worlds in and out at once than one launch takes (64), and sizes around a
+# block's 256 slots, against the same update through index lists.
+@pytest.mark.parametrize("sizes", [[2], [255, 256, 257, 700], [4] * 130])
+def test_swapped_worlds(sizes):
+    torch = pytest.importorskip("torch")
+    results = []
+    for lists in (False, True):
+        e = V.ServingEngine(capacity=4096, max_worlds=256, active_quantum=4096, graph=False)
+        if lists:
+            e._flush_updates = lambda e=e: flush_by_lists(e, torch)
+        t = e.load_templates([V.WorldTemplate(7 + n, n - 1, e.box_hull, e.ground_hull, e.hull_arrays)
+                              for n in sorted(set(sizes))])
+        rows = []
+        for step in range(4):
+            for k in range(len(sizes)):
+                e.admit(V.Request(step * 1000 + k, t[(k + step) % len(t)], 1 + k % 2, 0.0))
+            slot = e.slot
+            e.step()
+            c = e.counts()
+            rows += [np.array(list(c.values())), e.state.cpu().numpy(), e.motion.cpu().numpy(),
+                     e.counts_dev[slot].cpu().numpy()]
+        results.append(rows)
+        e.close()
+    assert len(sizes) == 1 or any(r.any() for r in results[0][3::4])
+    for a, b in zip(*results):
+        assert np.array_equal(a, b)
