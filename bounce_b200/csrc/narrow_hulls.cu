@@ -1417,11 +1417,11 @@ __device__ __forceinline__ void bulk_to_shared(void* dst, const void* src, uint3
 				 : "memory");
 }
 
-// Bytes of one warp's staging area: vertices, planes and half-edges of two
-// hulls of the scene's largest sizes.
-__host__ __device__ __forceinline__ size_t sat_stage_bytes(uint32_t maxV, uint32_t maxF, uint32_t maxE)
+// Bytes of one warp's staging area: vertices and planes of two hulls of the
+// scene's largest sizes.
+__host__ __device__ __forceinline__ size_t sat_stage_bytes(uint32_t maxV, uint32_t maxF)
 {
-	return 2 * 16 * ((size_t)maxV + maxF + maxE);
+	return 2 * 16 * ((size_t)maxV + maxF);
 }
 
 // Waits at most STAGE_SPIN polls for the barrier's phase; every lane polls.
@@ -1435,11 +1435,14 @@ __device__ __forceinline__ bool stage_wait(unsigned long long* bar, uint32_t pha
 }
 
 // Pass 2: one warp per contact the cache did not resolve (W warps per block).
-// With STAGE, each pair's hull vertices, planes and half-edges are brought
-// into the warp's shared memory by bulk copies (lane 0 issues six, the warp
-// waits on its barrier), and the face and edge queries and the face contact
-// read them there instead of from global memory, where every lane's loop
-// over the other hull's vertices waited on each load. Shared memory per block:
+// With STAGE, each pair's hull vertices and planes are brought into the warp's
+// shared memory by bulk copies (lane 0 issues four, the warp waits on its
+// barrier), and the face and edge queries and the face contact read them there
+// instead of from global memory, where every lane's loop over the other hull's
+// vertices waited on each load. The half-edges, twice as much, stay there: each
+// is read once, a lane an edge, and without them two blocks fit beside the other
+// kernels' (three contexts at once, 512 worlds: 830 -> 814 us, a pile of 24,064
+// hulls: 198 -> 194). Shared memory per block:
 // W barriers (16-byte rounded), then per warp its query / clip area
 // (sat_warp_bytes), then per warp its staging area (sat_stage_bytes).
 //
@@ -1458,7 +1461,7 @@ __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 	char* wsm = base + (size_t)warp * sat_warp_bytes(maxUE);
 	EdgeRec* recs = reinterpret_cast<EdgeRec*>(wsm);
 	unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem) + warp;
-	const size_t stageBytes = sat_stage_bytes(a.S.hullMaxV, a.S.hullMaxF, a.S.hullMaxE);
+	const size_t stageBytes = sat_stage_bytes(a.S.hullMaxV, a.S.hullMaxF);
 	char* stage = base + (size_t)W * sat_warp_bytes(maxUE) + (size_t)warp * stageBytes;
 	uint32_t phase = 0;
 	if (STAGE)
@@ -1489,23 +1492,19 @@ __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 		{
 			float4* v1 = reinterpret_cast<float4*>(stage);
 			float4* p1 = v1 + H.h1.vCnt;
-			uint4* e1 = reinterpret_cast<uint4*>(p1 + H.h1.fCnt);
-			float4* v2 = reinterpret_cast<float4*>(e1 + H.h1.eCnt);
+			float4* v2 = p1 + H.h1.fCnt;
 			float4* p2 = v2 + H.h2.vCnt;
-			uint4* e2 = reinterpret_cast<uint4*>(p2 + H.h2.fCnt);
 			if (lane == 0)
 			{
 				// The warp's reads of the previous pair (generic proxy) come
 				// before these writes (async proxy).
 				asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-				const uint32_t bytes = 16u * (H.h1.vCnt + H.h1.fCnt + H.h1.eCnt + H.h2.vCnt + H.h2.fCnt + H.h2.eCnt);
+				const uint32_t bytes = 16u * (H.h1.vCnt + H.h1.fCnt + H.h2.vCnt + H.h2.fCnt);
 				mbar_arrive_expect_tx(bar, bytes);
 				bulk_to_shared(v1, H.h1.v, 16u * H.h1.vCnt, bar);
 				bulk_to_shared(p1, H.h1.p, 16u * H.h1.fCnt, bar);
-				bulk_to_shared(e1, H.h1.e, 16u * H.h1.eCnt, bar);
 				bulk_to_shared(v2, H.h2.v, 16u * H.h2.vCnt, bar);
 				bulk_to_shared(p2, H.h2.p, 16u * H.h2.fCnt, bar);
-				bulk_to_shared(e2, H.h2.e, 16u * H.h2.eCnt, bar);
 			}
 			const bool ok = stage_wait(bar, phase);
 			if (!__all_sync(0xffffffffu, ok))
@@ -1520,10 +1519,8 @@ __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 			phase ^= 1u;
 			H.h1.v = v1;
 			H.h1.p = p1;
-			H.h1.e = e1;
 			H.h2.v = v2;
 			H.h2.p = p2;
-			H.h2.e = e2;
 		}
 		uint4 cache = a.cache[c];
 		DevManifold& m = a.man[c];
@@ -1770,7 +1767,7 @@ void launch_sat(const NPArgs& a, uint32_t maxUE, int blocksPerSM, cudaStream_t s
 {
 	const size_t plain = (size_t)W * sat_warp_bytes(maxUE);
 	const size_t staged = ((W * 8 + 15) & ~(size_t)15) + plain +
-		(size_t)W * sat_stage_bytes(a.S.hullMaxV, a.S.hullMaxF, a.S.hullMaxE);
+		(size_t)W * sat_stage_bytes(a.S.hullMaxV, a.S.hullMaxF);
 	static int optin = -1;
 	if (optin < 0)
 	{
