@@ -1831,13 +1831,13 @@ static void wait_copies(b3g_ctx* c, cudaStream_t s)
 		cudaStreamWaitEvent(s, c->copyDone, 0);
 }
 
-// Kernels of a pass's narrowphase: bucketing, the apart pairs, the convex
-// buckets (with the hull-sphere and hull-capsule follow-up kernels), the hull
+// Kernels of a pass's narrowphase: bucketing, the pairs apart or without a
+// hull, the other convex buckets (with the hull-sphere and hull-capsule follow-up kernels), the hull
 // probe and SAT, hull-triangle, and the mesh work.
 static uint32_t narrow_launches(const b3g_ctx* c)
 {
 	uint32_t k = 0;
-	for (int b = 0; b < B3G_CONVEX_KERNELS; ++b)
+	for (int b = CONVEX_PLAIN; b < B3G_CONVEX_KERNELS; ++b)
 		k += convex_bucket_possible(c, b) ? 1u : 0u;
 	return 1 + 1 + k + 2 + 2 + (c->anyTriangle ? 1u : 0u) + mesh_launches(c);
 }
@@ -3174,7 +3174,7 @@ extern "C" int b3g_autotune(b3g_ctx* c, uint32_t reps, void* stream, uint32_t* o
 	};
 	static const uint32_t convexBucket[B3G_CONVEX_KERNELS] = {BK_SPHERES, BK_CAPSULE_SPHERE, BK_CAPSULES,
 		BK_TRIANGLE_SPHERE, BK_TRIANGLE_CAPSULE, BK_HULL_SPHERE, BK_HULL_CAPSULE, BK_SENSOR, BK_INACTIVE};
-	for (int k = 0; k < B3G_CONVEX_KERNELS && rc == B3G_OK; ++k)
+	for (int k = CONVEX_PLAIN; k < B3G_CONVEX_KERNELS && rc == B3G_OK; ++k)
 	{
 		if (h[CTR_BUCKET0 + convexBucket[k]] == 0)
 			continue;

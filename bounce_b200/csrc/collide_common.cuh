@@ -967,7 +967,7 @@ __device__ __forceinline__ HullRef mesh_tri_ref(const MeshTri& t)
 	return r;
 }
 
-void launch_apart(const NPArgs& a, const uint32_t* list, const uint32_t* count, cudaStream_t s);
+void launch_plain(const NPArgs& a, const uint32_t* lists, const uint32_t* counts, uint32_t cap, cudaStream_t s);
 void launch_mesh_items_convex(const NPArgs& a, const Buffers& B, cudaStream_t s);
 void launch_mesh_items_hull(const NPArgs& a, const Buffers& B, uint32_t maxUE, const Tune& tune, cudaStream_t s);
 
@@ -977,6 +977,7 @@ void launch_convex_buckets(const NPArgs& base, const uint32_t* lists, const uint
 	const Tune& tune, cudaStream_t s);
 void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap,
 	const Tune& tune, cudaStream_t s);
+constexpr int CONVEX_PLAIN = 3; // the kernels before it run as one (launch_plain)
 constexpr int CONVEX_HULL_CAPSULE = 6, CONVEX_INACTIVE = 8;
 // Whether convex bucket kernel k (the order of B3G_TUNE_CONVEX) can have
 // contacts in this context's pass: the triangle buckets need triangle

@@ -796,7 +796,7 @@ __device__ GProxy shape_proxy(const DevScene& S, const ShapeP& s)
 // cull of collide_common.cuh, repeated here for contacts that reach these
 // kernels without k_bucket, i.e. wake-ups and b3g_collide_pairs).
 template <int BUCKET>
-__global__ void __launch_bounds__(128, 4) k_convex(NPArgs a)
+__device__ __forceinline__ void convex_bucket(const NPArgs& a)
 {
 	uint32_t n = *a.listCount;
 	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
@@ -868,6 +868,57 @@ __global__ void __launch_bounds__(128, 4) k_convex(NPArgs a)
 			collide_triangle_capsule(m, tri_ref(a.S, fa), xfA, sa, load_wings(a.S, fa), xfB, sb);
 		finish_convex(a, c, m);
 		a.cache[c] = make_uint4(B3G_NULL, B3G_NULL, B3G_NULL, B3G_NULL);
+	}
+}
+
+template <int BUCKET>
+__global__ void __launch_bounds__(128, 4) k_convex(NPArgs a)
+{
+	convex_bucket<BUCKET>(a);
+}
+
+// Convex contacts k_bucket found apart (spheres_apart): the routine would
+// return no point, so the manifold is empty; warm start and flags as above.
+__device__ __forceinline__ void apart_bucket(const NPArgs& a)
+{
+	uint32_t n = *a.listCount;
+	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+	{
+		uint32_t c = a.list[t];
+		DevManifold& m = a.man[c];
+		man_clear(m);
+		finish_convex(a, c, m);
+		a.cache[c] = make_uint4(B3G_NULL, B3G_NULL, B3G_NULL, B3G_NULL);
+	}
+}
+
+// The contacts without a hull, and those apart, a row of blocks per bucket:
+// each is a chain of dependent loads and little else (3 % of the issue slots),
+// so side by side they take as long as the longest. As four
+// launches: a host step of 64 mixed bodies 197 us, now 180; 2,001 with sleepers 333
+// and 318.
+constexpr int PLAIN_BUCKETS = 4;
+constexpr int PLAIN_BLOCKS = 4; // an SM and bucket
+__global__ void __launch_bounds__(128) k_plain(NPArgs a, const uint32_t* lists, const uint32_t* counts, uint32_t cap)
+{
+	const uint32_t bk = blockIdx.y == 0 ? BK_CAPSULES : blockIdx.y == 1 ? BK_CAPSULE_SPHERE : blockIdx.y == 2 ? BK_SPHERES
+																											 : BK_APART;
+	a.list = lists + (size_t)bk * cap;
+	a.listCount = counts + bk;
+	switch (bk)
+	{
+	case BK_CAPSULES:
+		convex_bucket<BK_CAPSULES>(a);
+		break;
+	case BK_CAPSULE_SPHERE:
+		convex_bucket<BK_CAPSULE_SPHERE>(a);
+		break;
+	case BK_SPHERES:
+		convex_bucket<BK_SPHERES>(a);
+		break;
+	default:
+		apart_bucket(a);
+		break;
 	}
 }
 
@@ -958,21 +1009,6 @@ __global__ void k_sensor(NPArgs a)
 		// with: e_empty (sat.h:69), the other fields unset.
 		bool hulls = a.S.fixType[fa] == B3G_SHAPE_HULL && a.S.fixType[fb] == B3G_SHAPE_HULL;
 		a.cache[c] = make_uint4(hulls ? 0u : B3G_NULL, B3G_NULL, B3G_NULL, B3G_NULL);
-	}
-}
-
-// Convex contacts k_bucket found apart (spheres_apart): the routine would
-// return no point, so the manifold is empty; warm start and flags as in k_convex.
-__global__ void k_apart(NPArgs a)
-{
-	uint32_t n = *a.listCount;
-	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-	{
-		uint32_t c = a.list[t];
-		DevManifold& m = a.man[c];
-		man_clear(m);
-		finish_convex(a, c, m);
-		a.cache[c] = make_uint4(B3G_NULL, B3G_NULL, B3G_NULL, B3G_NULL);
 	}
 }
 
@@ -1067,7 +1103,8 @@ __global__ void __launch_bounds__(128) k_mesh_items_convex(NPArgs a, Buffers B)
 } // namespace
 
 // Bucket kernel k of launch_convex_buckets (the order of B3G_TUNE_CONVEX). The
-// counts of the contacts handed on (hsPostCount, hcPostCount) start at 0.
+// counts of the contacts handed on (hsPostCount, hcPostCount) start at 0. The
+// first three, without hulls, run together (launch_plain).
 void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap,
 	const Tune& tune, cudaStream_t s)
 {
@@ -1080,15 +1117,6 @@ void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const u
 	const int blocks = work_blocks(cap, 128, (int)tune.v[B3G_TUNE_CONVEX + k]);
 	switch (k)
 	{
-	case 0:
-		k_convex<BK_SPHERES><<<blocks, 128, 0, s>>>(a);
-		break;
-	case 1:
-		k_convex<BK_CAPSULE_SPHERE><<<blocks, 128, 0, s>>>(a);
-		break;
-	case 2:
-		k_convex<BK_CAPSULES><<<blocks, 128, 0, s>>>(a);
-		break;
 	case 3:
 		k_convex<BK_TRIANGLE_SPHERE><<<blocks, 128, 0, s>>>(a);
 		break;
@@ -1112,19 +1140,19 @@ void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const u
 	}
 }
 
+// The buckets without hulls and the contacts apart.
+void launch_plain(const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap, cudaStream_t s)
+{
+	const dim3 grid(work_blocks(cap, 128, PLAIN_BLOCKS), PLAIN_BUCKETS);
+	k_plain<<<grid, 128, 0, s>>>(base, lists, counts, cap);
+}
+
 void launch_convex_buckets(const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap,
 	const Tune& tune, cudaStream_t s)
 {
-	for (int k = 0; k < B3G_CONVEX_KERNELS; ++k)
+	launch_plain(base, lists, counts, cap, s);
+	for (int k = CONVEX_PLAIN; k < B3G_CONVEX_KERNELS; ++k)
 		launch_convex_one(k, base, lists, counts, cap, tune, s);
-}
-
-void launch_apart(const NPArgs& base, const uint32_t* list, const uint32_t* count, cudaStream_t s)
-{
-	NPArgs a = base;
-	a.list = list;
-	a.listCount = count;
-	k_apart<<<work_blocks(a.hcPostCap, 128, 4), 128, 0, s>>>(a);
 }
 
 void launch_mesh_items_convex(const NPArgs& a, const Buffers& B, cudaStream_t s)
@@ -1135,10 +1163,9 @@ void launch_mesh_items_convex(const NPArgs& a, const Buffers& B, cudaStream_t s)
 void carveout_narrow_convex()
 {
 	set_carveout({
-		(const void*)k_convex<BK_SPHERES>, (const void*)k_convex<BK_CAPSULE_SPHERE>,
-		(const void*)k_convex<BK_CAPSULES>, (const void*)k_convex<BK_HULL_SPHERE>,
-		(const void*)k_convex<BK_HULL_CAPSULE>, (const void*)k_convex<BK_TRIANGLE_SPHERE>,
+		(const void*)k_plain, (const void*)k_convex<BK_HULL_SPHERE>, (const void*)k_convex<BK_HULL_CAPSULE>,
+		(const void*)k_convex<BK_TRIANGLE_SPHERE>,
 		(const void*)k_convex<BK_TRIANGLE_CAPSULE>, (const void*)k_sensor, (const void*)k_hull_sphere_gjk,
-		(const void*)k_hull_capsule_post<HC_POST_LANES>, (const void*)k_apart, (const void*)k_inactive,
+		(const void*)k_hull_capsule_post<HC_POST_LANES>, (const void*)k_inactive,
 		(const void*)k_mesh_items_convex});
 }

@@ -473,16 +473,16 @@ void launch_narrowphase(b3g_ctx* c, cudaStream_t s)
 	// bodies: 212, 338 and 647 us without the third branch, 176, 301 and 626
 	// with it).
 	const bool third = side != s && !meshSide;
+	launch_plain(a, B.bucketList, B.counters + CTR_BUCKET0, cap, s);
 	if (third)
 	{
 		cudaStreamWaitEvent(c->meshStream, c->forkEvent, 0);
 		launch_convex_one(CONVEX_HULL_CAPSULE, a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, c->meshStream);
 		cudaEventRecord(c->meshJoin, c->meshStream);
 	}
-	for (int k = 0; k < B3G_CONVEX_KERNELS; ++k)
+	for (int k = CONVEX_PLAIN; k < B3G_CONVEX_KERNELS; ++k)
 		if (convex_bucket_possible(c, k) && !(third && k == CONVEX_HULL_CAPSULE))
 			launch_convex_one(k, a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
-	launch_apart(a, B.bucketList + (size_t)BK_APART * cap, B.counters + CTR_BUCKET0 + BK_APART, s);
 	prof_mark(c, PM_CONVEX, s);
 	if (side != s)
 	{
