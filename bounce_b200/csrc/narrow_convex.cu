@@ -422,61 +422,66 @@ __device__ __forceinline__ bool hull_capsule_gjk(const DevScene& S, const XF& xf
 	return !(q.distance > totalRadius);
 }
 
-// The rest of b3CollideHullAndCapsule after its GJK, run by a group of G
-// lanes (gl the lane in the group): the support face or the SAT queries
-// spread over the lanes, the contact points built by lane 0, which alone
-// writes m.
+// b3CollideHullAndCapsule (collide_capsule_hull.cpp) after the GJK, in two
+// parts. The scans of a contact run on G lanes: at a distance, the hull's
+// support face along the GJK's normal e1; overlapping, the SAT of the hull
+// against the capsule segment (e1, e2) in its frame.
+struct HullCapsuleScan
+{
+	uint32_t face, edge;
+	float faceSep, edgeSep;
+};
+
 template <int G>
-__device__ void hull_capsule_after_gjk(DevManifold& m, const DevScene& S, const XF& xf1, const ShapeP& hs,
-	const XF& xf2, const ShapeP& k2, const GJKOut& q, uint32_t gl, uint32_t gmask)
+__device__ __forceinline__ HullCapsuleScan hull_capsule_scan(const HullRef& h, bool deep, V3 e1, V3 e2,
+	float totalRadius, uint32_t gl, uint32_t gmask)
+{
+	HullCapsuleScan r{0u, 0u, 0.0f, 0.0f};
+	if (!deep)
+		r.face = group_support_face<G>(h, e1, gl, gmask);
+	else
+	{
+		query_face_hull_capsule<G>(h, e1, e2, r.face, r.faceSep, gl, gmask);
+		if (!(r.faceSep > totalRadius))
+			query_edge_hull_capsule<G>(h, e1, e2, r.edge, r.edgeSep, gl, gmask);
+	}
+	return r;
+}
+
+// ... and its manifold, on one lane.
+__device__ __forceinline__ void hull_capsule_contact(DevManifold& m, const HullRef& h1, const XF& xf1,
+	const ShapeP& hs, const XF& xf2, const ShapeP& k2, const GJKOut& q, V3 localN1, const HullCapsuleScan& r)
 {
 	float r1 = hull_radius(hs), r2 = cap_radius(k2);
 	float totalRadius = r1 + r2;
-	HullRef h1 = hull_ref(S, hs.hull);
 	V3 v1 = cap_v1(k2), v2 = cap_v2(k2);
-	if (q.distance > 0.0f)
+	const bool deep = !(q.distance > 0.0f);
+	bool face, edge = false;
+	if (!deep)
 	{
-		V3 c1 = q.point1, c2 = q.point2;
-		float d = q.distance;
-		V3 N1 = (c2 - c1) / d;
-		V3 localN1 = rotc(xf1.q, N1);
-		uint32_t index1 = group_support_face<G>(h1, localN1, gl, gmask);
-		if (gl != 0)
-			return;
-		V3 localFaceN1 = hp(h1, index1).n;
 		const float kTol = 0.005f;
-		V3 N = cross(localN1, localFaceN1);
-		float L = dot(N, N);
-		if (L < kTol * kTol)
-		{
-			hull_capsule_face_contact(m, xf1, h1, index1, r1, xf2, v1, v2, r2);
-			if (m.pointCount == 2)
-				return;
-		}
-		m.pointCount = 1;
-		set_point(m.points[0], localN1, xmult(xf1, c1), xmult(xf2, c2));
-		set_id0(m.points[0]);
-		return;
+		V3 N = cross(localN1, hp(h1, r.face).n);
+		face = dot(N, N) < kTol * kTol;
 	}
-	// Deep overlap: SAT on the hull against the capsule segment.
-	XF xf = xmult(xf1, xf2);
-	V3 lv1 = xmul(xf, v1), lv2 = xmul(xf, v2);
-	uint32_t faceIndex;
-	float faceSep;
-	query_face_hull_capsule<G>(h1, lv1, lv2, faceIndex, faceSep, gl, gmask);
-	if (faceSep > totalRadius)
-		return;
-	uint32_t edgeIndex;
-	float edgeSep;
-	query_edge_hull_capsule<G>(h1, lv1, lv2, edgeIndex, edgeSep, gl, gmask);
-	if (edgeSep > totalRadius || gl != 0)
-		return;
-	const float kRelEdgeTol = 0.90f;
-	const float kAbsTol = 0.5f * B3G_LINEAR_SLOP;
-	if (edgeSep > kRelEdgeTol * faceSep + kAbsTol)
-		hull_capsule_edge_contact(m, xf1, h1, edgeIndex, xf2, v1, v2);
 	else
-		hull_capsule_face_contact(m, xf1, h1, faceIndex, r1, xf2, v1, v2, r2);
+	{
+		if (r.faceSep > totalRadius || r.edgeSep > totalRadius)
+			return;
+		const float kRelEdgeTol = 0.90f;
+		const float kAbsTol = 0.5f * B3G_LINEAR_SLOP;
+		edge = r.edgeSep > kRelEdgeTol * r.faceSep + kAbsTol;
+		face = !edge;
+	}
+	if (edge)
+		hull_capsule_edge_contact(m, xf1, h1, r.edge, xf2, v1, v2);
+	if (face)
+		hull_capsule_face_contact(m, xf1, h1, r.face, r1, xf2, v1, v2, r2);
+	if (!deep && !(face && m.pointCount == 2))
+	{
+		m.pointCount = 1;
+		set_point(m.points[0], localN1, xmult(xf1, q.point1), xmult(xf2, q.point2));
+		set_id0(m.points[0]);
+	}
 }
 
 // ---------------------------------------------------------------------------
@@ -947,10 +952,11 @@ __global__ void __launch_bounds__(128, 4) k_hull_sphere_gjk(NPArgs a)
 constexpr int HC_POST_LANES = 8;
 constexpr int HC_POST_BLOCKS = 6;
 
-// Hull-capsule contacts past their GJK (k_convex<BK_HULL_CAPSULE> lists them),
-// G lanes per contact: the support-face and SAT scans run on the group's
-// lanes, so a warp no longer walks, one lane at a time, the faces and edges
-// of every hull in it that needs them.
+// Hull-capsule contacts past their GJK (k_convex<BK_HULL_CAPSULE> lists them):
+// the scans of a contact's faces and edges run on G lanes, one contact of the
+// group after the other, then each lane builds the manifold of its own (built
+// on one lane of the group, 7.6 lanes of a warp were active: a pass of 65,536
+// mixed bodies, three contexts at once, 392 us, now 376).
 template <int G>
 __global__ void __launch_bounds__(128, HC_POST_BLOCKS) k_hull_capsule_post(NPArgs a)
 {
@@ -959,12 +965,20 @@ __global__ void __launch_bounds__(128, HC_POST_BLOCKS) k_hull_capsule_post(NPArg
 	const uint32_t nSep = a.hcPostCount[0];
 	const uint32_t n = nSep + a.hcPostCount[1];
 	const uint32_t lane = threadIdx.x & 31u;
-	const uint32_t gl = lane % G;
-	const uint32_t gmask = G == 32 ? 0xFFFFFFFFu : (((1u << G) - 1u) << (lane - gl));
-	const uint32_t groups = gridDim.x * (blockDim.x / G);
-	for (uint32_t t = blockIdx.x * (blockDim.x / G) + threadIdx.x / G; t < n; t += groups)
+	const uint32_t gl = lane % G, first = lane - gl;
+	const uint32_t gmask = G == 32 ? 0xFFFFFFFFu : (((1u << G) - 1u) << first);
+	// As many contacts a group as leave 8 warps an SM: one after the other takes
+	// longer than side by side where there are few (376 us; with 4 warps 378, and
+	// 542 instead of 511 alone; with 16 380).
+	const uint32_t each = min(max(n / (148u * 8u * (32u / G)), 1u), (uint32_t)G);
+	const uint32_t perWarp = each * (32u / G);
+	const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+	for (uint32_t t0 = (blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * perWarp; t0 < n; t0 += warps * perWarp)
 	{
-		const uint32_t j = t < nSep ? t : a.hcPostCap - 1u - (t - nSep);
+		const uint32_t t = t0 + (lane / G) * each + gl;
+		const bool mine = gl < each && t < n;
+		const uint32_t k = mine ? t : t0;
+		const uint32_t j = k < nSep ? k : a.hcPostCap - 1u - (k - nSep);
 		float4 q0 = a.hcPost[2 * (size_t)j], q1 = a.hcPost[2 * (size_t)j + 1];
 		uint32_t c = __float_as_uint(q1.w);
 		GJKOut q;
@@ -977,13 +991,41 @@ __global__ void __launch_bounds__(128, HC_POST_BLOCKS) k_hull_capsule_post(NPArg
 		XF xfA = a.exA ? load_xf7(a.exA + 7 * (size_t)c) : body_xf(a.S, ba);
 		XF xfB = a.exB ? load_xf7(a.exB + 7 * (size_t)c) : body_xf(a.S, bb);
 		ShapeP sa = load_shape(a.S, fa), sb = load_shape(a.S, fb);
-		DevManifold& m = a.man[c];
-		hull_capsule_after_gjk<G>(m, a.S, xfA, sa, xfB, sb, q, gl, gmask);
-		if (gl == 0)
+		const bool deep = !(q.distance > 0.0f);
+		const float totalRadius = hull_radius(sa) + cap_radius(sb);
+		V3 e1, e2;
+		if (!deep)
 		{
+			V3 N1 = (q.point2 - q.point1) / q.distance;
+			e1 = e2 = rotc(xfA.q, N1);
+		}
+		else
+		{
+			XF xf = xmult(xfA, xfB);
+			e1 = xmul(xf, cap_v1(sb));
+			e2 = xmul(xf, cap_v2(sb));
+		}
+		HullCapsuleScan scan{0u, 0u, 0.0f, 0.0f};
+		for (uint32_t r = 0; r < each; ++r)
+		{
+			auto from = [&](float x) { return __shfl_sync(0xffffffffu, x, first + r); };
+			const uint32_t hull = __shfl_sync(0xffffffffu, sa.hull, first + r);
+			const bool d = __shfl_sync(0xffffffffu, deep ? 1 : 0, first + r) != 0;
+			const V3 f1 = V3{from(e1.x), from(e1.y), from(e1.z)}, f2 = V3{from(e2.x), from(e2.y), from(e2.z)};
+			const float total = from(totalRadius);
+			const HullCapsuleScan s = hull_capsule_scan<G>(hull_ref(a.S, hull), d, f1, f2, total, gl, gmask);
+			if (gl == r)
+				scan = s;
+			__syncwarp();
+		}
+		if (mine)
+		{
+			DevManifold& m = a.man[c];
+			hull_capsule_contact(m, hull_ref(a.S, sa.hull), xfA, sa, xfB, sb, q, e1, scan);
 			finish_convex(a, c, m);
 			a.cache[c] = make_uint4(B3G_NULL, B3G_NULL, B3G_NULL, B3G_NULL);
 		}
+		__syncwarp();
 	}
 }
 

@@ -371,3 +371,41 @@ def test_swapped_worlds(sizes):
     assert len(sizes) == 1 or any(r.any() for r in results[0][3::4])
     for a, b in zip(*results):
         assert np.array_equal(a, b)
+
+
+# Hull-capsule pairs at a distance, touching and deep, one pair a world: however
+# many there are (a lane group takes 1 to 8), each is the pair alone.
+@pytest.mark.parametrize("worlds", [9, 31, 4737, 9475, 40001])
+def test_many_hull_capsule_pairs(worlds):
+    rng = np.random.default_rng(3)
+    kinds = 9
+    where = np.concatenate([rng.uniform(-0.5, 0.5, (kinds, 1)), np.linspace(0.1, 0.85, kinds)[:, None],
+                            rng.uniform(-0.5, 0.5, (kinds, 1))], 1)
+    turn = S.random_quats(rng, kinds)
+
+    def manifolds(n):
+        sc = S.Scene()
+        hull = sc.hulls.add_points(S.ellipsoid_points(np.random.default_rng(1), 20, np.array([0.6, 0.5, 0.7])))
+        box = sc.hulls.add_box(0.5, 0.4, 0.6)
+        for w in range(n):
+            b = sc.add_body(w, N.BODY_DYNAMIC, (0, 0, 0), (0, 0, 0, 1))
+            sc.add_fixture(b, N.SHAPE_HULL, [0.0], hull=(hull, box)[w % 2])
+            b = sc.add_body(w, N.BODY_DYNAMIC, where[w % kinds], turn[w % kinds])
+            sc.add_fixture(b, N.SHAPE_CAPSULE, [0, -0.5, 0, 0, 0.5, 0, 0.2])
+        sc.finalize()
+        pipe = CollisionPipeline(sc, max_contacts=2 * n + 64)
+        pipe.collide(S.KinematicDriver(sc).state17())
+        c, m = pipe.contacts(), pipe.manifolds()
+        pipe.close()
+        out = {}
+        for (a, _, _), x in zip(c, m):
+            points = int(x["pointCount"])
+            out[int(a) // 2] = (points, x["points"][:points].tobytes())
+        return out
+
+    few = manifolds(2 * kinds)
+    assert len(few) >= kinds and any(k for k, _ in few.values())
+    many = manifolds(worlds)
+    for w, m in many.items():
+        assert m == few[w % (2 * kinds)]
+    assert len(many) == sum(w % (2 * kinds) in few for w in range(worlds))
