@@ -8,10 +8,11 @@
 //   b3MeshShape::RayCast      mesh_shape.cpp:81-146, over b3StaticTree::RayCast
 //                             (static_tree.h:150-292)
 //
-// One thread per query walks the LBVH from the root along its ropes. The
-// reference walks its dynamic tree instead; the set of proxies a query meets
-// is the same (fat AABBs overlapping the box, or the segment), only the order
-// differs: QueryAABB and RayCast (every hit) are returned per query in LBVH
+// The calls that report every hit walk the LBVH from the root along its ropes,
+// a thread per query; those that report one meet its boxes nearest first, the
+// lanes of a warp in step. The reference walks its dynamic tree instead; the
+// set of proxies a query meets is the same (fat AABBs overlapping the box, or
+// the segment), only the order differs: QueryAABB and RayCast (every hit) are returned per query in LBVH
 // order, and RayCastSingle keeps the smallest fraction, the smaller fixture
 // index on an exact tie (the reference keeps the first one its tree meets).
 
