@@ -1462,7 +1462,9 @@ static cudaError_t refresh_awake(b3g_ctx* c)
 // Work on s that uses what b3g_load_impulses or b3g_set_awake has on the way.
 static cudaError_t wait_staged(b3g_ctx* c, cudaStream_t s)
 {
-	if (s == c->stream)
+	// Nothing is asked of a stream (it may be under capture) that has nothing to
+	// wait for.
+	if (s == c->stream || !c->staged)
 		return cudaSuccess;
 	cudaError_t e = cudaStreamWaitEvent(s, c->impulsesStaged, 0);
 	return e == cudaSuccess ? cudaStreamWaitEvent(s, c->awakeStaged, 0) : e;
@@ -1734,6 +1736,7 @@ extern "C" int b3g_set_awake(b3g_ctx* c, const uint8_t* awake)
 			std::memcpy(c->stageAwake, awake, c->nBodies);
 			CK(cudaMemcpyAsync(c->dBodyAwake, c->stageAwake, c->nBodies, cudaMemcpyHostToDevice, c->stream));
 			CK(cudaEventRecord(c->awakeStaged, c->stream));
+			c->staged = true;
 		}
 		else
 		{
@@ -2750,6 +2753,7 @@ extern "C" int b3g_load_impulses(b3g_ctx* c, const float* normal, const float* t
 		CK(cudaMemcpyAsync(c->buf.impulseTangent, at + 4 * (size_t)n, 8 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
 		CK(cudaMemcpyAsync(c->buf.impulseMotor, at + 6 * (size_t)n, 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
 		CK(cudaEventRecord(c->impulsesStaged, c->stream));
+		c->staged = true;
 	}
 	else if (n)
 	{

@@ -371,6 +371,7 @@ struct b3g_ctx
 	bool countsFetched;       // hCounters are those of the last pass, which has ended
 	char *stageOut, *stageImpulses, *stageAwake; // pinned, B3G_STAGE_BYTES each (allocated on first use)
 	cudaEvent_t impulsesStaged, awakeStaged;     // the copies from them
+	bool staged;                                 // one of them has been recorded
 	void* edgeBuf;            // b3g_fetch_fixture_contacts scratch (allocated on first use)
 	size_t edgeBytes;
 	cudaStream_t sideStream;  // hull-hull / hull-triangle narrowphase, beside the convex buckets
