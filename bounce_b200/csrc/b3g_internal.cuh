@@ -241,7 +241,7 @@ struct Buffers
 // and the caller's contact filter (b3ContactFilter::ShouldCollide, called by
 // AddPair, contact_manager.cpp:86-92, and for every contact by UpdateContacts,
 // :189-199). mode 0: none (the default pass); 1: joints and the per-contact
-// veto applied inside k_diff / k_kept; 2: as 1, plus new pairs the caller's
+// veto applied inside k_diff / k_order_scan; 2: as 1, plus new pairs the caller's
 // filter rejected, precomputed per overlapping pair in rawDrop.
 // With a filter in use a new contact also needs a proxy that moved this pass
 // (was re-inserted or created): FindPairs reports only pairs of moved proxies

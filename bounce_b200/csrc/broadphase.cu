@@ -10,9 +10,8 @@
 //  k_build       Karras (2012) radix tree over the sorted keys, with ropes
 //                (the next node in depth-first order after a subtree)
 //  k_refit       bottom-up node AABBs
-//  k_traverse    stackless rope traversal from each leaf's own rope, which
-//                visits exactly the leaves after it in sorted order, so each
-//                overlapping pair is met once; the AddPair filters
+//  k_traverse    each leaf's search of the subtrees after it in sorted order,
+//                so each overlapping pair is met once; the AddPair filters
 //                (contact_manager.cpp:98-160) and the b3Contact::Create A/B
 //                order (contact.cpp:290-322) are applied per pair
 //

@@ -5,11 +5,10 @@
 // Per pass, for every contact with a mesh fixture:
 //  k_mesh_sync    b3MeshContact::SynchronizeFixture / MoveAABB (or the
 //                 constructor's AABB for a new contact): the other shape's fat
-//                 AABB in mesh space (mesh_contact.cpp:26-231); then the
-//                 number of tree triangles it overlaps (b3StaticTree::QueryAABB)
-//  scan + k_mesh_emit
-//                 (contact, triangle) work items in the order the reference's
-//                 query reports them (FindPairs / Report, :233-297)
+//                 AABB in mesh space (mesh_contact.cpp:26-231); then the tree
+//                 triangles it overlaps (b3StaticTree::QueryAABB) as (contact,
+//                 triangle) work items, in the order the reference's query
+//                 reports them (FindPairs / Report, :233-297)
 //  evaluate       one work item = one b3Manifold of the child triangle
 //                 (b3MeshShape::GetChildTriangle + b3CollideTriangleAndSphere /
 //                 AndCapsule / b3CollideHullAndTriangle), points tagged with the

@@ -404,7 +404,7 @@ __device__ void hull_capsule_face_contact(DevManifold& m, const XF& xf1, const H
 // b3CollideHullAndCapsule (collide_hull_capsule.cpp:29-190), first part:
 // the GJK distance between the hull and the capsule's segment. False when it
 // is above the radii (an empty manifold); else the rest of the routine
-// (hull_capsule_after_gjk) builds the manifold from q.
+// (hull_capsule_scan, hull_capsule_contact) builds the manifold from q.
 __device__ __forceinline__ bool hull_capsule_gjk(const DevScene& S, const XF& xf1, const ShapeP& hs, const XF& xf2,
 	const ShapeP& k2, GJKOut& q)
 {
@@ -422,7 +422,7 @@ __device__ __forceinline__ bool hull_capsule_gjk(const DevScene& S, const XF& xf
 	return !(q.distance > totalRadius);
 }
 
-// b3CollideHullAndCapsule (collide_capsule_hull.cpp) after the GJK, in two
+// b3CollideHullAndCapsule (collide_hull_capsule.cpp:29-190) after the GJK, in two
 // parts. The scans of a contact run on G lanes: at a distance, the hull's
 // support face along the GJK's normal e1; overlapping, the SAT of the hull
 // against the capsule segment (e1, e2) in its frame.
