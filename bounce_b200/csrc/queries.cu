@@ -728,7 +728,7 @@ struct RayWarp
 {
 	unsigned long long best[64]; // per ray place: fraction bits, fixture; ~0: none
 	float p[6][64];
-	float normal[3][64];
+	float fraction[64], normal[3][64]; // of the best
 	uint32_t world[64];
 	uint32_t pending[64];         // queued leaves of the place's ray
 	uint32_t leaf[64];            // leaves reached
@@ -768,8 +768,8 @@ __global__ void __launch_bounds__(RAY_WARPS * 32, RAY_BLOCKS) k_ray_first(QueryC
 	__syncwarp();
 	auto finish = [&](uint32_t place, uint32_t& r) {
 		const unsigned long long key = W.best[place];
-		ray_write(outFix, outHit, r, warp_ray(W, place), key == ~0ull ? B3G_NULL : (uint32_t)key,
-			__uint_as_float((uint32_t)(key >> 32)), V3{W.normal[0][place], W.normal[1][place], W.normal[2][place]});
+		ray_write(outFix, outHit, r, warp_ray(W, place), key == ~0ull ? B3G_NULL : (uint32_t)key, W.fraction[place],
+			V3{W.normal[0][place], W.normal[1][place], W.normal[2][place]});
 		r = B3G_NULL;
 	};
 	for (;;)
@@ -916,9 +916,12 @@ __global__ void __launch_bounds__(RAY_WARPS * 32, RAY_BLOCKS) k_ray_first(QueryC
 			{
 				owner = W.owner[k][left + lane];
 				uint32_t f;
-				if (ray_hits(o, f, q, tree, warp_ray(W, owner), W.cast[k][left + lane]))
+				// A NaN fraction is below no other and never the first. The bits of
+				// the others order as the fractions do, but for -0 (a ray that starts
+				// in a triangle's plane): the key takes it as +0.
+				if (ray_hits(o, f, q, tree, warp_ray(W, owner), W.cast[k][left + lane]) && o.fraction < B3G_MAX_SCALAR)
 				{
-					mine = ((unsigned long long)__float_as_uint(o.fraction) << 32) | f;
+					mine = ((unsigned long long)__float_as_uint(o.fraction + 0.0f) << 32) | f;
 					atomicMin(&W.best[owner], mine);
 				}
 				atomicSub(&W.pending[owner], 1u);
@@ -926,7 +929,10 @@ __global__ void __launch_bounds__(RAY_WARPS * 32, RAY_BLOCKS) k_ray_first(QueryC
 			__syncwarp();
 			// A fixture is one leaf, so a key has one lane.
 			if (mine != ~0ull && W.best[owner] == mine)
+			{
+				W.fraction[owner] = o.fraction;
 				W.normal[0][owner] = o.normal.x, W.normal[1][owner] = o.normal.y, W.normal[2][owner] = o.normal.z;
+			}
 			__syncwarp();
 		}
 		if (walking == 0u && next >= end && leaves + qn[0] + qn[1] + qn[2] + qn[3] == 0u)
