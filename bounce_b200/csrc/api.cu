@@ -3,6 +3,7 @@
 // b3g_create for the configured capacities.
 
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -814,6 +815,25 @@ extern "C" const char* b3g_last_error(const b3g_ctx* c)
 	return c ? c->err.c_str() : "null context";
 }
 
+// Whether no vertex is more than 16 times as far from the centroid as the
+// nearest plane (HullDesc::blunt).
+static bool hull_blunt(uint32_t nv, const float* v, uint32_t np, const float* planes, const float* c)
+{
+	double far2 = 0.0, near = INFINITY;
+	for (uint32_t i = 0; i < nv; ++i)
+	{
+		const double x = (double)v[3 * i] - c[0], y = (double)v[3 * i + 1] - c[1], z = (double)v[3 * i + 2] - c[2];
+		far2 = std::max(far2, x * x + y * y + z * z);
+	}
+	for (uint32_t i = 0; i < np; ++i)
+	{
+		const float* p = planes + 4 * (size_t)i;
+		const double n = std::sqrt((double)p[0] * p[0] + (double)p[1] * p[1] + (double)p[2] * p[2]);
+		near = std::min(near, (p[3] - ((double)p[0] * c[0] + (double)p[1] * c[1] + (double)p[2] * c[2])) / n);
+	}
+	return near > 0.0 && far2 <= 256.0 * near * near;
+}
+
 extern "C" int b3g_set_hulls(b3g_ctx* c, uint32_t nh, const uint32_t* desc, const float* verts,
 	const uint32_t* edges, const uint32_t* faces, const float* planes, const float* centroids)
 {
@@ -853,8 +873,9 @@ extern "C" int b3g_set_hulls(b3g_ctx* c, uint32_t nh, const uint32_t* desc, cons
 				e = E[4];
 			} while (e != begin);
 		}
-		hd[h] = HullDesc{d[0], d[1], d[2], d[3], d[4], d[5], centroids[3 * h], centroids[3 * h + 1],
-			centroids[3 * h + 2], {0, 0, 0}};
+		const float* c3 = centroids + 3 * (size_t)h;
+		hd[h] = HullDesc{d[0], d[1], d[2], d[3], d[4], d[5], c3[0], c3[1], c3[2],
+			hull_blunt(d[1], verts + 3 * (size_t)d[0], d[5], planes + 4 * (size_t)d[4], c3) ? 1u : 0u, {0, 0}};
 		nv = std::max(nv, d[0] + d[1]);
 		ne = std::max(ne, d[2] + d[3]);
 		nf = std::max(nf, d[4] + d[5]);

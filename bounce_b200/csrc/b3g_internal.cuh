@@ -69,7 +69,8 @@ struct HullDesc
 {
 	uint32_t vOff, vCnt, eOff, eCnt, fOff, fCnt;
 	float cx, cy, cz;
-	uint32_t pad[3];
+	uint32_t blunt; // the vertices are at most 16 times as far from the centroid as the nearest plane (queries.cu)
+	uint32_t pad[2];
 };
 static_assert(sizeof(HullDesc) == 48, "HullDesc");
 

@@ -92,3 +92,54 @@ def test_tangent_and_endless(n):
     rays = surface_rays(points, directions, n, rng)
     rays[::4] = rng.normal(size=(len(rays[::4]), 6)) * 1e25
     same_first_hit(sc, rays)
+
+
+def tangent_rays(sc, n, rng):
+    """Rays of 50 to 1,000 m that pass the fixtures' bounding spheres, a
+    capsule's hemispheres or a hull's vertices at their surface."""
+    pick = rng.integers(0, sc.n_fixtures, n)
+    params = sc.fix_params.reshape(-1, 12)[pick]
+    kind = sc.fix_type[pick]
+    verts, desc = sc.hull_arrays["verts"].reshape(-1, 3), sc.hull_arrays["desc"].reshape(-1, 6)
+    local = np.zeros((n, 3), np.float32)
+    radius = np.where(kind == N.SHAPE_SPHERE, params[:, 3], np.where(kind == N.SHAPE_CAPSULE, params[:, 6], 0.0))
+    ends = np.where(rng.random(n)[:, None] < 0.5, params[:, 0:3], params[:, 3:6])
+    local[kind == N.SHAPE_CAPSULE] = ends[kind == N.SHAPE_CAPSULE]
+    for i in np.nonzero(kind == N.SHAPE_HULL)[0]:
+        d = desc[sc.fix_hull[pick[i]]]
+        local[i] = verts[d[0] + rng.integers(d[1])]
+    c = S.xf_apply(sc.body_pos[sc.fix_body[pick]], sc.body_quat[sc.fix_body[pick]], local)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    side = np.cross(d, rng.normal(size=(n, 3)))
+    side /= np.linalg.norm(side, axis=1)[:, None]
+    length = np.exp(rng.uniform(np.log(50.0), np.log(1000.0), n))
+    # As far outside as the rounding of a cast reaches: about a part in a
+    # million of the squared length over the radius.
+    off = radius + rng.uniform(-0.2, 1.0, n) * 1e-6 * length**2 / np.maximum(radius, 0.3)
+    p1 = c + side * off[:, None] - d * (length * rng.uniform(0.05, 0.95, n))[:, None]
+    return np.concatenate([p1, p1 + d * length[:, None]], axis=1)
+
+
+@pytest.mark.parametrize("n", BATCHES)
+def test_long_tangent_rays(n):
+    rng = np.random.default_rng(n)
+    sc = S.mixed_scene(seed=n, n=400, side=24.0).finalize()
+    same_first_hit(sc, tangent_rays(sc, n, rng))
+
+
+# Hulls with faces that meet at a sharp edge, and plates.
+@pytest.mark.parametrize("n", BATCHES)
+def test_long_rays_past_sharp_hulls(n):
+    rng = np.random.default_rng(n)
+    sc = S.Scene()
+    shapes = []
+    for w, t in ((4.0, 0.004), (3.0, 0.05), (2.0, 0.4)):
+        x = np.array([[-w, 0, -0.5], [-w, 0, 0.5], [w, -t, -0.5], [w, -t, 0.5], [w, t, -0.5], [w, t, 0.5]])
+        shapes.append(sc.hulls.add_points(x.astype(np.float32)))
+    q = S.random_quats(rng, 60)
+    for i in range(60):
+        b = sc.add_body(0, N.BODY_DYNAMIC, rng.uniform(-15, 15, 3), q[i])
+        sc.add_fixture(b, N.SHAPE_HULL, [0.0], hull=shapes[i % 3])
+    sc.finalize()
+    same_first_hit(sc, tangent_rays(sc, n, rng))
