@@ -530,7 +530,9 @@ constexpr uint32_t LEAF_NONE = 7u;
 // turned (when set): receives 1 if a live triangle fixture sits on a body away
 // from the identity transform. The reference ignores the transform in a
 // triangle's AABB (triangle_shape.cpp:59-67), so such a fixture lies outside
-// its box, and a shape cast may not skip boxes its motion does not meet.
+// its box: a hit on it says nothing of where the box is met, no box that a ray
+// meets is skipped for a hit before it, and a shape cast may not skip boxes its
+// motion does not meet.
 __global__ void k_walk_tree(QueryCtx q, float4* nodes, float4* leaves, uint32_t* turned)
 {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -694,7 +696,11 @@ __device__ __forceinline__ bool ray_hits(RayOut& o, uint32_t& f, const QueryCtx&
 // fraction, at most the root of a discriminant's: sqrt(16 eps/2) = 1e-3 of the
 // distance to the shape over the length, 3e-3 for shapes up to the ray's length.
 constexpr float RAY_SLACK = 0x1p-8f;
-__device__ __forceinline__ float ray_limit(float fraction) { return fminf(fraction + RAY_SLACK, 1.0f); }
+// turned: see k_walk_tree.
+__device__ __forceinline__ float ray_limit(float fraction, bool turned)
+{
+	return turned ? 1.0f : fminf(fraction + RAY_SLACK, 1.0f);
+}
 
 __device__ __forceinline__ void ray_slab(SlabTest& slab, const RayIn& in)
 {
@@ -767,9 +773,10 @@ __device__ __forceinline__ RayIn warp_ray(const RayWarp& W, uint32_t place)
 }
 
 __global__ void __launch_bounds__(RAY_WARPS * 32, RAY_BLOCKS) k_ray_first(QueryCtx q, WalkTree tree, const float* rays,
-	const uint32_t* worlds, uint32_t n, uint32_t share, uint32_t* outFix, float* outHit)
+	const uint32_t* worlds, uint32_t n, uint32_t share, const uint32_t* anyTurned, uint32_t* outFix, float* outHit)
 {
 	__shared__ RayWarp shared[RAY_WARPS];
+	const bool turned = anyTurned && *anyTurned;
 	const uint32_t lane = threadIdx.x & 31u;
 	RayWarp& W = shared[threadIdx.x >> 5];
 	const uint32_t warp = blockIdx.x * RAY_WARPS + (threadIdx.x >> 5);
@@ -832,7 +839,7 @@ __global__ void __launch_bounds__(RAY_WARPS * 32, RAY_BLOCKS) k_ray_first(QueryC
 		__syncwarp();
 		// Walk toward the next leaf, a few levels at a time.
 		const unsigned long long key = W.best[cur];
-		const float limit = key == ~0ull ? 1.0f : ray_limit(__uint_as_float((uint32_t)(key >> 32)));
+		const float limit = key == ~0ull ? 1.0f : ray_limit(__uint_as_float((uint32_t)(key >> 32)), turned);
 #pragma unroll 1
 		for (int k = 0; k < RAY_STEPS; ++k)
 		{
@@ -978,9 +985,10 @@ __global__ void __launch_bounds__(RAY_WARPS * 32, RAY_BLOCKS) k_ray_first(QueryC
 constexpr uint32_t RAY_FRONT = 1024; // stack entries per warp
 
 __global__ void __launch_bounds__(32) k_ray_first_warp(QueryCtx q, WalkTree tree, const float* rays,
-	const uint32_t* worlds, uint32_t n, uint32_t* outFix, float* outHit)
+	const uint32_t* worlds, uint32_t n, const uint32_t* anyTurned, uint32_t* outFix, float* outHit)
 {
 	__shared__ uint2 stack[RAY_FRONT]; // reference, entry fraction (float bits)
+	const bool turned = anyTurned && *anyTurned;
 	const uint32_t lane = threadIdx.x;
 	const uint32_t lt = (1u << lane) - 1u;
 	const uint32_t i = blockIdx.x;
@@ -1047,7 +1055,7 @@ __global__ void __launch_bounds__(32) k_ray_first_warp(QueryCtx q, WalkTree tree
 		if (hits >= 1u)
 			stack[size + __popc(one & ~lt) - 1u] = make_uint2(a, __float_as_uint(ta));
 		size += __popc(one);
-		float least = fminf(limit, ray_limit(bestOut.fraction));
+		float least = fminf(limit, ray_limit(bestOut.fraction, turned));
 		for (int o = 16; o > 0; o >>= 1)
 			least = fminf(least, __shfl_xor_sync(0xFFFFFFFFu, least, o));
 		limit = least;
@@ -1074,8 +1082,11 @@ __global__ void __launch_bounds__(32) k_ray_first_warp(QueryCtx q, WalkTree tree
 constexpr uint32_t RAY_WARP_MAX = 148u * 160u;
 
 // The tree laid out for the ordered walks, in the context's own records.
-WalkTree launch_walk_tree(b3g_ctx* c, const QueryCtx& q, uint32_t* turned, cudaStream_t s)
+// turned: see k_walk_tree; cleared by each pass and only set here, so that calls
+// on several streams, which write the same records, never see it go back to 0.
+WalkTree launch_walk_tree(b3g_ctx* c, const QueryCtx& q, uint32_t*& turned, cudaStream_t s)
 {
+	turned = c->anyTriangle ? c->buf.counters + CTR_WALK_TURNED : nullptr;
 	WalkTree t;
 	float4* nodes = c->buf.walkTree;
 	float4* leaves = nodes + 4 * (size_t)c->cfg.max_proxies;
@@ -1089,15 +1100,17 @@ WalkTree launch_walk_tree(b3g_ctx* c, const QueryCtx& q, uint32_t* turned, cudaS
 void launch_ray_first(b3g_ctx* c, const QueryCtx& q, const float* rays, const uint32_t* worlds, uint32_t n, uint32_t* fix,
 	float* hit, cudaStream_t s)
 {
-	const WalkTree t = launch_walk_tree(c, q, nullptr, s);
+	uint32_t* turned;
+	const WalkTree t = launch_walk_tree(c, q, turned, s);
 	if (n <= RAY_WARP_MAX)
-		k_ray_first_warp<<<n, 32, 0, s>>>(q, t, rays, worlds, n, fix, hit);
+		k_ray_first_warp<<<n, 32, 0, s>>>(q, t, rays, worlds, n, turned, fix, hit);
 	else
 	{
 		// Resident warps, each with an equal share of at least a warp's rays.
 		const uint32_t warps = std::min((n + 31u) / 32u, 148u * RAY_BLOCKS * RAY_WARPS);
 		const uint32_t share = (n + warps - 1u) / warps;
-		k_ray_first<<<(warps + RAY_WARPS - 1u) / RAY_WARPS, RAY_WARPS * 32, 0, s>>>(q, t, rays, worlds, n, share, fix, hit);
+		k_ray_first<<<(warps + RAY_WARPS - 1u) / RAY_WARPS, RAY_WARPS * 32, 0, s>>>(q, t, rays, worlds, n, share, turned,
+			fix, hit);
 	}
 }
 
@@ -1746,9 +1759,7 @@ __global__ void __launch_bounds__(CAST_WARPS * 32, CAST_BLOCKS) k_shape_cast_fir
 void launch_shape_cast_first(b3g_ctx* c, const QueryCtx& q, const float* casts, uint32_t n, uint32_t* fix, float* hit,
 	cudaStream_t s)
 {
-	// Cleared by each pass and only set here, so that calls on several streams,
-	// which write the same records, never see it go back to 0.
-	uint32_t* turned = c->anyTriangle ? c->buf.counters + CTR_WALK_TURNED : nullptr;
+	uint32_t* turned;
 	const WalkTree t = launch_walk_tree(c, q, turned, s);
 	// As many lanes to a cast as leave the GPU about 16 warps per SM: 16,384
 	// casts took 1.17 ms with 4 lanes each, 1.23 ms with 16.

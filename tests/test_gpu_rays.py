@@ -143,3 +143,20 @@ def test_long_rays_past_sharp_hulls(n):
         sc.add_fixture(b, N.SHAPE_HULL, [0.0], hull=shapes[i % 3])
     sc.finalize()
     same_first_hit(sc, tangent_rays(sc, n, rng))
+
+
+# Triangles of a body away from the identity are not where their boxes are
+# (triangle_shape.cpp:59-67): a ray can hit one, then a body, and only then
+# meet the triangle's box.
+@pytest.mark.parametrize("n", BATCHES)
+@pytest.mark.parametrize("shift", [(0.3, 2.0, -0.2), (0.0, -1.5, 0.0)])
+def test_triangles_outside_their_boxes(shift, n):
+    rng = np.random.default_rng(n)
+    sc = S.terrain_scene(seed=5, n=300)
+    sc.body_pos[0] = shift
+    sc.finalize()
+    p1 = rng.uniform(-8, 8, (n, 3))
+    p1[:, 1] = np.where(rng.random(n) < 0.5, 7.0, -7.0)
+    d = rng.normal(size=(n, 3)) * (1.0, 0.0, 1.0)
+    d[:, 1] = -2.0 * p1[:, 1]
+    same_first_hit(sc, np.concatenate([p1, p1 + d], axis=1))
