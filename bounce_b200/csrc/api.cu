@@ -183,20 +183,20 @@ __global__ void k_touch_scatter(const DevManifold* man, const DevManifold* extra
 // The packed touching output: k_pack_list finds every manifold with points in
 // contact order and its place (an exclusive scan of manifolds and 8-byte
 // words, 1,024 contacts a tile), k_pack_copy moves the records, 16 lanes each.
-// Two kernels that go by the device's counts, for what were two per-contact
+// Two kernels that go by the counts on the device, for what were two per-contact
 // kernels, two scans and their memsets after the host had seen the counts:
 // 85 us of a step of 65,536 mixed bodies with the gaps between them, now 33.
 //
 // A list entry: x = contact (bits 0-27; a contact takes 640 bytes of manifolds
 // alone), manifold (28-29) and points - 1 (30-31), y = its first word.
 __global__ void __launch_bounds__(SC_THREADS) k_pack_list(Buffers B, uint32_t cur, uint32_t cap,
-	unsigned long long* state, uint2* list)
+	const uint32_t* counts, unsigned long long* state, uint2* list)
 {
 	__shared__ uint32_t sTile;
 	__shared__ unsigned long long sPrefix;
 	constexpr uint32_t ITEMS = 4, TILE = SC_THREADS * ITEMS;
 	const uint32_t t = threadIdx.x;
-	const uint32_t n = min(B.counters[CTR_PAIRS], cap);
+	const uint32_t n = min(counts[CTR_PAIRS], cap);
 	const DevManifold* man = B.man[cur];
 	const DevManifold* extra = B.extraMan[cur];
 	for (;;)
@@ -257,12 +257,12 @@ __global__ void __launch_bounds__(SC_THREADS) k_pack_list(Buffers B, uint32_t cu
 }
 
 // Also clears the scan's states for the next call.
-__global__ void __launch_bounds__(256) k_pack_copy(Buffers B, uint32_t cur, uint32_t cap, unsigned long long* state,
-	uint32_t states, const uint2* list)
+__global__ void __launch_bounds__(256) k_pack_copy(Buffers B, uint32_t cur, uint32_t cap, const uint32_t* counts,
+	unsigned long long* state, uint32_t states, const uint2* list)
 {
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < states; i += gridDim.x * blockDim.x)
 		state[i] = 0ull;
-	const uint32_t n = min(B.counters[CTR_MANIFOLDS], cap);
+	const uint32_t n = min(counts[CTR_MANIFOLDS], cap);
 	unsigned long long* out = reinterpret_cast<unsigned long long*>(B.touchMan);
 	const uint32_t lane = threadIdx.x & 15u;
 	for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) / 16u; k < n; k += gridDim.x * blockDim.x / 16u)
@@ -771,6 +771,7 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 		cudaEventDestroy(c->copyReady);
 	dfree(c->packList);
 	dfree(c->packStates);
+	dfree(c->packCounts);
 	if (c->stageOut)
 		cudaFreeHost(c->stageOut);
 	for (cudaEvent_t e : {c->countsReady, c->impulsesStaged, c->awakeStaged})
@@ -1480,6 +1481,17 @@ static cudaError_t refresh_awake(b3g_ctx* c)
 	return e;
 }
 
+// A caller's stream s waits for e, if it is pending. Under capture e becomes a
+// node of the graph whether or not it is: the replays come later.
+static cudaError_t wait_event(cudaStream_t s, cudaEvent_t e, bool pending)
+{
+	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+	const cudaError_t rc = cudaStreamIsCapturing(s, &st);
+	if (rc == cudaSuccess && st == cudaStreamCaptureStatusActive)
+		return cudaStreamWaitEvent(s, e, cudaEventWaitExternal);
+	return rc == cudaSuccess && pending ? cudaStreamWaitEvent(s, e, 0) : rc;
+}
+
 // Work on s that uses what b3g_load_impulses or b3g_set_awake has on the way.
 static cudaError_t wait_staged(b3g_ctx* c, cudaStream_t s)
 {
@@ -1855,6 +1867,13 @@ static void wait_copies(b3g_ctx* c, cudaStream_t s)
 		cudaStreamWaitEvent(s, c->copyDone, 0);
 }
 
+// A pass on a caller's stream after one on the context's, whose results may
+// still be packed by its counters (b3g_fetch_results_packed_async).
+static cudaError_t wait_packing(b3g_ctx* c, cudaStream_t s)
+{
+	return s == c->stream ? cudaSuccess : wait_event(s, c->copyReady, c->packing);
+}
+
 // Kernels of a pass's narrowphase: bucketing, the pairs apart or without a
 // hull, the other convex buckets (with the hull-sphere and hull-capsule follow-up kernels), the hull
 // probe and SAT, hull-triangle, and the mesh work.
@@ -1912,6 +1931,8 @@ extern "C" int b3g_collide(b3g_ctx* c, const float* state, int onDevice, void* s
 		return fail(c, B3G_E_INVALID, "b3g_collide: the last pass waits for b3g_finish_pass");
 	c->countsFetched = false;
 	CK(wait_staged(c, s));
+	CK(wait_packing(c, s));
+	c->lastStream = s;
 	// Filters of this pass: the caller's contact filter (a host round trip in
 	// the middle of the pass), else joints or a contact veto (inside the pass).
 	c->filterMode = (c->cfg.flags & B3G_FLAG_CONTACT_FILTER) ? 2 : ((c->nJoints || c->nVeto) ? 1 : 0);
@@ -2406,24 +2427,37 @@ extern "C" int b3g_fetch_results_packed_async(b3g_ctx* c, uint32_t* contacts, ui
 	CK(cudaSetDevice(c->device));
 	Buffers& B = c->buf;
 	const uint32_t cap = c->cfg.max_contacts;
+	const uint32_t states = (cap + 1023u) / 1024u + 1u;
+	// The packing kernels run on the context's stream while the host goes on. A
+	// pass on the same stream follows them; one on a caller's stream clears its
+	// counters beside them, so they go by a copy of the last pass's (which adds
+	// 2-6 us to a host step) where passes run on such a stream, and a pass
+	// on one after a pass on the context's waits for them (wait_packing).
+	const bool beside = c->lastStream != c->stream;
+	if (touchCapacity && !c->packList)
+	{
+		CK(dalloc(&c->packCounts, CTR_BUCKET0));
+		CK(dalloc(&c->packStates, states));
+		CK(cudaMemsetAsync(c->packStates, 0, sizeof(unsigned long long) * states, c->stream));
+		CK(dalloc(&c->packList, cap));
+	}
 	CK(cudaMemcpyAsync(c->hCounters, B.counters, sizeof(uint32_t) * CTR_COUNT, cudaMemcpyDeviceToHost, c->stream));
+	if (touchCapacity && beside)
+		CK(cudaMemcpyAsync(c->packCounts, B.counters, sizeof(uint32_t) * CTR_BUCKET0, cudaMemcpyDeviceToDevice,
+			c->stream));
 	CK(cudaEventRecord(c->countsReady, c->stream));
 	if (touchCapacity)
 	{
-		// Packed while the host waits for the counts: the kernels go by the
-		// device's.
-		const uint32_t states = (cap + 1023u) / 1024u + 1u;
-		if (!c->packList)
-		{
-			CK(dalloc(&c->packList, cap));
-			CK(dalloc(&c->packStates, states));
-			CK(cudaMemsetAsync(c->packStates, 0, sizeof(unsigned long long) * states, c->stream));
-		}
+		const uint32_t* packCounts = beside ? c->packCounts : B.counters;
+		// The next pass writes the other parity's contacts, and the one after it
+		// waits for copyDone.
 		wait_copies(c, c->stream);
-		k_pack_list<<<work_blocks(cap, 1024, 4), SC_THREADS, 0, c->stream>>>(B, c->cur, cap, c->packStates, c->packList);
-		k_pack_copy<<<work_blocks(16ull * cap, 256, 8), 256, 0, c->stream>>>(B, c->cur, cap, c->packStates, states,
-			c->packList);
+		k_pack_list<<<work_blocks(cap, 1024, 4), SC_THREADS, 0, c->stream>>>(B, c->cur, cap, packCounts,
+			c->packStates, c->packList);
+		k_pack_copy<<<work_blocks(16ull * cap, 256, 8), 256, 0, c->stream>>>(B, c->cur, cap, packCounts,
+			c->packStates, states, c->packList);
 		CK(cudaEventRecord(c->copyReady, c->stream));
+		c->packing = !beside;
 	}
 	CK(cudaEventSynchronize(c->countsReady));
 	c->countsFetched = true;
@@ -2437,11 +2471,14 @@ extern "C" int b3g_fetch_results_packed_async(b3g_ctx* c, uint32_t* contacts, ui
 	counts->points = h[CTR_POINTS];
 	counts->moved = h[CTR_MOVED];
 	counts->status = status_code(h[CTR_STATUS]);
+	const uint32_t total = h[CTR_MANIFOLDS];
+	const uint64_t bytes = 32ull * total + 72ull * h[CTR_POINTS];
+	// Nothing is copied then, so that no later pass would wait for the packing.
+	if (touchCapacity && (counts->status || total > cap || total > touchCapacity || bytes > packedCapacity))
+		CK(cudaStreamSynchronize(c->stream));
 	if (counts->status)
 		return fail(c, -(int)counts->status, "pass status 0x%x (pairs %u, capacity %u)", h[CTR_STATUS], h[CTR_PAIRS],
 			c->cfg.max_contacts);
-	const uint32_t total = h[CTR_MANIFOLDS];
-	const uint64_t bytes = 32ull * total + 72ull * h[CTR_POINTS];
 	if (total > c->cfg.max_contacts)
 		return fail(c, B3G_E_CAPACITY, "b3g_fetch_results_packed_async: %u manifolds exceed the output buffer", total);
 	if (touchCapacity && (total > touchCapacity || bytes > packedCapacity))
@@ -2479,9 +2516,10 @@ extern "C" int b3g_fetch_results_packed_async(b3g_ctx* c, uint32_t* contacts, ui
 	CK(cudaStreamWaitEvent(c->copyStream, c->countsReady, 0));
 	if (nc)
 		CK(cudaMemcpyAsync(contacts, B.contactOut, contactBytes, cudaMemcpyDeviceToHost, c->copyStream));
+	if (touchCapacity)
+		CK(cudaStreamWaitEvent(c->copyStream, c->copyReady, 0));
 	if (nt)
 	{
-		CK(cudaStreamWaitEvent(c->copyStream, c->copyReady, 0));
 		CK(cudaMemcpyAsync(index, B.touchIndex, sizeof(uint32_t) * nt, cudaMemcpyDeviceToHost, c->copyStream));
 		CK(cudaMemcpyAsync(packed, B.touchMan, (size_t)bytes, cudaMemcpyDeviceToHost, c->copyStream));
 	}

@@ -368,6 +368,9 @@ struct b3g_ctx
 	bool copyPending;
 	uint2* packList;          // b3g_fetch_results_packed_async: manifolds with points (k_pack_list)
 	unsigned long long* packStates; // ... its scan's states, 0 between calls
+	uint32_t* packCounts;     // ... the pass's first counters, as the call found them
+	bool packing;             // it may still go by the counters themselves
+	cudaStream_t lastStream;  // of the last pass
 	cudaEvent_t countsReady;  // the last fetch's counts are on the host
 	bool countsFetched;       // hCounters are those of the last pass, which has ended
 	char *stageOut, *stageImpulses, *stageAwake; // pinned, B3G_STAGE_BYTES each (allocated on first use)

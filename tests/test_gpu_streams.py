@@ -1,0 +1,106 @@
+"""GPU: one context's calls over several streams and under capture: what a call
+leaves under way when it returns may not be overtaken by the next one, and what
+could be captured or run asynchronously still can."""
+import numpy as np
+import pytest
+
+from bounce_b200 import _native as N
+from bounce_b200 import scene as S
+from bounce_b200.pipeline import CollisionPipeline
+
+pytestmark = pytest.mark.gpu
+
+
+def mixed(n):
+    return S.mixed_scene(seed=n, n=n, side=max(3.0, 49.0 * (n / 65536.0) ** (1 / 3))).finalize()
+
+
+def states_of(sc, passes):
+    drv = S.KinematicDriver(sc)
+    out = []
+    for _ in range(passes):
+        out.append(drv.state17().copy())
+        drv.advance()
+    return out
+
+
+def packed_of(manifolds):
+    return b"".join(m.tobytes()[288:] + m["points"][: int(m["pointCount"])].tobytes() for m in manifolds)
+
+
+# The results of a pass are packed while the next pass already runs on the
+# caller's stream; the largest packs for longer than that pass takes to clear
+# its counters. Spheres apart: contacts, but nothing to pack.
+@pytest.mark.parametrize("kind,n", [("mixed", 30), ("mixed", 3000), ("mixed", 30000), ("apart", 2000)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_packed_results_beside_the_next_pass(kind, n, graph):
+    torch = pytest.importorskip("torch")
+    if kind == "mixed":
+        sc = mixed(n)
+    else:
+        sc = S.Scene()
+        for i in range(n):
+            b = sc.add_body(0, N.BODY_DYNAMIC, (1.1 * (i % 50), 1.1 * (i // 50), 0), (0, 0, 0, 1), lin=(0, 0, 1 + i % 3))
+            sc.add_fixture(b, N.SHAPE_SPHERE, [0, 0, 0, 0.5])
+        sc.finalize()
+    states = states_of(sc, 8)
+    ref = CollisionPipeline(sc)
+    want = []
+    for st in states:
+        ref.collide(st)
+        index, man = ref.touching()
+        want.append((ref.contacts(), index, packed_of(man)))
+    ref.close()
+    pipe = CollisionPipeline(sc, graph=graph)
+    s = torch.cuda.Stream()
+    on_device = [torch.from_numpy(st).cuda() for st in states]
+    room = max(len(w[2]) for w in want) + 8
+    make = lambda shape, dt: torch.zeros(shape, dtype=dt, pin_memory=True).numpy()
+    contacts = make((max(len(w[0]) for w in want), 3), torch.int32).view(np.uint32)
+    index = make((max(len(w[1]) for w in want) + 1,), torch.int32).view(np.uint32)
+    packed = make((room,), torch.uint8)
+    torch.cuda.synchronize()
+    pipe.collide(on_device[0].data_ptr(), on_device=True, stream=s.cuda_stream)
+    for k, (c, i, p) in enumerate(want):
+        s.synchronize()
+        counts = pipe.fetch_results_packed_async(contacts, index, packed)
+        if k + 1 < len(states):
+            pipe.collide(on_device[k + 1].data_ptr(), on_device=True, stream=s.cuda_stream)
+        pipe.wait_results()
+        assert counts["contacts"] == len(c) and counts["manifolds"] == len(i)
+        assert np.array_equal(contacts[: len(c)], c)
+        assert np.array_equal(index[: len(i)], i)
+        assert packed[: len(p)].tobytes() == p
+    pipe.close()
+
+
+# A pass on the context's own stream, its results being packed, then a pass on a
+# caller's.
+def test_packed_results_before_a_pass_on_another_stream():
+    torch = pytest.importorskip("torch")
+    sc = mixed(30000)
+    states = states_of(sc, 6)
+    ref = CollisionPipeline(sc)
+    pipe = CollisionPipeline(sc)
+    s = torch.cuda.Stream()
+    on_device = [torch.from_numpy(st).cuda() for st in states]
+    torch.cuda.synchronize()
+    make = lambda shape, dt: torch.zeros(shape, dtype=dt, pin_memory=True).numpy()
+    contacts = make((40 * sc.n_fixtures, 3), torch.int32).view(np.uint32)
+    index, packed = make((8 * sc.n_fixtures,), torch.int32).view(np.uint32), make((8 * sc.n_fixtures * 320,), torch.uint8)
+    for k in range(0, len(states), 2):
+        ref.collide(states[k])
+        want_index, man = ref.touching()
+        want, p = ref.contacts(), packed_of(man)
+        pipe.collide(on_device[k].data_ptr(), on_device=True)
+        counts = pipe.fetch_results_packed_async(contacts, index, packed)
+        pipe.collide(on_device[k + 1].data_ptr(), on_device=True, stream=s.cuda_stream)
+        pipe.wait_results()
+        assert np.array_equal(contacts[: counts["contacts"]], want)
+        assert np.array_equal(index[: counts["manifolds"]], want_index)
+        assert packed[: len(p)].tobytes() == p
+        ref.collide(states[k + 1])
+        s.synchronize()
+        assert np.array_equal(pipe.contacts(), ref.contacts())
+    ref.close()
+    pipe.close()
