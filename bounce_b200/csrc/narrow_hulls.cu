@@ -195,7 +195,9 @@ __host__ __device__ __forceinline__ uint32_t sat_warp_recs(uint32_t maxUE)
 
 // The warps that share one hull pair's edge query: this one is `part` of
 // `parts`, they meet at barrier `bar` of their block, and slot[] holds one
-// (separation, pair) per part in shared memory.
+// (separation, pair) per part in shared memory. The barrier has no limit: every
+// warp of the pair comes to it or none does, since they run the same queries on
+// the same values up to it.
 struct EdgeParts
 {
 	uint32_t part, parts, bar;
@@ -1473,18 +1475,17 @@ __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 		}
 		__syncwarp();
 	}
-	__shared__ float2 partBest[2][W];
+	__shared__ float2 partBest[W];
 	uint32_t n = *a.missCount;
 	uint32_t nw = gridDim.x * W;
 	const uint32_t parts = !a.convexCache ? 1u : (W >= 4 && 4u * n <= nw ? 4u : (2u * n <= nw ? 2u : 1u));
-	uint32_t turn = 0;
-	for (uint32_t t = (blockIdx.x * W + warp) / parts; t < n; t += nw / parts, turn ^= 1u)
+	// Warps that share have one pair each: parts * n <= nw.
+	for (uint32_t t = (blockIdx.x * W + warp) / parts; t < n; t += nw / parts)
 	{
 		uint32_t c = a.missList[t];
 		HullCtx H;
 		load_hull_ctx(a, c, H);
-		// The slots alternate: a warp may be a pair ahead of one still reading.
-		H.parts = EdgeParts{warp % parts, parts, 1u + warp / parts, &partBest[turn][warp / parts * parts]};
+		H.parts = EdgeParts{warp % parts, parts, 1u + warp / parts, &partBest[warp / parts * parts]};
 		H.recs = recs;
 		H.clip = reinterpret_cast<WarpClip*>(wsm);
 		H.maxUE = maxUE;
@@ -1510,11 +1511,24 @@ __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 			if (!__all_sync(0xffffffffu, ok))
 			{
 				// The copies did not land in time: report it, wait (bounded)
-				// for them before the shared memory goes away, and stop.
+				// for them before the shared memory goes away, and stop. A warp
+				// that shares its pair brings the hulls in itself (the same
+				// values) and goes on: the others wait for it where their edge
+				// queries meet.
 				if (lane == 0)
 					atomicOr(a.status, B3G_ST_WAIT_TIMEOUT);
 				stage_wait(bar, phase);
-				return;
+				if (parts == 1)
+					return;
+				for (uint32_t i = lane; i < H.h1.vCnt; i += 32)
+					v1[i] = H.h1.v[i];
+				for (uint32_t i = lane; i < H.h1.fCnt; i += 32)
+					p1[i] = H.h1.p[i];
+				for (uint32_t i = lane; i < H.h2.vCnt; i += 32)
+					v2[i] = H.h2.v[i];
+				for (uint32_t i = lane; i < H.h2.fCnt; i += 32)
+					p2[i] = H.h2.p[i];
+				__syncwarp();
 			}
 			phase ^= 1u;
 			H.h1.v = v1;
