@@ -1481,26 +1481,31 @@ static cudaError_t refresh_awake(b3g_ctx* c)
 	return e;
 }
 
+static bool in_capture(cudaStream_t s)
+{
+	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(s, &st) == cudaSuccess)
+		return st != cudaStreamCaptureStatusNone;
+	cudaGetLastError();
+	return false;
+}
+
 // A caller's stream s waits for e, if it is pending. Under capture e becomes a
 // node of the graph whether or not it is: the replays come later.
 static cudaError_t wait_event(cudaStream_t s, cudaEvent_t e, bool pending)
 {
-	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-	const cudaError_t rc = cudaStreamIsCapturing(s, &st);
-	if (rc == cudaSuccess && st == cudaStreamCaptureStatusActive)
+	if (in_capture(s))
 		return cudaStreamWaitEvent(s, e, cudaEventWaitExternal);
-	return rc == cudaSuccess && pending ? cudaStreamWaitEvent(s, e, 0) : rc;
+	return pending ? cudaStreamWaitEvent(s, e, 0) : cudaSuccess;
 }
 
 // Work on s that uses what b3g_load_impulses or b3g_set_awake has on the way.
 static cudaError_t wait_staged(b3g_ctx* c, cudaStream_t s)
 {
-	// Nothing is asked of a stream (it may be under capture) that has nothing to
-	// wait for.
-	if (s == c->stream || !c->staged)
+	if (s == c->stream)
 		return cudaSuccess;
-	cudaError_t e = cudaStreamWaitEvent(s, c->impulsesStaged, 0);
-	return e == cudaSuccess ? cudaStreamWaitEvent(s, c->awakeStaged, 0) : e;
+	const cudaError_t e = wait_event(s, c->impulsesStaged, c->staged);
+	return e == cudaSuccess ? wait_event(s, c->awakeStaged, c->staged) : e;
 }
 
 // After an update whose records the host has not seen.
@@ -1933,6 +1938,7 @@ extern "C" int b3g_collide(b3g_ctx* c, const float* state, int onDevice, void* s
 	CK(wait_staged(c, s));
 	CK(wait_packing(c, s));
 	c->lastStream = s;
+	c->captured = c->captured || in_capture(s);
 	// Filters of this pass: the caller's contact filter (a host round trip in
 	// the middle of the pass), else joints or a contact veto (inside the pass).
 	c->filterMode = (c->cfg.flags & B3G_FLAG_CONTACT_FILTER) ? 2 : ((c->nJoints || c->nVeto) ? 1 : 0);
@@ -2790,7 +2796,7 @@ extern "C" int b3g_load_impulses(b3g_ctx* c, const float* normal, const float* t
 		return fail(c, B3G_E_INVALID, "null argument");
 	uint32_t n;
 	CK(cudaSetDevice(c->device));
-	if (c->countsFetched && c->havePass)
+	if (c->countsFetched && c->havePass && !c->captured)
 		n = std::min(c->hCounters[CTR_PAIRS], c->cfg.max_contacts); // of a pass that has ended
 	else
 	{

@@ -104,3 +104,52 @@ def test_packed_results_before_a_pass_on_another_stream():
         assert np.array_equal(pipe.contacts(), ref.contacts())
     ref.close()
     pipe.close()
+
+
+# Two passes (one of each buffer parity) captured by the caller, after and before
+# flags and impulses have been handed in.
+@pytest.mark.parametrize("n", [40, 3000])
+def test_captured_passes(n):
+    torch = pytest.importorskip("torch")
+    sc = mixed(n)
+    states = states_of(sc, 12)
+    ref = CollisionPipeline(sc)
+    pipe = CollisionPipeline(sc)
+    awake = np.ones(sc.n_bodies, np.uint8)
+
+    def impulses(p, seed):
+        k = p.counts()["contacts"]
+        motor = np.random.default_rng(seed).uniform(0, 1, k).astype(np.float32)
+        p.load_impulses(np.zeros((k, 4), np.float32), np.zeros((k, 2), np.float32), motor)
+
+    for st in states[:2]:
+        for p in (ref, pipe):
+            p.set_awake(awake)
+            p.collide(st)
+    for p in (ref, pipe):
+        impulses(p, 0)
+        p.collide(states[2])
+        p.set_awake(awake)
+    slots = [torch.from_numpy(states[3]).cuda() for _ in range(2)]
+    graph = torch.cuda.CUDAGraph()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        for x in slots:
+            pipe.collide(x.data_ptr(), on_device=True, stream=stream.cuda_stream)
+    for k in range(3, 11, 2):
+        for p in (ref, pipe):
+            p.set_awake(awake)
+        for j, x in enumerate(slots):
+            x.copy_(torch.from_numpy(states[k + j]))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        ref.collide(states[k])
+        ref.collide(states[k + 1])
+        assert np.array_equal(pipe.contacts(), ref.contacts())
+        assert pipe.manifolds().tobytes() == ref.manifolds().tobytes()
+        assert np.array_equal(pipe.caches(), ref.caches())
+    graph.reset()
+    ref.close()
+    pipe.close()
