@@ -2179,6 +2179,7 @@ extern "C" int b3g_finish_pass(b3g_ctx* c, const uint8_t* keep, uint32_t count)
 			c->candFetched ? c->nCand : 0u);
 	CK(cudaSetDevice(c->device));
 	cudaStream_t s = c->passStream;
+	CK(wait_staged(c, s));
 	std::vector<uint32_t> rejected;
 	if (keep)
 		for (uint32_t i = 0; i < count; ++i)

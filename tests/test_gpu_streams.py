@@ -153,3 +153,35 @@ def test_captured_passes(n):
     graph.reset()
     ref.close()
     pipe.close()
+
+
+# Flags handed in between the halves of a filtered pass, on a caller's stream
+# as on the context's.
+def test_flags_between_the_halves_of_a_pass():
+    torch = pytest.importorskip("torch")
+    sc = mixed(20000)
+    states = states_of(sc, 5)
+    rng = np.random.default_rng(1)
+    flags = [(rng.random(sc.n_bodies) < 0.7).astype(np.uint8) for _ in states]
+    s = torch.cuda.Stream()
+    make = lambda shape, dt: torch.zeros(shape, dtype=dt, pin_memory=True).numpy()
+    contacts = make((40 * sc.n_fixtures, 3), torch.int32).view(np.uint32)
+    index, packed = make((8 * sc.n_fixtures,), torch.int32).view(np.uint32), make((8 * sc.n_fixtures * 320,), torch.uint8)
+    out = []
+    for stream in (None, s.cuda_stream):
+        pipe = CollisionPipeline(sc, contact_filter=True)
+        got = []
+        for st, awake in zip(states, flags):
+            x = torch.from_numpy(st).cuda()
+            torch.cuda.synchronize()
+            pipe.collide(x.data_ptr(), on_device=True, stream=stream)
+            pipe.new_pairs()
+            pipe.set_awake(awake)
+            pipe.finish_pass()
+            s.synchronize()
+            pipe.fetch_results_packed_async(contacts, index, packed)
+            got.append((pipe.contacts(), pipe.manifolds().tobytes(), pipe.awake()))
+        out.append(got)
+        pipe.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(a[2], b[2])
