@@ -528,6 +528,7 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 	step(cudaEventCreateWithFlags(&c->countsReady, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->impulsesStaged, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->awakeStaged, cudaEventDisableTiming), "cudaEventCreate");
+	step(cudaEventCreateWithFlags(&c->awakeOut, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->copyDone, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaStreamCreateWithFlags(&c->sideStream, cudaStreamNonBlocking), "cudaStreamCreate");
 	step(cudaEventCreateWithFlags(&c->forkEvent, cudaEventDisableTiming), "cudaEventCreate");
@@ -774,7 +775,7 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 	dfree(c->packCounts);
 	if (c->stageOut)
 		cudaFreeHost(c->stageOut);
-	for (cudaEvent_t e : {c->countsReady, c->impulsesStaged, c->awakeStaged})
+	for (cudaEvent_t e : {c->countsReady, c->impulsesStaged, c->awakeStaged, c->awakeOut})
 		if (e)
 			cudaEventDestroy(e);
 	if (c->edgeBuf)
@@ -1466,16 +1467,21 @@ static cudaError_t reserve_stage(b3g_ctx* c)
 	return e;
 }
 
-// The host copy of the awake flags, before a scene update changes some: a pass
-// with sleeping bodies leaves it behind.
+// The host copy of the awake flags, before the host changes some of it: a pass
+// with sleeping bodies leaves it behind. Waits for that pass's flags and for
+// nothing else (the side stream's work ended before them). An update from device
+// memory since may have set some flags; they count as awake then, and the sleep
+// count stays the upper bound that it is after such an update.
 static cudaError_t refresh_awake(b3g_ctx* c)
 {
 	if (c->awakeStale == 0)
 		return cudaSuccess;
-	cudaError_t e = cudaDeviceSynchronize();
+	cudaError_t e = cudaStreamWaitEvent(c->sideStream, c->awakeOut, 0);
 	if (e == cudaSuccess)
-		e = cudaMemcpy(c->hAwake.data(), c->dBodyAwake, std::min<size_t>(c->awakeStale, c->hAwake.size()),
-			cudaMemcpyDeviceToHost);
+		e = cudaMemcpyAsync(c->hAwake.data(), c->dBodyAwake, std::min<size_t>(c->awakeStale, c->hAwake.size()),
+			cudaMemcpyDeviceToHost, c->sideStream);
+	if (e == cudaSuccess)
+		e = cudaStreamSynchronize(c->sideStream);
 	if (e == cudaSuccess)
 		c->awakeStale = 0;
 	return e;
@@ -1554,7 +1560,6 @@ extern "C" int b3g_update_scene_device(b3g_ctx* c, uint32_t nb, const uint32_t* 
 	u.fFlags = flags;
 	u.fParams = params;
 	u.rIdx = retireIndex;
-	CK(refresh_awake(c));
 	CK(wait_staged(c, s));
 	launch_update(c, u, s);
 	CK(cudaGetLastError());
@@ -1584,7 +1589,6 @@ extern "C" int b3g_swap_worlds(b3g_ctx* c, uint32_t nRetire, const uint32_t* ret
 		return B3G_OK;
 	CK(cudaSetDevice(c->device));
 	cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-	CK(refresh_awake(c));
 	CK(wait_staged(c, s));
 	const UpdateLimits lim{c->capBodies, c->capFixtures, c->nWorlds, c->nHulls, c->dUpdateBad};
 	WorldRanges r;
@@ -1738,6 +1742,7 @@ extern "C" int b3g_set_active(b3g_ctx* c, uint32_t bodies, uint32_t fixtures)
 		return B3G_OK;
 	CK(cudaSetDevice(c->device));
 	CK(cudaDeviceSynchronize());
+	CK(refresh_awake(c));
 	destroy_graphs(c);
 	c->nBodies = bodies;
 	c->nFixtures = fixtures;

@@ -439,6 +439,7 @@ struct b3g_ctx
 	bool fixTypeStale;           // hFixType lags device-side scene updates
 	std::vector<uint8_t> hAwake; // host copy of the awake flags (sleep count)
 	uint32_t awakeStale;         // its first flags that the last pass may have changed (refresh_awake)
+	cudaEvent_t awakeOut;        // the flags as that pass left them
 	float4* dFixParams;
 	float4* dFixBound;
 

@@ -615,6 +615,8 @@ int resolve_wakeups(b3g_ctx* c, cudaStream_t s)
 	const int nbBlocks = (int)std::min<uint32_t>((c->nBodies + 255) / 256, 148u * 4u);
 	k_awake_out<<<nbBlocks, 256, 0, s>>>(c->scene, B, c->dBodyAwake, c->nBodies);
 	++launches;
+	if (cudaEventRecord(c->awakeOut, s) != cudaSuccess)
+		return B3G_E_CUDA;
 	c->awakeStale = std::max(c->awakeStale, c->nBodies);
 	// Bodies past the processed prefix keep their flags.
 	for (uint32_t b = c->nBodies; b < c->hAwake.size(); ++b)

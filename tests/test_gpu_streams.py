@@ -185,3 +185,62 @@ def test_flags_between_the_halves_of_a_pass():
         pipe.close()
     for a, b in zip(*out):
         assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(a[2], b[2])
+
+
+# Scene updates after a pass with sleeping bodies: asynchronous on their stream
+# (they wait for no work of others), and the next pass sees their bodies awake.
+@pytest.mark.parametrize("how", ["host", "device", "swap"])
+def test_updates_after_a_pass_with_sleepers(how):
+    torch = pytest.importorskip("torch")
+    sc = mixed(600)
+    states = states_of(sc, 4)
+    rng = np.random.default_rng(3)
+    awake = (rng.random(sc.n_bodies) < 0.5).astype(np.uint8)
+    first, count = 100, 30
+    b = np.arange(first, first + count, dtype=np.uint32)
+    world, btype = sc.body_world[b], sc.body_type[b]
+    ftype, fhull, fflags = sc.fix_type[b], sc.fix_hull[b], sc.fix_flags[b]
+    fparams = np.ascontiguousarray(sc.fix_params.reshape(-1, 12)[b])
+    assert np.array_equal(sc.fix_body[b], b)
+    other, mine = torch.cuda.Stream(), torch.cuda.Stream()
+    results = []
+    for busy in (False, True):
+        pipe = CollisionPipeline(sc)
+        pipe.collide(states[0])
+        pipe.set_awake(awake)
+        pipe.collide(states[1])
+        p = lambda a: a.ctypes.data_as(N.ctypes.c_void_p)
+        dev = [torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1)).cuda()
+               for a in (b, world, btype, b, b, ftype, fhull, fparams, fflags, b - first)]
+        d = [N.ctypes.c_void_p(x.data_ptr()) for x in dev]
+        rows = torch.zeros((sc.n_bodies, 17), device="cuda")
+        torch.cuda.synchronize()
+        if busy:
+            with torch.cuda.stream(other):
+                torch.cuda._sleep(400_000_000)
+        s = N.ctypes.c_void_p(mine.cuda_stream)
+        if how == "host":
+            u32, u8, f32 = N.ctypes.c_uint32, N.ctypes.c_uint8, N.ctypes.c_float
+            on = np.ones(count, np.uint8)
+            pipe._check(pipe.lib.b3g_update_scene(
+                pipe.ctx, count, N.ptr(b, u32), N.ptr(world, u32), N.ptr(btype, u32), N.ptr(on, u8), count,
+                N.ptr(b, u32), N.ptr(b, u32), N.ptr(ftype, u32), N.ptr(fhull, u32), N.ptr(fparams, f32),
+                N.ptr(fflags, u32), 0, None, s))
+        elif how == "device":
+            pipe._check(pipe.lib.b3g_update_scene_device(
+                pipe.ctx, count, d[0], d[1], d[2], count, d[3], d[4], d[5], d[6], d[7], d[8], 0, None, s))
+        else:
+            admit = np.array([[first, count, 0, 0]], np.uint32)
+            t = N.WorldTemplates(*(x.value for x in (d[2], d[9], d[5], d[6], d[8], d[7])), rows.data_ptr(), rows.data_ptr())
+            pipe._check(pipe.lib.b3g_swap_worlds(
+                pipe.ctx, 0, None, 1, p(admit), N.ctypes.byref(t), N.ctypes.c_void_p(rows.data_ptr()),
+                N.ctypes.c_void_p(rows.data_ptr()), s))
+        assert not busy or not other.query()
+        torch.cuda.synchronize()
+        assert pipe.awake()[b].all()
+        for st in states[2:]:
+            pipe.collide(st)
+        results.append((pipe.contacts(), pipe.awake(), pipe.pass_stats()["asleep"]))
+        assert results[-1][2] == int(((results[-1][1] == 0) & (sc.body_type != N.BODY_STATIC)).sum())
+        pipe.close()
+    assert np.array_equal(results[0][0], results[1][0]) and np.array_equal(results[0][1], results[1][1])
