@@ -529,6 +529,7 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 	step(cudaEventCreateWithFlags(&c->impulsesStaged, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->awakeStaged, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->awakeOut, cudaEventDisableTiming), "cudaEventCreate");
+	step(cudaEventCreateWithFlags(&c->walkDone, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->copyDone, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaStreamCreateWithFlags(&c->sideStream, cudaStreamNonBlocking), "cudaStreamCreate");
 	step(cudaEventCreateWithFlags(&c->forkEvent, cudaEventDisableTiming), "cudaEventCreate");
@@ -562,7 +563,7 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 	step(dalloc(&B.worldEnd, P), "alloc");
 	step(dalloc(&B.proxyInfo, P), "alloc");
 	step(dalloc(&B.outOff, C), "alloc");
-	step(dalloc(&B.walkTree, 8 * (size_t)P), "alloc");
+	step(dalloc(&B.walkTree, walk_tree_words(P)), "alloc");
 	const size_t scanWords = scan_aux_words(std::max(P, C) + 1);
 	step(dalloc(&B.scanAux, scanWords + scan_aux_words(P + 1) + scan_aux_words(C)), "alloc");
 	B.passScan = reinterpret_cast<unsigned long long*>(B.scanAux + scanWords);
@@ -775,7 +776,7 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 	dfree(c->packCounts);
 	if (c->stageOut)
 		cudaFreeHost(c->stageOut);
-	for (cudaEvent_t e : {c->countsReady, c->impulsesStaged, c->awakeStaged, c->awakeOut})
+	for (cudaEvent_t e : {c->countsReady, c->impulsesStaged, c->awakeStaged, c->awakeOut, c->walkDone})
 		if (e)
 			cudaEventDestroy(e);
 	if (c->edgeBuf)
@@ -1487,7 +1488,7 @@ static cudaError_t refresh_awake(b3g_ctx* c)
 	return e;
 }
 
-static bool in_capture(cudaStream_t s)
+bool in_capture(cudaStream_t s)
 {
 	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
 	if (cudaStreamIsCapturing(s, &st) == cudaSuccess)

@@ -171,7 +171,7 @@ struct Buffers
 	uint2* leafData;      // per sorted leaf: its proxy's proxyInfo word and fixture key
 	uint32_t* leafOf;     // per proxy: its sorted leaf (set when the LBVH is built)
 	uint32_t* outOff;     // per contact: offsets of the touching output
-	float4* walkTree;     // the tree as the world queries walk it: 8 float4 per proxy (queries.cu)
+	float4* walkTree;     // the tree as the world queries walk it (queries.cu)
 	uint32_t* scanAux;    // scan state
 	unsigned long long* passScan; // scan states of the contact list (order.cu), cleared when the pass begins
 	uint32_t* rawA;       // overlapping pairs in traversal order (this pass)
@@ -279,6 +279,8 @@ __device__ __forceinline__ bool joint_excluded(const FilterArgs& F, uint32_t ba,
 
 // The pairs of one leaf after which CTR_TRAV_OVERFLOW counts the rest.
 #define B3G_TRAV_SLOTS 32u
+// Words (float4) of Buffers::walkTree: two records of 4 per proxy, and a flag.
+constexpr size_t walk_tree_words(uint32_t proxies) { return 8 * (size_t)proxies + 1; }
 // Each of the pinned buffers of reserve_stage.
 #define B3G_STAGE_BYTES ((size_t)1 << 18)
 
@@ -313,7 +315,6 @@ enum
 	CTR_TRAV_OVERFLOW,  // pairs of a leaf past its first B3G_TRAV_SLOTS
 	CTR_CANDIDATES,     // new pairs handed to the caller's contact filter
 	CTR_MESH_ALL,       // mesh contacts of the pass, skipped ones included
-	CTR_WALK_TURNED,    // a triangle fixture lies outside its box (queries.cu)
 	CTR_WAKE_INACTIVE,  // contacts the pass skipped as inactive
 	CTR_WAKE_SAVE,      // the counters from CTR_BUCKET0 to CTR_WAKE_ACTIVATED as the pass left them
 	CTR_COUNT = CTR_WAKE_SAVE + (CTR_WAKE_ACTIVATED - CTR_BUCKET0) + 1
@@ -382,6 +383,8 @@ struct b3g_ctx
 	cudaStream_t sideStream;  // hull-hull / hull-triangle narrowphase, beside the convex buckets
 	cudaStream_t meshStream;  // mesh midphase (tree queries, work items), beside both
 	cudaEvent_t forkEvent, joinEvent, meshFork, meshJoin;
+	bool walkBeside;              // the last world query that wrote Buffers::walkTree ran on a caller's stream
+	cudaEvent_t walkDone;         // ... its end there
 	void* qScratch;       // device scratch of the world queries
 	size_t qScratchBytes;
 	float2* dFixMaterial;         // per fixture: friction, restitution (b3g_set_materials)
@@ -579,6 +582,8 @@ inline void set_carveout(std::initializer_list<const void*> kernels)
 		if (cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, CARVEOUT_PERCENT) != cudaSuccess)
 			cudaGetLastError(); // a preference only
 }
+bool in_capture(cudaStream_t s);
+
 void carveout_api();
 void carveout_broadphase();
 void carveout_pairs();

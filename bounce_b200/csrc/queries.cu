@@ -595,7 +595,9 @@ struct WalkTree
 {
 	const float4* nodes;
 	const float4* leaves;
-	uint32_t count; // leaves
+	const uint32_t* turned; // see k_walk_tree; nullptr: no triangles
+	uint32_t count;         // leaves
+	bool own;               // the records are this call's alone
 };
 
 // A path's keys share one bit more at every level (64 key bits, then 32 index
@@ -773,10 +775,10 @@ __device__ __forceinline__ RayIn warp_ray(const RayWarp& W, uint32_t place)
 }
 
 __global__ void __launch_bounds__(RAY_WARPS * 32, RAY_BLOCKS) k_ray_first(QueryCtx q, WalkTree tree, const float* rays,
-	const uint32_t* worlds, uint32_t n, uint32_t share, const uint32_t* anyTurned, uint32_t* outFix, float* outHit)
+	const uint32_t* worlds, uint32_t n, uint32_t share, uint32_t* outFix, float* outHit)
 {
 	__shared__ RayWarp shared[RAY_WARPS];
-	const bool turned = anyTurned && *anyTurned;
+	const bool turned = tree.turned && *tree.turned;
 	const uint32_t lane = threadIdx.x & 31u;
 	RayWarp& W = shared[threadIdx.x >> 5];
 	const uint32_t warp = blockIdx.x * RAY_WARPS + (threadIdx.x >> 5);
@@ -985,10 +987,10 @@ __global__ void __launch_bounds__(RAY_WARPS * 32, RAY_BLOCKS) k_ray_first(QueryC
 constexpr uint32_t RAY_FRONT = 1024; // stack entries per warp
 
 __global__ void __launch_bounds__(32) k_ray_first_warp(QueryCtx q, WalkTree tree, const float* rays,
-	const uint32_t* worlds, uint32_t n, const uint32_t* anyTurned, uint32_t* outFix, float* outHit)
+	const uint32_t* worlds, uint32_t n, uint32_t* outFix, float* outHit)
 {
 	__shared__ uint2 stack[RAY_FRONT]; // reference, entry fraction (float bits)
-	const bool turned = anyTurned && *anyTurned;
+	const bool turned = tree.turned && *tree.turned;
 	const uint32_t lane = threadIdx.x;
 	const uint32_t lt = (1u << lane) - 1u;
 	const uint32_t i = blockIdx.x;
@@ -1081,37 +1083,70 @@ __global__ void __launch_bounds__(32) k_ray_first_warp(QueryCtx q, WalkTree tree
 // 124 and 286 us; at 40,000: 459 and 317 us.
 constexpr uint32_t RAY_WARP_MAX = 148u * 160u;
 
-// The tree laid out for the ordered walks, in the context's own records.
-// turned: see k_walk_tree; cleared by each pass and only set here, so that calls
-// on several streams, which write the same records, never see it go back to 0.
-WalkTree launch_walk_tree(b3g_ctx* c, const QueryCtx& q, uint32_t*& turned, cudaStream_t s)
+// The tree laid out for the ordered walks, in records that no other call writes
+// while this one's walk reads them (as read-only memory). They are the
+// context's, and a call waits for the last one's walk where that ran on another
+// stream. A captured call, whose replays the host does not see, has records of
+// its own, as nodes of its graph.
+cudaError_t launch_walk_tree(b3g_ctx* c, const QueryCtx& q, WalkTree& t, cudaStream_t s)
 {
-	turned = c->anyTriangle ? c->buf.counters + CTR_WALK_TURNED : nullptr;
-	WalkTree t;
 	float4* nodes = c->buf.walkTree;
+	t.own = s != c->stream && in_capture(s);
+	cudaError_t e = cudaSuccess;
+	if (t.own)
+		e = cudaMallocAsync((void**)&nodes, sizeof(float4) * walk_tree_words(c->cfg.max_proxies), s);
+	else if (s != c->stream || c->walkBeside)
+	{
+		// A walk on a caller's stream was recorded there. The stream may be gone
+		// by now and another have its handle, so a caller's always waits.
+		if (!c->walkBeside)
+			e = cudaEventRecord(c->walkDone, c->stream);
+		if (e == cudaSuccess)
+			e = cudaStreamWaitEvent(s, c->walkDone, 0);
+		c->walkBeside = s != c->stream;
+	}
+	if (e != cudaSuccess)
+	{
+		cudaGetLastError();
+		return e;
+	}
 	float4* leaves = nodes + 4 * (size_t)c->cfg.max_proxies;
+	uint32_t* turned = c->anyTriangle ? reinterpret_cast<uint32_t*>(nodes + 8 * (size_t)c->cfg.max_proxies) : nullptr;
+	if (turned)
+		e = cudaMemsetAsync(turned, 0, sizeof(uint32_t), s);
 	t.nodes = nodes;
 	t.leaves = leaves;
+	t.turned = turned;
 	t.count = q.leaves;
 	k_walk_tree<<<(q.leaves + 127) / 128, 128, 0, s>>>(q, nodes, leaves, turned);
-	return t;
+	return e;
 }
 
-void launch_ray_first(b3g_ctx* c, const QueryCtx& q, const float* rays, const uint32_t* worlds, uint32_t n, uint32_t* fix,
+// The call's walk is launched.
+cudaError_t end_walk(b3g_ctx* c, const WalkTree& t, cudaStream_t s)
+{
+	if (t.own)
+		return cudaFreeAsync(const_cast<float4*>(t.nodes), s);
+	return s == c->stream ? cudaSuccess : cudaEventRecord(c->walkDone, s);
+}
+
+cudaError_t launch_ray_first(b3g_ctx* c, const QueryCtx& q, const float* rays, const uint32_t* worlds, uint32_t n, uint32_t* fix,
 	float* hit, cudaStream_t s)
 {
-	uint32_t* turned;
-	const WalkTree t = launch_walk_tree(c, q, turned, s);
+	WalkTree t;
+	cudaError_t e = launch_walk_tree(c, q, t, s);
+	if (e != cudaSuccess)
+		return e;
 	if (n <= RAY_WARP_MAX)
-		k_ray_first_warp<<<n, 32, 0, s>>>(q, t, rays, worlds, n, turned, fix, hit);
+		k_ray_first_warp<<<n, 32, 0, s>>>(q, t, rays, worlds, n, fix, hit);
 	else
 	{
 		// Resident warps, each with an equal share of at least a warp's rays.
 		const uint32_t warps = std::min((n + 31u) / 32u, 148u * RAY_BLOCKS * RAY_WARPS);
 		const uint32_t share = (n + warps - 1u) / warps;
-		k_ray_first<<<(warps + RAY_WARPS - 1u) / RAY_WARPS, RAY_WARPS * 32, 0, s>>>(q, t, rays, worlds, n, share, turned,
-			fix, hit);
+		k_ray_first<<<(warps + RAY_WARPS - 1u) / RAY_WARPS, RAY_WARPS * 32, 0, s>>>(q, t, rays, worlds, n, share, fix, hit);
 	}
+	return end_walk(c, t, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1515,7 +1550,7 @@ constexpr int CAST_WARPS = 2;
 constexpr int CAST_BLOCKS = 6; // per SM: 8 took 1.21 ms, 12 took 1.43 ms
 
 __global__ void __launch_bounds__(CAST_WARPS * 32, CAST_BLOCKS) k_shape_cast_first(QueryCtx q, WalkTree tree,
-	const float* casts, uint32_t n, uint32_t lanesPerCast, const uint32_t* turned, uint32_t* outSingle, float* outHit)
+	const float* casts, uint32_t n, uint32_t lanesPerCast, uint32_t* outSingle, float* outHit)
 {
 	__shared__ float simplex[CAST_WARPS][LANE_SIMPLEX_WORDS * LANE_ROW];
 	__shared__ uint32_t candFix[CAST_WARPS][32];
@@ -1548,7 +1583,7 @@ __global__ void __launch_bounds__(CAST_WARPS * 32, CAST_BLOCKS) k_shape_cast_fir
 		sw.hi = vmax(a1.hi, a2.hi);
 		// A cast triangle's box does not move with it (the reference's quirk
 		// above): the swept box is then met as a whole, at fraction 0.
-		prune = in.type != B3G_SHAPE_TRIANGLE && !(turned && *turned);
+		prune = in.type != B3G_SHAPE_TRIANGLE && !(tree.turned && *tree.turned);
 		const float pad = 4.0f * B3G_LINEAR_SLOP + 1e-5f * coord_mag(sw.lo, sw.hi);
 		if (prune)
 			slab.init(a1.lo, a1.hi, in.d, pad);
@@ -1756,18 +1791,21 @@ __global__ void __launch_bounds__(CAST_WARPS * 32, CAST_BLOCKS) k_shape_cast_fir
 	}
 }
 
-void launch_shape_cast_first(b3g_ctx* c, const QueryCtx& q, const float* casts, uint32_t n, uint32_t* fix, float* hit,
-	cudaStream_t s)
+cudaError_t launch_shape_cast_first(b3g_ctx* c, const QueryCtx& q, const float* casts, uint32_t n, uint32_t* fix,
+	float* hit, cudaStream_t s)
 {
-	uint32_t* turned;
-	const WalkTree t = launch_walk_tree(c, q, turned, s);
+	WalkTree t;
+	cudaError_t e = launch_walk_tree(c, q, t, s);
+	if (e != cudaSuccess)
+		return e;
 	// As many lanes to a cast as leave the GPU about 16 warps per SM: 16,384
 	// casts took 1.17 ms with 4 lanes each, 1.23 ms with 16.
 	uint32_t lanes = 32;
 	while (lanes > 1u && (unsigned long long)n * lanes > 32ull * 148ull * 16ull)
 		lanes >>= 1;
 	const uint32_t perBlock = CAST_WARPS * (32u / lanes);
-	k_shape_cast_first<<<(n + perBlock - 1) / perBlock, CAST_WARPS * 32, 0, s>>>(q, t, casts, n, lanes, turned, fix, hit);
+	k_shape_cast_first<<<(n + perBlock - 1) / perBlock, CAST_WARPS * 32, 0, s>>>(q, t, casts, n, lanes, fix, hit);
+	return end_walk(c, t, s);
 }
 
 __device__ __forceinline__ uint32_t cast_expand10(uint32_t v)
@@ -1971,7 +2009,8 @@ extern "C" int b3g_ray_cast_single(b3g_ctx* c, uint32_t n, const float* rays, co
 	float* dHit = (float*)(base + fixBytes);
 	cudaStream_t s = c->stream;
 	cudaMemsetAsync(c->buf.counters + CTR_SCRATCH, 0, 4, s);
-	launch_ray_first(c, q, (const float*)dIn, dWorlds, n, dFix, dHit, s);
+	if (launch_ray_first(c, q, (const float*)dIn, dWorlds, n, dFix, dHit, s) != cudaSuccess)
+		return qfail(c, B3G_E_CUDA, "b3g_ray_cast_single: launch");
 	rc = q_status(c);
 	if (rc)
 		return rc;
@@ -2003,8 +2042,7 @@ extern "C" int b3g_ray_cast_single_device(b3g_ctx* c, uint32_t n, const float* r
 	q.leaves = c->treeLeaves;
 	q.status = c->buf.counters + CTR_SCRATCH;
 	cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-	launch_ray_first(c, q, rays, worlds, n, fixture, hit, s);
-	if (cudaGetLastError() != cudaSuccess)
+	if (launch_ray_first(c, q, rays, worlds, n, fixture, hit, s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
 		return qfail(c, B3G_E_CUDA, "b3g_ray_cast_single_device: launch");
 	return B3G_OK;
 }
@@ -2130,7 +2168,8 @@ extern "C" int b3g_shape_cast_single(b3g_ctx* c, uint32_t n, const b3g_shape_cas
 	float* dHit = (float*)(base + fixBytes);
 	cudaStream_t s = c->stream;
 	cudaMemsetAsync(c->buf.counters + CTR_SCRATCH, 0, 4, s);
-	launch_shape_cast_first(c, q, (const float*)dIn, n, dFix, dHit, s);
+	if (launch_shape_cast_first(c, q, (const float*)dIn, n, dFix, dHit, s) != cudaSuccess)
+		return qfail(c, B3G_E_CUDA, "b3g_shape_cast_single: launch");
 	rc = q_status(c);
 	if (rc)
 		return rc;
@@ -2164,8 +2203,8 @@ extern "C" int b3g_shape_cast_single_device(b3g_ctx* c, uint32_t n, const b3g_sh
 	cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
 	if (n > std::max(c->cfg.max_proxies, c->cfg.max_contacts))
 		return qfail(c, B3G_E_CAPACITY, "world query: more queries than max(max_proxies, max_contacts) per call");
-	launch_shape_cast_first(c, q, (const float*)casts, n, fixture, hit, s);
-	if (cudaGetLastError() != cudaSuccess)
+	if (launch_shape_cast_first(c, q, (const float*)casts, n, fixture, hit, s) != cudaSuccess ||
+		cudaGetLastError() != cudaSuccess)
 		return qfail(c, B3G_E_CUDA, "b3g_shape_cast_single_device: launch");
 	return B3G_OK;
 }

@@ -578,7 +578,8 @@ int b3g_ray_cast_single(b3g_ctx* ctx, uint32_t n, const float* rays, const uint3
 /* b3g_ray_cast_single on device buffers (rays, worlds, fixture, hit as above,
  * all device memory; worlds may be NULL), asynchronous on stream (NULL: the
  * context's stream), for callers that keep their rays on the GPU. Nothing is
- * copied or allocated; the result is ready when the stream reaches it. */
+ * copied or allocated (a captured call's graph holds 128 bytes per proxy); the
+ * result is ready when the stream reaches it. */
 int b3g_ray_cast_single_device(b3g_ctx* ctx, uint32_t n, const float* rays, const uint32_t* worlds,
 	uint32_t* fixture, float* hit, void* stream);
 
@@ -620,7 +621,8 @@ int b3g_shape_cast_single(b3g_ctx* ctx, uint32_t n, const b3g_shape_cast_input* 
 /* b3g_shape_cast_single on device buffers (casts, fixture, hit as above, all
  * device memory), asynchronous on stream (NULL: the context's stream), for
  * callers that keep their casts on the GPU. The casts are not checked: every
- * hull index must be below the hull count. Nothing is copied or allocated. */
+ * hull index must be below the hull count. Nothing is copied or allocated (a
+ * captured call's graph holds 128 bytes per proxy). */
 int b3g_shape_cast_single_device(b3g_ctx* ctx, uint32_t n, const b3g_shape_cast_input* casts, uint32_t* fixture,
 	float* hit, void* stream);
 
