@@ -50,7 +50,6 @@ struct CIArgs
 	const uint32_t* fixBody;
 	const uint32_t* fixType;
 	const uint32_t* fixFlags;
-	bool sensors;             // some fixture is a sensor
 	const float4* fixParams;
 	const float2* material;   // per fixture: friction, restitution
 	const float4* bodies;     // b3g_solver_body records (7 float4 each)
@@ -109,7 +108,7 @@ __device__ __forceinline__ Item item_counts(const CIArgs& a, uint32_t i, uint32_
 	if (!a.list && (st & 1u) == 0)
 		return it;
 	const uint32_t fa = a.pairA[c], fb = a.pairB[c];
-	if (!a.list && a.sensors && ((a.fixFlags[fa] | a.fixFlags[fb]) & B3G_FIXTURE_SENSOR) != 0)
+	if (!a.list && ((a.fixFlags[fa] | a.fixFlags[fb]) & B3G_FIXTURE_SENSOR) != 0)
 		return it;
 	it.c = c;
 	it.flag = 1;
@@ -551,7 +550,6 @@ void launch_contact_constraints(b3g_ctx* c, const ConstraintCall& q, cudaStream_
 	a.fixBody = c->scene.fixBody;
 	a.fixType = c->scene.fixType;
 	a.fixFlags = c->scene.fixFlags;
-	a.sensors = c->anySensor;
 	a.fixParams = c->scene.fixParams;
 	a.material = q.material;
 	a.bodies = reinterpret_cast<const float4*>(q.bodies);

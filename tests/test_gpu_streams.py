@@ -244,3 +244,53 @@ def test_updates_after_a_pass_with_sleepers(how):
         assert results[-1][2] == int(((results[-1][1] == 0) & (sc.body_type != N.BODY_STATIC)).sum())
         pipe.close()
     assert np.array_equal(results[0][0], results[1][0]) and np.array_equal(results[0][1], results[1][1])
+
+
+# The constraints of a scene without sensors are captured; then some fixtures
+# become sensors, and the replay leaves their contacts out.
+def test_captured_constraints_see_new_sensors():
+    torch = pytest.importorskip("torch")
+    sc = mixed(1500)
+    states = states_of(sc, 6)
+    pipe = CollisionPipeline(sc)
+    bodies = np.zeros(sc.n_bodies, N.SOLVER_BODY_DTYPE)
+    bodies["x"], bodies["q"], bodies["invMass"] = sc.body_pos, sc.body_quat, 1.0
+    room = 8 * sc.n_fixtures
+    vp = N.ctypes.c_void_p
+    dev = [torch.from_numpy(bodies.view(np.uint8).copy()).cuda(), torch.zeros(room * 128, dtype=torch.uint8, device="cuda"),
+           torch.zeros(room * 464, dtype=torch.uint8, device="cuda"), torch.zeros(2, dtype=torch.int32, device="cuda")]
+    b, con, man, counts = (vp(x.data_ptr()) for x in dev)
+    stream = torch.cuda.Stream()
+
+    def build(s):
+        pipe._check(pipe.lib.b3g_contact_constraints_device(pipe.ctx, 0, None, b, 1.0, 1, con, room, man, room, counts, s))
+
+    for st in states[:2]:
+        pipe.collide(st)
+    torch.cuda.synchronize()
+    build(vp(stream.cuda_stream))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        build(vp(stream.cuda_stream))
+    before, _ = pipe.contact_constraints(bodies)
+    f = np.arange(0, sc.n_fixtures, 3, dtype=np.uint32)
+    u32, f32 = N.ctypes.c_uint32, N.ctypes.c_float
+    flags = np.full(len(f), N.FIXTURE_SENSOR, np.uint32)
+    arrays = [np.ascontiguousarray(a) for a in (sc.fix_body[f], sc.fix_type[f], sc.fix_hull[f])]
+    params = np.ascontiguousarray(sc.fix_params.reshape(-1, 12)[f])
+    pipe._check(pipe.lib.b3g_update_scene(
+        pipe.ctx, 0, None, None, None, None, len(f), N.ptr(f, u32), *(N.ptr(a, u32) for a in arrays),
+        N.ptr(params, f32), N.ptr(flags, u32), 0, None, None))
+    for st in states[2:4]:
+        pipe.collide(st)
+    want, want_man = pipe.contact_constraints(bodies)
+    assert 0 < len(want) < len(before)
+    graph.replay()
+    torch.cuda.synchronize()
+    n, m = dev[3].cpu().numpy().tolist()
+    assert (n, m) == (len(want), len(want_man))
+    assert dev[1].cpu().numpy()[: n * 128].tobytes() == want.tobytes()
+    assert dev[2].cpu().numpy()[: m * 464].tobytes() == want_man.tobytes()
+    graph.reset()
+    pipe.close()
