@@ -1515,12 +1515,22 @@ static cudaError_t wait_staged(b3g_ctx* c, cudaStream_t s)
 	return e == cudaSuccess ? wait_event(s, c->awakeStaged, c->staged) : e;
 }
 
+// A scene update may bring the first triangle or sensor: the captured passes
+// have no kernel for them.
+static void scene_may_have(b3g_ctx* c, bool triangle, bool sensor)
+{
+	if ((triangle && !c->anyTriangle) || (sensor && !c->anySensor))
+		destroy_graphs(c);
+	c->anyTriangle |= triangle;
+	c->anySensor |= sensor;
+}
+
 // After an update whose records the host has not seen.
 static void device_updated(b3g_ctx* c)
 {
 	c->treeForce = true; // fixtures created, replaced or retired: new leaves
 	// The written fixtures' types and flags stay on the device.
-	c->anyTriangle = c->anySensor = true;
+	scene_may_have(c, true, true);
 	// The host copy of fixture types is refreshed when the stand-alone
 	// narrowphase next needs it; written bodies are awake, so the sleep count
 	// can only have dropped (it stays an upper bound until the next wake-up
@@ -1717,8 +1727,7 @@ extern "C" int b3g_update_scene(b3g_ctx* c, uint32_t nb, const uint32_t* bodyInd
 	for (uint32_t i = 0; i < nf; ++i)
 	{
 		c->hFixType[fixIndex[i]] = shapeType[i];
-		c->anyTriangle |= shapeType[i] == B3G_SHAPE_TRIANGLE;
-		c->anySensor |= (flags[i] & B3G_FIXTURE_SENSOR) != 0;
+		scene_may_have(c, shapeType[i] == B3G_SHAPE_TRIANGLE, (flags[i] & B3G_FIXTURE_SENSOR) != 0);
 	}
 	for (uint32_t i = 0; i < nb; ++i)
 	{

@@ -294,3 +294,34 @@ def test_captured_constraints_see_new_sensors():
     assert dev[2].cpu().numpy()[: m * 464].tobytes() == want_man.tobytes()
     graph.reset()
     pipe.close()
+
+
+# The first sensors of a scene come with an update, after its passes have been
+# captured.
+def test_first_sensors_after_captured_passes():
+    torch = pytest.importorskip("torch")
+    sc = mixed(1500)
+    states = states_of(sc, 10)
+    f = np.arange(0, sc.n_fixtures, 2, dtype=np.uint32)
+    u32, f32 = N.ctypes.c_uint32, N.ctypes.c_float
+    flags = np.full(len(f), N.FIXTURE_SENSOR, np.uint32)
+    arrays = [np.ascontiguousarray(a) for a in (sc.fix_body[f], sc.fix_type[f], sc.fix_hull[f])]
+    params = np.ascontiguousarray(sc.fix_params.reshape(-1, 12)[f])
+    out = []
+    for graph in (False, True):
+        pipe = CollisionPipeline(sc, graph=graph)
+        got = []
+        for k, st in enumerate(states):
+            if k == 5:
+                pipe._check(pipe.lib.b3g_update_scene(
+                    pipe.ctx, 0, None, None, None, None, len(f), N.ptr(f, u32), *(N.ptr(a, u32) for a in arrays),
+                    N.ptr(params, f32), N.ptr(flags, u32), 0, None, None))
+            x = torch.from_numpy(st).cuda()
+            torch.cuda.synchronize()
+            pipe.collide(x.data_ptr(), on_device=True)
+            got.append((pipe.contacts(), pipe.manifolds().tobytes()))
+        assert (pipe.totals()["graph_passes"] > 0) == graph
+        out.append(got)
+        pipe.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a[0], b[0]) and a[1] == b[1]
