@@ -3259,12 +3259,17 @@ extern "C" int b3g_autotune(b3g_ctx* c, uint32_t reps, void* stream, uint32_t* o
 	};
 	static const uint32_t convexBucket[B3G_CONVEX_KERNELS] = {BK_SPHERES, BK_CAPSULE_SPHERE, BK_CAPSULES,
 		BK_TRIANGLE_SPHERE, BK_TRIANGLE_CAPSULE, BK_HULL_SPHERE, BK_HULL_CAPSULE, BK_SENSOR, BK_INACTIVE};
-	for (int k = CONVEX_PLAIN; k < B3G_CONVEX_KERNELS && rc == B3G_OK; ++k)
+	for (int k = 0; k < B3G_CONVEX_KERNELS && rc == B3G_OK; ++k)
 	{
 		if (h[CTR_BUCKET0 + convexBucket[k]] == 0)
 			continue;
 		pick(c->tune.v[B3G_TUNE_CONVEX + k], kBlocksPerSM, 5,
 			[&] {
+				if (k < CONVEX_PLAIN)
+				{
+					launch_plain(a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
+					return;
+				}
 				reset_post_counts(B, s);
 				launch_convex_one(k, a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
 			});

@@ -967,7 +967,8 @@ __device__ __forceinline__ HullRef mesh_tri_ref(const MeshTri& t)
 	return r;
 }
 
-void launch_plain(const NPArgs& a, const uint32_t* lists, const uint32_t* counts, uint32_t cap, cudaStream_t s);
+void launch_plain(const NPArgs& a, const uint32_t* lists, const uint32_t* counts, uint32_t cap, const Tune& tune,
+	cudaStream_t s);
 void launch_mesh_items_convex(const NPArgs& a, const Buffers& B, cudaStream_t s);
 void launch_mesh_items_hull(const NPArgs& a, const Buffers& B, uint32_t maxUE, const Tune& tune, cudaStream_t s);
 

@@ -799,12 +799,13 @@ __device__ GProxy shape_proxy(const DevScene& S, const ShapeP& s)
 
 // Contacts listed in one bucket, one thread each (spheres_apart: the exact
 // cull of collide_common.cuh, repeated here for contacts that reach these
-// kernels without k_bucket, i.e. wake-ups and b3g_collide_pairs).
+// kernels without k_bucket, i.e. wake-ups and b3g_collide_pairs). blocks: how
+// many take part.
 template <int BUCKET>
-__device__ __forceinline__ void convex_bucket(const NPArgs& a)
+__device__ __forceinline__ void convex_bucket(const NPArgs& a, uint32_t blocks)
 {
 	uint32_t n = *a.listCount;
-	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += blocks * blockDim.x)
 	{
 		uint32_t c = a.list[t];
 		uint32_t fa = a.pairA[c], fb = a.pairB[c];
@@ -879,15 +880,15 @@ __device__ __forceinline__ void convex_bucket(const NPArgs& a)
 template <int BUCKET>
 __global__ void __launch_bounds__(128, 4) k_convex(NPArgs a)
 {
-	convex_bucket<BUCKET>(a);
+	convex_bucket<BUCKET>(a, gridDim.x);
 }
 
 // Convex contacts k_bucket found apart (spheres_apart): the routine would
 // return no point, so the manifold is empty; warm start and flags as above.
-__device__ __forceinline__ void apart_bucket(const NPArgs& a)
+__device__ __forceinline__ void apart_bucket(const NPArgs& a, uint32_t blocks)
 {
 	uint32_t n = *a.listCount;
-	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += blocks * blockDim.x)
 	{
 		uint32_t c = a.list[t];
 		DevManifold& m = a.man[c];
@@ -903,26 +904,30 @@ __device__ __forceinline__ void apart_bucket(const NPArgs& a)
 // launches: a host step of 64 mixed bodies 197 us, now 180; 2,001 with sleepers 333
 // and 318.
 constexpr int PLAIN_BUCKETS = 4;
-constexpr int PLAIN_BLOCKS = 4; // an SM and bucket
-__global__ void __launch_bounds__(128) k_plain(NPArgs a, const uint32_t* lists, const uint32_t* counts, uint32_t cap)
+constexpr int APART_BLOCKS = 4; // an SM
+__global__ void __launch_bounds__(128) k_plain(NPArgs a, const uint32_t* lists, const uint32_t* counts, uint32_t cap,
+	uint4 blocks)
 {
 	const uint32_t bk = blockIdx.y == 0 ? BK_CAPSULES : blockIdx.y == 1 ? BK_CAPSULE_SPHERE : blockIdx.y == 2 ? BK_SPHERES
 																											 : BK_APART;
+	const uint32_t own = blockIdx.y == 0 ? blocks.x : blockIdx.y == 1 ? blocks.y : blockIdx.y == 2 ? blocks.z : blocks.w;
+	if (blockIdx.x >= own)
+		return;
 	a.list = lists + (size_t)bk * cap;
 	a.listCount = counts + bk;
 	switch (bk)
 	{
 	case BK_CAPSULES:
-		convex_bucket<BK_CAPSULES>(a);
+		convex_bucket<BK_CAPSULES>(a, own);
 		break;
 	case BK_CAPSULE_SPHERE:
-		convex_bucket<BK_CAPSULE_SPHERE>(a);
+		convex_bucket<BK_CAPSULE_SPHERE>(a, own);
 		break;
 	case BK_SPHERES:
-		convex_bucket<BK_SPHERES>(a);
+		convex_bucket<BK_SPHERES>(a, own);
 		break;
 	default:
-		apart_bucket(a);
+		apart_bucket(a, own);
 		break;
 	}
 }
@@ -1183,16 +1188,20 @@ void launch_convex_one(int k, const NPArgs& base, const uint32_t* lists, const u
 }
 
 // The buckets without hulls and the contacts apart.
-void launch_plain(const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap, cudaStream_t s)
+void launch_plain(const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap, const Tune& tune,
+	cudaStream_t s)
 {
-	const dim3 grid(work_blocks(cap, 128, PLAIN_BLOCKS), PLAIN_BUCKETS);
-	k_plain<<<grid, 128, 0, s>>>(base, lists, counts, cap);
+	auto blocks = [&](uint32_t perSM) { return (uint32_t)work_blocks(cap, 128, (int)perSM); };
+	const uint32_t* v = tune.v + B3G_TUNE_CONVEX; // spheres, capsule-sphere, capsules
+	const uint4 own = make_uint4(blocks(v[2]), blocks(v[1]), blocks(v[0]), blocks(APART_BLOCKS));
+	const dim3 grid(std::max(std::max(own.x, own.y), std::max(own.z, own.w)), PLAIN_BUCKETS);
+	k_plain<<<grid, 128, 0, s>>>(base, lists, counts, cap, own);
 }
 
 void launch_convex_buckets(const NPArgs& base, const uint32_t* lists, const uint32_t* counts, uint32_t cap,
 	const Tune& tune, cudaStream_t s)
 {
-	launch_plain(base, lists, counts, cap, s);
+	launch_plain(base, lists, counts, cap, tune, s);
 	for (int k = CONVEX_PLAIN; k < B3G_CONVEX_KERNELS; ++k)
 		launch_convex_one(k, base, lists, counts, cap, tune, s);
 }

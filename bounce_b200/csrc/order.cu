@@ -550,7 +550,7 @@ int resolve_wakeups(b3g_ctx* c, cudaStream_t s)
 			break;
 		if (act)
 		{
-			launch_plain(a, B.bucketList, B.counters + CTR_BUCKET0, cap, s);
+			launch_plain(a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
 			for (int k = CONVEX_PLAIN; k < B3G_CONVEX_KERNELS; ++k)
 				if (k != CONVEX_INACTIVE && convex_bucket_possible(c, k))
 				{

@@ -473,7 +473,7 @@ void launch_narrowphase(b3g_ctx* c, cudaStream_t s)
 	// bodies: 212, 338 and 647 us without the third branch, 176, 301 and 626
 	// with it).
 	const bool third = side != s && !meshSide;
-	launch_plain(a, B.bucketList, B.counters + CTR_BUCKET0, cap, s);
+	launch_plain(a, B.bucketList, B.counters + CTR_BUCKET0, cap, c->tune, s);
 	if (third)
 	{
 		cudaStreamWaitEvent(c->meshStream, c->forkEvent, 0);

@@ -475,7 +475,9 @@ const char* b3g_stage_name(uint32_t stage);
  *   [B3G_TUNE_CONVEX + k]  blocks per SM of the thread-per-pair kernel of
  *                          bucket k: spheres, capsule-sphere, capsules,
  *                          triangle-sphere, triangle-capsule, hull-sphere,
- *                          hull-capsule, sensor, inactive (128 threads per block)
+ *                          hull-capsule, sensor, inactive (128 threads per
+ *                          block; the first three run in one kernel, a row of
+ *                          blocks each)
  *   [B3G_TUNE_PROBE]       blocks per SM of the hull feature-cache probe
  *   [B3G_TUNE_SAT_WARPS]   warps per block of the hull-hull and hull-triangle
  *                          SAT kernels (2, 4, 8)
