@@ -1953,7 +1953,7 @@ extern "C" int b3g_collide(b3g_ctx* c, const float* state, int onDevice, void* s
 	CK(wait_staged(c, s));
 	CK(wait_packing(c, s));
 	c->lastStream = s;
-	c->captured = c->captured || in_capture(s);
+	c->captured = c->captured || (s != c->stream && in_capture(s));
 	// Filters of this pass: the caller's contact filter (a host round trip in
 	// the middle of the pass), else joints or a contact veto (inside the pass).
 	c->filterMode = (c->cfg.flags & B3G_FLAG_CONTACT_FILTER) ? 2 : ((c->nJoints || c->nVeto) ? 1 : 0);
@@ -2457,12 +2457,14 @@ extern "C" int b3g_fetch_results_packed_async(b3g_ctx* c, uint32_t* contacts, ui
 	// on one after a pass on the context's waits for them (wait_packing).
 	const bool beside = c->lastStream != c->stream;
 	if (touchCapacity && !c->packList)
+		CK(dalloc(&c->packList, cap));
+	if (touchCapacity && !c->packStates)
 	{
-		CK(dalloc(&c->packCounts, CTR_BUCKET0));
 		CK(dalloc(&c->packStates, states));
 		CK(cudaMemsetAsync(c->packStates, 0, sizeof(unsigned long long) * states, c->stream));
-		CK(dalloc(&c->packList, cap));
 	}
+	if (touchCapacity && beside && !c->packCounts)
+		CK(dalloc(&c->packCounts, CTR_BUCKET0));
 	CK(cudaMemcpyAsync(c->hCounters, B.counters, sizeof(uint32_t) * CTR_COUNT, cudaMemcpyDeviceToHost, c->stream));
 	if (touchCapacity && beside)
 		CK(cudaMemcpyAsync(c->packCounts, B.counters, sizeof(uint32_t) * CTR_BUCKET0, cudaMemcpyDeviceToDevice,
