@@ -3070,6 +3070,8 @@ extern "C" int b3g_collide_pairs(b3g_ctx* c, uint32_t n, const uint32_t* fixA, c
 					uint32_t* dOne = nullptr;
 					step(dalloc(&dOne, BK_COUNT));
 					step(cudaMemcpy(dOne, one.data(), 4 * BK_COUNT, cudaMemcpyHostToDevice));
+					// The contacts that the last bucket handed on are done.
+					step(cudaMemsetAsync(dMissCount + 1, 0, 12, c->stream));
 					launch_convex_buckets(a, dList + offs[b] - (size_t)b * n, dOne, n, c->tune, c->stream);
 					step(cudaStreamSynchronize(c->stream));
 					dfree(dOne);
