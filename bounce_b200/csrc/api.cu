@@ -517,7 +517,6 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 		carveout_broadphase();
 		carveout_pairs();
 		carveout_order();
-		carveout_narrow_convex();
 		carveout_narrow_hulls();
 		carveout_mesh();
 		carveout_solver_input();

@@ -567,14 +567,17 @@ struct ConstraintCall
 uint32_t contact_constraint_tiles(uint32_t items);
 void launch_contact_constraints(b3g_ctx* c, const ConstraintCall& q, cudaStream_t s);
 
-// The share of an SM's 228 KB of shared memory that every kernel of the pass
-// asks for: 100 KB. An SM changes the split between shared memory and L1 only
+// The share of an SM's 228 KB of shared memory that the kernels of the pass ask
+// for: 100 KB. An SM changes the split between shared memory and L1 only
 // when it is empty, so kernels that each leave it to the driver (none for one
 // kernel, 200 KB for the next) keep the passes of other contexts, and the
 // branches of one pass, off each other's SMs. Three contexts at once, a pass of
 // 65,536 mixed bodies / 512 worlds / a pile of 24,064 hulls took 464 / 1,011 /
 // 209 us so, 414 / 882 / 202 with 44 %, 418 / 884 / 198 with 58 % and 531 /
-// 1,115 / 212 with all of it (which leaves little L1).
+// 1,115 / 212 with all of it (which leaves little L1). The convex kernels, which
+// use none, leave it to the driver: on one stream those of 65,536 mixed bodies
+// take 223 us so and 238 with 44 %, and three contexts at once show no difference
+// (373 and 372 / 819 and 820 / 196 and 195 us); k_diff and k_bucket, see pairs.cu.
 constexpr int CARVEOUT_PERCENT = 44;
 inline void set_carveout(std::initializer_list<const void*> kernels)
 {
@@ -588,7 +591,6 @@ void carveout_api();
 void carveout_broadphase();
 void carveout_pairs();
 void carveout_order();
-void carveout_narrow_convex();
 void carveout_narrow_hulls();
 void carveout_mesh();
 void carveout_solver_input();

@@ -1210,13 +1210,3 @@ void launch_mesh_items_convex(const NPArgs& a, const Buffers& B, cudaStream_t s)
 {
 	k_mesh_items_convex<<<persistent_blocks(4), 128, 0, s>>>(a, B);
 }
-
-void carveout_narrow_convex()
-{
-	set_carveout({
-		(const void*)k_plain, (const void*)k_convex<BK_HULL_SPHERE>, (const void*)k_convex<BK_HULL_CAPSULE>,
-		(const void*)k_convex<BK_TRIANGLE_SPHERE>,
-		(const void*)k_convex<BK_TRIANGLE_CAPSULE>, (const void*)k_sensor, (const void*)k_hull_sphere_gjk,
-		(const void*)k_hull_capsule_post<HC_POST_LANES>, (const void*)k_inactive,
-		(const void*)k_mesh_items_convex});
-}
