@@ -845,6 +845,7 @@ extern "C" int b3g_set_hulls(b3g_ctx* c, uint32_t nh, const uint32_t* desc, cons
 	CK(cudaStreamSynchronize(c->stream));
 	destroy_graphs(c);
 	uint32_t nv = 0, ne = 0, nf = 0, maxUE = 0, maxV = 0, maxF = 0;
+	bool large = false;
 	std::vector<HullDesc> hd(nh);
 	for (uint32_t h = 0; h < nh; ++h)
 	{
@@ -859,6 +860,7 @@ extern "C" int b3g_set_hulls(b3g_ctx* c, uint32_t nh, const uint32_t* desc, cons
 			if (E[0] >= d[1] || E[2] >= d[5] || E[3] >= d[3] || E[4] >= d[3])
 				return fail(c, B3G_E_INVALID, "hull %u: half-edge %u out of range", h, e);
 		}
+		uint32_t maxFace = 0;
 		for (uint32_t f = 0; f < d[5]; ++f)
 		{
 			uint32_t begin = faces[d[4] + f];
@@ -874,10 +876,12 @@ extern "C" int b3g_set_hulls(b3g_ctx* c, uint32_t nh, const uint32_t* desc, cons
 					return fail(c, B3G_E_INVALID, "hull %u: face %u loop is broken", h, f);
 				e = E[4];
 			} while (e != begin);
+			maxFace = std::max(maxFace, steps);
 		}
 		const float* c3 = centroids + 3 * (size_t)h;
 		hd[h] = HullDesc{d[0], d[1], d[2], d[3], d[4], d[5], c3[0], c3[1], c3[2],
-			hull_blunt(d[1], verts + 3 * (size_t)d[0], d[5], planes + 4 * (size_t)d[4], c3) ? 1u : 0u, {0, 0}};
+			hull_blunt(d[1], verts + 3 * (size_t)d[0], d[5], planes + 4 * (size_t)d[4], c3) ? 1u : 0u, maxFace, 0};
+		large = large || !ring_holds(hd[h], hd[h]);
 		nv = std::max(nv, d[0] + d[1]);
 		ne = std::max(ne, d[2] + d[3]);
 		nf = std::max(nf, d[4] + d[5]);
@@ -923,6 +927,7 @@ extern "C" int b3g_set_hulls(b3g_ctx* c, uint32_t nh, const uint32_t* desc, cons
 	c->maxUniqueEdges = maxUE;
 	c->scene.hullMaxV = maxV;
 	c->scene.hullMaxF = maxF;
+	c->scene.hullsLarge = large;
 	c->scene.hulls = c->dHulls;
 	c->scene.hverts = c->dHverts;
 	c->scene.hedges = c->dHedges;
@@ -1899,7 +1904,7 @@ static uint32_t narrow_launches(const b3g_ctx* c)
 	uint32_t k = 0;
 	for (int b = CONVEX_PLAIN; b < B3G_CONVEX_KERNELS; ++b)
 		k += convex_bucket_possible(c, b) ? 1u : 0u;
-	return 1 + 1 + k + 2 + 2 + (c->anyTriangle ? 1u : 0u) + mesh_launches(c);
+	return 1 + 1 + k + 2 + (c->scene.hullsLarge ? 3 : 2) + (c->anyTriangle ? 1u : 0u) + mesh_launches(c);
 }
 
 // The LBVH bookkeeping once a pass's broadphase is issued.

@@ -70,7 +70,8 @@ struct HullDesc
 	uint32_t vOff, vCnt, eOff, eCnt, fOff, fCnt;
 	float cx, cy, cz;
 	uint32_t blunt; // the vertices are at most 16 times as far from the centroid as the nearest plane (queries.cu)
-	uint32_t pad[2];
+	uint32_t maxFace; // vertices of its largest face
+	uint32_t pad;
 };
 static_assert(sizeof(HullDesc) == 48, "HullDesc");
 
@@ -97,6 +98,7 @@ struct DevScene
 	const uint32_t* hfaces;
 	const float4* hplanes; // normal, offset
 	uint32_t hullMaxV, hullMaxF; // the largest hull's counts (shared-memory staging)
+	bool hullsLarge;      // some pair of hulls is one for k_hulls_probe_large
 
 	// bodies
 	const uint32_t* bodyWorld;

@@ -19,6 +19,16 @@ struct HullRef
 	V3 centroid;
 };
 
+// The clip polygons of k_hulls_probe hold this many vertices (narrow_hulls.cu);
+// a power of two.
+constexpr uint32_t CLIP_SLOTS = 8;
+// Whether a face of one hull clipped by the sides of a face of the other fits
+// them whatever the faces (each side adds a vertex at most), and edges 16 bits.
+__host__ __device__ __forceinline__ bool ring_holds(const HullDesc& h1, const HullDesc& h2)
+{
+	return h1.maxFace + h2.maxFace <= CLIP_SLOTS && h1.eCnt <= 0xFFFFu && h2.eCnt <= 0xFFFFu;
+}
+
 __device__ __forceinline__ HullRef hull_ref(const DevScene& S, uint32_t h)
 {
 	HullDesc d = S.hulls[h];

@@ -360,9 +360,8 @@ __device__ void build_edge_contact(DevManifold& m, const XF& xf1, uint32_t index
 	m.points[0].edgeContact = 1;
 }
 
-// b3BuildFaceContact (collide_hulls.cpp:75-187) on one thread, for the
-// polygons that do not fit the rings of rebuild_faces.
-__device__ __noinline__ void build_face_contact(DevManifold& m, const XF& xf1, uint32_t index1, const HullRef& h1, float r1,
+// b3BuildFaceContact (collide_hulls.cpp:75-187) on one thread.
+__device__ void build_face_contact(DevManifold& m, const XF& xf1, uint32_t index1, const HullRef& h1, float r1,
 	const XF& xf2, const HullRef& h2, float r2, bool flipNormal, uint32_t* status)
 {
 	float totalRadius = r1 + r2;
@@ -938,11 +937,8 @@ __device__ __forceinline__ void load_hull_ctx(const NPArgs& a, uint32_t c, HullC
 
 constexpr int PROBE_THREADS = 128;
 constexpr int PROBE_BLOCKS = 4;
-// A power of two. Faces have 3 or 4 vertices and gain one per side plane that
-// cuts them; with 16 slots the rings fill the SM's shared memory: three contexts
-// at once took 415 us a pass of 65,536 mixed bodies and 879 of 512 worlds, with
-// 8 they take 392 and 831, though more polygons are left to build_face_contact.
-constexpr uint32_t CLIP_SLOTS = 8;
+static_assert(CLIP_SLOTS == 8, "with 16 slots the rings fill the SM's shared memory: three contexts at once took 415 us a "
+	"pass of 65,536 mixed bodies and 879 of 512 worlds, with 8 they take 392 and 831");
 
 // A thread's clip polygon: a ring of vertices in shared memory, one column of
 // words per thread. A vertex's edge pair takes two words of two 16-bit edges
@@ -999,10 +995,7 @@ __device__ void rebuild_faces(const NPArgs& a, uint32_t c, bool live, ClipRings&
 	const uint32_t index1 = cache.z;
 	const PL plane1 = pmul(xf1, hp(h1, index1));
 	uint32_t head = 0, cnt = 0;
-	// A polygon that outgrows the ring, or edges that do not fit 16 bits: the
-	// thread builds the contact on its own.
-	bool big = h1.eCnt > 0xFFFFu || h2.eCnt > 0xFFFFu;
-	bool failed = false;
+	bool failed = false; // the polygon outgrows the ring: not with hulls that ring_holds
 	{
 		// b3BuildPolygon (clip.cpp:33-58).
 		V3 normal1 = rotc(xf2.q, plane1.n);
@@ -1010,9 +1003,8 @@ __device__ void rebuild_faces(const NPArgs& a, uint32_t c, bool live, ClipRings&
 		uint32_t edge = begin;
 		do
 		{
-			if (cnt == CLIP_SLOTS)
-				big = true;
-			if (big)
+			failed = cnt == CLIP_SLOTS;
+			if (failed)
 				break;
 			const uint4 e = h2.e[edge];
 			R.put(cnt++, xmul(xf2, hv(h2, e.x)), ~0u, ring_edges(e.z, edge));
@@ -1025,7 +1017,7 @@ __device__ void rebuild_faces(const NPArgs& a, uint32_t c, bool live, ClipRings&
 	// polygon grows behind its tail.
 	const uint32_t begin = h1.f[index1];
 	uint32_t edge = begin, guard = 0;
-	bool run = !big;
+	bool run = !failed;
 	while (__any_sync(0xffffffffu, run))
 	{
 		PL cp = plane1;
@@ -1062,7 +1054,7 @@ __device__ void rebuild_faces(const NPArgs& a, uint32_t c, bool live, ClipRings&
 				const uint32_t adds = (leaves || enters ? 1u : 0u) + (enters || stays ? 1u : 0u);
 				if (outN + adds + (n - i - 1) > CLIP_SLOTS)
 				{
-					big = true;
+					failed = true;
 					run = false;
 					n = 0;
 				}
@@ -1092,7 +1084,7 @@ __device__ void rebuild_faces(const NPArgs& a, uint32_t c, bool live, ClipRings&
 			run = cnt > 0 && edge != begin;
 		}
 	}
-	if (big || failed)
+	if (failed)
 		cnt = 0;
 	// The vertices on or behind the reference face, moved up to the head.
 	uint32_t n1 = 0, minIndex = 0;
@@ -1225,32 +1217,24 @@ __device__ void rebuild_faces(const NPArgs& a, uint32_t c, bool live, ClipRings&
 	if (!live)
 		return;
 	DevManifold& m = a.man[c];
-	if (big)
-	{
-		build_face_contact(m, xf1, index1, h1, flip ? H.r2 : H.r1, xf2, h2, flip ? H.r1 : H.r2, flip, a.status);
-		pc = m.pointCount;
-	}
-	else
-	{
-		if (failed)
-			atomicOr(a.status, B3G_ST_POLY_OVERFLOW);
-		const XF xm1 = flip ? xf2 : xf1, xm2 = flip ? xf1 : xf2;
-		const V3 normal = rotc(xm1.q, oriented);
+	if (failed)
+		atomicOr(a.status, B3G_ST_POLY_OVERFLOW);
+	const XF xm1 = flip ? xf2 : xf1, xm2 = flip ? xf1 : xf2;
+	const V3 normal = rotc(xm1.q, oriented);
 #pragma unroll
-		for (uint32_t i = 0; i < 4; ++i)
-		{
-			if (i >= pc)
-				break;
-			const uint32_t s = (head + at[i]) % CLIP_SLOTS;
-			const V3 v2 = R.pos(s);
-			const uint32_t e1 = R.pair1[s][threadIdx.x], e2 = R.pair2[s][threadIdx.x];
-			const uint32_t q1 = flip ? e2 : e1, q2 = flip ? e1 : e2;
-			set_point(m.points[i], normal, xmult(xm1, flip ? v2 : o[i]), xmult(xm2, flip ? o[i] : v2));
-			set_id(m.points[i], mkpair(ring_edge(q1 & 0xFFFFu), ring_edge(q1 >> 16), ring_edge(q2 & 0xFFFFu),
-				ring_edge(q2 >> 16)));
-		}
-		m.pointCount = pc;
+	for (uint32_t i = 0; i < 4; ++i)
+	{
+		if (i >= pc)
+			break;
+		const uint32_t s = (head + at[i]) % CLIP_SLOTS;
+		const V3 v2 = R.pos(s);
+		const uint32_t e1 = R.pair1[s][threadIdx.x], e2 = R.pair2[s][threadIdx.x];
+		const uint32_t q1 = flip ? e2 : e1, q2 = flip ? e1 : e2;
+		set_point(m.points[i], normal, xmult(xm1, flip ? v2 : o[i]), xmult(xm2, flip ? o[i] : v2));
+		set_id(m.points[i], mkpair(ring_edge(q1 & 0xFFFFu), ring_edge(q1 >> 16), ring_edge(q2 & 0xFFFFu),
+			ring_edge(q2 >> 16)));
 	}
+	m.pointCount = pc;
 	if (pc > 0)
 	{
 		a.cache[c] = cache; // overlap cache hit
@@ -1258,6 +1242,12 @@ __device__ void rebuild_faces(const NPArgs& a, uint32_t c, bool live, ClipRings&
 	}
 	else
 		probe_flush(a, c, cache);
+}
+
+// Whether the contact is one for k_hulls_probe_large.
+__device__ __forceinline__ bool probe_large(const NPArgs& a, uint32_t c)
+{
+	return !ring_holds(a.S.hulls[a.S.fixHull[a.pairA[c]]], a.S.hulls[a.S.fixHull[a.pairB[c]]]);
 }
 
 // Pass 1, the cache half of b3CollideHullsCache (collide_hulls.cpp:367-415):
@@ -1293,8 +1283,9 @@ __global__ void __launch_bounds__(PROBE_THREADS, PROBE_BLOCKS) k_hulls_probe(NPA
 			uint32_t c = 0;
 			bool face = false, edges = false;
 			if (base + tid < n)
-			{
 				c = a.list[base + tid];
+			if (base + tid < n && !(a.S.hullsLarge && probe_large(a, c)))
+			{
 				const int32_t prev = a.prevIndex[c];
 				const uint4 cache = prev >= 0 ? a.prevCache[prev] : make_uint4(CT_EMPTY, FT_FACE1, 0, 0);
 				man_clear(a.man[c]);
@@ -1380,6 +1371,66 @@ __global__ void __launch_bounds__(PROBE_THREADS, PROBE_BLOCKS) k_hulls_probe(NPA
 			sQueue = queued - take;
 		if (!more && queued == take)
 			break;
+	}
+}
+
+// The same for hulls whose polygons may outgrow the rings, a contact per thread
+// from its cache to its manifold: the polygons are in local memory, and without
+// the rings' shared memory more of them stay in L1. Contacts of 20,000 pairs of
+// 6, 8, 12 and 16-sided prisms take 83, 99, 143 and 206 us so (with the launch of
+// the other kernel), 93, 116, 174 and 246 built so in k_hulls_probe, and 104, 137,
+// 174 and 248 clipped in the ring there until they outgrew it.
+__global__ void __launch_bounds__(PROBE_THREADS) k_hulls_probe_large(NPArgs a)
+{
+	const uint32_t n = *a.listCount;
+	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+	{
+		const uint32_t c = a.list[t];
+		if (!probe_large(a, c))
+			continue;
+		const int32_t prev = a.prevIndex[c];
+		uint4 cache = prev >= 0 ? a.prevCache[prev] : make_uint4(CT_EMPTY, FT_FACE1, 0, 0);
+		DevManifold& m = a.man[c];
+		man_clear(m);
+		if (!a.convexCache)
+		{
+			probe_miss(a, c, cache);
+			continue;
+		}
+		bool done = false;
+		if (cache.x == CT_EMPTY)
+			cache = make_uint4(CT_EMPTY, FT_FACE1, 0, 0);
+		else
+		{
+			HullCtx H;
+			load_hull_ctx(a, c, H);
+			const bool face = cache.y == FT_FACE1 || cache.y == FT_FACE2;
+			// A face of either hull with the hulls in the face's order.
+			const bool f2 = cache.y == FT_FACE2;
+			const XF xa = f2 ? H.xf2 : H.xf1, xb = f2 ? H.xf1 : H.xf2;
+			const HullRef ha = f2 ? H.h2 : H.h1, hb = f2 ? H.h1 : H.h2;
+			uint32_t state = CT_EMPTY;
+			if (cache.y == FT_EDGES)
+				state = read_edges(H.xf1, H.h1, H.xf2, H.h2, cache.z, cache.w, H.r1 + H.r2);
+			else if (face)
+				state = read_face_thread(xa, ha, xb, hb, cache.z, H.r1 + H.r2);
+			done = cache.x == CT_SEPARATION && state == CT_SEPARATION;
+			if (cache.x == CT_OVERLAP && state == CT_OVERLAP)
+			{
+				if (!face)
+					rebuild_edge_contact(m, H.xf1, cache.z, H.h1, H.xf2, cache.w, H.h2);
+				else if (face_contact_persists(xa, xb, f2 ? H.xf02 : H.xf01, f2 ? H.xf01 : H.xf02))
+					build_face_contact(m, xa, cache.z, ha, f2 ? H.r2 : H.r1, xb, hb, f2 ? H.r1 : H.r2, f2, a.status);
+				done = m.pointCount > 0;
+			}
+		}
+		if (done)
+		{
+			a.cache[c] = cache;
+			finish_convex(a, c, m);
+		}
+		else
+			probe_flush(a, c, cache);
 	}
 }
 
@@ -1829,7 +1880,10 @@ void launch_hulls_probe(const NPArgs& base, const uint32_t* list, const uint32_t
 	NPArgs a = base;
 	a.list = list;
 	a.listCount = count;
-	k_hulls_probe<<<work_blocks(a.hcPostCap, PROBE_THREADS, (int)tune.v[B3G_TUNE_PROBE]), PROBE_THREADS, 0, s>>>(a);
+	const int blocks = work_blocks(a.hcPostCap, PROBE_THREADS, (int)tune.v[B3G_TUNE_PROBE]);
+	k_hulls_probe<<<blocks, PROBE_THREADS, 0, s>>>(a);
+	if (a.S.hullsLarge)
+		k_hulls_probe_large<<<blocks, PROBE_THREADS, 0, s>>>(a);
 }
 
 // Dynamic shared memory of the SAT kernel with `warps` warps per block.

@@ -564,7 +564,7 @@ int resolve_wakeups(b3g_ctx* c, cudaStream_t s)
 					B.counters + CTR_BUCKET0 + BK_HULL_TRIANGLE, c->maxUniqueEdges, c->tune, s);
 			launch_mesh_collide(c, B.bucketList + (size_t)BK_MESH * cap, B.counters + CTR_BUCKET0 + BK_MESH, s);
 			k_wake_events<<<most, 256, 0, s>>>(c->scene, B, cur, cap, B.wakeList, B.counters + CTR_WAKE_ACTIVATED, 0);
-			launches += 3 + (c->anyTriangle ? 1 : 0) + (c->nMeshFix ? 3 : 0) + 1;
+			launches += 3 + (c->scene.hullsLarge ? 1 : 0) + (c->anyTriangle ? 1 : 0) + (c->nMeshFix ? 3 : 0) + 1;
 		}
 	}
 	// The work lists are the pass's own where no skipped contact could wake,
