@@ -1047,11 +1047,10 @@ __global__ void k_traverse(DevScene S, Buffers B, uint32_t n, uint32_t leaves, u
 	walk_record(W, B, cap, on, on ? W.hitQuery[lane] : 0u, on ? W.hitLeaf[lane] : 0u, on ? W.hitProxy[lane] : 0u);
 }
 
-// Scan in place of *nPtr entries (at most cap) when nPtr is set, else nHost.
-__global__ void __launch_bounds__(SC_THREADS) k_scan_tiles(uint32_t* data, const uint32_t* nPtr, uint32_t nHost,
-	uint32_t cap, unsigned long long* state, uint32_t* total, uint32_t* err)
+// Scan in place.
+__global__ void __launch_bounds__(SC_THREADS) k_scan_tiles(uint32_t* data, uint32_t n, unsigned long long* state,
+	uint32_t* total, uint32_t* err)
 {
-	const uint32_t n = nPtr ? min(*nPtr, cap) : nHost;
 	scan_tile(
 		[=](uint32_t first, uint32_t* v) {
 #pragma unroll
@@ -1073,8 +1072,7 @@ void scan_exclusive(uint32_t* data, uint32_t n, uint32_t* aux, uint32_t* total, 
 {
 	const uint32_t tiles = scan_tiles(n);
 	cudaMemsetAsync(aux, 0, sizeof(unsigned long long) * (tiles + 1u), s);
-	k_scan_tiles<<<tiles ? tiles : 1u, SC_THREADS, 0, s>>>(data, nullptr, n, n,
-		reinterpret_cast<unsigned long long*>(aux), total, err);
+	k_scan_tiles<<<tiles ? tiles : 1u, SC_THREADS, 0, s>>>(data, n, reinterpret_cast<unsigned long long*>(aux), total, err);
 }
 
 // Stable sort of n (key, value) records by the low `bits` bits of the keys

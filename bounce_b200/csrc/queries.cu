@@ -742,9 +742,9 @@ __device__ __forceinline__ RayIn load_ray(const float* rays, uint32_t i)
 // two rays' places: it starts the next ray while the queues still hold leaves
 // of the one before. Each warp has a fixed share of the rays. Measured,
 // 524,288 rays of 10 m in the 65,536-body world: 6.2 ms with one thread per
-// ray on a walk without order, 1.17 ms now (62 levels, 11 leaves and 6 casts
-// a ray, at 15 of 32 lanes: issue of those and the waits for their loads
-// bound it, not the 46 MB read and written).
+// ray on a walk without order, 1.15 ms now (62 levels and 11 leaves a
+// ray, at 14 of 32 lanes: issue of those and the waits for their loads bound
+// it, not the 46 MB read and written).
 constexpr int RAY_WARPS = 4;
 constexpr int RAY_BLOCKS = 8;       // per SM: 6 took 1.21 ms, 4 took 1.34 ms
 constexpr int RAY_STEPS = 4;        // levels between two looks at the queues: 2 took 1.28 ms

@@ -519,7 +519,7 @@ __device__ __forceinline__ GProxy input_proxy(const DevScene& S, const float* w,
 // this code (5 of 32 active) and the kernel waited on the instruction cache
 // for 13 of 17 cycles per instruction; for the same reason the code is kept
 // small, with the query and its simplex in shared memory, where rolled loops
-// can index them. Bound by issue (a third of the cycles, 7 lanes) and the
+// can index them. Bound by issue (a third of the cycles, 9 lanes) and the
 // instruction cache. Measured, 262,144 queries of mixed shapes: 10.5 ms
 // before, 2.78 ms now (every lane one step of its own at a time: 3.10 ms).
 //

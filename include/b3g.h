@@ -321,8 +321,8 @@ int b3g_finish_pass(b3g_ctx* ctx, const uint8_t* keep, uint32_t count);
 
 /* Inner counters of the last pass, for diagnostics and work accounting: the
  * overlapping pairs the broadphase found, previous contacts kept, hull-hull
- * contacts the feature cache did not resolve (full SAT), traversal records
- * past a leaf's scratch slots, mesh (contact, triangle) work items, wake-up
+ * contacts the feature cache did not resolve (full SAT), pairs of a
+ * leaf of the traversal past its first 32, mesh (contact, triangle) work items, wake-up
  * events and the contacts they activated or destroyed, bodies asleep after
  * the pass, and the size of each narrowphase bucket (one per b3Contact
  * subclass of contact.cpp:256-267, then sensor, inactive and apart pairs).
