@@ -1487,6 +1487,22 @@ __device__ __forceinline__ bool stage_wait(unsigned long long* bar, uint32_t pha
 	return false;
 }
 
+// What the bulk copies bring in, by the warp's lanes. Out of line: it hardly
+// ever runs.
+__device__ __noinline__ void stage_by_lanes(float4* to, const HullRef& h1, const HullRef& h2, uint32_t lane)
+{
+	auto copy = [&](const float4* from, uint32_t n) {
+		for (uint32_t i = lane; i < n; i += 32)
+			to[i] = from[i];
+		to += n;
+	};
+	copy(h1.v, h1.vCnt);
+	copy(h1.p, h1.fCnt);
+	copy(h2.v, h2.vCnt);
+	copy(h2.p, h2.fCnt);
+	__syncwarp();
+}
+
 // Pass 2: one warp per contact the cache did not resolve (W warps per block).
 // With STAGE, each pair's hull vertices and planes are brought into the warp's
 // shared memory by bulk copies (lane 0 issues four, the warp waits on its
@@ -1571,15 +1587,7 @@ __global__ void __launch_bounds__(W * 32) k_hulls_sat(NPArgs a, uint32_t maxUE)
 				stage_wait(bar, phase);
 				if (parts == 1)
 					return;
-				for (uint32_t i = lane; i < H.h1.vCnt; i += 32)
-					v1[i] = H.h1.v[i];
-				for (uint32_t i = lane; i < H.h1.fCnt; i += 32)
-					p1[i] = H.h1.p[i];
-				for (uint32_t i = lane; i < H.h2.vCnt; i += 32)
-					v2[i] = H.h2.v[i];
-				for (uint32_t i = lane; i < H.h2.fCnt; i += 32)
-					p2[i] = H.h2.p[i];
-				__syncwarp();
+				stage_by_lanes(v1, H.h1, H.h2, lane);
 			}
 			phase ^= 1u;
 			H.h1.v = v1;
