@@ -1263,6 +1263,10 @@ __device__ __forceinline__ bool probe_large(const NPArgs& a, uint32_t c)
 // and the polygons lived in local memory: a pass of 512 worlds with 572,000 hull
 // pairs took 1,288 us, now 1,113. Blocks of 64 threads, or 5 blocks an SM
 // with 96 registers, take 10 % of that longer.
+//
+// LARGE: the scene has hulls for k_hulls_probe_large, whose contacts are not
+// this kernel's.
+template <bool LARGE>
 __global__ void __launch_bounds__(PROBE_THREADS, PROBE_BLOCKS) k_hulls_probe(NPArgs a)
 {
 	__shared__ ClipRings rings;
@@ -1284,7 +1288,7 @@ __global__ void __launch_bounds__(PROBE_THREADS, PROBE_BLOCKS) k_hulls_probe(NPA
 			bool face = false, edges = false;
 			if (base + tid < n)
 				c = a.list[base + tid];
-			if (base + tid < n && !(a.S.hullsLarge && probe_large(a, c)))
+			if (base + tid < n && !(LARGE && probe_large(a, c)))
 			{
 				const int32_t prev = a.prevIndex[c];
 				const uint4 cache = prev >= 0 ? a.prevCache[prev] : make_uint4(CT_EMPTY, FT_FACE1, 0, 0);
@@ -1889,9 +1893,13 @@ void launch_hulls_probe(const NPArgs& base, const uint32_t* list, const uint32_t
 	a.list = list;
 	a.listCount = count;
 	const int blocks = work_blocks(a.hcPostCap, PROBE_THREADS, (int)tune.v[B3G_TUNE_PROBE]);
-	k_hulls_probe<<<blocks, PROBE_THREADS, 0, s>>>(a);
-	if (a.S.hullsLarge)
-		k_hulls_probe_large<<<blocks, PROBE_THREADS, 0, s>>>(a);
+	if (!a.S.hullsLarge)
+	{
+		k_hulls_probe<false><<<blocks, PROBE_THREADS, 0, s>>>(a);
+		return;
+	}
+	k_hulls_probe<true><<<blocks, PROBE_THREADS, 0, s>>>(a);
+	k_hulls_probe_large<<<blocks, PROBE_THREADS, 0, s>>>(a);
 }
 
 // Dynamic shared memory of the SAT kernel with `warps` warps per block.
@@ -1910,7 +1918,7 @@ void launch_mesh_items_hull(const NPArgs& a, const Buffers& B, uint32_t maxUE, c
 void carveout_narrow_hulls()
 {
 	set_carveout({
-		(const void*)k_hulls_probe, (const void*)k_hulls_sat<2, true>, (const void*)k_hulls_sat<4, true>,
+		(const void*)k_hulls_probe<false>, (const void*)k_hulls_probe<true>, (const void*)k_hulls_sat<2, true>, (const void*)k_hulls_sat<4, true>,
 		(const void*)k_hulls_sat<8, true>, (const void*)k_hulls_sat<2, false>, (const void*)k_hulls_sat<4, false>,
 		(const void*)k_hulls_sat<8, false>, (const void*)k_hull_triangle<2>, (const void*)k_hull_triangle<4>,
 		(const void*)k_hull_triangle<8>, (const void*)k_mesh_items_hull<4>});
