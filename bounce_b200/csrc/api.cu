@@ -3,7 +3,6 @@
 // b3g_create for the configured capacities.
 
 #include <algorithm>
-#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -821,19 +820,21 @@ extern "C" const char* b3g_last_error(const b3g_ctx* c)
 // nearest plane (HullDesc::blunt).
 static bool hull_blunt(uint32_t nv, const float* v, uint32_t np, const float* planes, const float* c)
 {
-	double far2 = 0.0, near = INFINITY;
+	double far2 = 0.0;
 	for (uint32_t i = 0; i < nv; ++i)
 	{
 		const double x = (double)v[3 * i] - c[0], y = (double)v[3 * i + 1] - c[1], z = (double)v[3 * i + 2] - c[2];
 		far2 = std::max(far2, x * x + y * y + z * z);
 	}
+	bool blunt = true;
 	for (uint32_t i = 0; i < np; ++i)
 	{
 		const float* p = planes + 4 * (size_t)i;
-		const double n = std::sqrt((double)p[0] * p[0] + (double)p[1] * p[1] + (double)p[2] * p[2]);
-		near = std::min(near, (p[3] - ((double)p[0] * c[0] + (double)p[1] * c[1] + (double)p[2] * c[2])) / n);
+		const double n2 = (double)p[0] * p[0] + (double)p[1] * p[1] + (double)p[2] * p[2];
+		const double g = p[3] - ((double)p[0] * c[0] + (double)p[1] * c[1] + (double)p[2] * c[2]);
+		blunt = blunt && g > 0.0 && far2 * n2 <= 256.0 * g * g;
 	}
-	return near > 0.0 && far2 <= 256.0 * near * near;
+	return blunt;
 }
 
 extern "C" int b3g_set_hulls(b3g_ctx* c, uint32_t nh, const uint32_t* desc, const float* verts,
