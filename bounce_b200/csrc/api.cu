@@ -66,6 +66,7 @@ void destroy_graphs(b3g_ctx* c)
 	// Whatever made the captured passes stale may have changed the proxy set:
 	// the next pass rebuilds the LBVH.
 	c->treeForce = true;
+	c->graphsStale = false;
 	for (int i = 0; i < 2; ++i)
 		for (int j = 0; j < 2; ++j)
 			for (int r = 0; r < 2; ++r)
@@ -1519,11 +1520,11 @@ static cudaError_t wait_staged(b3g_ctx* c, cudaStream_t s)
 }
 
 // A scene update may bring the first triangle or sensor: the captured passes
-// have no kernel for them.
+// have no kernel for them (b3g_collide drops them: this call may itself be under
+// capture).
 static void scene_may_have(b3g_ctx* c, bool triangle, bool sensor)
 {
-	if ((triangle && !c->anyTriangle) || (sensor && !c->anySensor))
-		destroy_graphs(c);
+	c->graphsStale = c->graphsStale || (triangle && !c->anyTriangle) || (sensor && !c->anySensor);
 	c->anyTriangle |= triangle;
 	c->anySensor |= sensor;
 }
@@ -1971,6 +1972,8 @@ extern "C" int b3g_collide(b3g_ctx* c, const float* state, int onDevice, void* s
 	c->lastPassImpulses = c->impulsesLoaded;
 	if (graph)
 	{
+		if (c->graphsStale)
+			destroy_graphs(c);
 		c->cur ^= 1u;
 		// A pass of this parity is captured in both forms (tree rebuilt,
 		// tree refit) the first time either is needed, so a later pass never

@@ -376,6 +376,7 @@ struct b3g_ctx
 	cudaStream_t lastStream;  // of the last pass
 	cudaEvent_t countsReady;  // the last fetch's counts are on the host
 	bool countsFetched;       // hCounters are those of the last pass, which has ended
+	bool graphsStale;         // a scene update brought what the captured passes leave out
 	bool captured;            // a caller captured a pass: its replays are not seen here
 	char *stageOut, *stageImpulses, *stageAwake; // pinned, B3G_STAGE_BYTES each (allocated on first use)
 	cudaEvent_t impulsesStaged, awakeStaged;     // the copies from them

@@ -325,3 +325,49 @@ def test_first_sensors_after_captured_passes():
         pipe.close()
     for a, b in zip(*out):
         assert np.array_equal(a[0], b[0]) and a[1] == b[1]
+
+
+# An update from device memory captured after a pass with sleeping bodies, and
+# replayed (once: the tree is rebuilt for the call, the host sees no replay).
+@pytest.mark.parametrize("graph_passes", [False, True])
+def test_captured_update(graph_passes):
+    torch = pytest.importorskip("torch")
+    sc = mixed(600)
+    states = states_of(sc, 8)
+    pipe, ref = CollisionPipeline(sc, graph=graph_passes), CollisionPipeline(sc)
+    awake = np.ones(sc.n_bodies, np.uint8)
+    awake[::3] = 0
+    on_device = [torch.from_numpy(st).cuda() for st in states]
+    torch.cuda.synchronize()
+    for p in (pipe, ref):
+        for x in on_device[:3]:
+            p.collide(x.data_ptr(), on_device=True)
+        p.set_awake(awake)
+        p.collide(on_device[3].data_ptr(), on_device=True)
+    b = np.arange(0, 60, 2, dtype=np.uint32)
+    fixtures = [sc.fix_type[b], sc.fix_hull[b], np.ascontiguousarray(sc.fix_params.reshape(-1, 12)[b]), sc.fix_flags[b]]
+    dev = [torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1)).cuda()
+           for a in (b, sc.body_world[b], sc.body_type[b], *fixtures)]
+    idx, world, btype, ftype, fhull, fparams, fflags = (N.ctypes.c_void_p(x.data_ptr()) for x in dev)
+
+    def update(p, s):
+        p._check(p.lib.b3g_update_scene_device(p.ctx, len(b), idx, world, btype, len(b), idx, idx, ftype, fhull, fparams,
+                                               fflags, 0, None, s))
+
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        update(pipe, N.ctypes.c_void_p(stream.cuda_stream))
+    graph.replay()
+    update(ref, None)
+    torch.cuda.synchronize()
+    assert pipe.awake()[b].all()
+    for x in on_device[4:]:
+        pipe.collide(x.data_ptr(), on_device=True)
+        ref.collide(x.data_ptr(), on_device=True)
+        assert np.array_equal(pipe.contacts(), ref.contacts())
+        assert np.array_equal(pipe.awake(), ref.awake())
+        assert pipe.manifolds().tobytes() == ref.manifolds().tobytes()
+    graph.reset()
+    pipe.close()
+    ref.close()
