@@ -529,6 +529,7 @@ extern "C" int b3g_create(const b3g_config* cfg, b3g_ctx** out)
 	step(cudaEventCreateWithFlags(&c->awakeStaged, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->awakeOut, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->walkDone, cudaEventDisableTiming), "cudaEventCreate");
+	step(cudaEventCreateWithFlags(&c->passDone, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaEventCreateWithFlags(&c->copyDone, cudaEventDisableTiming), "cudaEventCreate");
 	step(cudaStreamCreateWithFlags(&c->sideStream, cudaStreamNonBlocking), "cudaStreamCreate");
 	step(cudaEventCreateWithFlags(&c->forkEvent, cudaEventDisableTiming), "cudaEventCreate");
@@ -775,7 +776,7 @@ extern "C" void b3g_destroy(b3g_ctx* c)
 	dfree(c->packCounts);
 	if (c->stageOut)
 		cudaFreeHost(c->stageOut);
-	for (cudaEvent_t e : {c->countsReady, c->impulsesStaged, c->awakeStaged, c->awakeOut, c->walkDone})
+	for (cudaEvent_t e : {c->countsReady, c->impulsesStaged, c->awakeStaged, c->awakeOut, c->walkDone, c->passDone})
 		if (e)
 			cudaEventDestroy(e);
 	if (c->edgeBuf)
@@ -1898,6 +1899,20 @@ static cudaError_t wait_packing(b3g_ctx* c, cudaStream_t s)
 	return s == c->stream ? cudaSuccess : wait_event(s, c->copyReady, c->packing);
 }
 
+// The end of a pass on a caller's stream, which the fetches on the context's
+// wait for. A captured pass records it in every replay.
+static cudaError_t pass_ended(b3g_ctx* c, cudaStream_t s)
+{
+	if (s == c->stream)
+		return cudaSuccess;
+	return cudaEventRecordWithFlags(c->passDone, s, in_capture(s) ? cudaEventRecordExternal : cudaEventRecordDefault);
+}
+
+static cudaError_t wait_pass(b3g_ctx* c)
+{
+	return c->lastStream == c->stream ? cudaSuccess : cudaStreamWaitEvent(c->stream, c->passDone, 0);
+}
+
 // Kernels of a pass's narrowphase: bucketing, the pairs apart or without a
 // hull, the other convex buckets (with the hull-sphere and hull-capsule follow-up kernels), the hull
 // probe and SAT, hull-triangle, and the mesh work.
@@ -2065,6 +2080,7 @@ extern "C" int b3g_collide(b3g_ctx* c, const float* state, int onDevice, void* s
 			++c->profPass;
 	}
 	c->launches += passLaunches;
+	CK(pass_ended(c, s));
 	CK(cudaGetLastError());
 	tree_pass_issued(c);
 	c->creationPass = false;
@@ -2229,6 +2245,7 @@ extern "C" int b3g_finish_pass(b3g_ctx* c, const uint8_t* keep, uint32_t count)
 		++c->profPass;
 	c->launches += pairs_diff_launches(c) + narrow_launches(c) + 1 +
 		(rejected.empty() ? 0 : 1);
+	CK(pass_ended(c, s));
 	CK(cudaGetLastError());
 	c->creationPass = false;
 	c->havePass = true;
@@ -2396,8 +2413,9 @@ extern "C" int b3g_fetch_results_async(b3g_ctx* c, uint32_t* contacts, uint32_t 
 	if (!c->havePass)
 		return fail(c, B3G_E_STATE, "no pass yet");
 	CK(cudaSetDevice(c->device));
-	// The pass's counters (sizes of the outputs); only the pass stream is
-	// waited for, so copies of earlier passes keep running.
+	// The pass's counters (sizes of the outputs); only the pass is waited for, so
+	// copies of earlier passes keep running.
+	CK(wait_pass(c));
 	CK(cudaMemcpyAsync(c->hCounters, c->buf.counters, sizeof(uint32_t) * CTR_COUNT, cudaMemcpyDeviceToHost,
 		c->stream));
 	CK(cudaStreamSynchronize(c->stream));
@@ -2471,6 +2489,7 @@ extern "C" int b3g_fetch_results_packed_async(b3g_ctx* c, uint32_t* contacts, ui
 	}
 	if (touchCapacity && beside && !c->packCounts)
 		CK(dalloc(&c->packCounts, CTR_BUCKET0));
+	CK(wait_pass(c));
 	CK(cudaMemcpyAsync(c->hCounters, B.counters, sizeof(uint32_t) * CTR_COUNT, cudaMemcpyDeviceToHost, c->stream));
 	if (touchCapacity && beside)
 		CK(cudaMemcpyAsync(c->packCounts, B.counters, sizeof(uint32_t) * CTR_BUCKET0, cudaMemcpyDeviceToDevice,

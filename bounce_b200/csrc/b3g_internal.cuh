@@ -374,6 +374,7 @@ struct b3g_ctx
 	uint32_t* packCounts;     // ... the pass's first counters, as the call found them
 	bool packing;             // it may still go by the counters themselves
 	cudaStream_t lastStream;  // of the last pass
+	cudaEvent_t passDone;     // its end, where that is a caller's stream
 	cudaEvent_t countsReady;  // the last fetch's counts are on the host
 	bool countsFetched;       // hCounters are those of the last pass, which has ended
 	bool graphsStale;         // a scene update brought what the captured passes leave out

@@ -371,3 +371,60 @@ def test_captured_update(graph_passes):
     graph.reset()
     pipe.close()
     ref.close()
+
+
+# The fetches wait for a pass on a caller's stream by themselves.
+@pytest.mark.parametrize("packed_form", [False, True])
+@pytest.mark.parametrize("how", ["launched", "graphs", "filtered"])
+def test_results_of_a_pass_under_way(packed_form, how):
+    torch = pytest.importorskip("torch")
+    sc = mixed(20000)
+    states = states_of(sc, 8)
+    ref = CollisionPipeline(sc)
+    pipe = CollisionPipeline(sc, graph=how == "graphs", contact_filter=how == "filtered")
+    make = lambda shape, dt: torch.zeros(shape, dtype=dt, pin_memory=True).numpy()
+    contacts = make((40 * sc.n_fixtures, 3), torch.int32).view(np.uint32)
+    index = make((4 * sc.n_fixtures,), torch.int32).view(np.uint32)
+    packed = make((4 * sc.n_fixtures * 320,), torch.uint8)
+    full = packed.view(N.MANIFOLD_DTYPE)
+    s = torch.cuda.Stream()
+    on_device = [torch.from_numpy(st).cuda() for st in states]
+    slots = [x.clone() for x in on_device[:2]]
+    torch.cuda.synchronize()
+
+    def check():
+        c = (pipe.fetch_results_packed_async(contacts, index, packed) if packed_form else
+             pipe.fetch_results_async(contacts, index, full))
+        pipe.wait_results()
+        want_index, man = ref.touching()
+        assert np.array_equal(contacts[: c["contacts"]], ref.contacts())
+        assert np.array_equal(index[: c["manifolds"]], want_index)
+        got = packed[: len(packed_of(man))].tobytes() if packed_form else packed_of(full[: c["manifolds"]])
+        assert got == packed_of(man)
+
+    graph = None
+    for k, (st, x) in enumerate(zip(states, on_device)):
+        ref.collide(st)
+        if how == "captured" and k >= 2:
+            if graph is None:
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=s):
+                    for y in slots:
+                        pipe.collide(y.data_ptr(), on_device=True, stream=s.cuda_stream)
+            if k & 1:
+                slots[0].copy_(on_device[k - 1])
+                slots[1].copy_(x)
+                torch.cuda.synchronize()
+                with torch.cuda.stream(s):
+                    graph.replay()
+                check()
+            continue
+        pipe.collide(x.data_ptr(), on_device=True, stream=s.cuda_stream)
+        if how == "filtered":
+            pipe.new_pairs()
+            pipe.finish_pass()
+        check()
+    if graph is not None:
+        graph.reset()
+    ref.close()
+    pipe.close()
