@@ -1888,7 +1888,9 @@ static void issue_pass(b3g_ctx* c, cudaStream_t s, const float* state, size_t by
 // the copies b3g_fetch_results_async started from them.
 static void wait_copies(b3g_ctx* c, cudaStream_t s)
 {
-	if (c->copyPending)
+	if (s != c->stream)
+		wait_event(s, c->copyDone, c->copyPending);
+	else if (c->copyPending)
 		cudaStreamWaitEvent(s, c->copyDone, 0);
 }
 

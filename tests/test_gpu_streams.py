@@ -375,7 +375,7 @@ def test_captured_update(graph_passes):
 
 # The fetches wait for a pass on a caller's stream by themselves.
 @pytest.mark.parametrize("packed_form", [False, True])
-@pytest.mark.parametrize("how", ["launched", "graphs", "filtered"])
+@pytest.mark.parametrize("how", ["launched", "graphs", "captured", "filtered"])
 def test_results_of_a_pass_under_way(packed_form, how):
     torch = pytest.importorskip("torch")
     sc = mixed(20000)
